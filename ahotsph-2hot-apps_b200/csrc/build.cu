@@ -15,8 +15,8 @@
 //   tables, rcrit     nln_cell_tables, nln_cell_rcrit (tree_math.h), one thread per cell
 //   sink groups       the runs of nlnhost.cpp's collect_groups: small children of every
 //                     large cell merged in order, sorted by first body
-//   walk              nln_walk_group (tree_math.h), one thread per group: a counting pass,
-//                     offsets, a filling pass
+//   walk              nln_walk_cell (tree_math.h), one warp per group: a counting pass,
+//                     offsets, a filling pass in nln_walk_group's order
 // Algorithms restated from the reference: nln/cofm.c:96-231,247-574 (moments,
 // critical radii), nln/mac.c:1774-1844 (DLRcritMAC), nln/mac.c:91-111 (images).
 #include <cuda_runtime.h>
@@ -482,82 +482,281 @@ __global__ void k_groups(int64_t ng, const int64_t *first, const int32_t *count,
 }
 
 // ------------------------------------------------------------ walk
-struct CountEmit {
-    int64_t np = 0, nq = 0, nh = 0, nc = 0, nb = 0;
-    __device__ void p(uint32_t, bool body) {
-        np++;
-        nb += body ? 1 : 0;
-    }
-    __device__ void q(uint32_t) { nq++; }
-    __device__ void h(uint32_t) { nh++; }
-    __device__ void c(uint32_t) { nc++; }
-};
+// One warp per group.  A warp keeps the group's pending cells on a stack in
+// shared memory, first in walk order on top, and every round takes the top
+// 32 of them, one per lane (nln_walk_cell, the host walk's own decision).
+// The counting pass needs no order: opened cells put their children back,
+// the rest is counted.  The filling pass must write the host walk's order:
+// the leading lanes that opened nothing are final and written at once,
+// coalesced, and the lanes behind the first opened cell go back in place, an
+// opened cell as its children, a decided one marked with its decision, so no
+// cell is decided twice.  Bounded by the FP64 decision and the scattered
+// 80-byte cell records, with the walk's parallelism 32 times the group count;
+// one thread per group had too few threads below a million bodies and wrote
+// every entry uncoalesced (100k-body sphere: 50.6 ms for both passes).
+constexpr int kWalkWarps = 4;
+// Stack entries per warp.  A round with w lanes adds at most 8 w entries, and
+// w falls to 1 (an ordinary depth-first walk, at most NLN_WALK_STACK deep)
+// before the stack could fill.
+constexpr int kWalkStack = 768;
 
-// Writes stay inside the group's counted ranges (ends E*): a walk that
-// produced more entries than it counted only moves its cursor on, and the
-// mismatch is reported.
-struct FillEmit {
-    uint32_t *P, *Q, *H, *Cl;
-    uint32_t *EP, *EQ, *EH, *EC;
-    __device__ void p(uint32_t e, bool) {
-        if (P < EP)
-            *P = e;
-        P++;
-    }
-    __device__ void q(uint32_t e) {
-        if (Q < EQ)
-            *Q = e;
-        Q++;
-    }
-    __device__ void h(uint32_t e) {
-        if (H < EH)
-            *H = e;
-        H++;
-    }
-    __device__ void c(uint32_t e) {
-        if (Cl < EC)
-            *Cl = e;
-        Cl++;
-    }
-};
+enum { W_OPEN = 0, W_MARK = 5 };  // 1..4: NLN_MONO..NLN_LEAF, decided; 5: a correction entry alone
+constexpr uint32_t kWalkCell = NLN_IDX_MASK;
+constexpr int kWalkType = 27;     // bits 27-29: W_OPEN, NLN_*, W_MARK
+constexpr int kWalkFlag = 30;     // undecided: bit 30 covered; decided: 1 cell, 2 bodies to the
+                                  // correction list
+constexpr uint8_t kOwnImages = 31;  // image code of a leaf whose bodies take their own images
 
-// cnt: 5 per group (point, quadrupole, order-4, correction entries, bodies among the points)
-__global__ void k_walk_count(const nln_wcell *__restrict__ wc, const float *spos, int64_t n,
-                             const nln_group *__restrict__ groups, int64_t ng, nln_mac P,
-                             int64_t *cnt, unsigned *err) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ng)
-        return;
-    int32_t stack[NLN_WALK_STACK];
-    CountEmit em;
-    const nln_group G = groups[g];
-    if (nln_walk_group(wc, spos, n, G, P, stack, NLN_WALK_STACK, em))
-        atomicOr(err, 1u);
-    cnt[5 * g] = em.np;
-    cnt[5 * g + 1] = em.nq;
-    cnt[5 * g + 2] = em.nh;
-    cnt[5 * g + 3] = em.nc;
-    cnt[5 * g + 4] = em.nb;
+__device__ __forceinline__ nln_wcell load_wcell(const nln_wcell *wc, uint32_t i) {
+    static_assert(sizeof(nln_wcell) == 80, "five 16-byte loads");
+    union {
+        double2 d[5];
+        nln_wcell c;
+    } u;
+    const double2 *s = reinterpret_cast<const double2 *>(wc + i);
+#pragma unroll
+    for (int k = 0; k < 5; k++) u.d[k] = __ldg(s + k);
+    return u.c;
 }
 
-__global__ void k_walk_fill(const nln_wcell *__restrict__ wc, const float *spos, int64_t n,
-                            const nln_group *__restrict__ groups, int64_t ng, nln_mac P,
-                            const int64_t *pp, const int64_t *qp, const int64_t *hp,
-                            const int64_t *cp, uint32_t *pl, uint32_t *ql, uint32_t *hl,
-                            uint32_t *cl, unsigned *err) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// inclusive warp scan
+__device__ __forceinline__ int warp_scan(int v, int lane) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d)
+            v += u;
+    }
+    return v;
+}
+
+__device__ __forceinline__ int64_t warp_sum(int64_t v) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    return v;
+}
+
+// The runs (first[l], n[l] entries) of the lanes, one after another, at
+// out[pos..end): entry j of a run is first + j with the run's image code, or
+// with kOwnImages the body's own image.  Returns the new position; writes
+// stay below end.
+__device__ __forceinline__ int64_t emit_runs(uint32_t *out, int64_t pos, int64_t end,
+                                             uint32_t first, int n, uint32_t code, int lane,
+                                             const float *spos, const nln_group &G, double box) {
+    const unsigned FULL = 0xffffffffu;
+    if (!__any_sync(FULL, n > 1)) {  // cells only: one entry per lane at most
+        const unsigned m = __ballot_sync(FULL, n == 1);
+        const int64_t k = pos + __popc(m & ((1u << lane) - 1u));
+        if (n == 1 && code != kOwnImages && k < end)
+            out[k] = first | code << NLN_IDX_BITS;
+        if (!__any_sync(FULL, n == 1 && code == kOwnImages))
+            return pos + __popc(m);
+    }
+    const int inc = warp_scan(n, lane);
+    const int total = __shfl_sync(FULL, inc, 31);
+    for (int j0 = 0; j0 < total; j0 += 32) {
+        const int j = j0 + lane;
+        int owner = 0;  // lanes whose runs all lie before j
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1)
+            if (__shfl_sync(FULL, inc, owner + step - 1) <= j)
+                owner += step;
+        owner = min(owner, 31);
+        const uint32_t f = __shfl_sync(FULL, first, owner);
+        const int b = __shfl_sync(FULL, inc - n, owner);
+        uint32_t c = __shfl_sync(FULL, code, owner);
+        if (j < total && pos + j < end) {
+            const uint32_t e = f + (uint32_t)(j - b);
+            if (c == kOwnImages) {
+                const float *x = spos + 3 * (int64_t)e;
+                int sb[3];
+                for (int d = 0; d < 3; d++) sb[d] = nln_image(x[d] - G.cen[d], box);
+                c = nln_shift_code(sb);
+            }
+            out[pos + j] = e | c << NLN_IDX_BITS;
+        }
+    }
+    return pos + total;
+}
+
+// FILL false: cnt[5 g ..] = point, quadrupole, order-4 and correction
+// entries, bodies among the points.  FILL true: the entries, at the offsets
+// pp, qp, hp, cp (ngroups + 1 each) of the four lists.
+template <bool FILL>
+__global__ void __launch_bounds__(32 * kWalkWarps)
+    k_walk(const nln_wcell *__restrict__ wc, const float *__restrict__ spos, int64_t n,
+           const nln_group *__restrict__ groups, int64_t ng, nln_mac P, int64_t *cnt,
+           const int64_t *pp, const int64_t *qp, const int64_t *hp, const int64_t *cp,
+           uint32_t *pl, uint32_t *ql, uint32_t *hl, uint32_t *cl, unsigned *err) {
+    __shared__ uint32_t s_item[kWalkWarps][kWalkStack];
+    __shared__ uint8_t s_code[kWalkWarps][FILL ? kWalkStack : 1];
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int64_t g = (int64_t)blockIdx.x * kWalkWarps + wib;
     if (g >= ng)
         return;
-    int32_t stack[NLN_WALK_STACK];
-    FillEmit em{pl + pp[g],     ql + qp[g],     hl + hp[g],     cl + cp[g],
-                pl + pp[g + 1], ql + qp[g + 1], hl + hp[g + 1], cl + cp[g + 1]};
+    uint32_t *item = s_item[wib];
+    uint8_t *codes = s_code[wib];
     const nln_group G = groups[g];
-    if (nln_walk_group(wc, spos, n, G, P, stack, NLN_WALK_STACK, em))
+    const uint32_t nb = (uint32_t)n;
+    const bool periodic = P.box > 0;
+    int64_t covered = 0;               // this lane's
+    int64_t np = 0, nbod = 0, nc = 0;  // counting: this lane's; filling: the warp's positions
+    int64_t nq = 0, nh = 0;
+    int64_t ep = 0, eq = 0, eh = 0, ec = 0;
+    if (FILL) {
+        np = pp[g], nq = qp[g], nh = hp[g], nc = cp[g];
+        ep = pp[g + 1], eq = qp[g + 1], eh = hp[g + 1], ec = cp[g + 1];
+    }
+    int sp = 1;
+    if (lane == 0)
+        item[0] = 0;
+    __syncwarp();
+    bool overflow = false;
+    while (sp > 0) {
+        const int room = (kWalkStack - NLN_WALK_STACK - sp) / 8;
+        const int w = min(min(32, sp), max(1, room));
+        const bool mine = lane < w;
+        uint32_t it = 0;
+        uint32_t code = NLN_SHIFT_NONE;
+        if (mine) {
+            it = item[sp - 1 - lane];
+            if (FILL)
+                code = codes[sp - 1 - lane];
+        }
+        const uint32_t ci = it & kWalkCell;
+        int type = mine ? (int)(it >> kWalkType & 7u) : W_MARK;
+        int cflag = FILL && mine ? (int)(it >> kWalkFlag) : 0;
+        int kids = 0, child = 0;
+        int32_t bodies = 0;
+        uint32_t first = 0;
+        bool covers = false, ccov = false, opened = false;
+        if (mine && type == W_OPEN) {
+            const nln_wcell c = load_wcell(wc, ci);
+            ccov = (it >> kWalkFlag & 1u) != 0;
+            const nln_visit v = nln_walk_cell(c, G, P, ccov);
+            covers = v.covers;
+            code = v.sc;
+            ccov |= covers;
+            first = (uint32_t)c.first;
+            bodies = c.count;
+            if (v.what == NLN_OPEN) {
+                opened = true;
+                child = c.child;
+                kids = c.nchild;
+            } else {
+                covered += c.count;
+                type = v.what;
+                // the correction list gets the cell, or an uncovered leaf's bodies
+                cflag = !periodic ? 0 : covers ? 1 : ccov ? 0 : type == NLN_LEAF ? 2 : 1;
+                if (type == NLN_LEAF && !v.inside)
+                    code = kOwnImages;
+            }
+            if (!FILL) {
+                np += type == NLN_LEAF ? bodies : type == NLN_MONO ? 1 : 0;
+                nbod += type == NLN_LEAF ? bodies : 0;
+                nq += type == NLN_QUAD;
+                nh += type == NLN_HEXA;
+                nc += covers ? 1 : opened ? 0 : cflag == 2 ? bodies : cflag;
+            }
+        } else if (FILL && mine && type == NLN_LEAF) {
+            first = (uint32_t)wc[ci].first;
+            bodies = wc[ci].count;
+        }
+        __syncwarp();  // the window is read: its entries may be overwritten
+        if (!FILL) {
+            const int inc = warp_scan(kids, lane);
+            const int total = __shfl_sync(FULL, inc, 31);
+            const int base = sp - w;
+            if (base + total > kWalkStack) {
+                overflow = true;
+                break;
+            }
+            const uint32_t flag = ccov ? 1u << kWalkFlag : 0u;
+            for (int k = 0; k < kids; k++)
+                item[base + inc - kids + k] = (uint32_t)(child + k) | flag;
+            sp = base + total;
+            __syncwarp();
+            continue;
+        }
+        const unsigned open = __ballot_sync(FULL, opened);
+        const int f = open ? __ffs(open) - 1 : w;
+        // lanes before f are final: write them in order
+        if (f > 0) {
+            const bool fin = lane < f;
+            const uint32_t self = nb + ci;
+            const int t = fin ? type : W_MARK;
+            const bool leaf = t == NLN_LEAF;
+            np = emit_runs(pl, np, ep, leaf ? first : self, leaf ? bodies : t == NLN_MONO ? 1 : 0,
+                           code, lane, spos, G, P.box);
+            const unsigned lt = (1u << lane) - 1u;
+            const unsigned mq = __ballot_sync(FULL, t == NLN_QUAD);
+            const unsigned mh = __ballot_sync(FULL, t == NLN_HEXA);
+            const uint32_t entry = ci | code << NLN_IDX_BITS;
+            if (t == NLN_QUAD && nq + __popc(mq & lt) < eq)
+                ql[nq + __popc(mq & lt)] = entry;
+            if (t == NLN_HEXA && nh + __popc(mh & lt) < eh)
+                hl[nh + __popc(mh & lt)] = entry;
+            nq += __popc(mq);
+            nh += __popc(mh);
+            if (periodic) {
+                const int cf = fin ? cflag : 0;
+                // a leaf that enters whole keeps the cell's own image code
+                uint32_t cc = code;
+                if (cf == 1 && code == kOwnImages)
+                    cc = nln_walk_cell(load_wcell(wc, ci), G, P, false).sc;
+                nc = emit_runs(cl, nc, ec, cf == 2 ? first : self, cf == 2 ? bodies : cf, cc, lane,
+                               spos, G, P.box);
+            }
+        }
+        // lanes f .. w-1 go back on the stack in place
+        const bool mark = opened && covers;
+        const int slots = lane < f || !mine ? 0 : opened ? kids + (mark ? 1 : 0) : 1;
+        const int inc = warp_scan(slots, lane);
+        const int total = __shfl_sync(FULL, inc, 31);
+        const int top = sp - w + total;
+        if (top > kWalkStack) {
+            overflow = true;
+            break;
+        }
+        if (slots) {
+            int at = top - (inc - slots) - 1;  // this lane's first entry, downwards
+            if (opened) {
+                if (mark) {
+                    item[at] = ci | (uint32_t)W_MARK << kWalkType | 1u << kWalkFlag;
+                    codes[at] = (uint8_t)code;
+                    at--;
+                }
+                const uint32_t flag = ccov ? 1u << kWalkFlag : 0u;
+                for (int k = 0; k < kids; k++) item[at - k] = (uint32_t)(child + k) | flag;
+            } else {
+                item[at] = ci | (uint32_t)type << kWalkType | (uint32_t)cflag << kWalkFlag;
+                codes[at] = (uint8_t)code;
+            }
+        }
+        sp = top;
+        __syncwarp();
+    }
+    covered = warp_sum(covered);
+    if ((overflow || covered != n) && lane == 0)
         atomicOr(err, 1u);
-    // the count pass sized every list: a walk that writes more or less is an error
-    if (em.P != pl + pp[g + 1] || em.Q != ql + qp[g + 1] || em.H != hl + hp[g + 1] ||
-        em.Cl != cl + cp[g + 1])
+    if (!FILL) {
+        np = warp_sum(np);
+        nq = warp_sum(nq);
+        nh = warp_sum(nh);
+        nc = warp_sum(nc);
+        nbod = warp_sum(nbod);
+        if (lane == 0) {
+            cnt[5 * g] = np;
+            cnt[5 * g + 1] = nq;
+            cnt[5 * g + 2] = nh;
+            cnt[5 * g + 3] = nc;
+            cnt[5 * g + 4] = nbod;
+        }
+    } else if (lane == 0 && (np != ep || nq != eq || nh != eh || nc != ec)) {
+        // the count pass sized every list: a walk that writes more or less is an error
         atomicOr(err, 2u);
+    }
 }
 
 template <typename T>
@@ -904,7 +1103,9 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     BC(B.get(&cnt, 5 * ng));
     BC(cudaMemsetAsync(cnt, 0, 5 * ng * sizeof(int64_t), st));
     BC(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
-    k_walk_count<<<grid_of(ng, 128), 128, 0, st>>>(wc, spos, n, out.groups, ng, P, cnt, flag);
+    k_walk<false><<<grid_of(ng, kWalkWarps), 32 * kWalkWarps, 0, st>>>(
+        wc, spos, n, out.groups, ng, P, cnt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+        nullptr, nullptr, flag);
     BC(cudaGetLastError());
     std::vector<int64_t> hc(5 * ng);
     BC(cudaMemcpyAsync(hc.data(), cnt, 5 * ng * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -943,9 +1144,9 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     out.seconds[5] = now_s() - t0;  // offsets and list allocation
     t0 = now_s();
     BC(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
-    k_walk_fill<<<grid_of(ng, 128), 128, 0, st>>>(wc, spos, n, out.groups, ng, P, dptr[0], dptr[1],
-                                              dptr[2], dptr[3], out.list[0], out.list[1],
-                                              out.list[2], out.list[3], flag);
+    k_walk<true><<<grid_of(ng, kWalkWarps), 32 * kWalkWarps, 0, st>>>(
+        wc, spos, n, out.groups, ng, P, nullptr, dptr[0], dptr[1], dptr[2], dptr[3], out.list[0],
+        out.list[1], out.list[2], out.list[3], flag);
     BC(cudaGetLastError());
     BC(cudaMemcpyAsync(&hbad, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     BC(cudaStreamSynchronize(st));

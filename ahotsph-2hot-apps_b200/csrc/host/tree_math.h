@@ -266,6 +266,72 @@ NLN_HD inline double nln_lattice_gap(const double y[3], double box) {
     return sqrt(D2);
 }
 
+// Image step of a displacement y: -nearbyint(y / box), the division only
+// where the quotient is near a half or beyond one and a half.
+NLN_HD inline int nln_image(double y, double box) {
+    const double a = fabs(y);
+    if (a < 0.499 * box)
+        return 0;
+    if (a > 0.501 * box && a < 1.499 * box)
+        return y > 0 ? -1 : 1;
+    return -(int)nearbyint(y / box);
+}
+
+// What the walk does with a cell: open it, expand it to its bodies (a leaf
+// that cannot be taken), or take it as a monopole, quadrupole or order-4 cell.
+enum { NLN_OPEN = 0, NLN_MONO = 1, NLN_QUAD = 2, NLN_HEXA = 3, NLN_LEAF = 4 };
+
+typedef struct nln_visit {
+    int what;
+    uint32_t sc;       // image code of the cell
+    bool inside;       // inside the correction's domain (a leaf that is not: each body its own image)
+    bool covers;       // the cell enters the correction list for its whole subtree
+} nln_visit;
+
+// One cell of a group's walk; ccov: an ancestor stands for it in the
+// correction list already.
+NLN_HD inline nln_visit nln_walk_cell(const nln_wcell &c, const nln_group &G, const nln_mac &P,
+                                      bool ccov) {
+    const double box = P.box;
+    const double theta = P.ewald_theta;
+    const int p2 = P.p2cut, p4 = P.p4cut;
+    nln_visit v;
+    double y[3];
+    int s[3] = {0, 0, 0};
+    for (int d = 0; d < 3; d++) {
+        y[d] = c.cen[d] - G.cen[d];
+        if (box > 0) {
+            s[d] = nln_image(y[d], box);
+            y[d] += s[d] * box;
+        }
+    }
+    const double dist = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
+    // Periodic: the cell is taken whole in the image nearest the group
+    // centre.  Every sink-body displacement it implies must stay inside
+    // the domain of the Ewald correction, |y_k| <= NLN_EWALD_REACH * box,
+    // where the correction is smooth; otherwise the cell is opened.
+    v.inside = true;
+    v.covers = false;
+    v.sc = nln_shift_code(s);
+    if (box > 0) {
+        const double ym = fmax(fabs(y[0]), fmax(fabs(y[1]), fabs(y[2])));
+        v.inside = ym + c.bmax + G.radius <= NLN_EWALD_REACH * box;
+        v.covers = !ccov && theta > 0 && c.count > 0 && ym + c.bmax < 0.5 * box * (1.0 - 1e-9) &&
+                   c.bmax + G.radius <= theta * nln_lattice_gap(y, box);
+    }
+    const double dd = dist - G.radius;
+    v.what = c.child >= 0 ? NLN_OPEN : NLN_LEAF;
+    if (v.inside && c.count > 0) {
+        if (dd > c.rc[0] + c.bmax)
+            v.what = NLN_MONO;
+        else if (p2 && c.count >= p2 && dd > c.rc[1] + c.bmax)
+            v.what = NLN_QUAD;
+        else if (p4 && c.count >= p4 && dd > c.rc[2] + c.bmax)
+            v.what = NLN_HEXA;
+    }
+    return v;
+}
+
 // The walk of one sink group (nln/mac.c:1703-1840 semantics: a cell is
 // taken at the lowest order whose critical radius it clears, else opened;
 // a leaf that cannot be taken expands to its bodies).  The MAC distance is
@@ -292,8 +358,6 @@ NLN_HD inline int nln_walk_group(const nln_wcell *cells, const float *spos, int6
                                  const nln_group &G, const nln_mac &P, int32_t *stack, int cap,
                                  Emit &em) {
     const double box = P.box;
-    const double theta = P.ewald_theta;
-    const int p2 = P.p2cut, p4 = P.p4cut;
     const uint32_t nb = (uint32_t)n;
     int64_t covered = 0;
     int sp = 0;
@@ -303,74 +367,47 @@ NLN_HD inline int nln_walk_group(const nln_wcell *cells, const float *spos, int6
         const int32_t ci = top >> 1;
         bool ccov = (top & 1) != 0;
         const nln_wcell &c = cells[ci];
-        double y[3];
-        int s[3] = {0, 0, 0};
-        for (int d = 0; d < 3; d++) {
-            y[d] = c.cen[d] - G.cen[d];
-            if (box > 0) {
-                s[d] = -(int)nearbyint(y[d] / box);
-                y[d] += s[d] * box;
-            }
-        }
-        const double dist = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
-        // Periodic: the cell is taken whole in the image nearest the group
-        // centre.  Every sink-body displacement it implies must stay inside
-        // the domain of the Ewald correction, |y_k| <= NLN_EWALD_REACH * box,
-        // where the correction is smooth; otherwise the cell is opened.
-        bool inside = true;
-        const uint32_t sc = nln_shift_code(s);
-        if (box > 0) {
-            const double ym = fmax(fabs(y[0]), fmax(fabs(y[1]), fabs(y[2])));
-            inside = ym + c.bmax + G.radius <= NLN_EWALD_REACH * box;
-            if (!ccov && theta > 0 && c.count > 0 && ym + c.bmax < 0.5 * box * (1.0 - 1e-9) &&
-                c.bmax + G.radius <= theta * nln_lattice_gap(y, box)) {
-                em.c((nb + (uint32_t)ci) | (sc << NLN_IDX_BITS));
-                ccov = true;
-            }
+        const nln_visit v = nln_walk_cell(c, G, P, ccov);
+        const uint32_t sc = v.sc, self = (nb + (uint32_t)ci) | (sc << NLN_IDX_BITS);
+        if (v.covers) {
+            em.c(self);
+            ccov = true;
         }
         const bool emit_c = box > 0 && !ccov;
-        const double dd = dist - G.radius;
-        if (inside && c.count > 0) {
-            const bool take = dd > c.rc[0] + c.bmax ||
-                              (p2 && c.count >= p2 && dd > c.rc[1] + c.bmax) ||
-                              (p4 && c.count >= p4 && dd > c.rc[2] + c.bmax);
-            if (take) {
-                if (dd > c.rc[0] + c.bmax) {
-                    em.p((nb + (uint32_t)ci) | (sc << NLN_IDX_BITS), false);
-                } else if (p2 && c.count >= p2 && dd > c.rc[1] + c.bmax) {
-                    em.q((uint32_t)ci | (sc << NLN_IDX_BITS));
-                } else {
-                    em.h((uint32_t)ci | (sc << NLN_IDX_BITS));
-                }
-                if (emit_c)
-                    em.c((nb + (uint32_t)ci) | (sc << NLN_IDX_BITS));
-                covered += c.count;
-                continue;
-            }
-        }
-        if (c.child >= 0) {
+        if (v.what == NLN_OPEN) {
             if (sp + c.nchild > cap)
                 return -2;
             for (int k = c.nchild - 1; k >= 0; k--) stack[sp++] = ((c.child + k) << 1) | (ccov ? 1 : 0);
             continue;
         }
+        covered += c.count;
+        if (v.what != NLN_LEAF) {
+            if (v.what == NLN_MONO)
+                em.p(self, false);
+            else if (v.what == NLN_QUAD)
+                em.q((uint32_t)ci | (sc << NLN_IDX_BITS));
+            else
+                em.h((uint32_t)ci | (sc << NLN_IDX_BITS));
+            if (emit_c)
+                em.c(self);
+            continue;
+        }
         // leaf: expand to bodies (nln/mac.c:1817-1832)
         for (int32_t k = 0; k < c.count; k++) {
             uint32_t e;
-            if (inside || box <= 0) {
+            if (v.inside) {
                 e = (uint32_t)(c.first + k) | (sc << NLN_IDX_BITS);
             } else {
                 // a leaf reaching out of the correction's domain: each body its own image
                 const float *x = spos + 3 * (c.first + k);
                 int sb[3];
-                for (int d = 0; d < 3; d++) sb[d] = -(int)nearbyint((x[d] - G.cen[d]) / box);
+                for (int d = 0; d < 3; d++) sb[d] = nln_image(x[d] - G.cen[d], box);
                 e = (uint32_t)(c.first + k) | (nln_shift_code(sb) << NLN_IDX_BITS);
             }
             em.p(e, true);
             if (emit_c)
                 em.c(e);
         }
-        covered += c.count;
     }
     return covered == n ? 0 : -1;
 }
