@@ -6,18 +6,19 @@
 // absolute FP32 copies, nln/mac.c:1421-1561):
 //   * each sink is held as an FP32 offset from its group's FP64 centre;
 //   * each source record is re-centred on the same FP64 centre (with its
-//     periodic image shift) as it is staged, so the inner loops subtract
+//     periodic image shift) as a lane takes it up, so the inner loops subtract
 //     two small FP32 numbers;
-//   * partial sums of one staged tile are plain FP32, folded into a
-//     compensated (hi, lo) accumulator per tile;
+//   * partial sums of one tile are plain FP32, folded into a compensated
+//     (hi, lo) accumulator per tile;
 //   * work-item partials are combined per group in FP64, in a fixed order.
 // Work decomposition: a work item is (group, kind, range of its list);
 // long lists are split so that small problems still fill the GPU; every
 // warp pulls items (costliest first) from its kind's queue until it is
-// empty.  One warp owns one item: lane = sink, 32 sources per staged tile;
-// tiles are staged by TMA row gathers (cp.async.bulk.tensor tile::gather4
-// over a 2-D tensor map of the table, one instruction per 4 records, issued
-// by one lane) into a 2-4 stage ring signalled by per-warp mbarriers.
+// empty.  One warp owns one item: lane = source records, a tile of 64 to 256
+// records in the lanes' registers, walked by the group's sinks (below).
+// Cell tiles are staged by TMA row gathers (cp.async.bulk.tensor
+// tile::gather4 over a 2-D tensor map of the table, one instruction per 4
+// records) signalled by per-warp mbarriers, points by per-lane cp.async.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -28,6 +29,7 @@
 #include <chrono>
 #include <mutex>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "build.cuh"
@@ -41,7 +43,23 @@
 namespace {
 
 enum { KP = 0, KQ = 1, KH = 2 };
-constexpr int TILE = 32;
+constexpr int kListWarps = 4;     // warps per block of the list kernels at most
+constexpr int kPointTile = 256;   // records of a staged tile: points
+constexpr int kQuadTile = 128;    // quadrupole cells
+constexpr int kHexaTile = 64;     // order-4 cells
+constexpr int kTile[3] = {kPointTile, kQuadTile, kHexaTile};
+
+// Resident blocks the list kernels' registers are held to (-D to rebuild
+// with others).
+#ifndef GRAV_H_MINB
+#define GRAV_H_MINB 3
+#endif
+#ifndef GRAV_Q_MINB
+#define GRAV_Q_MINB 4
+#endif
+#ifndef GRAV_P_MINB
+#define GRAV_P_MINB 4
+#endif
 
 struct Item {
     int32_t group;
@@ -85,87 +103,22 @@ struct DevProblem {
     float ew_trace;            // trace of the Hessian of C: -4 pi / L^3
     EwStored *ewm;             // per-group moments from k_ewald_moments
     // FP64 centres of the cells for the point table's monopole records (the
-    // mixed form re-centres them like every other source): a pre-staged cell
-    // table (centre x, y in floats 0-3, z in floats 10-11 of each record of
-    // cstride float4s), or null, where the FP32 point record is used
-    const float4 *cstage;
+    // mixed form re-centres them like every other source): a cell table (the
+    // centre is a record's first 24 bytes, one record every cstride bytes),
+    // or null, where the FP32 point record is used
+    const unsigned char *ccen;
     int cstride;
 };
 
-template <int KIND, bool PAIRED = false>
-struct KindOf {
-    static constexpr int rec_bytes = KIND == KP ? 16 : (KIND == KQ ? 64 : 128);
-    static constexpr int order = KIND == KP ? 0 : (KIND == KQ ? 2 : 4);
-    // pipeline depth: short per-record work needs more copies in flight; the
-    // paired order-4 path frees its one stage as soon as the tile is
-    // re-laid into the pair buffer, so the next copy overlaps the compute
-    static constexpr int stages = PAIRED ? 1 : (KIND == KP ? 4 : (KIND == KQ ? 3 : 2));
-    // one TMA row gather brings 4 records; each lands 128-byte aligned
-    static constexpr int group_bytes = 4 * rec_bytes < 128 ? 128 : 4 * rec_bytes;
-    static constexpr int stage_bytes = (TILE / 4) * group_bytes;
-    // paired tiles: 16 record pairs of 32 (order 4) or 10 (quadrupole)
-    // interleaved fields, one pair every 68 or 20 floats (16-byte aligned;
-    // the re-lay's 8-byte stores of a half-warp hit distinct banks)
-    static constexpr int pair_fields = KIND == KH ? 32 : 10;
-    static constexpr int pair_stride = pair_fields == 32 ? 68 : 20;
-    static constexpr int pair_bytes = PAIRED ? (TILE / 2) * pair_stride * 4 : 0;
-    // per-warp shared memory: stages of 32 records, the pair buffer,
-    // mbarriers, image codes
-    static constexpr int warp_bytes =
-        (stages * stage_bytes + pair_bytes + stages * 8 + stages * TILE * 4 + 127) / 128 * 128;
-    // byte offset of record r inside a stage
-    static __device__ __forceinline__ int rec_off(int r) {
-        return (r >> 2) * group_bytes + (r & 3) * rec_bytes;
-    }
-};
-
+// Image code (0..26) to the image's shift: (code / 9 - 1, code / 3 % 3 - 1,
+// code % 3 - 1) box.
 __device__ __forceinline__ void decode_shift(uint32_t code, double box, double &sx, double &sy,
                                              double &sz) {
-    sx = ((int)(code / 9) - 1) * box;
-    sy = ((int)(code / 3 % 3) - 1) * box;
-    sz = ((int)(code % 3) - 1) * box;
-}
-
-// Convert this lane's record (just landed by TMA) in place into the staged
-// form of interact.cuh, re-centred on the group centre c.  STAGED: the cell
-// tables are pre-staged (k_stage_cells) and only the 16-byte header (FP64
-// centre -> FP32 offset, mass) is rewritten; otherwise the raw nln_qcell /
-// nln_hcell record is scaled here.
-template <int KIND, bool STAGED>
-__device__ __forceinline__ void convert(unsigned char *slot, uint32_t code, const double *c,
-                                        double box) {
-    double sx, sy, sz;
-    decode_shift(code, box, sx, sy, sz);
-    float *o = reinterpret_cast<float *>(slot);
-    if (KIND == KP) {
-        float4 p = *reinterpret_cast<const float4 *>(slot);
-        o[0] = (float)((double)p.x + sx - c[0]);
-        o[1] = (float)((double)p.y + sy - c[1]);
-        o[2] = (float)((double)p.z + sz - c[2]);
-        o[3] = p.w;
-    } else if (STAGED) {
-        const double *d = reinterpret_cast<const double *>(slot);
-        const double cx = d[0], cy = d[1], cz = d[5];
-        const float m = o[KIND == KQ ? 12 : 31];
-        *reinterpret_cast<float4 *>(slot) =
-            make_float4((float)(cx + sx - c[0]), (float)(cy + sy - c[1]), (float)(cz + sz - c[2]), m);
-    } else if (KIND == KQ) {
-        const nln_qcell q = *reinterpret_cast<const nln_qcell *>(slot);
-        o[0] = (float)(q.cen[0] + sx - c[0]);
-        o[1] = (float)(q.cen[1] + sy - c[1]);
-        o[2] = (float)(q.cen[2] + sz - c[2]);
-        o[3] = q.mass;
-        float q2[5] = {q.qxx, q.qxy, q.qyy, q.qxz, q.qyz};
-        stage_quad(o, q.R, q2);
-    } else {
-        const nln_hcell h = *reinterpret_cast<const nln_hcell *>(slot);
-        o[0] = (float)(h.cen[0] + sx - c[0]);
-        o[1] = (float)(h.cen[1] + sy - c[1]);
-        o[2] = (float)(h.cen[2] + sz - c[2]);
-        o[3] = h.mass;
-        stage_quad(o, h.R, h.q2);
-        stage_hexa(o, h.R, h.q3, h.q4);
-    }
+    const uint32_t third = code * 171u >> 9, x = code * 57u >> 9;  // code / 3, code / 9
+    const uint32_t y = third - 3u * x, z = code - 3u * third;
+    sx = x == 0 ? -box : x == 2 ? box : 0.0;
+    sy = y == 0 ? -box : y == 2 ? box : 0.0;
+    sz = z == 0 ? -box : z == 2 ? box : 0.0;
 }
 
 // Unpack the run-packed lists (format in nlnlists.h) of groups g0..g1-1,
@@ -292,172 +245,249 @@ __global__ void k_check_lists(const uint32_t *__restrict__ list, const Item *__r
     }
 }
 
-// Pre-staged cell tables: the staged moments of interact.cuh at their
-// offsets, with the FP64 centre and the mass in the slots the inner loops
-// never read (centre x, y in floats 0-3 and z in floats 10-11; mass in
-// float 12 (quadrupole, 16 floats) or 31 (order 4, 32 floats)), so that a
-// tile's convert only rewrites the header.
-__global__ void k_stage_cells(const nln_qcell *__restrict__ qc, const nln_hcell *__restrict__ hc,
-                              int64_t n, float4 *__restrict__ qs, float4 *__restrict__ hs) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n)
-        return;
-    if (qs) {
-        const nln_qcell q = qc[c];
-        float o[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) o[k] = 0.f;
-        const float q2[5] = {q.qxx, q.qxy, q.qyy, q.qxz, q.qyz};
-        stage_quad(o, q.R, q2);
-        memcpy(&o[0], &q.cen[0], 8);
-        memcpy(&o[2], &q.cen[1], 8);
-        memcpy(&o[10], &q.cen[2], 8);
-        o[12] = q.mass;
-#pragma unroll
-        for (int k = 0; k < 4; k++) qs[c * 4 + k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+// ------------------------------------------------------------ list kernels
+//
+// A warp owns one work item: a range of one group's list.  Its lanes hold
+// the source records, R each in registers, and the warp walks the group's
+// sinks one by one: a sink's offsets are broadcast from shared memory, every
+// lane evaluates its own records, and the 32 lanes' sums are added by a
+// transposing butterfly that leaves sink s's sum in lane s.  So a group of c
+// sinks costs c steps and not 32 (22.5 sinks a group on spheres, 24 to 32 in
+// boxes), a record is read from shared memory once per tile and not once per
+// sink, and its image shift, FP64 re-centring and moment scaling are done
+// once for all sinks.  The butterfly costs about 10 FMA-pipe cycles a sink.
+// Against lanes as sinks (32 records broadcast from shared memory), 160^3
+// periodic box, MAC 2.5e-6: order 4 90.5 -> 65.5 ms, quadrupole 37.0 -> 30.0,
+// points 43.2 -> 34.0; Plummer 64k, points 0.418 -> 0.338 ms.  The order-4
+// kernel keeps the FMA pipe 73 % busy, where its operand reads allow 77 %.
+
+// A sink as splat pairs of its negated offsets from the group centre.
+struct __align__(16) Sink {
+    float4 xy;
+    float2 z, pad;
+};
+struct SinkTable {
+    Sink s[32];
+};
+
+// This lane's sink offset from the group centre c, into the table.
+__device__ __forceinline__ void stage_sinks(SinkTable &T, const DevProblem &P, const nln_group &G,
+                                            const double *c, int lane) {
+    __syncwarp();  // the previous item's sinks are no longer read
+    if (lane < G.count) {
+        const float4 s = P.points[G.first + lane];
+        const float nx = -(float)((double)s.x - c[0]), ny = -(float)((double)s.y - c[1]),
+                    nz = -(float)((double)s.z - c[2]);
+        T.s[lane].xy = make_float4(nx, nx, ny, ny);
+        T.s[lane].z = make_float2(nz, nz);
     }
-    if (hs) {
-        const nln_hcell h = hc[c];
-        float o[32];
-#pragma unroll
-        for (int k = 0; k < 32; k++) o[k] = 0.f;
-        stage_quad(o, h.R, h.q2);
-        stage_hexa(o, h.R, h.q3, h.q4);
-        memcpy(&o[0], &h.cen[0], 8);
-        memcpy(&o[2], &h.cen[1], 8);
-        memcpy(&o[10], &h.cen[2], 8);
-        o[31] = h.mass;
-#pragma unroll
-        for (int k = 0; k < 8; k++) hs[c * 8 + k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
-    }
+    __syncwarp();
 }
 
-// Re-lay this lane's pre-staged record (just landed by TMA at its stage
-// slot) into the pair-interleaved tile of quad2_plummer / hexa2_plummer:
-// header re-centred on the group centre c in the record's image; for order
-// 4 the octupole and four hexadecapole fields negated as that layout wants.
-// A lane past the tile's end writes a massless, momentless record far away,
-// which adds exactly zero.  Lanes 2p and 2p+1 write pair p: one shuffle per
-// field pair.
-template <int KIND>
-__device__ __forceinline__ void relay_pairs(const unsigned char *stage, uint32_t code, bool valid,
-                                            const double *c, double box, float *pbuf, int lane) {
-    using K = KindOf<KIND, true>;
-    constexpr int NF = K::pair_fields;
-    constexpr int NR = K::rec_bytes / 4;  // staged record floats
-    float g[NF];
-    if (valid) {
-        const float4 *src = reinterpret_cast<const float4 *>(stage + K::rec_off(lane));
-        float f[NR];
-#pragma unroll
-        for (int k = 0; k < NR / 4; k++) {
-            const float4 v = src[k];
-            f[4 * k] = v.x;
-            f[4 * k + 1] = v.y;
-            f[4 * k + 2] = v.z;
-            f[4 * k + 3] = v.w;
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+    const float2 u = add2(f2(a.x, a.y), f2(b.x, b.y)), v = add2(f2(a.z, a.w), f2(b.z, b.w));
+    return make_float4(u.x, u.y, v.x, v.y);
+}
+__device__ __forceinline__ float4 shfl_xor4(float4 v, int m) {
+    return make_float4(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m),
+                       __shfl_xor_sync(0xffffffffu, v.z, m), __shfl_xor_sync(0xffffffffu, v.w, m));
+}
+// Partial sums of a warp's sinks: row b holds sinks 4 b .. 4 b + 3, lane l's
+// entry a part of sink 4 b + (l & 3).  The pitch keeps two rows' reads on
+// different banks.
+struct SinkSums {
+    float4 row[8][36];
+};
+
+// Every sink's sum over the warp's records, added to lane s's (hi, lo) for
+// sink s; eval(sink) gives this lane's part.  In a full block of four sinks lane l starts with
+// sink l & 3, so that the two exchange levels need no selects: what it keeps
+// is always its own sink's.  The last three levels are summed from shared
+// memory once a tile.  The four evaluations of a block are one basic block
+// (a test per sink kept them from overlapping: 19.4 against 20.1 cycles per
+// point interaction, 18.5 with the registers to hold four of them).
+template <int FOLDS, bool PLAIN, class Eval>
+__device__ __forceinline__ void sum_sinks(const SinkTable &T, int nsink, int lane, SinkSums &buf,
+                                          float2 *hi, float2 *lo, Eval eval) {
+    const int sw = lane & 3, nb = nsink >> 2, rem = nsink & 3;
+    const Sink *p0 = T.s + sw, *p1 = T.s + (sw ^ 1), *p2 = T.s + (sw ^ 2), *p3 = T.s + (sw ^ 3);
+    float4 *out = &buf.row[0][lane];
+#pragma unroll 1
+    for (int b = 0; b < nb; b++) {
+        float4 r0 = eval(*p0), r1 = eval(*p1);
+        r0 = add4(r0, shfl_xor4(r1, 1));
+        float4 r2 = eval(*p2), r3 = eval(*p3);
+        r2 = add4(r2, shfl_xor4(r3, 1));
+        *out = add4(r0, shfl_xor4(r2, 2));
+        out += 36;
+        p0 += 4;
+        p1 += 4;
+        p2 += 4;
+        p3 += 4;
+    }
+    if (rem) {
+        float4 keep = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int i = 0; i < rem; i++) {
+            float4 r = eval(T.s[4 * nb + i]);
+            r = add4(r, shfl_xor4(r, 1));
+            r = add4(r, shfl_xor4(r, 2));
+            if (sw == i)
+                keep = r;
         }
+        *out = keep;
+    }
+    __syncwarp();
+    if (lane < nsink) {
+        const float4 *row = buf.row[lane >> 2] + sw;
+#pragma unroll
+        for (int f = 0; f < FOLDS; f++) {
+            float4 v = row[4 * f];
+#pragma unroll
+            for (int k = FOLDS; k < 8; k += FOLDS) v = add4(v, row[4 * (f + k)]);
+            const float2 t[2] = {f2(v.x, v.y), f2(v.z, v.w)};
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                if (PLAIN)
+                    hi[q] = add2(hi[q], t[q]);
+                else
+                    comp_add2(hi[q], lo[q], t[q]);
+            }
+        }
+    }
+    __syncwarp();  // read: the next tile may write
+}
+
+__device__ __forceinline__ void store_part(const DevProblem &P, const Item &item, int lane,
+                                           const float2 *hi, const float2 *lo) {
+    float4 *dst = P.part + ((size_t)item.slot * 32 + lane) * 2;
+    dst[0] = make_float4(hi[0].x, hi[0].y, hi[1].x, hi[1].y);
+    dst[1] = make_float4(lo[0].x, lo[0].y, lo[1].x, lo[1].y);
+}
+
+// Coordinate of an absent record, beyond any sink: with zero mass and
+// moments it adds exactly zero.
+constexpr float kFar = 1.0e18f;
+
+// A record's FP64 position in image `code` as an FP32 offset from c;
+// `shifted` (the same in every lane): some lane's image is not the box's own.
+__device__ __forceinline__ void recentre(double x, double y, double z, uint32_t code, bool shifted,
+                                         double box, const double *c, float *o) {
+    if (shifted) {
         double sx, sy, sz;
         decode_shift(code, box, sx, sy, sz);
-        const double cx = __hiloint2double(__float_as_int(f[1]), __float_as_int(f[0]));
-        const double cy = __hiloint2double(__float_as_int(f[3]), __float_as_int(f[2]));
-        const double cz = __hiloint2double(__float_as_int(f[11]), __float_as_int(f[10]));
-        g[0] = (float)(cx + sx - c[0]);
-        g[1] = (float)(cy + sy - c[1]);
-        g[2] = (float)(cz + sz - c[2]);
-        g[3] = f[KIND == KH ? 31 : 12];
-#pragma unroll
-        for (int k = 4; k < 10; k++) g[k] = f[k];
-        if (KIND == KH) {
-            // h_z's xxz and yyz coefficients with -Xxxyy folded in (its
-            // z z-trace terms): -(Xxxxx + Xxxyy), -(Xyyyy + Xxxyy)
-            g[10] = -(f[21] + f[23]);
-            g[11] = -(f[25] + f[23]);
-#pragma unroll
-            for (int k = 12; k < 19; k++) g[k] = -f[k];
-            g[19] = f[19];
-            g[20] = f[20];
-#pragma unroll
-            for (int k = 21; k < 30; k++) g[k] = f[k];
-            g[30] = -f[30];
-            g[31] = 0.f;
-        }
-    } else {
-#pragma unroll
-        for (int k = 0; k < NF; k++) g[k] = k < 3 ? 1.0e3f : 0.f;
+        x += sx;
+        y += sy;
+        z += sz;
     }
-    const int s = lane & 1;
-    float *dst = pbuf + (lane >> 1) * K::pair_stride + 2 * s;
+    o[0] = (float)(x - c[0]);
+    o[1] = (float)(y - c[1]);
+    o[2] = (float)(z - c[2]);
+}
+
+template <int KIND>
+struct CellKind {
+    using Rec = std::conditional_t<KIND == KH, nln_hcell, nln_qcell>;
+    using Pair = std::conditional_t<KIND == KH, HexaPair, QuadPair>;
+    static constexpr int rec_bytes = (int)sizeof(Rec);
+    static constexpr int pairs = kTile[KIND] / 64;  // record pairs per lane
+    static constexpr int stage_bytes = kTile[KIND] * rec_bytes;
+    // per warp: the stage (its swizzle pattern repeats every 1024 bytes), the
+    // sinks, their sums, the mbarrier
+    static constexpr int warp_bytes =
+        (stage_bytes + (int)(sizeof(SinkTable) + sizeof(SinkSums)) + 8 + 1023) / 1024 * 1024;
+    // 16-byte chunk k of row r: the TMA swizzle of the row's width spreads
+    // the lanes' own-row reads over all banks
+    static __device__ __forceinline__ int chunk(int r, int k) {
+        const int sw = KIND == KH ? r & 7 : (r >> 1) & 3;
+        return r * rec_bytes + ((k ^ sw) << 4);
+    }
+};
+
+// Half h (0: .x, 1: .y) of this lane's record pair from row r of the stage.
+__device__ __forceinline__ void set_half(float2 &p, int h, float v) {
+    if (h)
+        p.y = v;
+    else
+        p.x = v;
+}
+
+template <int KIND>
+__device__ __forceinline__ void load_cell(const unsigned char *stage, int r, bool valid,
+                                          uint32_t code, double box, const double *c,
+                                          typename CellKind<KIND>::Pair &p, int h) {
+    using K = CellKind<KIND>;
+    constexpr int NC = KIND == KH ? 8 : 4;
+    const bool shifted = __any_sync(0xffffffffu, code != NLN_SHIFT_NONE);
+    float f[4 * NC];
 #pragma unroll
-    for (int q = 0; q < NF / 2; q++) {
-        const float send = s ? g[2 * q] : g[2 * q + 1];
-        const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-        *reinterpret_cast<float2 *>(dst + 4 * q) =
-            s ? make_float2(recv, g[2 * q + 1]) : make_float2(g[2 * q], recv);
+    for (int k = 0; k < NC; k++) {
+        // the last chunk of a quadrupole record holds one field, of an order-4 record two
+        const float4 v = *reinterpret_cast<const float4 *>(stage + K::chunk(r, k));
+        f[4 * k] = v.x;
+        f[4 * k + 1] = v.y;
+        f[4 * k + 2] = v.z;
+        f[4 * k + 3] = v.w;
+    }
+    // floats 0-5 the FP64 centre, 6 mass, 7 R, then q2[5] (order 4: q3[7], q4[9])
+    auto d = [&](int k) { return __hiloint2double(__float_as_int(f[k + 1]), __float_as_int(f[k])); };
+    float o[3];
+    recentre(d(0), d(2), d(4), code, shifted, box, c, o);
+    auto put = [&](float2 &dst, float v) { set_half(dst, h, valid ? v : 0.f); };
+    set_half(p.x, h, valid ? o[0] : kFar);
+    set_half(p.y, h, valid ? o[1] : kFar);
+    set_half(p.z, h, valid ? o[2] : kFar);
+    put(p.m, f[6]);
+    const float R = f[7], c2 = -3.0f * R * R;
+#pragma unroll
+    for (int k = 0; k < 5; k++) put(p.q[k], c2 * f[8 + k]);
+    if constexpr (KIND == KQ) {
+        put(p.q[5], -(c2 * f[8] + c2 * f[10]));
+    } else {
+        const float c3 = 7.5f * R * R * R, c4 = -17.5f * R * R * R * R;
+        const float *q3 = f + 13, *q4 = f + 20;
+#pragma unroll
+        for (int k = 0; k < 7; k++) put(p.o[k], c3 * q3[k]);
+        put(p.o[7], -(c3 * q3[0] + c3 * q3[2]));
+        put(p.o[8], -(c3 * q3[1] + c3 * q3[3]));
+#pragma unroll
+        for (int k = 0; k < 9; k++) put(p.h[k], c4 * q4[k]);
+        put(p.h[9], -(c4 * q4[0] + c4 * q4[2]));
+        put(p.h[10], -(c4 * q4[4] + c4 * q4[2]));
+        put(p.h[11], -(c4 * q4[1] + c4 * q4[3]));
     }
 }
 
-// Compile-time shape of the paired kernels, as measured best on a B200
-// (-D to rebuild with others): unroll of the pair loop and minimum resident
-// blocks (register cap) for the order-4 (H2) and quadrupole (Q2) kernels;
-// GRAV_Q2_PAIRED=0 keeps the quadrupole kernel on the scalar loop.  Order 4:
-// unroll 2 held to 3 blocks (80 registers, a few spilled words) is 0.6 %
-// faster than unroll 1 and beat unroll 2 at its own 117 registers; minimum
-// blocks 0 leaves the register count to the compiler (a 1 there lets it
-// grow and cost occupancy).
-#ifndef GRAV_H2_UNROLL
-#define GRAV_H2_UNROLL 2
-#endif
-#ifndef GRAV_H2_MINB
-#define GRAV_H2_MINB 3
-#endif
-#ifndef GRAV_Q2_MINB
-#define GRAV_Q2_MINB 0
-#endif
-#ifndef GRAV_Q2_UNROLL
-#define GRAV_Q2_UNROLL 4
-#endif
-#ifndef GRAV_Q2_PAIRED
-#define GRAV_Q2_PAIRED 1
-#endif
-constexpr int kH2Unroll = GRAV_H2_UNROLL;
-constexpr int kQ2Unroll = GRAV_Q2_UNROLL;
+// Quadrupole and order-4 lists: tiles of 128 or 64 cells, two or one record
+// pairs per lane (a tile that ends short leaves out the second), gathered
+// from the cell table by TMA (row gathers of four records, issued by lane 0)
+// into one stage per warp, which is free for the next tile's copies as soon
+// as the lanes hold their records.
 // PLAIN: the plain FP32 form the reference's lists compute in (absolute FP32
 // coordinates, nln/mac.c:1421-1561 copies cell centres as floats): sinks and
 // sources are not re-centred on the group centre and tile sums are added
 // without compensation.  It exists to be compared with the mixed form.
-template <int KIND, bool STAGED, bool PLAIN = false>
-__global__ void __launch_bounds__(256, KIND == KH ? (STAGED ? GRAV_H2_MINB : 3)
-                                                  : (KIND == KQ && STAGED ? GRAV_Q2_MINB : 0))
-    k_batch(const __grid_constant__ CUtensorMap tmap, DevProblem P) {
-    // staged quadrupole and order-4 tables run the paired (f32x2)
-    // interaction on a pair-interleaved copy of each tile
-    constexpr bool PAIRED = (KIND == KH || (KIND == KQ && GRAV_Q2_PAIRED)) && STAGED;
-    using K = KindOf<KIND, PAIRED>;
-    constexpr int RB = K::rec_bytes;
-    constexpr int ORDER = K::order;
-    constexpr int NST = K::stages;
-    extern __shared__ __align__(128) unsigned char smem[];
+template <int KIND, bool PLAIN>
+__global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GRAV_Q_MINB)
+    k_cells(const __grid_constant__ CUtensorMap tmap, DevProblem P) {
+    using K = CellKind<KIND>;
+    constexpr int NP = K::pairs, NE = 2 * NP, CT = kTile[KIND];
+    extern __shared__ __align__(1024) unsigned char smem[];
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    unsigned char *wbuf = smem + (size_t)wib * K::warp_bytes;
-    float *pbuf = reinterpret_cast<float *>(wbuf + NST * K::stage_bytes);  // paired path
-    uint64_t *bar = reinterpret_cast<uint64_t *>(wbuf + NST * K::stage_bytes + K::pair_bytes);
-    uint32_t *codes = reinterpret_cast<uint32_t *>(bar + NST);  // [NST][TILE] image codes
+    unsigned char *stage = smem + (size_t)(threadIdx.x >> 5) * K::warp_bytes;
+    SinkTable &sinks = *reinterpret_cast<SinkTable *>(stage + K::stage_bytes);
+    SinkSums &sums = *reinterpret_cast<SinkSums *>(&sinks + 1);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(&sums + 1);
     if (lane == 0) {
-        for (int s = 0; s < NST; s++) mbar_init(&bar[s], 1);
+        mbar_init(bar, 1);
         fence_mbar_init();
     }
     __syncwarp();
-
     const uint32_t *list = P.list[KIND];
     const uint32_t ntab = (uint32_t)P.ntab[KIND];
-    // tiles issued (and later consumed, in the same order) by this warp:
-    // tile seq uses stage seq % NST with mbarrier parity (seq / NST) & 1
-    uint32_t tseq = 0;
-    bool alive = true;
-
-    while (alive) {
+    const float2 e2 = splat2(P.eps2);
+    uint32_t phase = 0;
+    for (;;) {
         int it = 0;
         if (lane == 0)
             it = atomicAdd(&P.counters[KIND], 1);
@@ -468,165 +498,127 @@ __global__ void __launch_bounds__(256, KIND == KH ? (STAGED ? GRAV_H2_MINB : 3)
         const nln_group G = P.groups[item.group];
         const double c[3] = {PLAIN ? 0.0 : G.cen[0], PLAIN ? 0.0 : G.cen[1],
                              PLAIN ? 0.0 : G.cen[2]};
-        // this lane's sink, as an FP32 offset from the group centre
-        float ux = 0.f, uy = 0.f, uz = 0.f;
-        if (lane < G.count) {
-            float4 s = P.points[G.first + lane];
-            ux = (float)((double)s.x - c[0]);
-            uy = (float)((double)s.y - c[1]);
-            uz = (float)((double)s.z - c[2]);
-        }
-        float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
         const int64_t nent = item.end - item.begin;
-        const int ntile = (int)((nent + TILE - 1) / TILE);
-
-        auto fetch = [&](int t) -> uint32_t {
-            int64_t k = item.begin + (int64_t)t * TILE + lane;
-            return (t < ntile && k < item.end) ? __ldg(list + k) : 0u;
+        const int ntile = (int)((nent + CT - 1) / CT);
+        // this lane's entries of tile t
+        auto fetch = [&](int t, uint32_t *e) {
+#pragma unroll
+            for (int h = 0; h < NE; h++) {
+                const int64_t k = item.begin + (int64_t)t * CT + 32 * h + lane;
+                e[h] = t < ntile && k < item.end ? __ldg(list + k) : 0u;
+            }
         };
-        // Start tile t (sequence number seq): each lane holds one entry; the
-        // row indices are gathered to lane 0, which issues one TMA row
-        // gather per 4 records.  Unused rows of a short tile repeat row 0.
-        auto issue = [&](int t, uint32_t ent, uint32_t seq) {
-            const int nt = (int)min((int64_t)TILE, nent - (int64_t)t * TILE);
+        // Start the copies of tile t: the row indices are gathered to lane 0;
+        // unused rows of the last gather repeat row 0.  code: the image codes
+        // of this lane's records.
+        auto issue = [&](int t, const uint32_t *e, uint32_t *code) {
+            const int nt = (int)min((int64_t)CT, nent - (int64_t)t * CT);
             const int ng4 = (nt + 3) >> 2;
-            const uint32_t st = seq % NST;
-            uint32_t idx = ent & NLN_IDX_MASK, code = ent >> NLN_IDX_BITS;
-            // entries are checked at upload, except in the pipelined end-to-end call
-            if (lane < nt && (idx >= ntab || code > 26u)) {
-                atomicOr(P.err, GC_DEV_BAD_INDEX);
-                idx = 0;
-                code = NLN_SHIFT_NONE;
-            }
-            if (lane >= nt)
-                idx = 0;
-            codes[st * TILE + lane] = code;
             if (lane == 0)
-                mbar_arrive_expect_tx(&bar[st], (uint32_t)(ng4 * 4 * RB));
-            unsigned char *dst = wbuf + st * K::stage_bytes;
+                mbar_arrive_expect_tx(bar, (uint32_t)(ng4 * 4 * K::rec_bytes));
 #pragma unroll
-            for (int g = 0; g < TILE / 4; g++) {
-                const int r0 = __shfl_sync(0xffffffffu, (int)idx, 4 * g);
-                const int r1 = __shfl_sync(0xffffffffu, (int)idx, 4 * g + 1);
-                const int r2 = __shfl_sync(0xffffffffu, (int)idx, 4 * g + 2);
-                const int r3 = __shfl_sync(0xffffffffu, (int)idx, 4 * g + 3);
-                if (lane == 0 && g < ng4)
-                    tma_gather4(dst + g * K::group_bytes, &tmap, r0, r1, r2, r3, &bar[st]);
+            for (int h = 0; h < NE; h++) {
+                uint32_t idx = e[h] & NLN_IDX_MASK;
+                const bool live = 32 * h + lane < nt;
+                code[h] = live ? e[h] >> NLN_IDX_BITS : NLN_SHIFT_NONE;
+                // entries are checked at upload, except in the pipelined end-to-end call
+                if (live && (idx >= ntab || code[h] > 26u)) {
+                    atomicOr(P.err, GC_DEV_BAD_INDEX);
+                    idx = 0;
+                    code[h] = NLN_SHIFT_NONE;
+                }
+                if (!live)
+                    idx = 0;
+                if (8 * h >= ng4)
+                    continue;
+#pragma unroll
+                for (int g = 0; g < 8; g++) {
+                    const int r0 = __shfl_sync(0xffffffffu, (int)idx, 4 * g);
+                    const int r1 = __shfl_sync(0xffffffffu, (int)idx, 4 * g + 1);
+                    const int r2 = __shfl_sync(0xffffffffu, (int)idx, 4 * g + 2);
+                    const int r3 = __shfl_sync(0xffffffffu, (int)idx, 4 * g + 3);
+                    if (lane == 0 && 8 * h + g < ng4)
+                        tma_gather4(stage + (8 * h + g) * 4 * K::rec_bytes, &tmap, r0, r1, r2, r3,
+                                    bar);
+                }
             }
         };
-        // tiles in flight ahead of the one being computed
-        constexpr int AHEAD = PAIRED ? 1 : NST - 1;
+        uint32_t ent[NE], code[NE];
 #pragma unroll
-        for (int p = 0; p < AHEAD; p++)
-            if (p < ntile)
-                issue(p, fetch(p), tseq + p);
-        uint32_t ent_next = fetch(AHEAD);
+        for (int h = 0; h < NE; h++) code[h] = NLN_SHIFT_NONE;
+        fetch(0, ent);
+        if (ntile > 0)
+            issue(0, ent, code);
+        fetch(1, ent);
+        stage_sinks(sinks, P, G, c, lane);
+        float2 hi[2] = {splat2(0.f), splat2(0.f)}, lo[2] = {splat2(0.f), splat2(0.f)};
         for (int t = 0; t < ntile; t++) {
-            const uint32_t seq = tseq + t;
-            if (!PAIRED) {
-                if (t + NST - 1 < ntile)
-                    issue(t + NST - 1, ent_next, seq + NST - 1);
-                ent_next = fetch(t + NST);
-            }
-            const int nt = (int)min((int64_t)TILE, nent - (int64_t)t * TILE);
-            const uint32_t st = seq % NST;
-            bool ok = mbar_wait_bounded(&bar[st], (seq / NST) & 1, P.err);
-            if (!__all_sync(0xffffffffu, ok)) {
-                // give the copies still in flight a bounded chance to land
-                for (int u = t + 1; u < ntile && u < t + NST; u++)
-                    mbar_wait_bounded(&bar[(tseq + u) % NST], ((tseq + u) / NST) & 1, P.err,
-                                      1u << 10);
-                alive = false;
-                break;
-            }
-            unsigned char *bt = wbuf + st * K::stage_bytes;
-            Acc4 a{0.f, 0.f, 0.f, 0.f};
-            if constexpr (PAIRED) {
-                relay_pairs<KIND>(bt, codes[st * TILE + lane], lane < nt, c, P.box, pbuf, lane);
-                __syncwarp();  // the stage is free: start the next copy, then compute
-                if (t + 1 < ntile)
-                    issue(t + 1, ent_next, seq + 1);
-                ent_next = fetch(t + 2);
-                const float2 nsx = splat2(-ux), nsy = splat2(-uy), nsz = splat2(-uz);
-                const float2 e2 = splat2(P.eps2), nqsh = splat2(-P.qsh);
-                Acc2h A{splat2(0.f), splat2(0.f), splat2(0.f), splat2(0.f)};
-                const int npair = (nt + 1) >> 1;
-                auto pair = [&](int q) {
-                    if (KIND == KH)
-                        hexa2_plummer(pbuf + q * K::pair_stride, nsx, nsy, nsz, e2, nqsh, A);
-                    else
-                        quad2_plummer(pbuf + q * K::pair_stride, nsx, nsy, nsz, e2, nqsh, A);
-                };
-                constexpr int kUnroll = KIND == KH ? kH2Unroll : kQ2Unroll;
-                if (npair == TILE / 2) {
-#pragma unroll kUnroll
-                    for (int q = 0; q < TILE / 2; q++) pair(q);
-                } else {
-                    for (int q = 0; q < npair; q++) pair(q);
-                }
-                a.ax = A.ax.x + A.ax.y;
-                a.ay = A.ay.x + A.ay.y;
-                a.az = A.az.x + A.az.y;
-                a.phi = -(A.nphi.x + A.nphi.y);
-            } else {
-            if (lane < nt)
-                convert<KIND, STAGED>(bt + K::rec_off(lane), codes[st * TILE + lane], c, P.box);
-            __syncwarp();
-            if (nt == TILE) {
-#pragma unroll 4
-                for (int r = 0; r < TILE; r++)
-                    interact<ORDER, SOFT_PLUMMER>(reinterpret_cast<const float *>(bt + K::rec_off(r)),
-                                                  ux, uy, uz, P.eps2, P.qsh, a);
-            } else {
-                for (int r = 0; r < nt; r++)
-                    interact<ORDER, SOFT_PLUMMER>(reinterpret_cast<const float *>(bt + K::rec_off(r)),
-                                                  ux, uy, uz, P.eps2, P.qsh, a);
-            }
-            }
-            if (PLAIN) {
-                hi[0] += a.ax;
-                hi[1] += a.ay;
-                hi[2] += a.az;
-                hi[3] += a.phi;
-            } else {
-                comp_add(hi[0], lo[0], a.ax);
-                comp_add(hi[1], lo[1], a.ay);
-                comp_add(hi[2], lo[2], a.az);
-                comp_add(hi[3], lo[3], a.phi);
-            }
-            __syncwarp();  // every lane is done with this stage before it is refilled
+            const int nt = (int)min((int64_t)CT, nent - (int64_t)t * CT);
+            const bool ok = mbar_wait_bounded(bar, phase, P.err);
+            if (!__all_sync(0xffffffffu, ok))
+                return;  // a lost copy: the error word is set, nothing else is in flight
+            phase ^= 1;
+            typename K::Pair rec[NP];
+#pragma unroll
+            for (int h = 0; h < NE; h++)
+                if (h < 2 || nt > 64 * (h >> 1))
+                    load_cell<KIND>(stage, 32 * h + lane, 32 * h + lane < nt, code[h], P.box, c,
+                                    rec[h >> 1], h & 1);
+            __syncwarp();  // the stage is free: start the next copies, then compute
+            if (t + 1 < ntile)
+                issue(t + 1, ent, code);
+            fetch(t + 2, ent);
+            // the forms of a tile are told apart outside the sink loop
+            auto sums_of = [&](auto form) {
+                constexpr bool F = decltype(form)::value;
+                sum_sinks<KIND == KH ? 2 : 4, PLAIN>(sinks, G.count, lane, sums, hi, lo, [&](const Sink &k) {
+                    const float2 nx = f2(k.xy.x, k.xy.y), ny = f2(k.xy.z, k.xy.w), nz = k.z;
+                    Sum2 A;
+                    if constexpr (KIND == KH) {
+                        cell_pair<F>(rec[0], nx, ny, nz, e2, P.qsh, A);
+                    } else {
+                        cell_pair<true>(rec[0], nx, ny, nz, e2, P.qsh, A);
+                        if (F)
+                            cell_pair<false>(rec[1], nx, ny, nz, e2, P.qsh, A);
+                    }
+                    return A.total();
+                });
+            };
+            const bool form = KIND == KH ? P.qsh == 0.5f : nt > 64;
+            if (form)
+                sums_of(std::true_type());
+            else
+                sums_of(std::false_type());
         }
-        tseq += ntile;
-        if (!alive)
-            break;
-        float4 *dst = P.part + ((size_t)item.slot * 32 + lane) * 2;
-        dst[0] = make_float4(hi[0], hi[1], hi[2], hi[3]);
-        dst[1] = make_float4(lo[0], lo[1], lo[2], lo[3]);
+        store_part(P, item, lane, hi, lo);
     }
 }
 
-// Point records (bodies and cell monopoles, 16 B each) are staged without
-// TMA: every lane loads its own record with a plain read-only load, one tile
-// ahead of use (the list entry two tiles ahead), re-centres it in registers
-// and writes it to the warp's shared tile; the row-gather path costs more
-// than it saves for records this small.  The tile is laid out in record
-// pairs, field by field (pair j: npx0 npx1 npy0 npy1 | npz0 npz1 m0 m1, with
-// np the negated offset), so that each 16-byte shared read yields two ready
-// operand pairs for the paired FP32 instructions of mono2_plummer.
-template <bool PLAIN = false>
-__global__ void __launch_bounds__(256) k_points(DevProblem P) {
-    __shared__ __align__(16) float stile[8][TILE * 4];
+// Point lists (bodies and cell monopoles): tiles of 256 records, eight per
+// lane in four pairs.  Every lane copies its own next records (a body's 16
+// bytes, a cell's FP64 centre and mass: 32) to its own slots of the warp's
+// stage by cp.async while the warp computes the current tile, with the list
+// words one tile further ahead; the registers that hold four evaluations at
+// once leave 16 warps on an SM, too few to cover the loads otherwise.
+struct PointStage {
+    float4 chunk[kPointTile / 32][2][32];  // [record of the lane][half][lane]
+};
+constexpr int kPointWarpBytes = (int)(sizeof(PointStage) + sizeof(SinkTable) + sizeof(SinkSums));
+
+template <bool PLAIN>
+__global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProblem P) {
+    extern __shared__ __align__(16) unsigned char psm[];
     const int lane = threadIdx.x & 31;
-    float *tile = stile[threadIdx.x >> 5];
-    const float4 *tile4 = reinterpret_cast<const float4 *>(tile);
-    // this lane's record slot in the pair layout
-    float *mine = tile + (lane >> 1) * 8 + (lane & 1);
+    PointStage &stage = *reinterpret_cast<PointStage *>(psm + (size_t)(threadIdx.x >> 5) * kPointWarpBytes);
+    SinkTable &sinks = *reinterpret_cast<SinkTable *>(&stage + 1);
+    SinkSums &sums = *reinterpret_cast<SinkSums *>(&sinks + 1);
     const uint32_t *list = P.list[KP];
     const uint32_t ntab = (uint32_t)P.ntab[KP];
-    const uint32_t nb = ntab - (uint32_t)P.ncells;
-    const bool periodic = P.box > 0;
-    const float2 e2 = make_float2(P.eps2, P.eps2);
-    while (true) {
+    const uint32_t nb = PLAIN || !P.ccen ? ntab : ntab - (uint32_t)P.ncells;  // cells from here on
+    const float2 e2 = splat2(P.eps2);
+    constexpr int NP = kPointTile / 64, NE = 2 * NP;  // record pairs, records per lane
+    constexpr uint32_t kNone = 0xffffffffu;           // no entry
+    for (;;) {
         int it = 0;
         if (lane == 0)
             it = atomicAdd(&P.counters[KP], 1);
@@ -637,106 +629,96 @@ __global__ void __launch_bounds__(256) k_points(DevProblem P) {
         const nln_group G = P.groups[item.group];
         const double c[3] = {PLAIN ? 0.0 : G.cen[0], PLAIN ? 0.0 : G.cen[1],
                              PLAIN ? 0.0 : G.cen[2]};
-        float ux = 0.f, uy = 0.f, uz = 0.f;
-        if (lane < G.count) {
-            float4 sk = P.points[G.first + lane];
-            ux = (float)((double)sk.x - c[0]);
-            uy = (float)((double)sk.y - c[1]);
-            uz = (float)((double)sk.z - c[2]);
-        }
-        const float2 sx = make_float2(ux, ux), sy = make_float2(uy, uy), sz = make_float2(uz, uz);
-        float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
-        const int64_t nent = item.end - item.begin;
-        const int ntile = (int)((nent + TILE - 1) / TILE);
-        constexpr uint32_t kNone = 0xffffffffu;  // no entry in this lane
-        auto entry = [&](int t) -> uint32_t {
-            const int64_t k = item.begin + (int64_t)t * TILE + lane;
-            return (t < ntile && k < item.end) ? __ldg(list + k) : kNone;
+        auto fetch = [&](int64_t k0, uint32_t *e) {
+#pragma unroll
+            for (int j = 0; j < NE; j++) {
+                const int64_t k = k0 + 32 * j + lane;
+                e[j] = k < item.end ? __ldg(list + k) : kNone;
+            }
         };
-        // a record's position (FP64: a cell monopole's centre from the staged
-        // cell table in the mixed form) and mass
-        struct Rec {
-            double x, y, z;
-            float m;
-        };
-        auto record = [&](uint32_t &e) -> Rec {
-            if (e == kNone)
-                return Rec{0.0, 0.0, 0.0, 0.f};
-            uint32_t idx = e & NLN_IDX_MASK;
-            // entries are checked at upload, except in the pipelined end-to-end call
-            if (idx >= ntab || (e >> NLN_IDX_BITS) > 26u) {
+        // Start this lane's copies of its entries' records.  Entries are
+        // checked at upload, except in the pipelined end-to-end call: a bad
+        // one becomes body 0 in the box's own image.
+        auto copy = [&](uint32_t *e) {
+            bool bad = false;
+#pragma unroll
+            for (int j = 0; j < NE; j++) {
+                if (e[j] == kNone)
+                    continue;
+                if ((e[j] & NLN_IDX_MASK) >= ntab || (e[j] >> NLN_IDX_BITS) > 26u) {
+                    bad = true;
+                    e[j] = NLN_SHIFT_NONE << NLN_IDX_BITS;
+                }
+                const uint32_t idx = e[j] & NLN_IDX_MASK;
+                if (idx < nb) {
+                    cp_async16(&stage.chunk[j][0][lane], P.points + idx);
+                } else {
+                    const unsigned char *r = P.ccen + (size_t)(idx - nb) * P.cstride;
+                    cp_async16(&stage.chunk[j][0][lane], r);
+                    cp_async16(&stage.chunk[j][1][lane], r + 16);
+                }
+            }
+            cp_async_commit();
+            if (bad)
                 atomicOr(P.err, GC_DEV_BAD_INDEX);
-                idx = 0;
-                e = NLN_SHIFT_NONE << NLN_IDX_BITS;
-            }
-            const float4 p = __ldg(P.points + idx);
-            if (!PLAIN && P.cstage && idx >= nb) {
-                const float4 *cs = P.cstage + (size_t)(idx - nb) * P.cstride;
-                const float4 a = __ldg(cs), b = __ldg(cs + 2);
-                return Rec{__hiloint2double(__float_as_int(a.y), __float_as_int(a.x)),
-                           __hiloint2double(__float_as_int(a.w), __float_as_int(a.z)),
-                           __hiloint2double(__float_as_int(b.w), __float_as_int(b.z)), p.w};
-            }
-            return Rec{(double)p.x, (double)p.y, (double)p.z, p.w};
         };
-        uint32_t e_cur = entry(0);
-        Rec r_cur = record(e_cur);
-        uint32_t e_nxt = entry(1);
-        for (int t = 0; t < ntile; t++) {
-            const Rec r_nxt = record(e_nxt);  // consumed next tile
-            const uint32_t e_nn = entry(t + 2);
-            const int nt = (int)min((int64_t)TILE, nent - (int64_t)t * TILE);
-            // an absent record: massless and far from every sink
-            float npx = -1.0e3f, npy = -1.0e3f, npz = -1.0e3f, m = 0.f;
-            if (e_cur != kNone) {
-                double sxs = 0.0, sys = 0.0, szs = 0.0;
-                if (periodic)
-                    decode_shift(e_cur >> NLN_IDX_BITS, P.box, sxs, sys, szs);
-                npx = (float)(c[0] - (r_cur.x + sxs));
-                npy = (float)(c[1] - (r_cur.y + sys));
-                npz = (float)(c[2] - (r_cur.z + szs));
-                m = r_cur.m;
-            }
-            __syncwarp();  // the previous tile is no longer read
-            mine[0] = npx;
-            mine[2] = npy;
-            mine[4] = npz;
-            mine[6] = m;
-            __syncwarp();
-            Acc2 a2{make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f),
-                    make_float2(0.f, 0.f)};
-            if (nt == TILE) {
-#pragma unroll 8
-                for (int j = 0; j < TILE / 2; j++) {
-                    const float4 A = tile4[2 * j], B = tile4[2 * j + 1];
-                    mono2_plummer(make_float2(A.x, A.y), make_float2(A.z, A.w),
-                                  make_float2(B.x, B.y), make_float2(B.z, B.w), sx, sy, sz, e2, a2);
+        uint32_t cur[NE], nxt[NE];
+        fetch(item.begin, cur);
+        copy(cur);
+        fetch(item.begin + kPointTile, nxt);
+        stage_sinks(sinks, P, G, c, lane);
+        float2 hi[2] = {splat2(0.f), splat2(0.f)}, lo[2] = {splat2(0.f), splat2(0.f)};
+        for (int64_t k0 = item.begin; k0 < item.end; k0 += kPointTile) {
+            const int np = (int)min((int64_t)NP, (item.end - k0 + 63) / 64);  // pairs in use
+            MonoPair rec[NP];
+            cp_async_wait<0>();  // this lane's records have landed
+#pragma unroll
+            for (int j = 0; j < NE; j++) {
+                if ((j >> 2) > (np - 1) >> 1)
+                    break;
+                const bool live = cur[j] != kNone;
+                const uint32_t idx = cur[j] & NLN_IDX_MASK;
+                const uint32_t code = live ? cur[j] >> NLN_IDX_BITS : NLN_SHIFT_NONE;
+                const float4 u = stage.chunk[j][0][lane];
+                double x = u.x, y = u.y, z = u.z;
+                float m = u.w;
+                if (idx >= nb) {
+                    const float4 w = stage.chunk[j][1][lane];
+                    x = __hiloint2double(__float_as_int(u.y), __float_as_int(u.x));
+                    y = __hiloint2double(__float_as_int(u.w), __float_as_int(u.z));
+                    z = __hiloint2double(__float_as_int(w.y), __float_as_int(w.x));
+                    m = w.z;
                 }
-            } else {
-                for (int j = 0; j < (nt + 1) / 2; j++) {
-                    const float4 A = tile4[2 * j], B = tile4[2 * j + 1];
-                    mono2_plummer(make_float2(A.x, A.y), make_float2(A.z, A.w),
-                                  make_float2(B.x, B.y), make_float2(B.z, B.w), sx, sy, sz, e2, a2);
-                }
+                float o[3];
+                recentre(x, y, z, code, __any_sync(0xffffffffu, code != NLN_SHIFT_NONE), P.box, c,
+                         o);
+                set_half(rec[j >> 1].x, j & 1, live ? o[0] : kFar);
+                set_half(rec[j >> 1].y, j & 1, live ? o[1] : kFar);
+                set_half(rec[j >> 1].z, j & 1, live ? o[2] : kFar);
+                set_half(rec[j >> 1].m, j & 1, live ? m : 0.f);
             }
-            if (PLAIN) {
-                hi[0] -= a2.nax.x + a2.nax.y;
-                hi[1] -= a2.nay.x + a2.nay.y;
-                hi[2] -= a2.naz.x + a2.naz.y;
-                hi[3] -= a2.nphi.x + a2.nphi.y;
-            } else {
-                comp_add(hi[0], lo[0], -(a2.nax.x + a2.nax.y));
-                comp_add(hi[1], lo[1], -(a2.nay.x + a2.nay.y));
-                comp_add(hi[2], lo[2], -(a2.naz.x + a2.naz.y));
-                comp_add(hi[3], lo[3], -(a2.nphi.x + a2.nphi.y));
-            }
-            e_cur = e_nxt;
-            r_cur = r_nxt;
-            e_nxt = e_nn;
+            copy(nxt);
+#pragma unroll
+            for (int j = 0; j < NE; j++) cur[j] = nxt[j];
+            fetch(k0 + 2 * kPointTile, nxt);
+            // a tile of at most 128 records leaves out the other two pairs
+            auto sums_of = [&](auto n) {
+                sum_sinks<8, PLAIN>(sinks, G.count, lane, sums, hi, lo, [&](const Sink &k) {
+                    const float2 nx = f2(k.xy.x, k.xy.y), ny = f2(k.xy.z, k.xy.w), nz = k.z;
+                    Sum2 A;
+                    mono_pair<true>(rec[0], nx, ny, nz, e2, A);
+#pragma unroll
+                    for (int q = 1; q < decltype(n)::value; q++)
+                        mono_pair<false>(rec[q], nx, ny, nz, e2, A);
+                    return A.total();
+                });
+            };
+            if (np > 2)
+                sums_of(std::integral_constant<int, 4>());
+            else
+                sums_of(std::integral_constant<int, 2>());
         }
-        float4 *dst = P.part + ((size_t)item.slot * 32 + lane) * 2;
-        dst[0] = make_float4(hi[0], hi[1], hi[2], hi[3]);
-        dst[1] = make_float4(lo[0], lo[1], lo[2], lo[3]);
+        store_part(P, item, lane, hi, lo);
     }
 }
 
@@ -1055,18 +1037,16 @@ struct grav_plan {
     int nsm = 148;
     int launches = 0;
     int64_t nslots = 0;
-    CUtensorMap tmap[3];    // row-gather views of the point, quadrupole and order-4 tables
+    CUtensorMap tmap[3];    // row-gather views of the quadrupole and order-4 tables
     int timing = 0;         // record events around each kernel of an evaluation
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     std::vector<int64_t> lists_ptr[4];  // host copies of the P, Q, H (queue rebuilds) and
                                         // correction list offsets
     int64_t *order = nullptr;           // device-built plans: tree position -> input index
-    bool staged = false;                // the Q/H tensor maps view pre-staged tables
     bool plain = false;                 // plain FP32 kernels (grav_problem.precision = 1)
     int integrator = 0;                 // 0: Integrate, 1: CosmoIntegrate (step.cuh)
     bool evaluated = false;             // grav_groups_eval_CUDA has been enqueued (the
                                         // correction moments the adjoint reads are set)
-    float4 *qstage = nullptr, *hstage = nullptr;  // pre-staged cell tables (k_stage_cells)
     grav_step_state *step = nullptr;  // tree links, refit scratch and the step graph
     grav_adjoint_state *adj = nullptr;  // adjoint scratch
     // periodic: the side stream of k_ewald_moments, its fork/join events and
@@ -1090,9 +1070,11 @@ struct grav_plan {
 
 namespace {
 
-// A 2-D tensor map over `rows` records of `row_bytes` (a multiple of 16),
-// box = one full record (one row high, as the row gather requires).
-int encode_rows(CUtensorMap *m, const void *base, uint64_t rows, uint32_t row_bytes) {
+// A 2-D tensor map over the records of a cell table, box = one full record
+// (one row high, as the row gather requires), swizzled over the record's
+// width (CellKind::chunk).
+template <int KIND>
+int encode_cells(CUtensorMap *m, const void *base, int64_t rows) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
         void *fn = nullptr;
@@ -1102,19 +1084,26 @@ int encode_rows(CUtensorMap *m, const void *base, uint64_t rows, uint32_t row_by
             return gc::set_status(-1, "cuTensorMapEncodeTiled unavailable");
         encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
-    const uint32_t w = row_bytes / 4;
-    cuuint64_t dims[2] = {w, rows};
-    cuuint64_t strides[1] = {row_bytes};
+    constexpr uint32_t bytes = CellKind<KIND>::rec_bytes, w = bytes / 4;
+    cuuint64_t dims[2] = {w, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {bytes};
     cuuint32_t box[2] = {w, 1};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(base), dims,
                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                        KIND == KH ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
-        return gc::set_status(-1, "cuTensorMapEncodeTiled failed (%d) for %llu rows of %u bytes",
-                              (int)r, (unsigned long long)rows, row_bytes);
+        return gc::set_status(-1, "cuTensorMapEncodeTiled failed (%d) for %lld rows of %u bytes",
+                              (int)r, (long long)rows, bytes);
     return 0;
+}
+
+// The table k_points reads FP64 cell centres from, and its record size.
+const unsigned char *cell_centres(const DevProblem &d, bool quad, int &stride) {
+    stride = quad ? (int)sizeof(nln_qcell) : (int)sizeof(nln_hcell);
+    return quad ? reinterpret_cast<const unsigned char *>(d.qcells)
+                : reinterpret_cast<const unsigned char *>(d.hcells);
 }
 
 template <typename T>
@@ -1168,14 +1157,16 @@ grav_tuning default_tuning() {
 }
 
 // Split lists so that there are at least ~8 work items per resident warp
-// (about 148 SMs x 32 warps), in whole tiles, no shorter than `lo`.
-int auto_chunk(int64_t total, int64_t ngroups, int nsm, int64_t lo) {
-    const int64_t warps = (int64_t)nsm * 32;
+// (about 148 SMs x 16 warps), in whole tiles: shorter items spend more on
+// their start than the idle warps are worth (8,000 bodies: 43 us a point
+// kernel in items of 64 or 128, 33 us in tiles of 256).
+int auto_chunk(int64_t total, int64_t ngroups, int nsm, int kind) {
+    const int64_t warps = (int64_t)nsm * 16;
     int64_t ng = std::max<int64_t>(ngroups, 1);
     int64_t per = std::max<int64_t>(1, (8 * warps + ng - 1) / ng);
     int64_t avg = std::max<int64_t>(1, total / ng);
-    int64_t c = std::max<int64_t>(lo, avg / per);
-    c = (c + TILE - 1) / TILE * TILE;
+    const int64_t tile = kTile[kind];
+    const int64_t c = (std::max<int64_t>(tile, avg / per) + tile - 1) / tile * tile;
     return (int)std::min<int64_t>(1 << 24, c);
 }
 
@@ -1447,11 +1438,11 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     if (pl->tune.warps_per_block < 1 || pl->tune.warps_per_block > 8)
         pl->tune.warps_per_block = 8;
     if (pl->tune.chunk_p <= 0)
-        pl->tune.chunk_p = auto_chunk(eptr[ng], ng, pl->nsm, 128);
+        pl->tune.chunk_p = auto_chunk(eptr[ng], ng, pl->nsm, KP);
     if (pl->tune.chunk_q <= 0)
-        pl->tune.chunk_q = auto_chunk(hp->qptr ? hp->qptr[ng] : 0, ng, pl->nsm, 64);
+        pl->tune.chunk_q = auto_chunk(hp->qptr ? hp->qptr[ng] : 0, ng, pl->nsm, KQ);
     if (pl->tune.chunk_h <= 0)
-        pl->tune.chunk_h = auto_chunk(hp->hptr ? hp->hptr[ng] : 0, ng, pl->nsm, 32);
+        pl->tune.chunk_h = auto_chunk(hp->hptr ? hp->hptr[ng] : 0, ng, pl->nsm, KH);
 
     // work items, created group by group (slot order), then sorted per kind by cost
     std::vector<Item> items[3];
@@ -1703,28 +1694,13 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
         pl->counts[1] = (int64_t)h[2];
     }
     memset(pl->tmap, 0, sizeof(pl->tmap));
-    // pre-staged copies of the cell tables the Q and H lists gather from
-    if (d.qcells && hp->qptr && hp->qptr[ng])
-        rc |= dev_copy<float4>(pl, nullptr, (size_t)hp->ncells * 4, &pl->qstage);
-    if (d.hcells && hp->hptr && hp->hptr[ng])
-        rc |= dev_copy<float4>(pl, nullptr, (size_t)hp->ncells * 8, &pl->hstage);
-    if (!rc && (pl->qstage || pl->hstage)) {
-        k_stage_cells<<<(unsigned)((hp->ncells + 127) / 128), 128>>>(d.qcells, d.hcells, hp->ncells,
-                                                                       pl->qstage, pl->hstage);
-        const cudaError_t e = cudaDeviceSynchronize();
-        if (e != cudaSuccess) {
-            grav_plan_free(pl);
-            return gc::cuda_status(e, "grav_groups_upload_CUDA: staging the cell tables");
-        }
-        pl->staged = true;
-    }
-    d.cstage = pl->qstage ? pl->qstage : pl->hstage;
-    d.cstride = pl->qstage ? 4 : 8;
-    rc |= encode_rows(&pl->tmap[KP], d.points, (uint64_t)np, 16);
-    if (pl->qstage)
-        rc |= encode_rows(&pl->tmap[KQ], pl->qstage, (uint64_t)hp->ncells, sizeof(nln_qcell));
-    if (pl->hstage)
-        rc |= encode_rows(&pl->tmap[KH], pl->hstage, (uint64_t)hp->ncells, sizeof(nln_hcell));
+    const bool has_q = d.qcells && hp->qptr && hp->qptr[ng];
+    const bool has_h = d.hcells && hp->hptr && hp->hptr[ng];
+    d.ccen = has_q || has_h ? cell_centres(d, has_q, d.cstride) : nullptr;
+    if (has_q)
+        rc |= encode_cells<KQ>(&pl->tmap[KQ], d.qcells, hp->ncells);
+    if (has_h)
+        rc |= encode_cells<KH>(&pl->tmap[KH], d.hcells, hp->ncells);
     if (rc) {
         grav_plan_free(pl);
         return rc;
@@ -1766,32 +1742,25 @@ template <int KIND>
 int launch_kind(grav_plan *pl, const DevProblem &dp, cudaStream_t st) {
     if (dp.nitems[KIND] == 0)
         return 0;
-    const int wpb = pl->tune.warps_per_block;
-    if (KIND == KP) {
-        auto kp = pl->plain ? k_points<true> : k_points<false>;
-        int fit = 0;
-        GC_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kp, 256, 0));
-        int per_sm = pl->tune.blocks_per_sm > 0 ? std::min(pl->tune.blocks_per_sm, fit) : fit;
-        int blocks = std::max(1, per_sm) * pl->nsm;
-        blocks = std::min(blocks, (dp.nitems[KP] + 7) / 8);
-        kp<<<blocks, 256, 0, st>>>(dp);
-        GC_CHECK(cudaGetLastError());
-        pl->launches++;
-        return 0;
+    const int wpb = std::min(pl->tune.warps_per_block, kListWarps);
+    size_t smem;
+    const void *kern;
+    if constexpr (KIND == KP) {
+        smem = (size_t)wpb * kPointWarpBytes;
+        kern = pl->plain ? (const void *)k_points<true> : (const void *)k_points<false>;
+    } else {
+        smem = (size_t)wpb * CellKind<KIND>::warp_bytes;
+        kern = pl->plain ? (const void *)k_cells<KIND, true> : (const void *)k_cells<KIND, false>;
     }
-    constexpr bool paired = KIND == KH || (KIND == KQ && GRAV_Q2_PAIRED);
-    const size_t smem = (size_t)wpb * (pl->staged ? KindOf<KIND, paired>::warp_bytes
-                                                  : KindOf<KIND>::warp_bytes);
-    auto kern = pl->staged ? (pl->plain ? k_batch<KIND, true, true> : k_batch<KIND, true, false>)
-                           : (pl->plain ? k_batch<KIND, false, true> : k_batch<KIND, false, false>);
     GC_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int fit = 0;
     GC_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, wpb * 32, smem));
-    int per_sm = pl->tune.blocks_per_sm > 0 ? std::min(pl->tune.blocks_per_sm, fit) : fit;
-    int blocks = std::max(1, per_sm) * pl->nsm;
-    blocks = std::min(blocks, (dp.nitems[KIND] + wpb - 1) / wpb);
-    kern<<<blocks, wpb * 32, smem, st>>>(pl->tmap[KIND], dp);
-    GC_CHECK(cudaGetLastError());
+    const int per_sm = pl->tune.blocks_per_sm > 0 ? std::min(pl->tune.blocks_per_sm, fit) : fit;
+    const int blocks = std::min(std::max(1, per_sm) * pl->nsm, (dp.nitems[KIND] + wpb - 1) / wpb);
+    CUtensorMap tm = pl->tmap[KIND];
+    DevProblem d = dp;
+    void *pargs[] = {&d}, *cargs[] = {&tm, &d};
+    GC_CHECK(cudaLaunchKernel(kern, dim3(blocks), dim3(wpb * 32), KIND == KP ? pargs : cargs, smem, st));
     pl->launches++;
     return 0;
 }
@@ -1940,11 +1909,11 @@ extern "C" int grav_plan_retune_CUDA(grav_plan *pl, const grav_tuning *tuning) {
                             pl->lists_ptr[1].empty() ? 0 : pl->lists_ptr[1][ng],
                             pl->lists_ptr[2].empty() ? 0 : pl->lists_ptr[2][ng]};
     if (t.chunk_p <= 0)
-        t.chunk_p = auto_chunk(tot[0], ng, pl->nsm, 128);
+        t.chunk_p = auto_chunk(tot[0], ng, pl->nsm, KP);
     if (t.chunk_q <= 0)
-        t.chunk_q = auto_chunk(tot[1], ng, pl->nsm, 64);
+        t.chunk_q = auto_chunk(tot[1], ng, pl->nsm, KQ);
     if (t.chunk_h <= 0)
-        t.chunk_h = auto_chunk(tot[2], ng, pl->nsm, 32);
+        t.chunk_h = auto_chunk(tot[2], ng, pl->nsm, KH);
     t.ewald_n = pl->tune.ewald_n;  // the correction table is not rebuilt
     pl->tune = t;
     std::vector<Item> items[3];
@@ -2451,8 +2420,8 @@ size_t dev_scratch_bytes(int64_t ng, int nk) {
 }
 
 // Once per device, with that device current: the scratch's address, the
-// device's SM count and the shared-memory attribute of the two row-gather
-// kernels this entry launches (point lists run in k_points, which needs none).
+// device's SM count and the shared-memory attribute of the list kernels this
+// entry launches.
 int dev_scratch_base(void **out, int *nsm) {
     static std::mutex mu;
     static void *base[kMaxDevices] = {};
@@ -2475,10 +2444,12 @@ int dev_scratch_base(void **out, int *nsm) {
             return gc::cuda_status(e, "grav_groups_eval_dev_CUDA: SM count");
         if (n <= 0)
             return gc::set_status(-1, "grav_groups_eval_dev_CUDA: device %d reports no SMs", dev);
-        GC_CHECK(cudaFuncSetAttribute(k_batch<KQ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      8 * KindOf<KQ>::warp_bytes));
-        GC_CHECK(cudaFuncSetAttribute(k_batch<KH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      8 * KindOf<KH>::warp_bytes));
+        GC_CHECK(cudaFuncSetAttribute(k_points<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kListWarps * kPointWarpBytes));
+        GC_CHECK(cudaFuncSetAttribute(k_cells<KQ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kListWarps * CellKind<KQ>::warp_bytes));
+        GC_CHECK(cudaFuncSetAttribute(k_cells<KH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kListWarps * CellKind<KH>::warp_bytes));
         sms[dev] = n;
         base[dev] = p;
     }
@@ -2603,11 +2574,11 @@ extern "C" int grav_groups_eval_dev_CUDA(const grav_problem *dp, float *acc_phi,
     d.clist = nullptr;
     d.ewald = 0;
     memset(pl.tmap, 0, sizeof(pl.tmap));
-    int rc = encode_rows(&pl.tmap[KP], d.points, (uint64_t)np, 16);
-    if (!rc && d.qcells)
-        rc = encode_rows(&pl.tmap[KQ], d.qcells, (uint64_t)dp->ncells, sizeof(nln_qcell));
+    int rc = 0;
+    if (d.qcells)
+        rc = encode_cells<KQ>(&pl.tmap[KQ], d.qcells, dp->ncells);
     if (!rc && d.hcells)
-        rc = encode_rows(&pl.tmap[KH], d.hcells, (uint64_t)dp->ncells, sizeof(nln_hcell));
+        rc = encode_cells<KH>(&pl.tmap[KH], d.hcells, dp->ncells);
     if (rc)
         return rc;
 

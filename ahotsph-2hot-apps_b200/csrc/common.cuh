@@ -132,18 +132,3 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-
-// Knuth two-sum: s + e == a + b exactly.
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-    s = a + b;
-    float bp = s - a;
-    e = (a - (s - bp)) + (b - bp);
-}
-
-// Fold a tile partial sum t into the compensated accumulator (hi, lo).
-__device__ __forceinline__ void comp_add(float &hi, float &lo, float t) {
-    float s, e;
-    two_sum(hi, t, s, e);
-    hi = s;
-    lo += e;
-}

@@ -205,179 +205,157 @@ __device__ __forceinline__ void interact(const float *__restrict__ r, float sx, 
     a.az = fmaf(z, K, fmaf(-ri5, tz, a.az));
 }
 
-// Two point records against one sink with Blackwell's paired FP32
-// instructions (fma/add/mul .f32x2): the .x halves belong to one record,
-// the .y halves to the other.  The records are staged as negated offsets,
-// np = -(source - group centre), so d = s + np needs no negation; the
-// accumulators hold +m/r and +d m/r^3 (the caller negates once per tile).
-// Same Plummer arithmetic as mono<SOFT_PLUMMER>, element by element.
-struct Acc2 {
-    float2 nax, nay, naz, nphi;
-};
-
-__device__ __forceinline__ void mono2_plummer(float2 npx, float2 npy, float2 npz, float2 m,
-                                              float2 sx, float2 sy, float2 sz, float2 e2,
-                                              Acc2 &acc) {
-    const float2 dx = __fadd2_rn(sx, npx), dy = __fadd2_rn(sy, npy), dz = __fadd2_rn(sz, npz);
-    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-    const float2 ri = make_float2(rsqrt_fast(r2.x), rsqrt_fast(r2.y));
-    const float2 ri2 = __fmul2_rn(ri, ri);
-    const float2 mri = __fmul2_rn(m, ri);
-    const float2 mri3 = __fmul2_rn(mri, ri2);
-    acc.nphi = __fadd2_rn(acc.nphi, mri);
-    acc.nax = __ffma2_rn(dx, mri3, acc.nax);
-    acc.nay = __ffma2_rn(dy, mri3, acc.nay);
-    acc.naz = __ffma2_rn(dz, mri3, acc.naz);
-}
-
-// Two order-4 records against one sink with the paired FP32 instructions,
-// on a pair-interleaved tile: field f of records a (.x) and b (.y) sits at
-// floats 2f, 2f+1 of the pair.  Fields: 0-2 position (group-centred), 3
-// mass, 4-9 Q as in the staged record, 10 -(Xxxxx + Xxxyy), 11 -(Xyyyy +
-// Xxxyy) (h_z's xxz and yyz coefficients, the traceless moment's zz-pair
-// components folded in), 12-18 -O (the octupole negated), 19-20 the
-// octupole sums (not negated), 21-29 X, 30 -XS, 31 unused.  Working in v = source - sink = -d with those signs folded in
-// leaves no negation in the loop:
-//   e'(v) = -O:vv (so v.e' = d.e), h(v) = -h(d), U = Q.v + r^-2 (e' + r^-2 h),
-//   a   = v (m/r^3 - r^-2 (5/2 eq_2.d + 7/3 eq_3.d + 9/4 eq_4.d)) + r^-5 U,
-//   -phi = m/r - qsh eq_2.d - eq_3.d/3 - eq_4.d/4   (accumulated negated),
-// the terms of interact<4, SOFT_PLUMMER> in another order, element by element.
-struct Acc2h {
-    float2 ax, ay, az, nphi;
-};
-
-// The quadrupole counterpart on a pair-interleaved tile of 10 fields
-// (position, mass, Q as staged): with v = -d and U = Q.v,
-//   a = v (m/r^3 - 5/2 r^-2 eq_2.d) + r^-5 U,  -phi = m/r - qsh eq_2.d.
-__device__ __forceinline__ void quad2_plummer(const float *__restrict__ pr, float2 nsx, float2 nsy,
-                                              float2 nsz, float2 eps2, float2 nqsh, Acc2h &A);
-
+// ---------------------------------------------------------------- record pairs
+//
+// Two source records against one sink with Blackwell's paired FP32
+// instructions (fma/add/mul .f32x2): the .x halves belong to one record, the
+// .y halves to the other.  Both records stay in this lane's registers while
+// the warp walks its group's sinks, whose negated offsets come in as splat
+// pairs (nsx, nsx).  Everything works in v = source - sink = -d.
+//
+// What bounds them is the register file, not the FMA pipe: on a B200 a
+// paired FMA with three distinct operands takes three cycles a warp (two
+// with two; 49 of 74 TFLOP/s), a scalar one about 1.4.  So the forms below
+// count operand reads, not only operations.
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 splat2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 rsqrt2(float2 a) { return f2(rsqrt_fast(a.x), rsqrt_fast(a.y)); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-__device__ __forceinline__ void hexa2_plummer(const float *__restrict__ pr, float2 nsx, float2 nsy,
-                                              float2 nsz, float2 eps2, float2 nqsh, Acc2h &A) {
-    const float4 *q = reinterpret_cast<const float4 *>(pr);
-    float4 w = q[0];
-    const float2 vx = __fadd2_rn(f2(w.x, w.y), nsx);
-    const float2 vy = __fadd2_rn(f2(w.z, w.w), nsy);
-    w = q[1];
-    const float2 vz = __fadd2_rn(f2(w.x, w.y), nsz);
-    const float2 m = f2(w.z, w.w);
-    // monopole
-    const float2 r2 = __ffma2_rn(vx, vx, __ffma2_rn(vy, vy, __ffma2_rn(vz, vz, eps2)));
-    const float2 ri = f2(rsqrt_fast(r2.x), rsqrt_fast(r2.y));
-    const float2 ri2 = __fmul2_rn(ri, ri);
-    const float2 ri3 = __fmul2_rn(ri, ri2);  // shared by the monopole and the higher orders
-    const float2 mri3 = __fmul2_rn(m, ri3);
-    A.nphi = __ffma2_rn(m, ri, A.nphi);
-    // quadrupole
-    w = q[2];
-    const float2 Qxx = f2(w.x, w.y), Qxy = f2(w.z, w.w);
-    w = q[3];
-    const float2 Qyy = f2(w.x, w.y), Qxz = f2(w.z, w.w);
-    w = q[4];
-    const float2 Qyz = f2(w.x, w.y), Qzz = f2(w.z, w.w);
-    float2 Ux = __ffma2_rn(Qxx, vx, __ffma2_rn(Qxy, vy, __fmul2_rn(Qxz, vz)));
-    float2 Uy = __ffma2_rn(Qxy, vx, __ffma2_rn(Qyy, vy, __fmul2_rn(Qyz, vz)));
-    float2 Uz = __ffma2_rn(Qxz, vx, __ffma2_rn(Qyz, vy, __fmul2_rn(Qzz, vz)));
-    const float2 vQv = __ffma2_rn(vx, Ux, __ffma2_rn(vy, Uy, __fmul2_rn(vz, Uz)));
-    const float2 ri5 = __fmul2_rn(ri3, ri2);
-    const float2 eqd2 = __fmul2_rn(ri5, vQv);
-    // monomials of v (hexa_vec's, with -zz in place of zz)
-    const float2 third = splat2(1.0f / 3.0f);
-    float2 xx = __fmul2_rn(__fmul2_rn(splat2(0.5f), vx), vx);
-    float2 yy = __fmul2_rn(__fmul2_rn(splat2(0.5f), vy), vy);
-    const float2 nzz = __fmul2_rn(__fmul2_rn(splat2(-0.5f), vz), vz);
-    const float2 xy = __fmul2_rn(vx, vy), xz = __fmul2_rn(vx, vz), yz = __fmul2_rn(vy, vz);
-    const float2 xxx = __fmul2_rn(vx, __ffma2_rn(xx, third, nzz));
-    const float2 xxz = __fmul2_rn(vz, __ffma2_rn(nzz, third, xx));
-    const float2 yyy = __fmul2_rn(vy, __ffma2_rn(yy, third, nzz));
-    const float2 yyz = __fmul2_rn(vz, __ffma2_rn(nzz, third, yy));
-    xx = __fadd2_rn(xx, nzz);
-    yy = __fadd2_rn(yy, nzz);
-    // octupole (negated moments): e' and d3 = v.e'
-    w = q[6];
-    const float2 O0 = f2(w.x, w.y), O1 = f2(w.z, w.w);  // Oxxx Oxxy
-    w = q[7];
-    const float2 O2 = f2(w.x, w.y), O3 = f2(w.z, w.w);  // Oxyy Oyyy
-    w = q[8];
-    const float2 O4 = f2(w.x, w.y), O5 = f2(w.z, w.w);  // Oxxz Oxyz
-    w = q[9];
-    const float2 O6 = f2(w.x, w.y), S1 = f2(w.z, w.w);  // Oyyz, Oxxx+Oxyy
-    w = q[10];
-    const float2 S2 = f2(w.x, w.y), X0 = f2(w.z, w.w);  // Oxxy+Oyyy, Xxxxx
-    const float2 e0 = __ffma2_rn(O0, xx, __ffma2_rn(O2, yy, __ffma2_rn(O1, xy, __ffma2_rn(O4, xz, __fmul2_rn(O5, yz)))));
-    const float2 e1 = __ffma2_rn(O2, xy, __ffma2_rn(O1, xx, __ffma2_rn(O3, yy, __ffma2_rn(O6, yz, __fmul2_rn(O5, xz)))));
-    const float2 e2 = __ffma2_rn(S1, xz, __ffma2_rn(S2, yz, __ffma2_rn(O4, xx, __ffma2_rn(O6, yy, __fmul2_rn(O5, xy)))));
-    const float2 d3 = __ffma2_rn(vx, e0, __ffma2_rn(vy, e1, __fmul2_rn(vz, e2)));
-    // hexadecapole: h(v) and d4 = v.h
-    w = q[11];
-    const float2 X1 = f2(w.x, w.y), X2 = f2(w.z, w.w);  // Xxxxy Xxxyy
-    w = q[12];
-    const float2 X3 = f2(w.x, w.y), X4 = f2(w.z, w.w);  // Xxyyy Xyyyy
-    w = q[13];
-    const float2 X5 = f2(w.x, w.y), X6 = f2(w.z, w.w);  // Xxxxz Xxxyz
-    w = q[14];
-    const float2 X7 = f2(w.x, w.y), X8 = f2(w.z, w.w);  // Xxyyz Xyyyz
-    w = q[15];
-    const float2 nXS = f2(w.x, w.y);
-    w = q[5];
-    const float2 nX02 = f2(w.x, w.y), nX42 = f2(w.z, w.w);
-    const float2 xxy = __fmul2_rn(vy, xx), xyy = __fmul2_rn(vx, yy), xyz = __fmul2_rn(xy, vz);
-    // each chain starts from xyz, the monomial ready first (two operations
-    // from v; the others take four)
-    const float2 h0 = __ffma2_rn(X0, xxx, __ffma2_rn(X3, yyy, __ffma2_rn(X1, xxy, __ffma2_rn(X5, xxz,
-                      __ffma2_rn(X2, xyy, __ffma2_rn(X7, yyz, __fmul2_rn(X6, xyz)))))));
-    const float2 h1 = __ffma2_rn(X3, xyy, __ffma2_rn(X1, xxx, __ffma2_rn(X4, yyy, __ffma2_rn(X8, yyz,
-                      __ffma2_rn(X2, xxy, __ffma2_rn(X6, xxz, __fmul2_rn(X7, xyz)))))));
-    const float2 h2 = __ffma2_rn(nX02, xxz, __ffma2_rn(nX42, yyz, __ffma2_rn(X5, xxx, __ffma2_rn(X8, yyy,
-                      __ffma2_rn(X6, xxy, __ffma2_rn(X7, xyy, __fmul2_rn(nXS, xyz)))))));
-    const float2 d4 = __ffma2_rn(vx, h0, __ffma2_rn(vy, h1, __fmul2_rn(vz, h2)));
-    // sums of the orders
-    const float2 ri7 = __fmul2_rn(ri5, ri2), ri9 = __fmul2_rn(ri7, ri2);
-    const float2 eqd3 = __fmul2_rn(ri7, d3), eqd4 = __fmul2_rn(ri9, d4);
-    A.nphi = __ffma2_rn(splat2(-0.25f), eqd4,
-             __ffma2_rn(splat2(-1.0f / 3.0f), eqd3, __ffma2_rn(nqsh, eqd2, A.nphi)));
-    const float2 Kn = __ffma2_rn(ri2, __ffma2_rn(splat2(-2.25f), eqd4,
-                      __ffma2_rn(splat2(-7.0f / 3.0f), eqd3, __fmul2_rn(splat2(-2.5f), eqd2))), mri3);
-    Ux = __ffma2_rn(ri2, __ffma2_rn(ri2, h0, e0), Ux);
-    Uy = __ffma2_rn(ri2, __ffma2_rn(ri2, h1, e1), Uy);
-    Uz = __ffma2_rn(ri2, __ffma2_rn(ri2, h2, e2), Uz);
-    A.ax = __ffma2_rn(vx, Kn, __ffma2_rn(ri5, Ux, A.ax));
-    A.ay = __ffma2_rn(vy, Kn, __ffma2_rn(ri5, Uy, A.ay));
-    A.az = __ffma2_rn(vz, Kn, __ffma2_rn(ri5, Uz, A.az));
+// Fold t into the compensated accumulator (hi, lo), half by half: Knuth's
+// two-sum, s + e == hi + t exactly.
+__device__ __forceinline__ void comp_add2(float2 &hi, float2 &lo, float2 t) {
+    const float2 s = add2(hi, t), bp = add2(s, neg2(hi));
+    lo = add2(lo, add2(add2(hi, neg2(add2(s, neg2(bp)))), add2(t, neg2(bp))));
+    hi = s;
 }
 
-__device__ __forceinline__ void quad2_plummer(const float *__restrict__ pr, float2 nsx, float2 nsy,
-                                              float2 nsz, float2 eps2, float2 nqsh, Acc2h &A) {
-    const float4 *q = reinterpret_cast<const float4 *>(pr);
-    float4 w = q[0];
-    const float2 vx = __fadd2_rn(f2(w.x, w.y), nsx);
-    const float2 vy = __fadd2_rn(f2(w.z, w.w), nsy);
-    w = q[1];
-    const float2 vz = __fadd2_rn(f2(w.x, w.y), nsz);
-    const float2 m = f2(w.z, w.w);
-    const float2 r2 = __ffma2_rn(vx, vx, __ffma2_rn(vy, vy, __ffma2_rn(vz, vz, eps2)));
-    const float2 ri = f2(rsqrt_fast(r2.x), rsqrt_fast(r2.y));
-    const float2 ri2 = __fmul2_rn(ri, ri);
-    const float2 ri3 = __fmul2_rn(ri, ri2);  // shared by the monopole and quadrupole terms
-    const float2 mri3 = __fmul2_rn(m, ri3);
-    w = q[2];
-    const float2 Qxx = f2(w.x, w.y), Qxy = f2(w.z, w.w);
-    w = q[3];
-    const float2 Qyy = f2(w.x, w.y), Qxz = f2(w.z, w.w);
-    w = q[4];
-    const float2 Qyz = f2(w.x, w.y), Qzz = f2(w.z, w.w);
-    const float2 Ux = __ffma2_rn(Qxx, vx, __ffma2_rn(Qxy, vy, __fmul2_rn(Qxz, vz)));
-    const float2 Uy = __ffma2_rn(Qxy, vx, __ffma2_rn(Qyy, vy, __fmul2_rn(Qyz, vz)));
-    const float2 Uz = __ffma2_rn(Qxz, vx, __ffma2_rn(Qyz, vy, __fmul2_rn(Qzz, vz)));
-    const float2 vQv = __ffma2_rn(vx, Ux, __ffma2_rn(vy, Uy, __fmul2_rn(vz, Uz)));
-    const float2 ri5 = __fmul2_rn(ri3, ri2);
-    const float2 eqd2 = __fmul2_rn(ri5, vQv);
-    A.nphi = __ffma2_rn(nqsh, eqd2, __ffma2_rn(m, ri, A.nphi));
-    const float2 Kn = __ffma2_rn(__fmul2_rn(splat2(-2.5f), ri2), eqd2, mri3);
-    A.ax = __ffma2_rn(vx, Kn, __ffma2_rn(ri5, Ux, A.ax));
-    A.ay = __ffma2_rn(vy, Kn, __ffma2_rn(ri5, Uy, A.ay));
-    A.az = __ffma2_rn(vz, Kn, __ffma2_rn(ri5, Uz, A.az));
+// Running sums of one sink over this lane's records (nphi: -phi).
+struct Sum2 {
+    float2 ax, ay, az, nphi;
+    // (ax, ay, az, phi) of both halves together
+    __device__ __forceinline__ float4 total() const {
+        return make_float4(ax.x + ax.y, ay.x + ay.y, az.x + az.y, -(nphi.x + nphi.y));
+    }
+};
+
+struct MonoPair {
+    float2 x, y, z, m;
+};
+
+// Monopoles, the arithmetic of mono<SOFT_PLUMMER>; FIRST starts the sums.
+template <bool FIRST>
+__device__ __forceinline__ void mono_pair(const MonoPair &r, float2 nsx, float2 nsy, float2 nsz,
+                                          float2 e2, Sum2 &A) {
+    const float2 x = add2(r.x, nsx), y = add2(r.y, nsy), z = add2(r.z, nsz);
+    const float2 ri = rsqrt2(fma2(x, x, fma2(y, y, fma2(z, z, e2))));
+    const float2 mri = mul2(r.m, ri), mri3 = mul2(mri, mul2(ri, ri));
+    if (FIRST) {
+        A.nphi = mri;
+        A.ax = mul2(x, mri3);
+        A.ay = mul2(y, mri3);
+        A.az = mul2(z, mri3);
+    } else {
+        A.nphi = add2(A.nphi, mri);
+        A.ax = fma2(x, mri3, A.ax);
+        A.ay = fma2(y, mri3, A.ay);
+        A.az = fma2(z, mri3, A.az);
+    }
+}
+
+// Quadrupole cells: q = Qxx Qxy Qyy Qxz Qyz Qzz with Q = -3 R^2 q2.  With
+// U = Q.v:  a = v (m r^-3 - 5/2 r^-2 eq_2.d) + r^-5 U,  -phi = m/r - qsh eq_2.d.
+struct QuadPair {
+    float2 x, y, z, m, q[6];
+};
+
+template <bool FIRST>
+__device__ __forceinline__ void cell_pair(const QuadPair &r, float2 nsx, float2 nsy, float2 nsz,
+                                          float2 e2, float qsh, Sum2 &A) {
+    const float2 x = add2(r.x, nsx), y = add2(r.y, nsy), z = add2(r.z, nsz);
+    const float2 ri = rsqrt2(fma2(x, x, fma2(y, y, fma2(z, z, e2))));
+    const float2 ri2 = mul2(ri, ri), ri3 = mul2(ri, ri2), ri5 = mul2(ri3, ri2);
+    const float2 Ux = fma2(r.q[0], x, fma2(r.q[1], y, mul2(r.q[3], z)));
+    const float2 Uy = fma2(r.q[1], x, fma2(r.q[2], y, mul2(r.q[4], z)));
+    const float2 Uz = fma2(r.q[3], x, fma2(r.q[4], y, mul2(r.q[5], z)));
+    const float2 eqd = mul2(ri5, fma2(x, Ux, fma2(y, Uy, mul2(z, Uz))));
+    A.nphi = fma2(r.m, ri, FIRST ? mul2(splat2(-qsh), eqd) : fma2(splat2(-qsh), eqd, A.nphi));
+    const float2 K = fma2(mul2(splat2(-2.5f), ri2), eqd, mul2(r.m, ri3));
+    A.ax = fma2(x, K, FIRST ? mul2(ri5, Ux) : fma2(ri5, Ux, A.ax));
+    A.ay = fma2(y, K, FIRST ? mul2(ri5, Uy) : fma2(ri5, Uy, A.ay));
+    A.az = fma2(z, K, FIRST ? mul2(ri5, Uz) : fma2(ri5, Uz, A.az));
+}
+
+// Order-4 cells.  Staged per record: q = Q (xx xy yy xz yz), o = -O/2 (the
+// seven of stage_hexa) and the two sums (Oxxx+Oxyy)/2, (Oxxy+Oyyy)/2, h = X/6
+// (nine) and -(Xxxxx+Xxxyy)/6, -(Xyyyy+Xxxyy)/6, -(Xxxxy+Xxyyy)/6 (the xxzz,
+// yyzz and xyzz components).  With the harmonic second-degree monomials
+// s = (x^2 - z^2, y^2 - z^2, 2xy, 2xz, 2yz):
+//   e = o : s          v.e = d3     (octupole vector)
+//   M = h : s          M : s = d4   (hexadecapole as a traceless matrix)
+//   U = (Q + r^-4 M).v + r^-2 e,    v.U = T = d2 + r^-2 d3 + r^-4 d4
+// and with t = r^-2 (d3 + 3/2 r^-2 d4), P = T - t/3 (twice the multipole
+// potential over r^-5):
+//   -phi = m/r - r^-5 P / 2,   a = v (m r^-3 - r^-7 (4 T + P) / 2) + r^-5 U.
+// Contracting the hexadecapole to a matrix once folds its 3x3 product into
+// the quadrupole's: 105 operations against 111 for separate order-2, 3 and 4
+// vectors, 274 against 285 cycles a pair by the operand reads.
+struct HexaPair {
+    float2 x, y, z, m, q[5], o[9], h[12];
+};
+
+__device__ __forceinline__ float2 dot5(const float2 *c, const float2 *s) {
+    return fma2(c[0], s[0], fma2(c[1], s[1], fma2(c[2], s[2], fma2(c[3], s[3], mul2(c[4], s[4])))));
+}
+
+// PHYS: the physical potential (qsh = 1/2); otherwise the quadrupole's enters
+// with qsh, the other sign convention.
+template <bool PHYS>
+__device__ __forceinline__ void cell_pair(const HexaPair &r, float2 nsx, float2 nsy, float2 nsz,
+                                          float2 e2, float qsh, Sum2 &A) {
+    const float2 x = add2(r.x, nsx), y = add2(r.y, nsy), z = add2(r.z, nsz);
+    const float2 ri = rsqrt2(fma2(x, x, fma2(y, y, fma2(z, z, e2))));
+    const float2 nzz = neg2(mul2(z, z)), x2 = add2(x, x), y2 = add2(y, y);
+    const float2 s[5] = {fma2(x, x, nzz), fma2(y, y, nzz), mul2(x2, y), mul2(x2, z), mul2(y2, z)};
+    // o: xxx xxy xyy yyy xxz xyz yyz, sums; h: xxxx xxxy xxyy xyyy yyyy xxxz xxyz xyyz yyyz,
+    // xxzz yyzz xyzz
+    const float2 *o = r.o, *h = r.h;
+    const float2 c0[5] = {o[0], o[2], o[1], o[4], o[5]}, c1[5] = {o[1], o[3], o[2], o[5], o[6]},
+                 c2[5] = {o[4], o[6], o[5], o[7], o[8]};
+    const float2 ex = dot5(c0, s), ey = dot5(c1, s), ez = dot5(c2, s);
+    const float2 mxx[5] = {h[0], h[2], h[1], h[5], h[6]}, mxy[5] = {h[1], h[3], h[2], h[6], h[7]},
+                 myy[5] = {h[2], h[4], h[3], h[7], h[8]}, mxz[5] = {h[5], h[7], h[6], h[9], h[11]},
+                 myz[5] = {h[6], h[8], h[7], h[11], h[10]};
+    const float2 M[5] = {dot5(mxx, s), dot5(myy, s), dot5(mxy, s), dot5(mxz, s), dot5(myz, s)};
+    const float2 ri2 = mul2(ri, ri), ri4 = mul2(ri2, ri2), ri5 = mul2(ri4, ri);
+    const float2 mri = mul2(r.m, ri);
+    const float2 d3 = fma2(x, ex, fma2(y, ey, mul2(z, ez)));
+    const float2 d4 = dot5(M, s);
+    const float2 qxx = fma2(ri4, M[0], r.q[0]), qyy = fma2(ri4, M[1], r.q[2]),
+                 qxy = fma2(ri4, M[2], r.q[1]), qxz = fma2(ri4, M[3], r.q[3]),
+                 qyz = fma2(ri4, M[4], r.q[4]);
+    float2 Ux = fma2(qxx, x, fma2(qxy, y, mul2(qxz, z)));
+    float2 Uy = fma2(qxy, x, fma2(qyy, y, mul2(qyz, z)));
+    float2 Uz = fma2(qxz, x, fma2(qyz, y, mul2(neg2(add2(qxx, qyy)), z)));
+    Ux = fma2(ri2, ex, Ux);
+    Uy = fma2(ri2, ey, Uy);
+    Uz = fma2(ri2, ez, Uz);
+    const float2 T = fma2(x, Ux, fma2(y, Uy, mul2(z, Uz)));
+    const float2 q1 = mul2(ri2, d4);
+    const float2 t = mul2(ri2, fma2(splat2(1.5f), q1, d3));
+    float2 P = fma2(splat2(-1.f / 3.f), t, T);
+    const float2 c = fma2(splat2(4.f), T, P);
+    if (!PHYS) {
+        const float2 d2 = fma2(neg2(ri2), add2(d3, q1), T);
+        P = fma2(splat2(2.f * qsh - 1.f), d2, P);
+    }
+    const float2 nri5h = mul2(splat2(-0.5f), ri5);
+    A.nphi = fma2(nri5h, P, mri);
+    const float2 K = fma2(mul2(nri5h, c), ri2, mul2(mri, ri2));
+    A.ax = fma2(x, K, mul2(ri5, Ux));
+    A.ay = fma2(y, K, mul2(ri5, Uy));
+    A.az = fma2(z, K, mul2(ri5, Uz));
 }
