@@ -102,6 +102,9 @@ struct DevProblem {
     float ew_self;             // C(0) - pi/(alpha^2 L^3): the self term ewald() leaves out
     float ew_trace;            // trace of the Hessian of C: -4 pi / L^3
     EwStored *ewm;             // per-group moments from k_ewald_moments
+    EwStored *ewpart;          // its units' moments where a group's list is split (ewsplit > 1)
+    int *ewdone;               // finished units per group, zero between evaluations
+    int ewsplit;               // units per group
     // FP64 centres of the cells for the point table's monopole records (the
     // mixed form re-centres them like every other source): a cell table (the
     // centre is a record's first 24 bytes, one record every cstride bytes),
@@ -723,34 +726,154 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
 }
 
 // Periodic correction moments (ewald.cuh) of groups gbegin..ngroups-1, one
-// warp per group from a queue (counter 3), lanes striding the group's
-// correction list, stored per group for k_finish.  Bodies count as masses; a
-// cell adds its traceless second to fourth moments (the list's cells
+// warp per unit from a queue (counter 3), lanes striding the unit's part of
+// its group's correction list; a group has ewsplit units.  Bodies count as
+// masses; a cell adds its traceless second to fourth moments (the list's cells
 // include coarse ones standing for whole subtrees, and cells a tenth of the
 // box wide near the half-box, where C varies on the scale of the cell), and
 // its second-moment trace B2/3 against the constant Laplacian of C.
-//
-// The loads are what bound this loop: each entry needs its table node
-// (224 B) and its cell record (128 B) from scattered addresses, and the node
-// depends on the record's centre.  So every lane runs a three-deep pipeline
-// of its own entries: list word three tiles ahead, the source's FP64 centre
-// (a plain load) two tiles ahead, and one tile ahead a per-lane cp.async of
-// the node and the record into this warp's shared-memory stage, laid out
-// chunk-major ([chunk][lane] float4) so that the compute's reads are
-// conflict-free.  Each lane reads only what it copied itself.
-constexpr int kEwNodeChunks = 14;  // 56 floats: C and its derivatives of orders 0..5
-constexpr int kEwRecChunks = 7;    // floats 4..31 of an order-4 cell record (nln_hcell); the
-                                   // centre in floats 0..5 comes with the pipeline's registers
-struct EwStage {
-    float4 node[kEwNodeChunks][32];
-    float4 rec[kEwRecChunks][32];
-};
-constexpr int kEwWarpBytes = 2 * (int)sizeof(EwStage);  // two stages per warp: 21,504 B
 
-__global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
-    extern __shared__ __align__(16) unsigned char ewsm[];
-    const int lane = threadIdx.x & 31;
-    EwStage *stg = reinterpret_cast<EwStage *>(ewsm + (size_t)(threadIdx.x >> 5) * kEwWarpBytes);
+// Unit u of the moments' queue: group and tile range [t0, t1) of its list.
+struct EwUnit {
+    int64_t g, cb, ce;
+    int t0, t1;
+};
+
+__device__ __forceinline__ EwUnit ew_unit(const DevProblem &P, int64_t u) {
+    EwUnit r;
+    const int part = (int)(u % P.ewsplit);
+    r.g = P.gbegin + u / P.ewsplit;
+    if (r.g >= P.ngroups)
+        return r;
+    r.cb = P.cptr[r.g];
+    r.ce = P.cptr[r.g + 1];
+    const int64_t nt = (r.ce - r.cb + 31) / 32;
+    r.t0 = (int)(nt * part / P.ewsplit);
+    r.t1 = (int)(nt * (part + 1) / P.ewsplit);
+    return r;
+}
+
+// Store a unit's moments (already summed over the warp) as its group's, or,
+// where the list is split, as a part: the warp that finishes the group's
+// last unit adds the parts in order.
+__device__ __forceinline__ void ew_store(const DevProblem &P, int64_t u, int64_t g, int lane,
+                                         const EwMoments &M) {
+    EwStored *E = P.ewsplit > 1 ? P.ewpart + (g * P.ewsplit + u % P.ewsplit) : P.ewm + g;
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 10; q++) E->lo[q] = M.lo[q];
+#pragma unroll
+        for (int q = 0; q < 25; q++) E->hi[q] = M.hi[q];
+    }
+    if (P.ewsplit == 1)
+        return;
+    __threadfence();
+    int before = 0;
+    if (lane == 0)
+        before = atomicAdd(&P.ewdone[g], 1);
+    if (__shfl_sync(0xffffffffu, before, 0) != P.ewsplit - 1)
+        return;
+    __threadfence();
+    const EwStored *S = P.ewpart + g * P.ewsplit;
+    EwStored &D = P.ewm[g];
+    if (lane < 10) {
+        double v = __ldcg(&S[0].lo[lane]);
+        for (int k = 1; k < P.ewsplit; k++) v += __ldcg(&S[k].lo[lane]);
+        D.lo[lane] = v;
+    }
+    if (lane < 25) {
+        float v = __ldcg(&S[0].hi[lane]);
+        for (int k = 1; k < P.ewsplit; k++) v += __ldcg(&S[k].hi[lane]);
+        D.hi[lane] = v;
+    }
+    if (lane == 0)
+        P.ewdone[g] = 0;
+}
+
+// One entry's terms from its node values V (56 floats) and, for a cell, its
+// record r (nln_hcell as floats: mass 6, R 7, q2 8..12, q3 13..19, q4 20..28,
+// B2 29); m: a body's mass.
+template <class Node, class Record>
+__device__ __forceinline__ void ew_entry(EwMoments &M, const DevProblem &P, const EwNode &N,
+                                         bool cell, float m, Node node, Record record) {
+    // orders 0..4 (35 values) for the expansion; order 5 is read after it, so
+    // the two are never in registers together
+    float V[36];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const float4 v = node(k);
+        V[4 * k] = v.x;
+        V[4 * k + 1] = v.y;
+        V[4 * k + 2] = v.z;
+        V[4 * k + 3] = v.w;
+    }
+    float o[ew::kNQ4], f5[21];
+    ew_expand<false>(V, N, o, nullptr);
+    if (!cell) {
+        ew_add_mass(M, m, o);
+    } else {
+        float V5[24];  // node floats 32..55; order 5 starts at 35
+#pragma unroll
+        for (int k = 8; k < 14; k++) {
+            const float4 v = node(k);
+            V5[4 * (k - 8)] = v.x;
+            V5[4 * (k - 8) + 1] = v.y;
+            V5[4 * (k - 8) + 2] = v.z;
+            V5[4 * (k - 8) + 3] = v.w;
+        }
+        ew_fifth(V5 + 3, N, f5);
+        float r[32];
+#pragma unroll
+        for (int k = 1; k < 8; k++) {
+            const float4 v = record(k);
+            r[4 * k] = v.x;
+            r[4 * k + 1] = v.y;
+            r[4 * k + 2] = v.z;
+            r[4 * k + 3] = v.w;
+        }
+        const float R = r[7];
+        ew_add_mass(M, r[6], o);
+        float S[15];
+        ew_quad(R, r + 8, S);
+        ew_fold<2, 3>(M, S, o, f5);
+        ew_oct(R, r + 13, S);
+        ew_fold<3, 2>(M, S, o, f5);
+        ew_hex(R, r + 20, S);
+        ew_fold<4, 1>(M, S, o, f5);
+        M.at(0) = fmaf(__fmul_rn(r[29], 1.f / 6.f), P.ew_trace, M.at(0));
+    }
+    M.end_entry();
+}
+
+// Every entry needs its table node (224 B) and its cell record (128 B) from
+// scattered addresses, and the node depends on the record's centre: list word
+// three tiles ahead, the source's FP64 centre (plain loads) two tiles ahead,
+// and one tile ahead the tile's 32 nodes and records by TMA row gathers, four
+// rows an instruction, into one of two stages of the warp.  Copying the rows
+// by per-lane cp.async instead touched 32 cache lines with every one of its
+// 21 instructions and held the kernel to the L1's rate (160^3 box: 30.7 ms with the finish pass, now
+// 24.7).
+constexpr int kEwNodeBytes = 32 * 4 * ew::kNode;             // 7,168
+constexpr int kEwRecBytes = 32 * (int)sizeof(nln_hcell);     // 4,096, swizzled
+constexpr int kEwWarpBytes = 2 * (kEwNodeBytes + kEwRecBytes) + 16;
+
+__global__ void __launch_bounds__(128)
+    k_ewald_moments(const __grid_constant__ CUtensorMap tnode,
+                    const __grid_constant__ CUtensorMap trec, DevProblem P) {
+    extern __shared__ __align__(1024) unsigned char ewsm[];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    // the block's record stages first (their swizzle repeats every 1024
+    // bytes), then the node stages, then the mbarriers
+    unsigned char *recs = ewsm + (size_t)wib * 2 * kEwRecBytes;
+    unsigned char *nodes = ewsm + (size_t)nw * 2 * kEwRecBytes + (size_t)wib * 2 * kEwNodeBytes;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(ewsm + (size_t)nw * 2 * (kEwRecBytes + kEwNodeBytes)) +
+                    2 * wib;
+    if (lane == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_mbar_init();
+    }
+    __syncwarp();
     const uint32_t ntab = (uint32_t)P.ntab[0];
     const uint32_t nb = ntab - (uint32_t)P.ncells;
     constexpr uint32_t kNone = 0xffffffffu;
@@ -761,29 +884,29 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
         double x, y, z;
         float m;
     };
+    uint32_t seq = 0;  // tiles started by this warp: stage seq & 1, parity seq >> 1 & 1
     for (;;) {
         int it = 0;
         if (lane == 0)
             it = atomicAdd(&P.counters[3], 1);
         it = __shfl_sync(0xffffffffu, it, 0);
-        const int64_t g = P.gbegin + it;
-        if (g >= P.ngroups)
+        const EwUnit U = ew_unit(P, it);
+        if (U.g >= P.ngroups)
             break;
-        const nln_group G = P.groups[g];
+        const nln_group G = P.groups[U.g];
         const double c[3] = {G.cen[0], G.cen[1], G.cen[2]};
-        const int64_t cb = P.cptr[g], ce = P.cptr[g + 1];
-        const int ntile = (int)((ce - cb + 31) / 32);
+        const int ntile = U.t1 - U.t0;
         // the list word is checked where it is used, a tile after its load
         auto entry = [&](int t) -> uint32_t {
-            const int64_t k = cb + (int64_t)t * 32 + lane;
-            return (t < ntile && k < ce) ? __ldg(P.clist + k) : kNone;
+            const int64_t k = U.cb + (int64_t)(U.t0 + t) * 32 + lane;
+            return (t < ntile && k < U.ce) ? __ldg(P.clist + k) : kNone;
         };
         auto source = [&](uint32_t e) -> Src {
             Src r{kNone, 0.0, 0.0, 0.0, 0.f};
             if (e == kNone)
                 return r;
             const uint32_t idx = e & NLN_IDX_MASK;
-            if (idx >= ntab || (e >> NLN_IDX_BITS) > 26u) {  // as in k_batch
+            if (idx >= ntab || (e >> NLN_IDX_BITS) > 26u) {  // as in the list kernels
                 atomicOr(P.err, GC_DEV_BAD_INDEX);
                 return r;
             }
@@ -796,8 +919,9 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
                 r.m = p.w;
             } else {
                 const double *cen = P.hcells[idx - nb].cen;
-                r.x = __ldg(cen);
-                r.y = __ldg(cen + 1);
+                const double2 a = __ldg(reinterpret_cast<const double2 *>(cen));
+                r.x = a.x;
+                r.y = a.y;
                 r.z = __ldg(cen + 2);
             }
             return r;
@@ -808,174 +932,136 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
             return ew_node(P.ew, (float)(q.x + sx - c[0]), (float)(q.y + sy - c[1]),
                            (float)(q.z + sz - c[2]));
         };
-        auto issue = [&](const Src &q, EwStage &S) {
-            if (q.e == kNone)
-                return;
-            const uint32_t idx = q.e & NLN_IDX_MASK;
-            const float4 *node =
-                reinterpret_cast<const float4 *>(P.ew.t + (size_t)node_of(q).node * ew::kNode);
+        // Start the copies of a tile (sequence number s): lane 0 gathers the
+        // row numbers; lanes without an entry repeat row 0.
+        auto issue = [&](const Src &q, uint32_t s) {
+            const bool live = q.e != kNone;
+            const bool cell = live && (q.e & NLN_IDX_MASK) >= nb;
+            const int node = live ? node_of(q).node : 0;
+            const int rec = cell ? (int)((q.e & NLN_IDX_MASK) - nb) : 0;
+            const unsigned any = __ballot_sync(0xffffffffu, live);
+            const unsigned cells = __ballot_sync(0xffffffffu, cell);
+            uint64_t *b = &bar[s & 1];
+            unsigned char *dn = nodes + (s & 1) * kEwNodeBytes, *dr = recs + (s & 1) * kEwRecBytes;
+            if (lane == 0) {
+                uint32_t bytes = 0;
+                for (int g = 0; g < 8; g++) {
+                    bytes += any >> (4 * g) & 15u ? 16u * ew::kNode : 0u;
+                    bytes += cells >> (4 * g) & 15u ? 4u * (uint32_t)sizeof(nln_hcell) : 0u;
+                }
+                mbar_arrive_expect_tx(b, bytes);
+            }
 #pragma unroll
-            for (int k = 0; k < kEwNodeChunks; k++) cp_async16(&S.node[k][lane], node + k);
-            if (idx >= nb) {
-                const float4 *rec = reinterpret_cast<const float4 *>(P.hcells + (idx - nb)) + 1;
+            for (int g = 0; g < 8; g++) {
+                int rn[4], rr[4];
 #pragma unroll
-                for (int k = 0; k < kEwRecChunks; k++) cp_async16(&S.rec[k][lane], rec + k);
+                for (int j = 0; j < 4; j++) {
+                    rn[j] = __shfl_sync(0xffffffffu, node, 4 * g + j);
+                    rr[j] = __shfl_sync(0xffffffffu, rec, 4 * g + j);
+                }
+                if (lane == 0) {
+                    if (any >> (4 * g) & 15u)
+                        tma_gather4(dn + g * 16 * ew::kNode, &tnode, rn[0], rn[1], rn[2], rn[3], b);
+                    if (cells >> (4 * g) & 15u)
+                        tma_gather4(dr + g * 4 * (int)sizeof(nln_hcell), &trec, rr[0], rr[1], rr[2],
+                                    rr[3], b);
+                }
             }
         };
         EwMoments M;
         M.zero();
         Src s0 = source(entry(0));
-        issue(s0, stg[0]);
-        cp_async_commit();
+        if (ntile > 0)
+            issue(s0, seq);
         Src s1 = source(entry(1));
         uint32_t e2 = entry(2);
         for (int t = 0; t < ntile; t++) {
+            __syncwarp();  // the other stage is no longer read
             if (t + 1 < ntile)
-                issue(s1, stg[(t + 1) & 1]);
-            cp_async_commit();
+                issue(s1, seq + t + 1);
             const Src s2 = source(e2);  // consumed by the next tile's issue
             e2 = entry(t + 3);
-            cp_async_wait<1>();  // this lane's copies for tile t have landed
+            const uint32_t s = seq + t;
+            const bool ok = mbar_wait_bounded(&bar[s & 1], s >> 1 & 1, P.err);
+            if (!__all_sync(0xffffffffu, ok)) {
+                // give the copies still in flight a bounded chance to land
+                if (t + 1 < ntile)
+                    mbar_wait_bounded(&bar[(s + 1) & 1], (s + 1) >> 1 & 1, P.err, 1u << 10);
+                return;
+            }
             if (s0.e != kNone) {
-                const EwStage &S = stg[t & 1];
-                const EwNode N = node_of(s0);
-                // orders 0..4 (35 values) for the expansion; order 5 is read
-                // after it, so the two are never in registers together
-                float V[36];
-#pragma unroll
-                for (int k = 0; k < 9; k++) {
-                    const float4 v = S.node[k][lane];
-                    V[4 * k] = v.x;
-                    V[4 * k + 1] = v.y;
-                    V[4 * k + 2] = v.z;
-                    V[4 * k + 3] = v.w;
-                }
-                float o[ew::kNQ4], f5[21];
-                ew_expand<false>(V, N, o, nullptr);
-                if ((s0.e & NLN_IDX_MASK) < nb) {
-                    ew_add_mass(M, s0.m, o);
-                } else {
-                    float V5[24];  // node floats 32..55; order 5 starts at 35
-#pragma unroll
-                    for (int k = 8; k < kEwNodeChunks; k++) {
-                        const float4 v = S.node[k][lane];
-                        V5[4 * (k - 8)] = v.x;
-                        V5[4 * (k - 8) + 1] = v.y;
-                        V5[4 * (k - 8) + 2] = v.z;
-                        V5[4 * (k - 8) + 3] = v.w;
-                    }
-                    ew_fifth(V5 + 3, N, f5);
-                    float r[32];
-#pragma unroll
-                    for (int k = 0; k < kEwRecChunks; k++) {
-                        const float4 v = S.rec[k][lane];
-                        r[4 * (k + 1)] = v.x;
-                        r[4 * (k + 1) + 1] = v.y;
-                        r[4 * (k + 1) + 2] = v.z;
-                        r[4 * (k + 1) + 3] = v.w;
-                    }
-                    // nln_hcell floats: mass 6, R 7, q2 8..12, q3 13..19, q4 20..28, B2 29
-                    const float R = r[7];
-                    ew_add_mass(M, r[6], o);
-                    float Sm[15];
-                    ew_quad(R, r + 8, Sm);
-                    ew_fold<2, 3>(M, Sm, o, f5);
-                    ew_oct(R, r + 13, Sm);
-                    ew_fold<3, 2>(M, Sm, o, f5);
-                    ew_hex(R, r + 20, Sm);
-                    ew_fold<4, 1>(M, Sm, o, f5);
-                    M.add(0, __fmul_rn(__fmul_rn(r[29], 1.f / 6.f), P.ew_trace));
-                }
-                M.end_entry();
+                const float4 *node =
+                    reinterpret_cast<const float4 *>(nodes + (s & 1) * kEwNodeBytes + lane * 4 * ew::kNode);
+                const unsigned char *rec = recs + (s & 1) * kEwRecBytes;
+                ew_entry(M, P, node_of(s0), (s0.e & NLN_IDX_MASK) >= nb, s0.m,
+                         [&](int k) { return node[k]; },
+                         [&](int k) {
+                             return *reinterpret_cast<const float4 *>(rec + CellKind<KH>::chunk(lane, k));
+                         });
             }
             s0 = s1;
             s1 = s2;
         }
-        cp_async_wait<0>();
+        seq += ntile;
         M.warp_sum();
-        if (lane == 0) {
-            EwStored &E = P.ewm[g];
-#pragma unroll
-            for (int q = 0; q < 10; q++) E.lo[q] = M.lo[q];
-#pragma unroll
-            for (int q = 0; q < 25; q++) E.hi[q] = M.hi[q];
-        }
+        ew_store(P, it, U.g, lane, M);
     }
 }
 
-// The same correction moments of group g by a plain loop over the list,
-// lanes striding it, every load on demand: no shared memory and fewer
-// registers than k_ewald_moments, which suits a kernel that shares the SMs
-// with the list kernels (the side stream).  The arithmetic and its order are
-// k_ewald_moments', so the two store identical moments.  Bodies count as masses; a cell adds its
-// traceless second to fourth moments (the list's cells include coarse
-// ones standing for whole subtrees, and cells a tenth of the box wide near
-// the half-box, where C varies on the scale of the cell), and its
-// second-moment trace B2/3 against the constant Laplacian of C.
-__device__ __forceinline__ void ewald_moments_loop(const DevProblem &P, int64_t g, const double *c,
-                                              int lane, EwMoments &M) {
-    M.zero();
-    float o[ew::kNQ4], f5[21];
-    const uint32_t nb = (uint32_t)P.ntab[0] - (uint32_t)P.ncells;
-    for (int64_t k = P.cptr[g] + lane; k < P.cptr[g + 1]; k += 32) {
-        const uint32_t ent = P.clist[k];
-        const uint32_t idx = ent & NLN_IDX_MASK;
-        if (idx >= (uint32_t)P.ntab[0] || (ent >> NLN_IDX_BITS) > 26u) {  // as in k_batch
-            atomicOr(P.err, GC_DEV_BAD_INDEX);
-            continue;
-        }
-        double sx, sy, sz;
-        decode_shift(ent >> NLN_IDX_BITS, P.box, sx, sy, sz);
-        if (idx < nb) {
-            const float4 p = P.points[idx];
-            ew_lookup<false>(P.ew, (float)((double)p.x + sx - c[0]),
-                             (float)((double)p.y + sy - c[1]), (float)((double)p.z + sz - c[2]),
-                             o, nullptr);
-            ew_add_mass(M, p.w, o);
-        } else {
-            const nln_hcell &h = P.hcells[idx - nb];
-            ew_lookup<true>(P.ew, (float)(h.cen[0] + sx - c[0]), (float)(h.cen[1] + sy - c[1]),
-                            (float)(h.cen[2] + sz - c[2]), o, f5);
-            ew_add_mass(M, h.mass, o);
-            float S[15];
-            ew_quad(h.R, h.q2, S);
-            ew_fold<2, 3>(M, S, o, f5);
-            ew_oct(h.R, h.q3, S);
-            ew_fold<3, 2>(M, S, o, f5);
-            ew_hex(h.R, h.q4, S);
-            ew_fold<4, 1>(M, S, o, f5);
-            M.add(0, __fmul_rn(__fmul_rn(h.B2, 1.f / 6.f), P.ew_trace));
-        }
-        M.end_entry();
-    }
-    M.warp_sum();
-}
-
-// The correction moments of groups gbegin..ngroups-1 by ewald_moments_loop,
-// stored per group for k_finish: one warp per group from a queue (counter
-// 3), run on a side stream beside the list kernels, which it does not
-// depend on.
+// The same moments by a plain loop over the list, every load on demand: no
+// shared memory, which suits a kernel that shares the SMs with the list
+// kernels (the side stream).  The arithmetic and its order are
+// k_ewald_moments', so the two store identical moments.
 __global__ void __launch_bounds__(64) k_ewald_side(DevProblem P) {
     const int lane = threadIdx.x & 31;
+    const uint32_t ntab = (uint32_t)P.ntab[0];
+    const uint32_t nb = ntab - (uint32_t)P.ncells;
     for (;;) {
         int it = 0;
         if (lane == 0)
             it = atomicAdd(&P.counters[3], 1);
         it = __shfl_sync(0xffffffffu, it, 0);
-        const int64_t g = P.gbegin + it;
-        if (g >= P.ngroups)
+        const EwUnit U = ew_unit(P, it);
+        if (U.g >= P.ngroups)
             break;
-        const nln_group G = P.groups[g];
-        const double c[3] = {G.cen[0], G.cen[1], G.cen[2]};
+        const nln_group G = P.groups[U.g];
         EwMoments M;
-        ewald_moments_loop(P, g, c, lane, M);
-        if (lane == 0) {
-            EwStored &E = P.ewm[g];
-#pragma unroll
-            for (int q = 0; q < 10; q++) E.lo[q] = M.lo[q];
-#pragma unroll
-            for (int q = 0; q < 25; q++) E.hi[q] = M.hi[q];
+        M.zero();
+        const int64_t end = min(U.ce, U.cb + (int64_t)U.t1 * 32);
+        for (int64_t k = U.cb + (int64_t)U.t0 * 32 + lane; k < end; k += 32) {
+            const uint32_t ent = P.clist[k];
+            const uint32_t idx = ent & NLN_IDX_MASK;
+            if (idx >= ntab || (ent >> NLN_IDX_BITS) > 26u) {  // as in the list kernels
+                atomicOr(P.err, GC_DEV_BAD_INDEX);
+                continue;
+            }
+            const bool cell = idx >= nb;
+            double x, y, z;
+            float m = 0.f;
+            const float4 *rec = nullptr;
+            if (cell) {
+                const nln_hcell &h = P.hcells[idx - nb];
+                x = h.cen[0];
+                y = h.cen[1];
+                z = h.cen[2];
+                rec = reinterpret_cast<const float4 *>(&h);
+            } else {
+                const float4 p = P.points[idx];
+                x = p.x;
+                y = p.y;
+                z = p.z;
+                m = p.w;
+            }
+            double sx, sy, sz;
+            decode_shift(ent >> NLN_IDX_BITS, P.box, sx, sy, sz);
+            const EwNode N = ew_node(P.ew, (float)(x + sx - G.cen[0]), (float)(y + sy - G.cen[1]),
+                                     (float)(z + sz - G.cen[2]));
+            const float4 *node = reinterpret_cast<const float4 *>(P.ew.t + (size_t)N.node * ew::kNode);
+            ew_entry(M, P, N, cell, m, [&](int q) { return __ldg(node + q); },
+                     [&](int q) { return __ldg(rec + q); });
         }
+        M.warp_sum();
+        ew_store(P, it, U.g, lane, M);
     }
 }
 
@@ -1037,7 +1123,8 @@ struct grav_plan {
     int nsm = 148;
     int launches = 0;
     int64_t nslots = 0;
-    CUtensorMap tmap[3];    // row-gather views of the quadrupole and order-4 tables
+    CUtensorMap tmap[4];    // row-gather views: 1, 2 the quadrupole and order-4 tables, 3 the
+                            // Ewald table
     int timing = 0;         // record events around each kernel of an evaluation
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     std::vector<int64_t> lists_ptr[4];  // host copies of the P, Q, H (queue rebuilds) and
@@ -1070,11 +1157,10 @@ struct grav_plan {
 
 namespace {
 
-// A 2-D tensor map over the records of a cell table, box = one full record
-// (one row high, as the row gather requires), swizzled over the record's
-// width (CellKind::chunk).
-template <int KIND>
-int encode_cells(CUtensorMap *m, const void *base, int64_t rows) {
+// A 2-D tensor map over `rows` records of `bytes` (a multiple of 16), box =
+// one full record (one row high, as the row gather requires).
+int encode_rows(CUtensorMap *m, const void *base, int64_t rows, uint32_t bytes,
+                CUtensorMapSwizzle swizzle) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
         void *fn = nullptr;
@@ -1084,19 +1170,26 @@ int encode_cells(CUtensorMap *m, const void *base, int64_t rows) {
             return gc::set_status(-1, "cuTensorMapEncodeTiled unavailable");
         encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
-    constexpr uint32_t bytes = CellKind<KIND>::rec_bytes, w = bytes / 4;
+    const uint32_t w = bytes / 4;
     cuuint64_t dims[2] = {w, (cuuint64_t)rows};
     cuuint64_t strides[1] = {bytes};
     cuuint32_t box[2] = {w, 1};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(base), dims,
-                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        KIND == KH ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return gc::set_status(-1, "cuTensorMapEncodeTiled failed (%d) for %lld rows of %u bytes",
                               (int)r, (long long)rows, bytes);
     return 0;
+}
+
+// The row-gather view of a cell table, swizzled over the record's width
+// (CellKind::chunk).
+template <int KIND>
+int encode_cells(CUtensorMap *m, const void *base, int64_t rows) {
+    return encode_rows(m, base, rows, CellKind<KIND>::rec_bytes,
+                       KIND == KH ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 // The table k_points reads FP64 cell centres from, and its record size.
@@ -1632,6 +1725,18 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
         d.ewald = 1;
         rc |= dev_copy<EwStored>(pl, nullptr, (size_t)ng, &pl->ewm);
         pl->ewald_entries = hp->cptr[ng];
+        // Lists are split until there are ~4 units per resident warp (10 per
+        // SM), but not below 8 tiles a unit: a 16^3 box has 156 groups for
+        // 1,480 warps (moments 0.16 -> 0.07 ms), a 64^3 box enough as it is.
+        const int64_t tiles = hp->cptr[ng] / (32 * ng);
+        d.ewsplit = (int)std::max<int64_t>(1, std::min<int64_t>((40 * (int64_t)pl->nsm + ng - 1) / ng,
+                                                                tiles / 8));
+        if (d.ewsplit > 1) {
+            rc |= dev_copy<EwStored>(pl, nullptr, (size_t)(ng * d.ewsplit), &d.ewpart);
+            rc |= dev_copy<int>(pl, nullptr, (size_t)ng, &d.ewdone);
+            if (d.ewdone)
+                cudaMemset(d.ewdone, 0, (size_t)ng * sizeof(int));
+        }
         cudaError_t e = cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking);
         if (e == cudaSuccess)
             e = cudaEventCreateWithFlags(&pl->fork, cudaEventDisableTiming);
@@ -1699,8 +1804,11 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     d.ccen = has_q || has_h ? cell_centres(d, has_q, d.cstride) : nullptr;
     if (has_q)
         rc |= encode_cells<KQ>(&pl->tmap[KQ], d.qcells, hp->ncells);
-    if (has_h)
+    if (d.hcells && hp->ncells > 0 && (has_h || want_ewald))
         rc |= encode_cells<KH>(&pl->tmap[KH], d.hcells, hp->ncells);
+    if (want_ewald)
+        rc |= encode_rows(&pl->tmap[3], d.ew.t, (int64_t)d.ew.n * d.ew.n * d.ew.n, 4 * ew::kNode,
+                          CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) {
         grav_plan_free(pl);
         return rc;
@@ -1765,11 +1873,11 @@ int launch_kind(grav_plan *pl, const DevProblem &dp, cudaStream_t st) {
     return 0;
 }
 
-// k_ewald_moments: `warps` warps per block, each with two 11 KiB stages,
-// blocks_per_sm x SM count blocks (0: as many as fit), at most one warp per
-// group; over dp's groups, on stream s.
+// k_ewald_moments: `warps` warps per block, blocks_per_sm x SM count blocks
+// (0: as many as fit), at most one warp per unit; over dp's groups, on
+// stream s.
 int launch_moments(grav_plan *pl, const DevProblem &dp, cudaStream_t s, int per_sm, int warps) {
-    const int64_t n = dp.ngroups - dp.gbegin;
+    const int64_t n = (dp.ngroups - dp.gbegin) * dp.ewsplit;
     if (n <= 0)
         return 0;
     const size_t smem = (size_t)warps * kEwWarpBytes;
@@ -1785,7 +1893,7 @@ int launch_moments(grav_plan *pl, const DevProblem &dp, cudaStream_t s, int per_
     d.ewm = pl->ewm;
     const unsigned blocks = (unsigned)std::max<int64_t>(
         1, std::min<int64_t>((n + warps - 1) / warps, (int64_t)per_sm * pl->nsm));
-    k_ewald_moments<<<blocks, warps * 32, smem, s>>>(d);
+    k_ewald_moments<<<blocks, warps * 32, smem, s>>>(pl->tmap[3], pl->tmap[KH], d);
     GC_CHECK(cudaGetLastError());
     pl->launches++;
     return 0;
@@ -1826,7 +1934,7 @@ int side_fork(grav_plan *pl, const DevProblem &dp, cudaStream_t st, bool &forked
     GC_CHECK(cudaStreamWaitEvent(pl->side, pl->fork, 0));
     DevProblem d = dp;
     d.ewm = pl->ewm;
-    const int64_t n = dp.ngroups - dp.gbegin;
+    const int64_t n = (dp.ngroups - dp.gbegin) * dp.ewsplit;
     const unsigned blocks =
         (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 1) / 2, (int64_t)per_sm * pl->nsm));
     k_ewald_side<<<blocks, 64, 0, pl->side>>>(d);

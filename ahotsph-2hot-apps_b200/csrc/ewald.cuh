@@ -168,6 +168,8 @@ __device__ __forceinline__ void ew_lookup(const EwTab &E, float yx, float yy, fl
 // 0..2 (its mass and up to four folds) are first summed in FP32 (`cur`),
 // which carries their own FP32 rounding anyway, and reach the FP64 sums once
 // per entry (end_entry): one FP64 add per component and entry, not five.
+// Every term is one explicit fused multiply-add, so every kernel that sums
+// moments in this order stores the same bits.
 struct EwMoments {
     double lo[10];
     float hi[25];
@@ -180,14 +182,8 @@ struct EwMoments {
 #pragma unroll
         for (int q = 0; q < 10; q++) cur[q] = 0.f;
     }
-    // rounded adds (never contracted with the product that forms v), so
-    // every kernel that sums moments stores the same bits
-    __device__ __forceinline__ void add(int q, float v) {
-        if (q < 10)
-            cur[q] = __fadd_rn(cur[q], v);
-        else
-            hi[q - 10] = __fadd_rn(hi[q - 10], v);
-    }
+    // the FP32 sum component q is accumulated in
+    __device__ __forceinline__ float &at(int q) { return q < 10 ? cur[q] : hi[q - 10]; }
     __device__ __forceinline__ void end_entry() {
 #pragma unroll
         for (int q = 0; q < 10; q++) {
@@ -219,7 +215,7 @@ __device__ __forceinline__ void ew_fold(EwMoments &M, const float *S, const floa
             for (int a2 = 0; a2 <= SMAX; a2++) {
                 if (a0 + a1 + a2 > SMAX)
                     continue;
-                float acc = 0.f;
+                float &acc = M.at(ew::idx(a0, a1, a2));
 #pragma unroll
                 for (int b0 = 0; b0 <= K; b0++)
 #pragma unroll
@@ -233,14 +229,13 @@ __device__ __forceinline__ void ew_fold(EwMoments &M, const float *S, const floa
                                        (ew::ifact(b0) * ew::ifact(b1) * ew::ifact(b2)),
                                    D, acc);
                     }
-                M.add(ew::idx(a0, a1, a2), acc);
             }
 }
 
 // A source of mass m at the looked-up point: M_s += m D^alpha C.
 __device__ __forceinline__ void ew_add_mass(EwMoments &M, float m, const float *o) {
 #pragma unroll
-    for (int q = 0; q < ew::kNQ4; q++) M.add(q, __fmul_rn(m, o[q]));
+    for (int q = 0; q < ew::kNQ4; q++) M.at(q) = fmaf(m, o[q], M.at(q));
 }
 
 // Traceless second moment (multi-index layout xx xy xz yy yz zz) from the
