@@ -85,7 +85,7 @@ struct AdjProblem {
     const int64_t *cptr;
     const uint32_t *clist;
     EwTab ew;
-    float ew_self, ew_trace;
+    float ew_self;
     const EwStored *ewm;     // the forward's per-group moments
     double *mbar;            // 35 per group: dL/dM[alpha]
     double *gstf;            // kStfIndep per cell: the correction's trace-free moment duals
@@ -842,7 +842,7 @@ __global__ void k_adjoint_ewald_groups(AdjProblem P) {
 //   N[g] = m Mbar[g] + sum_K sum_{|b|=K, b<=g} A_K[b]/b! Mbar[g - b],
 //   dL/dA_K[b] = (1/K!) sum_a Mbar[a] D[a + b] over the forward's terms
 //                (|a| <= 3, 2, 1 for K = 2, 3, 4),
-//   dL/dB2 = Mbar[0] ew_trace / 6.
+//   dL/dB2 = Mbar[0] tr(D^2 C) / 6.
 __device__ __forceinline__ float ew_D(const float *o, const float *f5, int q) {
     return q < ew::kNQ4 ? o[q] : f5[q - ew::kNQ4];
 }
@@ -980,7 +980,7 @@ __global__ void __launch_bounds__(64) k_adjoint_ewald_entries(AdjProblem P) {
             ew_adj_conv<4>(S, Mb, N);
             ew_adj_moment<4, 1>(Mb, o, f5, G);
             add_indep<4>(G, gi + 12);
-            atomicAdd(gc + kAdjB2, (double)(Mb[0] * (1.f / 6.f) * P.ew_trace));
+            atomicAdd(gc + kAdjB2, (double)(Mb[0] * (1.f / 6.f) * P.ew.trace));
         }
         float dX[3] = {0.f, 0.f, 0.f};
 #pragma unroll
@@ -1260,7 +1260,6 @@ extern "C" int grav_plan_adjoint_CUDA(grav_plan *pl, const float *wu, float *gra
     P.clist = pl->dp.clist;
     P.ew = pl->dp.ew;
     P.ew_self = pl->dp.ew_self;
-    P.ew_trace = pl->dp.ew_trace;
     P.ewm = pl->ewm;
     P.mbar = A->mbar;
     P.gstf = A->gstf;

@@ -100,7 +100,6 @@ struct DevProblem {
     int ewald;
     EwTab ew;
     float ew_self;             // C(0) - pi/(alpha^2 L^3): the self term ewald() leaves out
-    float ew_trace;            // trace of the Hessian of C: -4 pi / L^3
     EwStored *ewm;             // per-group moments from k_ewald_moments
     EwStored *ewpart;          // its units' moments where a group's list is split (ewsplit > 1)
     int *ewdone;               // finished units per group, zero between evaluations
@@ -757,9 +756,10 @@ __device__ __forceinline__ EwUnit ew_unit(const DevProblem &P, int64_t u) {
 // where the list is split, as a part: the warp that finishes the group's
 // last unit adds the parts in order.
 __device__ __forceinline__ void ew_store(const DevProblem &P, int64_t u, int64_t g, int lane,
-                                         const EwMoments &M) {
+                                         const EwSums &T) {
     EwStored *E = P.ewsplit > 1 ? P.ewpart + (g * P.ewsplit + u % P.ewsplit) : P.ewm + g;
     if (lane == 0) {
+        const EwMoments M = T.full(P.ew.trace);
 #pragma unroll
         for (int q = 0; q < 10; q++) E->lo[q] = M.lo[q];
 #pragma unroll
@@ -790,90 +790,28 @@ __device__ __forceinline__ void ew_store(const DevProblem &P, int64_t u, int64_t
         P.ewdone[g] = 0;
 }
 
-// One entry's terms from its node values V (56 floats) and, for a cell, its
-// record r (nln_hcell as floats: mass 6, R 7, q2 8..12, q3 13..19, q4 20..28,
-// B2 29); m: a body's mass.
-template <class Node, class Record>
-__device__ __forceinline__ void ew_entry(EwMoments &M, const DevProblem &P, const EwNode &N,
-                                         bool cell, float m, Node node, Record record) {
-    // orders 0..4 (35 values) for the expansion; order 5 is read after it, so
-    // the two are never in registers together
-    float V[36];
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        const float4 v = node(k);
-        V[4 * k] = v.x;
-        V[4 * k + 1] = v.y;
-        V[4 * k + 2] = v.z;
-        V[4 * k + 3] = v.w;
-    }
-    float o[ew::kNQ4], f5[21];
-    ew_expand<false>(V, N, o, nullptr);
-    if (!cell) {
-        ew_add_mass(M, m, o);
-    } else {
-        float V5[24];  // node floats 32..55; order 5 starts at 35
-#pragma unroll
-        for (int k = 8; k < 14; k++) {
-            const float4 v = node(k);
-            V5[4 * (k - 8)] = v.x;
-            V5[4 * (k - 8) + 1] = v.y;
-            V5[4 * (k - 8) + 2] = v.z;
-            V5[4 * (k - 8) + 3] = v.w;
-        }
-        ew_fifth(V5 + 3, N, f5);
-        float r[32];
-#pragma unroll
-        for (int k = 1; k < 8; k++) {
-            const float4 v = record(k);
-            r[4 * k] = v.x;
-            r[4 * k + 1] = v.y;
-            r[4 * k + 2] = v.z;
-            r[4 * k + 3] = v.w;
-        }
-        const float R = r[7];
-        ew_add_mass(M, r[6], o);
-        float S[15];
-        ew_quad(R, r + 8, S);
-        ew_fold<2, 3>(M, S, o, f5);
-        ew_oct(R, r + 13, S);
-        ew_fold<3, 2>(M, S, o, f5);
-        ew_hex(R, r + 20, S);
-        ew_fold<4, 1>(M, S, o, f5);
-        M.at(0) = fmaf(__fmul_rn(r[29], 1.f / 6.f), P.ew_trace, M.at(0));
-    }
-    M.end_entry();
-}
+// Every entry needs its table node (144 B) and its cell record (112 of 128 B)
+// from scattered addresses, and the node depends on the record's centre: list
+// word three tiles ahead, the source's FP64 centre (plain loads) two tiles
+// ahead, and one tile ahead the tile's 32 nodes and records by cp.async into
+// one of two stages of the warp.  The warp copies them row by row, neighbour
+// lanes neighbour chunks of a row: with each lane copying its own rows every
+// instruction touched 32 cache lines and the L1's rate held the kernel (160^3
+// box: 30.7 ms with the finish pass); TMA row gathers, the other way, cost 270
+// of 1,500 instructions a tile to start (24.7 ms; now 13.9).  Rows of 9 and 7 chunks
+// are read back without bank conflicts.
+constexpr int kEwNodeChunks = ew::kNode / 4;   // 9
+constexpr int kEwRecChunks = 7;                // floats 4..31 of nln_hcell
+struct EwStage {
+    float4 node[32 * kEwNodeChunks];
+    float4 rec[32 * kEwRecChunks];
+};
+constexpr int kEwWarpBytes = 2 * (int)sizeof(EwStage);  // 16 KB
 
-// Every entry needs its table node (224 B) and its cell record (128 B) from
-// scattered addresses, and the node depends on the record's centre: list word
-// three tiles ahead, the source's FP64 centre (plain loads) two tiles ahead,
-// and one tile ahead the tile's 32 nodes and records by TMA row gathers, four
-// rows an instruction, into one of two stages of the warp.  Copying the rows
-// by per-lane cp.async instead touched 32 cache lines with every one of its
-// 21 instructions and held the kernel to the L1's rate (160^3 box: 30.7 ms with the finish pass, now
-// 24.7).
-constexpr int kEwNodeBytes = 32 * 4 * ew::kNode;             // 7,168
-constexpr int kEwRecBytes = 32 * (int)sizeof(nln_hcell);     // 4,096, swizzled
-constexpr int kEwWarpBytes = 2 * (kEwNodeBytes + kEwRecBytes) + 16;
-
-__global__ void __launch_bounds__(128)
-    k_ewald_moments(const __grid_constant__ CUtensorMap tnode,
-                    const __grid_constant__ CUtensorMap trec, DevProblem P) {
-    extern __shared__ __align__(1024) unsigned char ewsm[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // the block's record stages first (their swizzle repeats every 1024
-    // bytes), then the node stages, then the mbarriers
-    unsigned char *recs = ewsm + (size_t)wib * 2 * kEwRecBytes;
-    unsigned char *nodes = ewsm + (size_t)nw * 2 * kEwRecBytes + (size_t)wib * 2 * kEwNodeBytes;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(ewsm + (size_t)nw * 2 * (kEwRecBytes + kEwNodeBytes)) +
-                    2 * wib;
-    if (lane == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
+__global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
+    extern __shared__ __align__(16) unsigned char ewsm[];
+    const int lane = threadIdx.x & 31;
+    EwStage *stg = reinterpret_cast<EwStage *>(ewsm + (size_t)(threadIdx.x >> 5) * kEwWarpBytes);
     const uint32_t ntab = (uint32_t)P.ntab[0];
     const uint32_t nb = ntab - (uint32_t)P.ncells;
     constexpr uint32_t kNone = 0xffffffffu;
@@ -884,7 +822,12 @@ __global__ void __launch_bounds__(128)
         double x, y, z;
         float m;
     };
-    uint32_t seq = 0;  // tiles started by this warp: stage seq & 1, parity seq >> 1 & 1
+    // the entry whose rows are staged: its node and what kind it is
+    struct Staged {
+        EwNode N;
+        bool live, cell;
+        float m;
+    };
     for (;;) {
         int it = 0;
         if (lane == 0)
@@ -926,83 +869,67 @@ __global__ void __launch_bounds__(128)
             }
             return r;
         };
-        auto node_of = [&](const Src &q) -> EwNode {
-            double sx, sy, sz;
-            decode_shift(q.e >> NLN_IDX_BITS, P.box, sx, sy, sz);
-            return ew_node(P.ew, (float)(q.x + sx - c[0]), (float)(q.y + sy - c[1]),
-                           (float)(q.z + sz - c[2]));
-        };
-        // Start the copies of a tile (sequence number s): lane 0 gathers the
-        // row numbers; lanes without an entry repeat row 0.
-        auto issue = [&](const Src &q, uint32_t s) {
-            const bool live = q.e != kNone;
-            const bool cell = live && (q.e & NLN_IDX_MASK) >= nb;
-            const int node = live ? node_of(q).node : 0;
-            const int rec = cell ? (int)((q.e & NLN_IDX_MASK) - nb) : 0;
-            const unsigned any = __ballot_sync(0xffffffffu, live);
-            const unsigned cells = __ballot_sync(0xffffffffu, cell);
-            uint64_t *b = &bar[s & 1];
-            unsigned char *dn = nodes + (s & 1) * kEwNodeBytes, *dr = recs + (s & 1) * kEwRecBytes;
-            if (lane == 0) {
-                uint32_t bytes = 0;
-                for (int g = 0; g < 8; g++) {
-                    bytes += any >> (4 * g) & 15u ? 16u * ew::kNode : 0u;
-                    bytes += cells >> (4 * g) & 15u ? 4u * (uint32_t)sizeof(nln_hcell) : 0u;
-                }
-                mbar_arrive_expect_tx(b, bytes);
+        // Start the copies of a tile: chunk i of its 32 rows is chunk i % 9 (or
+        // i % 7) of row i / 9 (or 7), whose lane names it.
+        auto issue = [&](const Src &q, EwStage &S) -> Staged {
+            Staged r;
+            r.live = q.e != kNone;
+            r.m = q.m;
+            const uint32_t idx = q.e & NLN_IDX_MASK;
+            r.cell = r.live && idx >= nb;
+            int node = 0;
+            if (r.live) {
+                double sx, sy, sz;
+                decode_shift(q.e >> NLN_IDX_BITS, P.box, sx, sy, sz);
+                r.N = ew_node(P.ew, (float)(q.x + sx - c[0]), (float)(q.y + sy - c[1]),
+                              (float)(q.z + sz - c[2]));
+                node = r.N.node;
             }
+            const unsigned live = __ballot_sync(0xffffffffu, r.live);
+            const unsigned cells = __ballot_sync(0xffffffffu, r.cell);
+            const int rec = r.cell ? (int)(idx - nb) : 0;
 #pragma unroll
-            for (int g = 0; g < 8; g++) {
-                int rn[4], rr[4];
+            for (int k = 0; k < kEwNodeChunks; k++) {
+                const int i = 32 * k + lane, row = i / kEwNodeChunks;
+                const int from = __shfl_sync(0xffffffffu, node, row);
+                if (live >> row & 1u)
+                    cp_async16(&S.node[i], P.ew.t + (size_t)from * ew::kNode + 4 * (i - row * kEwNodeChunks));
+            }
+            if (cells) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    rn[j] = __shfl_sync(0xffffffffu, node, 4 * g + j);
-                    rr[j] = __shfl_sync(0xffffffffu, rec, 4 * g + j);
-                }
-                if (lane == 0) {
-                    if (any >> (4 * g) & 15u)
-                        tma_gather4(dn + g * 16 * ew::kNode, &tnode, rn[0], rn[1], rn[2], rn[3], b);
-                    if (cells >> (4 * g) & 15u)
-                        tma_gather4(dr + g * 4 * (int)sizeof(nln_hcell), &trec, rr[0], rr[1], rr[2],
-                                    rr[3], b);
+                for (int k = 0; k < kEwRecChunks; k++) {
+                    const int i = 32 * k + lane, row = i / kEwRecChunks;
+                    const int from = __shfl_sync(0xffffffffu, rec, row);
+                    if (cells >> row & 1u)
+                        cp_async16(&S.rec[i], reinterpret_cast<const float4 *>(P.hcells + from) + 1 +
+                                                  (i - row * kEwRecChunks));
                 }
             }
+            cp_async_commit();
+            return r;
         };
-        EwMoments M;
+        EwSums M;
         M.zero();
-        Src s0 = source(entry(0));
-        if (ntile > 0)
-            issue(s0, seq);
+        Staged now = issue(source(entry(0)), stg[0]), next;
         Src s1 = source(entry(1));
         uint32_t e2 = entry(2);
         for (int t = 0; t < ntile; t++) {
             __syncwarp();  // the other stage is no longer read
-            if (t + 1 < ntile)
-                issue(s1, seq + t + 1);
-            const Src s2 = source(e2);  // consumed by the next tile's issue
+            next = issue(s1, stg[(t + 1) & 1]);
+            s1 = source(e2);  // consumed by the next tile's issue
             e2 = entry(t + 3);
-            const uint32_t s = seq + t;
-            const bool ok = mbar_wait_bounded(&bar[s & 1], s >> 1 & 1, P.err);
-            if (!__all_sync(0xffffffffu, ok)) {
-                // give the copies still in flight a bounded chance to land
-                if (t + 1 < ntile)
-                    mbar_wait_bounded(&bar[(s + 1) & 1], (s + 1) >> 1 & 1, P.err, 1u << 10);
-                return;
+            cp_async_wait<1>();  // this lane's copies for tile t have landed
+            __syncwarp();        // and the other lanes'
+            if (now.live) {
+                const float4 *node = stg[t & 1].node + lane * kEwNodeChunks;
+                const float4 *rec = stg[t & 1].rec + lane * kEwRecChunks - 1;
+                ew_entry(M, P.ew.trace, now.N, now.cell, now.m, [&](int k) { return node[k]; },
+                         [&](int k) { return rec[k]; });
             }
-            if (s0.e != kNone) {
-                const float4 *node =
-                    reinterpret_cast<const float4 *>(nodes + (s & 1) * kEwNodeBytes + lane * 4 * ew::kNode);
-                const unsigned char *rec = recs + (s & 1) * kEwRecBytes;
-                ew_entry(M, P, node_of(s0), (s0.e & NLN_IDX_MASK) >= nb, s0.m,
-                         [&](int k) { return node[k]; },
-                         [&](int k) {
-                             return *reinterpret_cast<const float4 *>(rec + CellKind<KH>::chunk(lane, k));
-                         });
-            }
-            s0 = s1;
-            s1 = s2;
+            now = next;
         }
-        seq += ntile;
+        cp_async_wait<0>();
+        __syncwarp();
         M.warp_sum();
         ew_store(P, it, U.g, lane, M);
     }
@@ -1025,7 +952,7 @@ __global__ void __launch_bounds__(64) k_ewald_side(DevProblem P) {
         if (U.g >= P.ngroups)
             break;
         const nln_group G = P.groups[U.g];
-        EwMoments M;
+        EwSums M;
         M.zero();
         const int64_t end = min(U.ce, U.cb + (int64_t)U.t1 * 32);
         for (int64_t k = U.cb + (int64_t)U.t0 * 32 + lane; k < end; k += 32) {
@@ -1057,7 +984,7 @@ __global__ void __launch_bounds__(64) k_ewald_side(DevProblem P) {
             const EwNode N = ew_node(P.ew, (float)(x + sx - G.cen[0]), (float)(y + sy - G.cen[1]),
                                      (float)(z + sz - G.cen[2]));
             const float4 *node = reinterpret_cast<const float4 *>(P.ew.t + (size_t)N.node * ew::kNode);
-            ew_entry(M, P, N, cell, m, [&](int q) { return __ldg(node + q); },
+            ew_entry(M, P.ew.trace, N, cell, m, [&](int q) { return __ldg(node + q); },
                      [&](int q) { return __ldg(rec + q); });
         }
         M.warp_sum();
@@ -1123,8 +1050,7 @@ struct grav_plan {
     int nsm = 148;
     int launches = 0;
     int64_t nslots = 0;
-    CUtensorMap tmap[4];    // row-gather views: 1, 2 the quadrupole and order-4 tables, 3 the
-                            // Ewald table
+    CUtensorMap tmap[3];    // row-gather views of the quadrupole and order-4 tables
     int timing = 0;         // record events around each kernel of an evaluation
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     std::vector<int64_t> lists_ptr[4];  // host copies of the P, Q, H (queue rebuilds) and
@@ -1157,10 +1083,11 @@ struct grav_plan {
 
 namespace {
 
-// A 2-D tensor map over `rows` records of `bytes` (a multiple of 16), box =
-// one full record (one row high, as the row gather requires).
-int encode_rows(CUtensorMap *m, const void *base, int64_t rows, uint32_t bytes,
-                CUtensorMapSwizzle swizzle) {
+// The row-gather view of a cell table: box = one full record (one row high,
+// as the row gather requires), swizzled over the record's width
+// (CellKind::chunk).
+template <int KIND>
+int encode_cells(CUtensorMap *m, const void *base, int64_t rows) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
         void *fn = nullptr;
@@ -1170,26 +1097,19 @@ int encode_rows(CUtensorMap *m, const void *base, int64_t rows, uint32_t bytes,
             return gc::set_status(-1, "cuTensorMapEncodeTiled unavailable");
         encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
-    const uint32_t w = bytes / 4;
+    constexpr uint32_t bytes = CellKind<KIND>::rec_bytes, w = bytes / 4;
     cuuint64_t dims[2] = {w, (cuuint64_t)rows};
     cuuint64_t strides[1] = {bytes};
     cuuint32_t box[2] = {w, 1};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(base), dims,
-                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        KIND == KH ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return gc::set_status(-1, "cuTensorMapEncodeTiled failed (%d) for %lld rows of %u bytes",
                               (int)r, (long long)rows, bytes);
     return 0;
-}
-
-// The row-gather view of a cell table, swizzled over the record's width
-// (CellKind::chunk).
-template <int KIND>
-int encode_cells(CUtensorMap *m, const void *base, int64_t rows) {
-    return encode_rows(m, base, rows, CellKind<KIND>::rec_bytes,
-                       KIND == KH ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 // The table k_points reads FP64 cell centres from, and its record size.
@@ -1714,14 +1634,20 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
                 cache_n = n;
             }
         }
-        std::vector<float> t32(t64.begin(), t64.end());
+        std::vector<float> t32((size_t)n * n * n * ew::kNode);
+        for (size_t node = 0; node < (size_t)n * n * n; node++)
+            for (int l = 0; l <= 5; l++)
+                for (int az = 0; az <= (l ? 1 : 0); az++)
+                    for (int ay = 0; ay <= l - az; ay++)
+                        t32[node * ew::kNode + ew::hidx(l - az - ay, ay, az)] =
+                            (float)t64[node * NLN_EWALD_NQ + ew::idx(l - az - ay, ay, az)];
         float *tab = nullptr;
         rc |= dev_copy(pl, t32.data(), t32.size(), &tab);
         const double h = NLN_EWALD_REACH * hp->box / (n - 1);
-        d.ew = EwTab{tab, n, (float)h, (float)(1.0 / h)};
+        d.ew = EwTab{tab, n, (float)h, (float)(1.0 / h),
+                     (float)(-4.0 * M_PI / (hp->box * hp->box * hp->box))};
         const double alpha = 2.0 / hp->box;
         d.ew_self = (float)(t64[0] - M_PI / (alpha * alpha * hp->box * hp->box * hp->box));
-        d.ew_trace = (float)(-4.0 * M_PI / (hp->box * hp->box * hp->box));
         d.ewald = 1;
         rc |= dev_copy<EwStored>(pl, nullptr, (size_t)ng, &pl->ewm);
         pl->ewald_entries = hp->cptr[ng];
@@ -1804,11 +1730,8 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     d.ccen = has_q || has_h ? cell_centres(d, has_q, d.cstride) : nullptr;
     if (has_q)
         rc |= encode_cells<KQ>(&pl->tmap[KQ], d.qcells, hp->ncells);
-    if (d.hcells && hp->ncells > 0 && (has_h || want_ewald))
+    if (has_h)
         rc |= encode_cells<KH>(&pl->tmap[KH], d.hcells, hp->ncells);
-    if (want_ewald)
-        rc |= encode_rows(&pl->tmap[3], d.ew.t, (int64_t)d.ew.n * d.ew.n * d.ew.n, 4 * ew::kNode,
-                          CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) {
         grav_plan_free(pl);
         return rc;
@@ -1893,7 +1816,7 @@ int launch_moments(grav_plan *pl, const DevProblem &dp, cudaStream_t s, int per_
     d.ewm = pl->ewm;
     const unsigned blocks = (unsigned)std::max<int64_t>(
         1, std::min<int64_t>((n + warps - 1) / warps, (int64_t)per_sm * pl->nsm));
-    k_ewald_moments<<<blocks, warps * 32, smem, s>>>(pl->tmap[3], pl->tmap[KH], d);
+    k_ewald_moments<<<blocks, warps * 32, smem, s>>>(d);
     GC_CHECK(cudaGetLastError());
     pl->launches++;
     return 0;
