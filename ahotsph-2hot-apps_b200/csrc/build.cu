@@ -493,11 +493,14 @@ __global__ void k_groups(int64_t ng, const int64_t *first, const int32_t *count,
 // cell is decided twice.  Bounded by the FP64 decision and the scattered
 // 80-byte cell records, with the walk's parallelism 32 times the group count;
 // one thread per group had too few threads below a million bodies and wrote
-// every entry uncoalesced (100k-body sphere: 50.6 ms for both passes).
+// every entry uncoalesced (both passes, 100k-body sphere 50.6 -> 2.7 ms, 96^3
+// box 71 -> 17 ms, 160^3 238 -> 121 ms).  Issue slots are 62 to 71 % busy;
+// single-precision bounds in place of the FP64 square roots changed nothing.
 constexpr int kWalkWarps = 4;
-// Stack entries per warp.  A round with w lanes adds at most 8 w entries, and
-// w falls to 1 (an ordinary depth-first walk, at most NLN_WALK_STACK deep)
-// before the stack could fill.
+// Stack entries per warp, of which the last NLN_WALK_STACK are kept for an
+// ordinary depth-first walk: lanes whose children would reach into them go
+// back undecided, all but the first, so a round always gets on and the stack
+// never fills.
 constexpr int kWalkStack = 768;
 
 enum { W_OPEN = 0, W_MARK = 5 };  // 1..4: NLN_MONO..NLN_LEAF, decided; 5: a correction entry alone
@@ -554,29 +557,53 @@ __device__ __forceinline__ int64_t emit_runs(uint32_t *out, int64_t pos, int64_t
     }
     const int inc = warp_scan(n, lane);
     const int total = __shfl_sync(FULL, inc, 31);
-    for (int j0 = 0; j0 < total; j0 += 32) {
-        const int j = j0 + lane;
-        int owner = 0;  // lanes whose runs all lie before j
+    constexpr int U = 4;  // searches in flight
+    for (int j0 = 0; j0 < total; j0 += 32 * U) {
+        int owner[U];  // lanes whose runs all lie before entry j0 + 32 u + lane
+#pragma unroll
+        for (int u = 0; u < U; u++) owner[u] = 0;
 #pragma unroll
         for (int step = 16; step >= 1; step >>= 1)
-            if (__shfl_sync(FULL, inc, owner + step - 1) <= j)
-                owner += step;
-        owner = min(owner, 31);
-        const uint32_t f = __shfl_sync(FULL, first, owner);
-        const int b = __shfl_sync(FULL, inc - n, owner);
-        uint32_t c = __shfl_sync(FULL, code, owner);
-        if (j < total && pos + j < end) {
-            const uint32_t e = f + (uint32_t)(j - b);
-            if (c == kOwnImages) {
-                const float *x = spos + 3 * (int64_t)e;
-                int sb[3];
-                for (int d = 0; d < 3; d++) sb[d] = nln_image(x[d] - G.cen[d], box);
-                c = nln_shift_code(sb);
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (__shfl_sync(FULL, inc, owner[u] + step - 1) <= j0 + 32 * u + lane)
+                    owner[u] += step;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int j = j0 + 32 * u + lane, o = min(owner[u], 31);
+            const uint32_t f = __shfl_sync(FULL, first, o);
+            const int b = __shfl_sync(FULL, inc - n, o);
+            uint32_t c = __shfl_sync(FULL, code, o);
+            if (j < total && pos + j < end) {
+                const uint32_t e = f + (uint32_t)(j - b);
+                if (c == kOwnImages) {
+                    const float *x = spos + 3 * (int64_t)e;
+                    int sb[3];
+                    for (int d = 0; d < 3; d++) sb[d] = nln_image(x[d] - G.cen[d], box);
+                    c = nln_shift_code(sb);
+                }
+                out[pos + j] = e | c << NLN_IDX_BITS;
             }
-            out[pos + j] = e | c << NLN_IDX_BITS;
         }
     }
     return pos + total;
+}
+
+// Groups in the walk's order: first those whose radius is a sixteenth of the
+// cube or more (a sphere's sparse outskirts), which open most of the tree and
+// would end last alone, then the others, both as they lie in space.
+__global__ void k_wide_groups(const nln_group *__restrict__ groups, int64_t ng, double wide,
+                              int64_t *flag) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g <= ng)
+        flag[g] = g < ng && groups[g].radius >= wide ? 1 : 0;
+}
+
+__global__ void k_walk_order(const nln_group *__restrict__ groups, int64_t ng, double wide,
+                             const int64_t *__restrict__ before, int32_t *order) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < ng)
+        order[groups[g].radius >= wide ? before[g] : before[ng] + g - before[g]] = (int32_t)g;
 }
 
 // FILL false: cnt[5 g ..] = point, quadrupole, order-4 and correction
@@ -585,16 +612,17 @@ __device__ __forceinline__ int64_t emit_runs(uint32_t *out, int64_t pos, int64_t
 template <bool FILL>
 __global__ void __launch_bounds__(32 * kWalkWarps)
     k_walk(const nln_wcell *__restrict__ wc, const float *__restrict__ spos, int64_t n,
-           const nln_group *__restrict__ groups, int64_t ng, nln_mac P, int64_t *cnt,
-           const int64_t *pp, const int64_t *qp, const int64_t *hp, const int64_t *cp,
+           const nln_group *__restrict__ groups, const int32_t *__restrict__ order, int64_t ng,
+           nln_mac P, int64_t *cnt, const int64_t *pp, const int64_t *qp, const int64_t *hp, const int64_t *cp,
            uint32_t *pl, uint32_t *ql, uint32_t *hl, uint32_t *cl, unsigned *err) {
     __shared__ uint32_t s_item[kWalkWarps][kWalkStack];
     __shared__ uint8_t s_code[kWalkWarps][FILL ? kWalkStack : 1];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int64_t g = (int64_t)blockIdx.x * kWalkWarps + wib;
-    if (g >= ng)
+    const int64_t slot = (int64_t)blockIdx.x * kWalkWarps + wib;
+    if (slot >= ng)
         return;
+    const int64_t g = order[slot];
     uint32_t *item = s_item[wib];
     uint8_t *codes = s_code[wib];
     const nln_group G = groups[g];
@@ -614,8 +642,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
     __syncwarp();
     bool overflow = false;
     while (sp > 0) {
-        const int room = (kWalkStack - NLN_WALK_STACK - sp) / 8;
-        const int w = min(min(32, sp), max(1, room));
+        int w = min(32, sp);
         const bool mine = lane < w;
         uint32_t it = 0;
         uint32_t code = NLN_SHIFT_NONE;
@@ -630,7 +657,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
         int kids = 0, child = 0;
         int32_t bodies = 0;
         uint32_t first = 0;
-        bool covers = false, ccov = false, opened = false;
+        bool covers = false, ccov = false, opened = false, decided = false;
         if (mine && type == W_OPEN) {
             const nln_wcell c = load_wcell(wc, ci);
             ccov = (it >> kWalkFlag & 1u) != 0;
@@ -645,41 +672,52 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
                 child = c.child;
                 kids = c.nchild;
             } else {
-                covered += c.count;
+                decided = true;
                 type = v.what;
                 // the correction list gets the cell, or an uncovered leaf's bodies
                 cflag = !periodic ? 0 : covers ? 1 : ccov ? 0 : type == NLN_LEAF ? 2 : 1;
                 if (type == NLN_LEAF && !v.inside)
                     code = kOwnImages;
             }
-            if (!FILL) {
+        } else if (FILL && mine && type == NLN_LEAF) {
+            first = (uint32_t)wc[ci].first;
+            bodies = wc[ci].count;
+        }
+        __syncwarp();  // the window is read: its entries may be overwritten
+        // entries each lane puts back, and the lanes whose entries fit with one
+        // for each lane behind them: the others stay as they were
+        const int slots0 = !mine ? 0 : FILL ? (opened ? kids + (covers ? 1 : 0) : 1) : kids;
+        const int inc0 = warp_scan(slots0, lane);
+        const bool fits = sp - w + inc0 + (w - 1 - lane) <= kWalkStack - NLN_WALK_STACK;
+        const unsigned fit = __ballot_sync(FULL, mine && (fits || lane == 0));
+        const int keep = fit == FULL ? 32 : __ffs(~fit) - 1;  // lanes that go through
+        w = keep;
+        const bool through = lane < w;
+        if (through && decided)
+            covered += bodies;
+        if (!FILL) {
+            if (through && mine) {
                 np += type == NLN_LEAF ? bodies : type == NLN_MONO ? 1 : 0;
                 nbod += type == NLN_LEAF ? bodies : 0;
                 nq += type == NLN_QUAD;
                 nh += type == NLN_HEXA;
                 nc += covers ? 1 : opened ? 0 : cflag == 2 ? bodies : cflag;
             }
-        } else if (FILL && mine && type == NLN_LEAF) {
-            first = (uint32_t)wc[ci].first;
-            bodies = wc[ci].count;
-        }
-        __syncwarp();  // the window is read: its entries may be overwritten
-        if (!FILL) {
-            const int inc = warp_scan(kids, lane);
-            const int total = __shfl_sync(FULL, inc, 31);
+            const int total = __shfl_sync(FULL, inc0, w - 1);
             const int base = sp - w;
             if (base + total > kWalkStack) {
                 overflow = true;
                 break;
             }
             const uint32_t flag = ccov ? 1u << kWalkFlag : 0u;
-            for (int k = 0; k < kids; k++)
-                item[base + inc - kids + k] = (uint32_t)(child + k) | flag;
+            if (through)
+                for (int k = 0; k < kids; k++)
+                    item[base + inc0 - kids + k] = (uint32_t)(child + k) | flag;
             sp = base + total;
             __syncwarp();
             continue;
         }
-        const unsigned open = __ballot_sync(FULL, opened);
+        const unsigned open = __ballot_sync(FULL, opened && through);
         const int f = open ? __ffs(open) - 1 : w;
         // lanes before f are final: write them in order
         if (f > 0) {
@@ -711,10 +749,10 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
         }
         // lanes f .. w-1 go back on the stack in place
         const bool mark = opened && covers;
-        const int slots = lane < f || !mine ? 0 : opened ? kids + (mark ? 1 : 0) : 1;
-        const int inc = warp_scan(slots, lane);
-        const int total = __shfl_sync(FULL, inc, 31);
-        const int top = sp - w + total;
+        const int slots = lane < f || !through ? 0 : slots0;
+        const int gone = f > 0 ? __shfl_sync(FULL, inc0, f - 1) : 0;  // the final lanes' entries
+        const int inc = inc0 - gone;
+        const int top = sp - w + __shfl_sync(FULL, inc, w - 1);
         if (top > kWalkStack) {
             overflow = true;
             break;
@@ -1103,8 +1141,21 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     BC(B.get(&cnt, 5 * ng));
     BC(cudaMemsetAsync(cnt, 0, 5 * ng * sizeof(int64_t), st));
     BC(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
+    int32_t *worder = nullptr;
+    {
+        int64_t *wide = nullptr, *before = nullptr;
+        BC(B.get(&wide, ng + 1));
+        BC(B.get(&before, ng + 1));
+        BC(B.get(&worder, ng));
+        k_wide_groups<<<grid_of(ng + 1), kThreads, 0, st>>>(out.groups, ng, side / 16, wide);
+        BC(cudaGetLastError());
+        if (int rc = exclusive_scan(B, wide, before, ng + 1, st))
+            return rc;
+        k_walk_order<<<grid_of(ng), kThreads, 0, st>>>(out.groups, ng, side / 16, before, worder);
+        BC(cudaGetLastError());
+    }
     k_walk<false><<<grid_of(ng, kWalkWarps), 32 * kWalkWarps, 0, st>>>(
-        wc, spos, n, out.groups, ng, P, cnt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+        wc, spos, n, out.groups, worder, ng, P, cnt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
         nullptr, nullptr, flag);
     BC(cudaGetLastError());
     std::vector<int64_t> hc(5 * ng);
@@ -1145,7 +1196,7 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     t0 = now_s();
     BC(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
     k_walk<true><<<grid_of(ng, kWalkWarps), 32 * kWalkWarps, 0, st>>>(
-        wc, spos, n, out.groups, ng, P, nullptr, dptr[0], dptr[1], dptr[2], dptr[3], out.list[0],
+        wc, spos, n, out.groups, worder, ng, P, nullptr, dptr[0], dptr[1], dptr[2], dptr[3], out.list[0],
         out.list[1], out.list[2], out.list[3], flag);
     BC(cudaGetLastError());
     BC(cudaMemcpyAsync(&hbad, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
