@@ -61,12 +61,6 @@ constexpr int kTile[3] = {kPointTile, kQuadTile, kHexaTile};
 #define GRAV_P_MINB 4
 #endif
 
-struct Item {
-    int32_t group;
-    int32_t slot;      // partial-result slot (creation order: grouped by group)
-    int64_t begin, end;
-};
-
 // One group's correction moments as k_ewald_moments stores them (EwMoments).
 struct EwStored {
     double lo[10];
@@ -1326,7 +1320,7 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
         // failures included (grav_plan_free releases them)
         void *own[] = {adopt->points, adopt->qcells, adopt->hcells, adopt->groups,
                        adopt->list[0], adopt->list[1], adopt->list[2], adopt->list[3],
-                       adopt->order};
+                       adopt->order, adopt->ptr[0], adopt->ptr[1], adopt->ptr[2], adopt->ptr[3]};
         for (void *q : own)
             if (q)
                 pl->allocs.push_back(q);
@@ -1500,7 +1494,10 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
         }
         pl->chunk_group.push_back(ng);
     }
-    pl->nslots = make_queue(pl, items, gslot);
+    if (!adopt)
+        pl->nslots = make_queue(pl, items, gslot);
+    else
+        pl->chunk_group = {0, ng};
 
     // interaction counts (sinks x sources); the point list's split into
     // bodies and cell monopoles is counted on the device (k_check_lists)
@@ -1575,11 +1572,30 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     d.list[2] = l2;
     d.ntab[0] = np;
     d.ntab[1] = d.ntab[2] = hp->ncells;
-    for (int k = 0; k < 3; k++) {
-        Item *it = nullptr;
-        rc |= dev_copy(pl, items[k].data(), items[k].size(), &it);
-        d.items[k] = it;
-        d.nitems[k] = (int)items[k].size();
+    int64_t *gs = nullptr;
+    if (adopt) {
+        // the offsets are on the device: so is the queue made there (96^3 box: 3.9 ms on the
+        // host with its copies, 0.3 ms)
+        const int64_t *const dptr[3] = {adopt->ptr[0], adopt->ptr[1], adopt->ptr[2]};
+        const int64_t chunk[3] = {pl->tune.chunk_p, pl->tune.chunk_q, pl->tune.chunk_h};
+        Item *it[3];
+        rc |= gpu_make_queue(dptr, ng, chunk, 0, pl->pool, it, d.nitems, &gs, &pl->nslots);
+        for (int k = 0; k < 3; k++) {
+            d.items[k] = it[k];
+            if (it[k])
+                pl->allocs.push_back(it[k]);
+            pl->chunk_item[k] = {0, d.nitems[k]};
+        }
+        if (gs)
+            pl->allocs.push_back(gs);
+    } else {
+        for (int k = 0; k < 3; k++) {
+            Item *it = nullptr;
+            rc |= dev_copy(pl, items[k].data(), items[k].size(), &it);
+            d.items[k] = it;
+            d.nitems[k] = (int)items[k].size();
+        }
+        rc |= dev_copy(pl, gslot.data(), gslot.size(), &gs);
     }
     int *ctr = nullptr;  // 4 queue heads per group range
     rc |= dev_copy<int>(pl, nullptr, 4 * (pl->chunk_group.size() - 1), &ctr);
@@ -1587,15 +1603,16 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     float4 *part = nullptr;
     rc |= dev_copy<float4>(pl, nullptr, (size_t)std::max<int64_t>(1, pl->nslots) * 64, &part);
     d.part = part;
-    int64_t *gs = nullptr;
-    rc |= dev_copy(pl, gslot.data(), gslot.size(), &gs);
     d.gslot = gs;
     d.cptr = nullptr;
     d.clist = nullptr;
     if (want_ewald) {
         int64_t *cp = nullptr;
         uint32_t *cl = nullptr;
-        rc |= dev_copy(pl, hp->cptr, (size_t)ng + 1, &cp);
+        if (adopt)
+            cp = adopt->ptr[3];
+        else
+            rc |= dev_copy(pl, hp->cptr, (size_t)ng + 1, &cp);
         if (hp->lists_in_host) {
             cl = const_cast<uint32_t *>(mapped_host(hp->clist));
             if (!cl) {
@@ -1617,37 +1634,40 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     if (want_ewald) {
         // FP64 table on the host, FP32 copy on the device
         const int n = pl->tune.ewald_n > 1 ? pl->tune.ewald_n : 32;
-        // the table depends only on (box, n): build it once per process
+        // the table depends only on (box, n): build it once per process, with its FP32 values
         static std::mutex cache_mu;
-        static double cache_box = 0;
+        static double cache_box = 0, cache_c0 = 0;
         static int cache_n = 0;
-        static std::vector<double> t64;
+        static std::vector<float> t32;
+        float *tab = nullptr;
+        double c0 = 0;
         {
             std::lock_guard<std::mutex> lk(cache_mu);
             if (cache_box != hp->box || cache_n != n) {
-                t64.assign((size_t)n * n * n * NLN_EWALD_NQ, 0.0);
+                std::vector<double> t64((size_t)n * n * n * NLN_EWALD_NQ, 0.0);
                 if (ewald_table(hp->box, n, NLN_EWALD_REACH, t64.data())) {
                     grav_plan_free(pl);
                     return gc::set_status(-1, "Ewald table build failed");
                 }
+                t32.resize((size_t)n * n * n * ew::kNode);
+                for (size_t node = 0; node < (size_t)n * n * n; node++)
+                    for (int l = 0; l <= 5; l++)
+                        for (int az = 0; az <= (l ? 1 : 0); az++)
+                            for (int ay = 0; ay <= l - az; ay++)
+                                t32[node * ew::kNode + ew::hidx(l - az - ay, ay, az)] =
+                                    (float)t64[node * NLN_EWALD_NQ + ew::idx(l - az - ay, ay, az)];
+                cache_c0 = t64[0];
                 cache_box = hp->box;
                 cache_n = n;
             }
+            c0 = cache_c0;
+            rc |= dev_copy(pl, t32.data(), t32.size(), &tab);
         }
-        std::vector<float> t32((size_t)n * n * n * ew::kNode);
-        for (size_t node = 0; node < (size_t)n * n * n; node++)
-            for (int l = 0; l <= 5; l++)
-                for (int az = 0; az <= (l ? 1 : 0); az++)
-                    for (int ay = 0; ay <= l - az; ay++)
-                        t32[node * ew::kNode + ew::hidx(l - az - ay, ay, az)] =
-                            (float)t64[node * NLN_EWALD_NQ + ew::idx(l - az - ay, ay, az)];
-        float *tab = nullptr;
-        rc |= dev_copy(pl, t32.data(), t32.size(), &tab);
         const double h = NLN_EWALD_REACH * hp->box / (n - 1);
         d.ew = EwTab{tab, n, (float)h, (float)(1.0 / h),
                      (float)(-4.0 * M_PI / (hp->box * hp->box * hp->box))};
         const double alpha = 2.0 / hp->box;
-        d.ew_self = (float)(t64[0] - M_PI / (alpha * alpha * hp->box * hp->box * hp->box));
+        d.ew_self = (float)(c0 - M_PI / (alpha * alpha * hp->box * hp->box * hp->box));
         d.ewald = 1;
         rc |= dev_copy<EwStored>(pl, nullptr, (size_t)ng, &pl->ewm);
         pl->ewald_entries = hp->cptr[ng];
@@ -2062,8 +2082,7 @@ extern "C" void grav_plan_free(grav_plan *pl) {
 }
 
 // step.cuh: the plan's step state adopts a device-built tree's links
-int set_tree_adopt(grav_plan *pl, int64_t *cell_first, int32_t *cell_count, int32_t *cell_child,
-                   int32_t *cell_nchild, const int32_t *cell_level, cudaMemPool_t pool);
+int set_tree_adopt(grav_plan *pl, const DevTree &T, cudaMemPool_t pool);
 
 namespace {
 // The device build and the plan that adopts it; buffers from the device's
@@ -2100,25 +2119,19 @@ int build_plan(const nln_params *params, const float4 *bodies, int64_t n, double
     hp.ewald = params->box > 0 && ewald;
     hp.cptr = T.ptr_h[3].data();
     hp.clist = T.list[3];
-    // the tree's links (for the device refit and the adjoint) stay on the
-    // device: the plan's step state adopts them
-    int64_t *cfirst = T.cell_first;
-    int32_t *ccount = T.cell_count, *cchild = T.cell_child, *cnchild = T.cell_nchild,
-            *clevel = T.cell_level;
-    T.cell_first = nullptr;
-    T.cell_count = T.cell_child = T.cell_nchild = T.cell_level = nullptr;
     grav_plan *pl = nullptr;
     if (int rc = upload_impl(&hp, tuning, &pl, 0, &T)) {
-        for (void *q : {(void *)cfirst, (void *)ccount, (void *)cchild, (void *)cnchild,
-                        (void *)clevel})
+        // upload_impl took the tree's buffers over and released them, but for its links
+        for (void *q : {(void *)T.cell_first, (void *)T.cell_count, (void *)T.cell_child,
+                        (void *)T.cell_nchild})
             cudaFreeAsync(q, 0);
-        return rc;  // upload_impl took the tree's other buffers over and released them
+        return rc;
     }
-    const int rc_links = set_tree_adopt(pl, cfirst, ccount, cchild, cnchild, clevel, pool);
-    cudaFreeAsync(clevel, 0);
-    if (rc_links) {
+    // the tree's links (for the device refit and the adjoint) stay on the
+    // device: the plan's step state adopts them
+    if (int rc = set_tree_adopt(pl, T, pool)) {
         grav_plan_free(pl);
-        return rc_links;
+        return rc;
     }
     t_build = now_s() - t0;
     for (int k = 0; k < 6; k++) t_build_phase[k] = T.seconds[k];

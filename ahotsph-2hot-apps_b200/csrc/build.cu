@@ -254,6 +254,15 @@ __global__ void k_split_write(Cells C, int64_t lo, int64_t nf, const int64_t *__
 // (K = NLN_NMOM, + 1 max): raw moments about the centre of mass.  Level 0:
 // one thread per block of 64 bodies of a cell; level 1: per block of 64
 // level-0 partials; level 2: per cell, its level-1 partials in order.
+__global__ void k_sum_blocks(const Cells C, int64_t ncells, int64_t *b0, int64_t *b1) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c > ncells)
+        return;
+    const int64_t n = c < ncells ? (C.count[c] + kSumBlock - 1) / kSumBlock : 0;
+    b0[c] = n;
+    b1[c] = (n + kSumBlock - 1) / kSumBlock;
+}
+
 template <int K>
 __device__ inline void body_terms(const float *spos, const float *smass, int64_t b,
                                   const double *ctr, double *a, double &mx) {
@@ -813,7 +822,7 @@ int exclusive_scan(Bufs &B, const T *in, T *out, int64_t n, cudaStream_t st) {
 void dev_tree_free(DevTree &t, cudaMemPool_t pool) {
     void *ps[] = {t.points, t.qcells, t.hcells, t.groups, t.list[0], t.list[1], t.list[2],
                   t.list[3], t.order, t.cell_first, t.cell_count, t.cell_child, t.cell_nchild,
-                  t.cell_level};
+                  t.ptr[0], t.ptr[1], t.ptr[2], t.ptr[3]};
     for (void *p : ps)
         if (p) {
             if (pool)
@@ -942,6 +951,7 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     }
     int64_t lo = 0, hi = 1;
     while (hi > lo) {
+        out.level_start.push_back(lo);
         const int64_t nf = hi - lo;
         int64_t *nk = nullptr, *bounds = nullptr, *off = nullptr;
         BC(B.get(&nk, nf));
@@ -985,6 +995,7 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
         hi += total;
     }
     const int64_t nc = hi;
+    out.level_start.push_back(nc);
     if (n + nc + 1 >= (int64_t)NLN_IDX_MASK)
         return gc::set_status(-1, "GPU tree build: bodies plus cells exceed 27-bit list indices");
     out.n = n;
@@ -995,23 +1006,21 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     t0 = now_s();
 
     // ---- moments: block offsets of the canonical sums
-    int64_t *o0 = nullptr, *o1 = nullptr, *nb = nullptr;
+    int64_t *o0 = nullptr, *o1 = nullptr, *nb = nullptr, *nb1 = nullptr;
     BC(B.get(&o0, nc + 1));
     BC(B.get(&o1, nc + 1));
     BC(B.get(&nb, nc + 1));
-    std::vector<int32_t> hcount(nc);
-    BC(cudaMemcpyAsync(hcount.data(), C.count, nc * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    BC(B.get(&nb1, nc + 1));
+    k_sum_blocks<<<grid_of(nc + 1), kThreads, 0, st>>>(C, nc, nb, nb1);
+    BC(cudaGetLastError());
+    if (int rc = exclusive_scan(B, nb, o0, nc + 1, st))
+        return rc;
+    if (int rc = exclusive_scan(B, nb1, o1, nc + 1, st))
+        return rc;
+    int64_t B0 = 0, B1 = 0;
+    BC(cudaMemcpyAsync(&B0, o0 + nc, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    BC(cudaMemcpyAsync(&B1, o1 + nc, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     BC(cudaStreamSynchronize(st));
-    std::vector<int64_t> ho0(nc + 1), ho1(nc + 1);
-    ho0[0] = ho1[0] = 0;
-    for (int64_t c = 0; c < nc; c++) {
-        const int64_t b0 = (hcount[c] + kSumBlock - 1) / kSumBlock;
-        ho0[c + 1] = ho0[c] + b0;
-        ho1[c + 1] = ho1[c] + (b0 + kSumBlock - 1) / kSumBlock;
-    }
-    BC(cudaMemcpyAsync(o0, ho0.data(), (nc + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    BC(cudaMemcpyAsync(o1, ho1.data(), (nc + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    const int64_t B0 = ho0[nc], B1 = ho1[nc];
     double *cen = nullptr, *mass = nullptr, *p0 = nullptr, *p1 = nullptr;
     BC(B.get(&cen, 3 * nc));
     BC(B.get(&mass, nc));
@@ -1063,6 +1072,7 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     B.drop(o0);
     B.drop(o1);
     B.drop(nb);
+    B.drop(nb1);
     out.seconds[2] = now_s() - t0;
     t0 = now_s();
 
@@ -1205,15 +1215,166 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
         return gc::set_status(-1, "GPU tree build: the filling walk differs from the counting "
                                   "walk (0x%x)", hbad);
     out.seconds[4] = t_count + (now_s() - t0);
-    // ---- the tree links, handed on
+    // ---- the tree links and list offsets, handed on
     out.cell_first = C.first;
     out.cell_count = C.count;
     out.cell_child = C.child;
     out.cell_nchild = C.nchild;
-    out.cell_level = C.level;
+    for (int k = 0; k < 4; k++) out.ptr[k] = dptr[k];
     void *keep[] = {out.points, out.qcells, out.hcells, out.groups, out.list[0], out.list[1],
                     out.list[2], out.list[3], out.order, C.first, C.count, C.child, C.nchild,
-                    C.level};
+                    dptr[0], dptr[1], dptr[2], dptr[3]};
     for (void *q : keep) B.release(q);
+    return 0;
+}
+
+// ------------------------------------------------------------ work queue
+namespace {
+
+struct QueueIn {
+    const int64_t *ptr[3];
+    int64_t chunk[3];
+};
+
+// Per group: full chunks of each kind (nfull[k (ng + 1) + g]), the length of
+// its remainder (0: none) with the group itself for the sort, and all its
+// items (its slots).
+__global__ void k_queue_count(QueueIn Q, int64_t ng, int64_t *nfull, uint32_t *rem, int32_t *gid,
+                              int64_t *nall) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g > ng)
+        return;
+    int64_t all = 0;
+    for (int k = 0; k < 3; k++) {
+        const int64_t len = g < ng && Q.ptr[k] ? Q.ptr[k][g + 1] - Q.ptr[k][g] : 0;
+        const int64_t f = len / Q.chunk[k], r = len % Q.chunk[k];
+        nfull[k * (ng + 1) + g] = f;
+        all += f + (r ? 1 : 0);
+        if (g < ng) {
+            rem[k * ng + g] = (uint32_t)r;
+            gid[k * ng + g] = (int32_t)g;
+        }
+    }
+    nall[g] = all;
+}
+
+// Group g's first slot of kind k: after its items of the kinds before.
+__device__ inline int64_t kind_slot(const QueueIn &Q, int64_t g, int k, const int64_t *gslot) {
+    int64_t s = gslot[g];
+    for (int j = 0; j < k; j++)
+        if (Q.ptr[j])
+            s += (Q.ptr[j][g + 1] - Q.ptr[j][g] + Q.chunk[j] - 1) / Q.chunk[j];
+    return s;
+}
+
+// Remainders per kind, one atomic per warp.
+__global__ void k_queue_nrem(const uint32_t *__restrict__ rem, int64_t ng, unsigned long long *n) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int k = 0; k < 3; k++) {
+        const unsigned m = __ballot_sync(0xffffffffu, g < ng && rem[k * ng + g] != 0);
+        if ((threadIdx.x & 31) == 0 && m)
+            atomicAdd(&n[k], (unsigned long long)__popc(m));
+    }
+}
+
+__global__ void k_queue_full(QueueIn Q, int k, int64_t ng, const int64_t *__restrict__ off,
+                             const int64_t *__restrict__ gslot, Item *items) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= ng)
+        return;
+    const int64_t b = Q.ptr[k][g];
+    int64_t slot = kind_slot(Q, g, k, gslot);
+    Item *out = items + off[g];
+    for (int64_t j = 0; j < off[g + 1] - off[g]; j++)
+        out[j] = Item{(int32_t)g, (int32_t)slot++, b + j * Q.chunk[k], b + (j + 1) * Q.chunk[k]};
+}
+
+__global__ void k_queue_rem(QueueIn Q, int k, int64_t nrem, const int32_t *__restrict__ gid,
+                            const int64_t *__restrict__ gslot, Item *items) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nrem)
+        return;
+    const int32_t g = gid[i];
+    const int64_t b = Q.ptr[k][g], e = Q.ptr[k][g + 1], f = (e - b) / Q.chunk[k];
+    items[i] = Item{g, (int32_t)(kind_slot(Q, g, k, gslot) + f), b + f * Q.chunk[k], e};
+}
+
+}  // namespace
+
+int gpu_make_queue(const int64_t *const ptr[3], int64_t ng, const int64_t chunk[3], cudaStream_t st,
+                   cudaMemPool_t pool, Item *items[3], int nitems[3], int64_t **gslot,
+                   int64_t *nslots) {
+    Bufs B;
+    B.pool = pool;
+    B.st = st;
+    QueueIn Q;
+    int64_t most = 1;
+    for (int k = 0; k < 3; k++) {
+        Q.ptr[k] = ptr[k];
+        Q.chunk[k] = chunk[k];
+        most = std::max(most, chunk[k]);
+        items[k] = nullptr;
+        nitems[k] = 0;
+    }
+    int64_t *nfull = nullptr, *off = nullptr, *nall = nullptr, *slots = nullptr;
+    uint32_t *rem = nullptr, *rem_s = nullptr;
+    int32_t *gid = nullptr, *gid_s = nullptr;
+    BC(B.get(&nfull, 3 * (ng + 1)));
+    BC(B.get(&off, 3 * (ng + 1)));
+    BC(B.get(&nall, ng + 1));
+    BC(B.get(&slots, ng + 1));
+    BC(B.get(&rem, 3 * ng));
+    BC(B.get(&rem_s, 3 * ng));
+    BC(B.get(&gid, 3 * ng));
+    BC(B.get(&gid_s, 3 * ng));
+    k_queue_count<<<grid_of(ng + 1), kThreads, 0, st>>>(Q, ng, nfull, rem, gid, nall);
+    BC(cudaGetLastError());
+    if (int rc = exclusive_scan(B, nall, slots, ng + 1, st))
+        return rc;
+    int bits = 1;
+    while (bits < 32 && (int64_t)1 << bits < most) bits++;
+    int64_t tot[4] = {0, 0, 0, 0};
+    for (int k = 0; k < 3; k++) {
+        if (!ptr[k])
+            continue;
+        if (int rc = exclusive_scan(B, nfull + k * (ng + 1), off + k * (ng + 1), ng + 1, st))
+            return rc;
+        size_t bytes = 0;
+        BC(cub::DeviceRadixSort::SortPairsDescending(nullptr, bytes, rem + k * ng, rem_s + k * ng,
+                                                     gid + k * ng, gid_s + k * ng, (int)ng, 0, bits, st));
+        unsigned char *tmp = nullptr;
+        BC(B.get(&tmp, bytes));
+        BC(cub::DeviceRadixSort::SortPairsDescending(tmp, bytes, rem + k * ng, rem_s + k * ng,
+                                                     gid + k * ng, gid_s + k * ng, (int)ng, 0, bits, st));
+        B.drop(tmp);
+        BC(cudaMemcpyAsync(&tot[k], off + k * (ng + 1) + ng, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    }
+    BC(cudaMemcpyAsync(&tot[3], slots + ng, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    int64_t *nrem_d = nullptr;  // remainders per kind
+    BC(B.get(&nrem_d, 3));
+    BC(cudaMemsetAsync(nrem_d, 0, 3 * sizeof(int64_t), st));
+    k_queue_nrem<<<grid_of(ng), kThreads, 0, st>>>(rem, ng, reinterpret_cast<unsigned long long *>(nrem_d));
+    BC(cudaGetLastError());
+    int64_t nrem[3];
+    BC(cudaMemcpyAsync(nrem, nrem_d, sizeof(nrem), cudaMemcpyDeviceToHost, st));
+    BC(cudaStreamSynchronize(st));
+    for (int k = 0; k < 3; k++) {
+        if (!ptr[k] || tot[k] + nrem[k] == 0)
+            continue;
+        BC(B.get(&items[k], tot[k] + nrem[k]));
+        nitems[k] = (int)(tot[k] + nrem[k]);
+        k_queue_full<<<grid_of(ng), kThreads, 0, st>>>(Q, k, ng, off + k * (ng + 1), slots, items[k]);
+        BC(cudaGetLastError());
+        if (nrem[k] > 0) {
+            k_queue_rem<<<grid_of(nrem[k]), kThreads, 0, st>>>(Q, k, nrem[k], gid_s + k * ng, slots,
+                                                                items[k] + tot[k]);
+            BC(cudaGetLastError());
+        }
+    }
+    BC(cudaStreamSynchronize(st));
+    *gslot = slots;
+    *nslots = tot[3];
+    for (int k = 0; k < 3; k++) B.release(items[k]);
+    B.release(slots);
     return 0;
 }

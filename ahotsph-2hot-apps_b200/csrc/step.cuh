@@ -45,7 +45,7 @@ __global__ void k_refit_level(const float4 *__restrict__ pts, const int64_t *__r
     const int64_t i = lo + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= hi)
         return;
-    const int32_t c = order[i];
+    const int32_t c = order ? order[i] : (int32_t)i;
     double R[kRaw];
 #pragma unroll
     for (int q = 0; q < kRaw; q++) R[q] = 0.0;
@@ -316,7 +316,9 @@ struct grav_step_state {
     int64_t ncells = 0;
     int64_t *cfirst = nullptr;
     int32_t *ccount = nullptr, *cchild = nullptr, *cnchild = nullptr, *order = nullptr;
-    std::vector<int64_t> level_ptr;  // host: cells of depth level, deepest first, in `order`
+    // cells of each depth, deepest first: ranges of `order`, or of the cells
+    // themselves where that is null
+    std::vector<std::pair<int64_t, int64_t>> levels;
     double *raw = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -344,9 +346,8 @@ namespace {
 
 int refit_enqueue(grav_plan *pl, cudaStream_t st) {
     grav_step_state *S = pl->step;
-    const int64_t nl = (int64_t)S->level_ptr.size() - 1;
-    for (int64_t l = 0; l < nl; l++) {
-        const int64_t lo = S->level_ptr[l], hi = S->level_ptr[l + 1];
+    for (const auto &level : S->levels) {
+        const int64_t lo = level.first, hi = level.second;
         if (hi <= lo)
             continue;
         k_refit_level<<<(unsigned)((hi - lo + 127) / 128), 128, 0, st>>>(
@@ -403,50 +404,25 @@ void step_graph_reset(grav_step_state *S) {
 // the deepest-first order is those ranges in reverse; only the depths are
 // read back, to find the ranges.  The adopted arrays belong to the plan
 // from here on, also when this fails.
-int set_tree_adopt(grav_plan *pl, int64_t *cell_first, int32_t *cell_count, int32_t *cell_child,
-                   int32_t *cell_nchild, const int32_t *cell_level, cudaMemPool_t pool) {
+int set_tree_adopt(grav_plan *pl, const DevTree &T, cudaMemPool_t pool) {
     const int64_t nc = pl->hp.ncells;
     auto *S = new grav_step_state();
     S->pool = pool;
     S->ncells = nc;
-    S->cfirst = cell_first;
-    S->ccount = cell_count;
-    S->cchild = cell_child;
-    S->cnchild = cell_nchild;
-    std::vector<int32_t> level((size_t)std::max<int64_t>(nc, 1));
-    cudaError_t e = nc > 0 ? cudaMemcpy(level.data(), cell_level, nc * sizeof(int32_t),
-                                        cudaMemcpyDeviceToHost)
-                           : cudaSuccess;
-    if (e != cudaSuccess || nc <= 0) {
+    S->cfirst = T.cell_first;
+    S->ccount = T.cell_count;
+    S->cchild = T.cell_child;
+    S->cnchild = T.cell_nchild;
+    if (nc <= 0) {
         delete S;
-        return e != cudaSuccess ? gc::cuda_status(e, "grav_plan_build_CUDA: tree depths")
-                                : gc::set_status(-1, "grav_plan_build_CUDA: the plan has no cells");
+        return gc::set_status(-1, "grav_plan_build_CUDA: the plan has no cells");
     }
-    std::vector<int64_t> start;  // start[l]: first cell of depth l
-    for (int64_t c = 0; c < nc; c++) {
-        if (level[c] < 0 || (c > 0 && level[c] < level[c - 1]) || level[c] > (int32_t)start.size()) {
-            delete S;
-            return gc::set_status(-1, "grav_plan_build_CUDA: cells not in depth order at %lld",
-                                  (long long)c);
-        }
-        if (level[c] == (int32_t)start.size())
-            start.push_back(c);
-    }
-    start.push_back(nc);
-    std::vector<int32_t> order;
-    order.reserve(nc);
-    S->level_ptr.assign(1, 0);
-    for (int64_t l = (int64_t)start.size() - 2; l >= 0; l--) {
-        for (int64_t c = start[l]; c < start[l + 1]; c++) order.push_back((int32_t)c);
-        S->level_ptr.push_back((int64_t)order.size());
-    }
-    e = cudaMallocFromPoolAsync((void **)&S->order, nc * sizeof(int32_t), pool, 0);
+    // the builder makes cells level by level: no order array is needed
+    for (size_t l = T.level_start.size() - 1; l-- > 0;)
+        S->levels.push_back({T.level_start[l], T.level_start[l + 1]});
+    cudaError_t e = cudaMallocFromPoolAsync((void **)&S->raw, (size_t)nc * kRaw * sizeof(double), pool, 0);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(S->order, order.data(), nc * sizeof(int32_t), cudaMemcpyHostToDevice, 0);
-    if (e == cudaSuccess)
-        e = cudaMallocFromPoolAsync((void **)&S->raw, (size_t)nc * kRaw * sizeof(double), pool, 0);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(0);  // `order` is read before the host vector goes
+        e = cudaStreamSynchronize(0);  // other streams use it
     if (e != cudaSuccess) {
         delete S;
         return gc::cuda_status(e, "grav_plan_build_CUDA: tree links");
@@ -485,13 +461,12 @@ extern "C" int grav_plan_set_tree_CUDA(grav_plan *pl, const int64_t *cell_first,
     order.reserve(nc);
     auto *S = new grav_step_state();
     S->ncells = nc;
-    S->level_ptr.assign(1, 0);
     {
         std::vector<std::vector<int32_t>> by(maxl + 1);
         for (int64_t c = 0; c < nc; c++) by[cell_level[c]].push_back((int32_t)c);
         for (int l = maxl; l >= 0; l--) {
+            S->levels.push_back({(int64_t)order.size(), (int64_t)(order.size() + by[l].size())});
             order.insert(order.end(), by[l].begin(), by[l].end());
-            S->level_ptr.push_back((int64_t)order.size());
         }
     }
     cudaError_t e = cudaSuccess;
