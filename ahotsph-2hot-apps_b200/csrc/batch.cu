@@ -469,6 +469,7 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
     using K = CellKind<KIND>;
     constexpr int NP = K::pairs, NE = 2 * NP, CT = kTile[KIND];
     extern __shared__ __align__(1024) unsigned char smem[];
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     unsigned char *stage = smem + (size_t)(threadIdx.x >> 5) * K::warp_bytes;
     SinkTable &sinks = *reinterpret_cast<SinkTable *>(stage + K::stage_bytes);
@@ -551,8 +552,10 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
         for (int t = 0; t < ntile; t++) {
             const int nt = (int)min((int64_t)CT, nent - (int64_t)t * CT);
             const bool ok = mbar_wait_bounded(bar, phase, P.err);
-            if (!__all_sync(0xffffffffu, ok))
+            if (!__all_sync(0xffffffffu, ok)) {
+                pdl_wait();
                 return;  // a lost copy: the error word is set, nothing else is in flight
+            }
             phase ^= 1;
             typename K::Pair rec[NP];
 #pragma unroll
@@ -588,6 +591,7 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
         }
         store_part(P, item, lane, hi, lo);
     }
+    pdl_wait();
 }
 
 // Point lists (bodies and cell monopoles): tiles of 256 records, eight per
@@ -604,6 +608,7 @@ constexpr int kPointWarpBytes = (int)(sizeof(PointStage) + sizeof(SinkTable) + s
 template <bool PLAIN>
 __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProblem P) {
     extern __shared__ __align__(16) unsigned char psm[];
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     PointStage &stage = *reinterpret_cast<PointStage *>(psm + (size_t)(threadIdx.x >> 5) * kPointWarpBytes);
     SinkTable &sinks = *reinterpret_cast<SinkTable *>(&stage + 1);
@@ -716,6 +721,7 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
         }
         store_part(P, item, lane, hi, lo);
     }
+    pdl_wait();
 }
 
 // Periodic correction moments (ewald.cuh) of groups gbegin..ngroups-1, one
@@ -804,6 +810,7 @@ constexpr int kEwWarpBytes = 2 * (int)sizeof(EwStage);  // 16 KB
 
 __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
     extern __shared__ __align__(16) unsigned char ewsm[];
+    pdl_trigger();
     const int lane = threadIdx.x & 31;
     EwStage *stg = reinterpret_cast<EwStage *>(ewsm + (size_t)(threadIdx.x >> 5) * kEwWarpBytes);
     const uint32_t ntab = (uint32_t)P.ntab[0];
@@ -927,6 +934,7 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
         M.warp_sum();
         ew_store(P, it, U.g, lane, M);
     }
+    pdl_wait();
 }
 
 // The same moments by a plain loop over the list, every load on demand: no
@@ -989,6 +997,7 @@ __global__ void __launch_bounds__(64) k_ewald_side(DevProblem P) {
 // Per group, in slot order: sum the partials of its work items in FP64,
 // add the periodic correction, and write (ax, ay, az, phi) of each sink.
 __global__ void k_finish(DevProblem P) {
+    pdl_wait();
     const int64_t g = P.gbegin + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (g >= P.ngroups)
@@ -1789,8 +1798,30 @@ extern "C" int grav_groups_upload_CUDA(const grav_problem *hp, const grav_tuning
 }
 
 namespace {
+// The kernels of one evaluation do not read one another's results, but for
+// the finish pass: with `after` a kernel may start as soon as every block of
+// the one before it on the stream has, and fill the SMs that one's last wave
+// leaves (2,000 bodies: 26.5 -> 16.5 us an evaluation).  Each waits for its
+// predecessor before it ends, so the last one's end is the end of all.
+int launch_after(const void *kern, unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
+                 bool after, void **args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = after ? 1 : 0;
+    GC_CHECK(cudaLaunchKernelExC(&cfg, kern, args));
+    return 0;
+}
+
+// `after`: see launch_after; set once a kernel has been launched.
 template <int KIND>
-int launch_kind(grav_plan *pl, const DevProblem &dp, cudaStream_t st) {
+int launch_kind(grav_plan *pl, const DevProblem &dp, cudaStream_t st, bool *after = nullptr) {
     if (dp.nitems[KIND] == 0)
         return 0;
     const int wpb = std::min(pl->tune.warps_per_block, kListWarps);
@@ -1811,7 +1842,10 @@ int launch_kind(grav_plan *pl, const DevProblem &dp, cudaStream_t st) {
     CUtensorMap tm = pl->tmap[KIND];
     DevProblem d = dp;
     void *pargs[] = {&d}, *cargs[] = {&tm, &d};
-    GC_CHECK(cudaLaunchKernel(kern, dim3(blocks), dim3(wpb * 32), KIND == KP ? pargs : cargs, smem, st));
+    if (int rc = launch_after(kern, blocks, wpb * 32, smem, st, after && *after, KIND == KP ? pargs : cargs))
+        return rc;
+    if (after)
+        *after = true;
     pl->launches++;
     return 0;
 }
@@ -1819,7 +1853,8 @@ int launch_kind(grav_plan *pl, const DevProblem &dp, cudaStream_t st) {
 // k_ewald_moments: `warps` warps per block, blocks_per_sm x SM count blocks
 // (0: as many as fit), at most one warp per unit; over dp's groups, on
 // stream s.
-int launch_moments(grav_plan *pl, const DevProblem &dp, cudaStream_t s, int per_sm, int warps) {
+int launch_moments(grav_plan *pl, const DevProblem &dp, cudaStream_t s, int per_sm, int warps,
+                   bool after) {
     const int64_t n = (dp.ngroups - dp.gbegin) * dp.ewsplit;
     if (n <= 0)
         return 0;
@@ -1836,8 +1871,9 @@ int launch_moments(grav_plan *pl, const DevProblem &dp, cudaStream_t s, int per_
     d.ewm = pl->ewm;
     const unsigned blocks = (unsigned)std::max<int64_t>(
         1, std::min<int64_t>((n + warps - 1) / warps, (int64_t)per_sm * pl->nsm));
-    k_ewald_moments<<<blocks, warps * 32, smem, s>>>(d);
-    GC_CHECK(cudaGetLastError());
+    void *args[] = {&d};
+    if (int rc = launch_after((const void *)k_ewald_moments, blocks, warps * 32, smem, s, after, args))
+        return rc;
     pl->launches++;
     return 0;
 }
@@ -1895,16 +1931,20 @@ int side_join(grav_plan *pl, cudaStream_t st) {
 
 // The finish pass, after the correction moments when they did not run on
 // the side stream (forked).
-int launch_finish(grav_plan *pl, const DevProblem &dp, cudaStream_t st, bool forked) {
+int launch_finish(grav_plan *pl, const DevProblem &dp, cudaStream_t st, bool forked,
+                  bool after = false) {
     if (dp.ewald && !forked)
-        if (int rc = launch_moments(pl, dp, st, 0, main_moments_warps(pl)))
+        if (int rc = launch_moments(pl, dp, st, 0, main_moments_warps(pl), after))
             return rc;
     const int wpb = 2;
     const int64_t n = dp.ngroups - dp.gbegin;
     if (n <= 0)
         return 0;
-    k_finish<<<(unsigned)((n + wpb - 1) / wpb), wpb * 32, 0, st>>>(dp);
-    GC_CHECK(cudaGetLastError());
+    DevProblem d = dp;
+    void *args[] = {&d};
+    if (int rc = launch_after((const void *)k_finish, (unsigned)((n + wpb - 1) / wpb), wpb * 32, 0, st,
+                              after && !forked, args))
+        return rc;
     pl->launches++;
     return 0;
 }
@@ -1923,18 +1963,19 @@ extern "C" int grav_groups_eval_CUDA(grav_plan *pl, void *stream) {
     GC_CHECK(cudaMemsetAsync(pl->dp.counters, 0, 4 * sizeof(int), st));
     if (int rc = mark(0))
         return rc;
-    bool forked = false;
+    bool forked = false, after = false;
+    bool *chain = pl->timing ? nullptr : &after;  // events between them time whole kernels
     if (int rc = side_fork(pl, pl->dp, st, forked))
         return rc;
-    if (int rc = launch_kind<KH>(pl, pl->dp, st))
+    if (int rc = launch_kind<KH>(pl, pl->dp, st, chain))
         return rc;
     if (int rc = mark(1))
         return rc;
-    if (int rc = launch_kind<KQ>(pl, pl->dp, st))
+    if (int rc = launch_kind<KQ>(pl, pl->dp, st, chain))
         return rc;
     if (int rc = mark(2))
         return rc;
-    if (int rc = launch_kind<KP>(pl, pl->dp, st))
+    if (int rc = launch_kind<KP>(pl, pl->dp, st, chain))
         return rc;
     if (int rc = mark(3))
         return rc;
@@ -1943,7 +1984,7 @@ extern "C" int grav_groups_eval_CUDA(grav_plan *pl, void *stream) {
     if (forked)
         if (int rc = side_join(pl, st))
             return rc;
-    if (int rc = launch_finish(pl, df, st, forked))
+    if (int rc = launch_finish(pl, df, st, forked, after))
         return rc;
     pl->evaluated = true;
     return mark(4);

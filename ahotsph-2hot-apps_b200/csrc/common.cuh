@@ -124,6 +124,15 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Programmatic dependent launch: let the kernel after this one on the stream
+// start (its blocks take the room this one leaves), and wait for the kernel
+// before it to be complete and its writes visible.  Both do nothing in a
+// kernel launched without the attribute.
+__device__ __forceinline__ void pdl_trigger() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Single MUFU reciprocal square root (approximate, flush-to-zero); the
 // reference uses an 11-bit rsqrtps refined by one Newton step
 // (nln/do_grav_avx8.c:2188-2201), which this matches in accuracy.
