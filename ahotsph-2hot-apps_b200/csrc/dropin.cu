@@ -124,7 +124,9 @@ __device__ void stage_aosoa(float *o, const float *raw, int sz, int s) {
 
 // Sinks [base_sink, base_sink+m) against list blocks [c0, c1) of f, c0/c1
 // from blockIdx.y.  Dynamic shared memory: 2 raw tiles + staged records + 2 mbarriers.
-template <int ORDER, int SOFT>
+// INPLACE: f is page-locked host memory, read by the threads as 16-byte words
+// (past the caches: the next call rewrites it), not a device copy staged by TMA.
+template <int ORDER, int SOFT, bool INPLACE>
 __global__ void __launch_bounds__(128) k_list(const float *__restrict__ pos, float4 *accp, int m,
                                               const float *__restrict__ f, int nblk, int sz,
                                               int blk_per_chunk, float e, float qsh,
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__(128) k_list(const float *__restrict__ pos, flo
     const int ntile = (c1 - c0 + TBLK - 1) / TBLK;
     const int tid = threadIdx.x;
 
-    if (tid == 0) {
+    if (!INPLACE && tid == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
         fence_mbar_init();
@@ -156,7 +158,13 @@ __global__ void __launch_bounds__(128) k_list(const float *__restrict__ pos, flo
         mbar_arrive_expect_tx(&bar[t & 1], bytes);
         tma_bulk_g2s(dst, f + (size_t)b0 * sz * 8, bytes, &bar[t & 1]);
     };
-    if (tid == 0 && ntile > 0)
+    auto fetch = [&](int t) {
+        const int b0 = c0 + t * TBLK;
+        const int n4 = min(TBLK, c1 - b0) * sz * 2;
+        const float4 *src = reinterpret_cast<const float4 *>(f + (size_t)b0 * sz * 8);
+        for (int i = tid; i < n4; i += blockDim.x) reinterpret_cast<float4 *>(raw0)[i] = __ldcv(src + i);
+    };
+    if (!INPLACE && tid == 0 && ntile > 0)
         issue(0);
 
     float sx[SPT], sy[SPT], sz_[SPT];
@@ -175,15 +183,20 @@ __global__ void __launch_bounds__(128) k_list(const float *__restrict__ pos, flo
     bool ok = true;
     int failed_at = -1;
     for (int t = 0; t < ntile; t++) {
-        if (tid == 0 && t + 1 < ntile)
-            issue(t + 1);
-        ok = mbar_wait_bounded(&bar[t & 1], (t >> 1) & 1, err);
-        if (!__syncthreads_and(ok)) {
-            ok = false;
-            failed_at = t;
-            break;
+        if (INPLACE) {
+            fetch(t);
+            __syncthreads();
+        } else {
+            if (tid == 0 && t + 1 < ntile)
+                issue(t + 1);
+            ok = mbar_wait_bounded(&bar[t & 1], (t >> 1) & 1, err);
+            if (!__syncthreads_and(ok)) {
+                ok = false;
+                failed_at = t;
+                break;
+            }
         }
-        const float *rt = (t & 1) ? raw1 : raw0;
+        const float *rt = !INPLACE && (t & 1) ? raw1 : raw0;
         const int nsrc = min(TBLK, c1 - (c0 + t * TBLK)) * 8;
         for (int s = tid; s < nsrc; s += blockDim.x) stage_aosoa<ORDER>(rec + s * REC, rt, sz, s);
         __syncthreads();
@@ -354,8 +367,9 @@ struct Slot {
     // 2 its copy to the device issued (copied[k] recorded)
     std::atomic<int> bstate[2] = {{0}, {0}};
     std::atomic<int> queued{0};  // jobs of this slot not yet issued
-    // recorded by the submitter after each launch; kpending = 1 until the
-    // submitter has seen it complete (then qallocCUDA needs no stream query)
+    // recorded by the submitter after each launch (an in-place one records
+    // copied[k] alone); kpending = 1, or 3 + k, until the submitter has seen it
+    // complete (then qallocCUDA needs no stream query)
     cudaEvent_t kdone = nullptr;
     std::atomic<int> kpending{0};
     int turn = 0;
@@ -384,8 +398,14 @@ struct State {
     float *Btab = nullptr;
     int bstride = 0;
     int64_t nobj = 0;
-    float *devpos = nullptr;     // 3 floats per sink
-    float4 *devaccp = nullptr;   // ax ay az phi per sink
+    // 3 floats and (ax, ay, az, phi) per sink: set while a sink table is
+    // registered; the buffers behind them are kept for the next walk until
+    // one needs larger ones or CUDA_Finalize
+    float *devpos = nullptr;
+    float4 *devaccp = nullptr;
+    float *pos_buf = nullptr;
+    float4 *acc_buf = nullptr;
+    int64_t sink_cap = 0;
     float *qdev = nullptr;       // cell table for pQQ1, 10 floats per cell
     int64_t ncells = 0;
     unsigned *derr = nullptr;    // device error word
@@ -654,7 +674,7 @@ int check_device_error(const char *what) {
     return 0;
 }
 
-template <int ORDER, int SOFT>
+template <int ORDER, int SOFT, bool INPLACE>
 int launch_list(cudaStream_t st, const float *pos, float4 *acc, int m, const float *f, int nblk,
                 int sz, float e, float qsh) {
     constexpr int REC = RecOf<ORDER>::v;
@@ -666,7 +686,7 @@ int launch_list(cudaStream_t st, const float *pos, float4 *acc, int m, const flo
     bpc = (bpc + TBLK - 1) / TBLK * TBLK;
     int gy = (nblk + bpc - 1) / bpc;
     size_t smem = (size_t)2 * TBLK * sz * 8 * 4 + (size_t)TSRC * REC * 4 + 16;
-    auto kern = k_list<ORDER, SOFT>;
+    auto kern = k_list<ORDER, SOFT, INPLACE>;
     // the largest dynamic shared memory set for this kernel so far (once per size)
     static int smem_set = 0;
     if ((int)smem > smem_set) {
@@ -691,10 +711,11 @@ const Routine kRoutines[] = {
 };
 
 int dispatch_list(const Routine &r, cudaStream_t st, const float *pos, float4 *acc, int m,
-                  const float *f, int nblk, int sz, float e) {
-#define GC_CASE(O, SO)                                                        \
-    if (r.order == O && r.soft == SO)                                         \
-        return launch_list<O, SO>(st, pos, acc, m, f, nblk, sz, e, r.qsh);
+                  const float *f, int nblk, int sz, float e, bool inplace) {
+#define GC_CASE(O, SO)                                                                    \
+    if (r.order == O && r.soft == SO)                                                     \
+        return inplace ? launch_list<O, SO, true>(st, pos, acc, m, f, nblk, sz, e, r.qsh) \
+                       : launch_list<O, SO, false>(st, pos, acc, m, f, nblk, sz, e, r.qsh);
     GC_CASE(0, SOFT_NONE)
     GC_CASE(2, SOFT_NONE)
     GC_CASE(4, SOFT_NONE)
@@ -706,6 +727,12 @@ int dispatch_list(const Routine &r, cudaStream_t st, const float *pos, float4 *a
 #undef GC_CASE
     return gc::set_status(-1, "no kernel for routine %s", r.name);
 }
+
+// Lists up to this size are read by the kernels from page-locked memory (-D
+// to rebuild with another).
+#ifndef GRAV_INPLACE_BYTES
+#define GRAV_INPLACE_BYTES (128 << 10)
+#endif
 
 // ---- deferred issue: the submitter thread ----
 // grav_mn_CUDA copies its list into a slot's staging buffer and queues a
@@ -740,9 +767,9 @@ struct Submitter {
     void poll_slots() {
         for (int q = 0; q < NQ; q++) {
             Slot &s = S.q[q];
-            if (s.kpending.load(std::memory_order_acquire) == 1 &&
-                s.queued.load(std::memory_order_acquire) == 0 &&
-                cudaEventQuery(s.kdone) == cudaSuccess)
+            const int kp = s.kpending.load(std::memory_order_acquire);
+            if ((kp == 1 || kp >= 3) && s.queued.load(std::memory_order_acquire) == 0 &&
+                cudaEventQuery(kp == 1 ? s.kdone : s.copied[kp - 3]) == cudaSuccess)
                 s.kpending.store(0, std::memory_order_release);
         }
     }
@@ -765,19 +792,32 @@ struct Submitter {
     void issue(const Job &j) {
         const int64_t t0 = now_ns();
         Slot &s = S.q[j.q];
-        cudaError_t e = cudaMemcpyAsync(s.dev, s.hbuf[j.turn], j.bytes, cudaMemcpyHostToDevice,
-                                        s.stream);
-        if (e == cudaSuccess)
-            e = cudaEventRecord(s.copied[j.turn], s.stream);
-        s.bstate[j.turn].store(2, std::memory_order_release);
-        if (issued_head - issued_tail < (uint64_t)kCap)
-            issued[issued_head++ % kCap] = {j.q, j.turn};
+        // A short list whose sinks fill one column of blocks is read where it
+        // lies: the copy to the device and its event cost the submitter more
+        // than the kernel's reads over the bus (8k-body sphere, lists of 58 and
+        // 3 KB, a pass: 9.5 ms copied, 7.1 in place; 4 MB as the limit 7.0, and
+        // 64k bodies 41 ms against 40).
+        const bool inplace = j.bytes <= (size_t)GRAV_INPLACE_BYTES && j.n <= 128 * SPT;
+        cudaError_t e = cudaSuccess;
+        if (!inplace) {
+            e = cudaMemcpyAsync(s.dev, s.hbuf[j.turn], j.bytes, cudaMemcpyHostToDevice, s.stream);
+            if (e == cudaSuccess)
+                e = cudaEventRecord(s.copied[j.turn], s.stream);
+        }
         int rc = e == cudaSuccess ? 0 : gc::cuda_status(e, "grav_mn_CUDA: list copy");
         if (!rc)
             rc = dispatch_list(*j.r, s.stream, S.devpos + 3 * j.first, S.devaccp + j.first, j.n,
-                               (const float *)s.dev, j.nblk, j.sz, j.e);
-        if (!rc && cudaEventRecord(s.kdone, s.stream) == cudaSuccess)
+                               (const float *)(inplace ? s.hbuf[j.turn] : s.dev), j.nblk, j.sz, j.e,
+                               inplace);
+        if (inplace) {  // read by the kernel: its end frees the staging buffer and the slot
+            if (cudaEventRecord(s.copied[j.turn], s.stream) == cudaSuccess && !rc)
+                s.kpending.store(3 + j.turn, std::memory_order_release);
+        } else if (!rc && cudaEventRecord(s.kdone, s.stream) == cudaSuccess) {
             s.kpending.store(1, std::memory_order_release);
+        }
+        s.bstate[j.turn].store(2, std::memory_order_release);
+        if (issued_head - issued_tail < (uint64_t)kCap)
+            issued[issued_head++ % kCap] = {j.q, j.turn};
         if (rc) {
             int zero = 0;
             err.compare_exchange_strong(zero, rc);
@@ -912,8 +952,8 @@ extern "C" void CUDA_Init(void *device_prop) {
     (void)device_prop;
     if (ensure_init())
         return;
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, 0) == cudaSuccess && getenv("GRAVCUDA_VERBOSE"))
+    cudaDeviceProp prop;  // takes about 2 ms to read: only to be shown
+    if (getenv("GRAVCUDA_VERBOSE") && cudaGetDeviceProperties(&prop, 0) == cudaSuccess)
         fprintf(stderr, "CUDA_Init: %s, sm_%d%d, %d SMs, %.1f GB\n", prop.name, prop.major,
                 prop.minor, prop.multiProcessorCount, prop.totalGlobalMem / 1e9);
 }
@@ -942,8 +982,11 @@ extern "C" void CUDA_Finalize(void) {
             cudaFree(s.dev);
         s.reset();
     }
-    cudaFree(S.devpos);
-    cudaFree(S.devaccp);
+    cudaFree(S.pos_buf);
+    cudaFree(S.acc_buf);
+    S.pos_buf = nullptr;
+    S.acc_buf = nullptr;
+    S.sink_cap = 0;
     cudaFree(S.qdev);
     cudaFree(S.derr);
     S.init = false;
@@ -1053,20 +1096,32 @@ extern "C" void WalkInitSinkCUDA(float *btab, int stride, int64_t nobj) {
         gc::set_status(-1, "WalkInitSinkCUDA: bad table");
         return;
     }
-    cudaFree(S.devpos);
-    cudaFree(S.devaccp);
     S.devpos = nullptr;
     S.devaccp = nullptr;
+    if (S.sink_cap < nobj) {
+        cudaFree(S.pos_buf);
+        cudaFree(S.acc_buf);
+        S.pos_buf = nullptr;
+        S.acc_buf = nullptr;
+        S.sink_cap = 0;
+        if (cudaMalloc(&S.pos_buf, (size_t)nobj * 3 * sizeof(float)) != cudaSuccess ||
+            cudaMalloc(&S.acc_buf, (size_t)nobj * sizeof(float4)) != cudaSuccess) {
+            gc::set_status(-1, "WalkInitSinkCUDA: device allocation failed");
+            return;
+        }
+        S.sink_cap = nobj;
+    }
     std::vector<float> h((size_t)nobj * 3);
     for (int64_t i = 0; i < nobj; i++)
         for (int d = 0; d < 3; d++) h[3 * i + d] = btab[(size_t)i * stride + 1 + d];
-    if (cudaMalloc(&S.devpos, h.size() * 4) != cudaSuccess ||
-        cudaMalloc(&S.devaccp, (size_t)nobj * sizeof(float4)) != cudaSuccess ||
-        cudaMemcpy(S.devpos, h.data(), h.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(S.devaccp, 0, (size_t)nobj * sizeof(float4)) != cudaSuccess) {
-        gc::set_status(-1, "WalkInitSinkCUDA: device allocation failed");
+    if (cudaMemcpy(S.pos_buf, h.data(), h.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemset(S.acc_buf, 0, (size_t)nobj * sizeof(float4)) != cudaSuccess ||
+        cudaStreamSynchronize(0) != cudaSuccess) {  // the slots' streams do not wait for this one
+        gc::set_status(-1, "WalkInitSinkCUDA: copying the sinks failed");
         return;
     }
+    S.devpos = S.pos_buf;
+    S.devaccp = S.acc_buf;
     S.Btab = btab;
     S.bstride = stride;
     S.nobj = nobj;
@@ -1109,8 +1164,6 @@ extern "C" void WalkTerminateSinkCUDA(float *btab, int stride, int64_t nobj) {
         return;
     for (int64_t i = 0; i < nobj; i++)
         for (int k = 0; k < 4; k++) btab[(size_t)i * stride + 7 + k] += h[4 * i + k];
-    cudaFree(S.devpos);
-    cudaFree(S.devaccp);
     S.devpos = nullptr;
     S.devaccp = nullptr;
     S.Btab = nullptr;
