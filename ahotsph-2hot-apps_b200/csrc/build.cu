@@ -598,9 +598,13 @@ __device__ __forceinline__ int64_t emit_runs(uint32_t *out, int64_t pos, int64_t
     return pos + total;
 }
 
-// Groups in the walk's order: first those whose radius is a sixteenth of the
-// cube or more (a sphere's sparse outskirts), which open most of the tree and
-// would end last alone, then the others, both as they lie in space.
+// The walk's units in order: first the groups whose radius is a sixteenth of
+// the cube or more (a sphere's sparse outskirts, any group of a small
+// problem), which open most of the tree and would end last alone: eight units
+// each, one per child of the root.  Then the others, a unit each.  Both as the
+// groups lie in space.
+constexpr int kWalkParts = 8;
+
 __global__ void k_wide_groups(const nln_group *__restrict__ groups, int64_t ng, double wide,
                               int64_t *flag) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -615,23 +619,29 @@ __global__ void k_walk_order(const nln_group *__restrict__ groups, int64_t ng, d
         order[groups[g].radius >= wide ? before[g] : before[ng] + g - before[g]] = (int32_t)g;
 }
 
-// FILL false: cnt[5 g ..] = point, quadrupole, order-4 and correction
-// entries, bodies among the points.  FILL true: the entries, at the offsets
-// pp, qp, hp, cp (ngroups + 1 each) of the four lists.
-template <bool FILL>
+// FILL false: cnt[6 g ..] = point, quadrupole, order-4 and correction
+// entries, bodies among the points, bodies covered; ucnt[5 u ..] the first five
+// of unit u of the wide groups.  FILL true: the entries, at the offsets pp, qp,
+// hp, cp (ngroups + 1 each) of the four lists.
+// PARTS: there are wide groups (nwide > 0); without them the kernel keeps to
+// fewer registers.
+template <bool FILL, bool PARTS>
 __global__ void __launch_bounds__(32 * kWalkWarps)
     k_walk(const nln_wcell *__restrict__ wc, const float *__restrict__ spos, int64_t n,
            const nln_group *__restrict__ groups, const int32_t *__restrict__ order, int64_t ng,
-           nln_mac P, int64_t *cnt, const int64_t *pp, const int64_t *qp, const int64_t *hp, const int64_t *cp,
+           int64_t nwide, nln_mac P, int64_t *cnt, int64_t *ucnt, const int64_t *pp, const int64_t *qp, const int64_t *hp, const int64_t *cp,
            uint32_t *pl, uint32_t *ql, uint32_t *hl, uint32_t *cl, unsigned *err) {
     __shared__ uint32_t s_item[kWalkWarps][kWalkStack];
     __shared__ uint8_t s_code[kWalkWarps][FILL ? kWalkStack : 1];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int64_t slot = (int64_t)blockIdx.x * kWalkWarps + wib;
+    const int64_t u = (int64_t)blockIdx.x * kWalkWarps + wib;
+    const bool parts = PARTS && u < kWalkParts * nwide;
+    const int64_t slot = parts ? u / kWalkParts : PARTS ? u - (kWalkParts - 1) * nwide : u;
     if (slot >= ng)
         return;
-    const int64_t g = order[slot];
+    const int part = (int)(u % kWalkParts);
+    const int64_t g = PARTS ? order[slot] : slot;
     uint32_t *item = s_item[wib];
     uint8_t *codes = s_code[wib];
     const nln_group G = groups[g];
@@ -644,10 +654,37 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
     if (FILL) {
         np = pp[g], nq = qp[g], nh = hp[g], nc = cp[g];
         ep = pp[g + 1], eq = qp[g + 1], eh = hp[g + 1], ec = cp[g + 1];
+        if (parts) {  // this part's range follows the parts before it
+            const int64_t *c = ucnt + 5 * (u - part);
+            for (int k = 0; k < part; k++)
+                np += c[5 * k], nq += c[5 * k + 1], nh += c[5 * k + 2], nc += c[5 * k + 3];
+        }
     }
     int sp = 1;
     if (lane == 0)
         item[0] = 0;
+    if (parts) {
+        // the root decides alike in every part: opened, part k walks its child
+        // k; else part 0 walks the root itself
+        const nln_wcell root = load_wcell(wc, 0);
+        const nln_visit v = nln_walk_cell(root, G, P, false);
+        if (v.what == NLN_OPEN) {
+            sp = part < root.nchild ? 1 : 0;
+            if (lane == 0)
+                item[0] = (uint32_t)(root.child + part) | (v.covers ? 1u << kWalkFlag : 0u);
+            if (v.covers && part == 0) {  // the root's own correction entry
+                if (FILL) {
+                    if (lane == 0 && nc < ec)
+                        cl[nc] = nb | v.sc << NLN_IDX_BITS;
+                    nc++;
+                } else if (lane == 0) {
+                    nc = 1;
+                }
+            }
+        } else if (part > 0) {
+            sp = 0;
+        }
+    }
     __syncwarp();
     bool overflow = false;
     while (sp > 0) {
@@ -785,7 +822,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
         __syncwarp();
     }
     covered = warp_sum(covered);
-    if ((overflow || covered != n) && lane == 0)
+    if ((overflow || (!parts && covered != n)) && lane == 0)
         atomicOr(err, 1u);
     if (!FILL) {
         np = warp_sum(np);
@@ -794,15 +831,27 @@ __global__ void __launch_bounds__(32 * kWalkWarps)
         nc = warp_sum(nc);
         nbod = warp_sum(nbod);
         if (lane == 0) {
-            cnt[5 * g] = np;
-            cnt[5 * g + 1] = nq;
-            cnt[5 * g + 2] = nh;
-            cnt[5 * g + 3] = nc;
-            cnt[5 * g + 4] = nbod;
+            const int64_t v[6] = {np, nq, nh, nc, nbod, covered};
+            for (int k = 0; k < 6; k++) {
+                if (!parts)
+                    cnt[6 * g + k] = v[k];
+                else
+                    atomicAdd(reinterpret_cast<unsigned long long *>(cnt + 6 * g + k),
+                              (unsigned long long)v[k]);
+                if (parts && k < 5)
+                    ucnt[5 * u + k] = v[k];
+            }
         }
-    } else if (lane == 0 && (np != ep || nq != eq || nh != eh || nc != ec)) {
+    } else if (lane == 0) {
         // the count pass sized every list: a walk that writes more or less is an error
-        atomicOr(err, 2u);
+        if (parts) {  // where the next part starts
+            const int64_t *c = ucnt + 5 * (u - part);
+            ep = pp[g], eq = qp[g], eh = hp[g], ec = cp[g];
+            for (int k = 0; k <= part; k++)
+                ep += c[5 * k], eq += c[5 * k + 1], eh += c[5 * k + 2], ec += c[5 * k + 3];
+        }
+        if (np != ep || nq != eq || nh != eh || nc != ec)
+            atomicOr(err, 2u);
     }
 }
 
@@ -1147,11 +1196,12 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     t0 = now_s();
 
     // ---- walk: count, offsets, fill
-    int64_t *cnt = nullptr;
-    BC(B.get(&cnt, 5 * ng));
-    BC(cudaMemsetAsync(cnt, 0, 5 * ng * sizeof(int64_t), st));
+    int64_t *cnt = nullptr, *ucnt = nullptr;
+    BC(B.get(&cnt, 6 * ng));
+    BC(cudaMemsetAsync(cnt, 0, 6 * ng * sizeof(int64_t), st));
     BC(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
     int32_t *worder = nullptr;
+    int64_t nwide = 0;
     {
         int64_t *wide = nullptr, *before = nullptr;
         BC(B.get(&wide, ng + 1));
@@ -1163,18 +1213,29 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
             return rc;
         k_walk_order<<<grid_of(ng), kThreads, 0, st>>>(out.groups, ng, side / 16, before, worder);
         BC(cudaGetLastError());
+        BC(cudaMemcpyAsync(&nwide, before + ng, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        BC(cudaStreamSynchronize(st));
     }
-    k_walk<false><<<grid_of(ng, kWalkWarps), 32 * kWalkWarps, 0, st>>>(
-        wc, spos, n, out.groups, worder, ng, P, cnt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-        nullptr, nullptr, flag);
+    if (4 * nwide > ng)  // enough of them to fill the GPU whole
+        nwide = 0;
+    const int64_t units = ng + (kWalkParts - 1) * nwide;
+    BC(B.get(&ucnt, 5 * kWalkParts * nwide));
+    const auto count_pass = nwide ? k_walk<false, true> : k_walk<false, false>;
+    const auto fill_pass = nwide ? k_walk<true, true> : k_walk<true, false>;
+    count_pass<<<grid_of(units, kWalkWarps), 32 * kWalkWarps, 0, st>>>(
+        wc, spos, n, out.groups, worder, ng, nwide, P, cnt, ucnt, nullptr, nullptr, nullptr, nullptr,
+        nullptr, nullptr, nullptr, nullptr, flag);
     BC(cudaGetLastError());
-    std::vector<int64_t> hc(5 * ng);
-    BC(cudaMemcpyAsync(hc.data(), cnt, 5 * ng * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    std::vector<int64_t> hc(6 * ng);
+    BC(cudaMemcpyAsync(hc.data(), cnt, 6 * ng * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     BC(cudaMemcpyAsync(&hbad, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     out.groups_h.resize(ng);
     BC(cudaMemcpyAsync(out.groups_h.data(), out.groups, ng * sizeof(nln_group),
                        cudaMemcpyDeviceToHost, st));
     BC(cudaStreamSynchronize(st));
+    for (int64_t g = 0; g < ng; g++)
+        if (hc[6 * g + 5] != n)
+            hbad |= 1u;
     if (hbad)
         return gc::set_status(-1, "GPU tree build: a group's walk did not cover every body "
                                   "exactly once, or overflowed its stack");
@@ -1184,15 +1245,15 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     for (int64_t g = 0; g < ng; g++) {
         // a group's lists cover every body once: no kind can exceed the point table
         for (int k = 0; k < 5; k++)
-            if (hc[5 * g + k] < 0 || hc[5 * g + k] > n + nc)
+            if (hc[6 * g + k] < 0 || hc[6 * g + k] > n + nc)
                 return gc::set_status(-1, "GPU tree build: group %lld counted %lld entries",
-                                      (long long)g, (long long)hc[5 * g + k]);
-        for (int k = 0; k < 4; k++) out.ptr_h[k][g + 1] = out.ptr_h[k][g] + hc[5 * g + k];
-        const int64_t c = out.groups_h[g].count, nbod = hc[5 * g + 4];
+                                      (long long)g, (long long)hc[6 * g + k]);
+        for (int k = 0; k < 4; k++) out.ptr_h[k][g + 1] = out.ptr_h[k][g] + hc[6 * g + k];
+        const int64_t c = out.groups_h[g].count, nbod = hc[6 * g + 4];
         out.counts[0] += c * nbod;
-        out.counts[1] += c * (hc[5 * g] - nbod);
-        out.counts[2] += c * hc[5 * g + 1];
-        out.counts[3] += c * hc[5 * g + 2];
+        out.counts[1] += c * (hc[6 * g] - nbod);
+        out.counts[2] += c * hc[6 * g + 1];
+        out.counts[3] += c * hc[6 * g + 2];
     }
     int64_t *dptr[4];
     for (int k = 0; k < 4; k++) {
@@ -1205,9 +1266,9 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     out.seconds[5] = now_s() - t0;  // offsets and list allocation
     t0 = now_s();
     BC(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
-    k_walk<true><<<grid_of(ng, kWalkWarps), 32 * kWalkWarps, 0, st>>>(
-        wc, spos, n, out.groups, worder, ng, P, nullptr, dptr[0], dptr[1], dptr[2], dptr[3], out.list[0],
-        out.list[1], out.list[2], out.list[3], flag);
+    fill_pass<<<grid_of(units, kWalkWarps), 32 * kWalkWarps, 0, st>>>(
+        wc, spos, n, out.groups, worder, ng, nwide, P, nullptr, ucnt, dptr[0], dptr[1], dptr[2],
+        dptr[3], out.list[0], out.list[1], out.list[2], out.list[3], flag);
     BC(cudaGetLastError());
     BC(cudaMemcpyAsync(&hbad, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     BC(cudaStreamSynchronize(st));
