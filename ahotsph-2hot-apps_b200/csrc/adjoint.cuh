@@ -1143,18 +1143,46 @@ __global__ void k_adjoint_bodies(const float4 *__restrict__ pts, const int32_t *
     out[b] = make_float4((float)g[0], (float)g[1], (float)g[2], (float)g[3]);
 }
 
+// The parent of every cell and the leaf of every body from the tree's links,
+// a thread per cell (both arrays -1 before).
+__global__ void k_adjoint_links(const int64_t *__restrict__ first, const int32_t *__restrict__ count,
+                                const int32_t *__restrict__ child, const int32_t *__restrict__ nchild,
+                                int64_t nc, int32_t *parent, int32_t *leaf) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= nc)
+        return;
+    if (child[c] >= 0) {
+        for (int32_t k = 0; k < nchild[c]; k++) parent[child[c] + k] = (int32_t)c;
+    } else {
+        for (int64_t b = first[c]; b < first[c] + count[c]; b++) leaf[b] = (int32_t)c;
+    }
+}
+
 }  // namespace
 
-// Per-plan adjoint state (owned by the plan).
+// Per-plan adjoint state (owned by the plan), from the plan's pool where it
+// has one.
 struct grav_adjoint_state {
+    cudaMemPool_t pool = nullptr;
     int32_t *leaf = nullptr, *parent = nullptr;
     int *flag = nullptr;
     double *gbody = nullptr, *gcell = nullptr, *mbar = nullptr, *gstf = nullptr;
+    template <typename T>
+    cudaError_t get(T **p, size_t n) {
+        return pool ? cudaMallocFromPoolAsync((void **)p, n * sizeof(T), pool, 0)
+                    : cudaMalloc((void **)p, n * sizeof(T));
+    }
     ~grav_adjoint_state() {
+        if (pool)
+            cudaDeviceSynchronize();  // an adjoint on any stream may still use them
         for (void *p : {(void *)leaf, (void *)parent, (void *)flag, (void *)gbody, (void *)gcell,
                         (void *)mbar, (void *)gstf})
-            if (p)
-                cudaFree(p);
+            if (p) {
+                if (pool)
+                    cudaFreeAsync(p, 0);
+                else
+                    cudaFree(p);
+            }
     }
 };
 
@@ -1183,45 +1211,31 @@ extern "C" int grav_plan_adjoint_CUDA(grav_plan *pl, const float *wu, float *gra
     grav_step_state *S = pl->step;
     if (!pl->adj) {
         auto *A = new grav_adjoint_state();
-        // leaf of every body and parent of every cell, from the links
-        std::vector<int32_t> child(nc), nchild(nc), parent(nc, -1), leaf(nb, -1);
-        std::vector<int64_t> first(nc);
-        std::vector<int32_t> count(nc);
-        cudaError_t e = cudaMemcpy(child.data(), S->cchild, nc * 4, cudaMemcpyDeviceToHost);
+        A->pool = pl->pool;
+        cudaError_t e = A->get(&A->leaf, nb);
         if (e == cudaSuccess)
-            e = cudaMemcpy(nchild.data(), S->cnchild, nc * 4, cudaMemcpyDeviceToHost);
+            e = A->get(&A->parent, nc);
         if (e == cudaSuccess)
-            e = cudaMemcpy(first.data(), S->cfirst, nc * 8, cudaMemcpyDeviceToHost);
+            e = A->get(&A->flag, nc);
         if (e == cudaSuccess)
-            e = cudaMemcpy(count.data(), S->ccount, nc * 4, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) {
-            delete A;
-            return gc::cuda_status(e, "grav_plan_adjoint_CUDA: links");
-        }
-        for (int64_t c = 0; c < nc; c++) {
-            if (child[c] >= 0) {
-                for (int32_t k = 0; k < nchild[c]; k++) parent[child[c] + k] = (int32_t)c;
-            } else {
-                for (int64_t b = first[c]; b < first[c] + count[c]; b++) leaf[b] = (int32_t)c;
-            }
-        }
-        e = cudaMalloc((void **)&A->leaf, nb * 4);
+            e = A->get(&A->gbody, nb * 4);
         if (e == cudaSuccess)
-            e = cudaMemcpy(A->leaf, leaf.data(), nb * 4, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMalloc((void **)&A->parent, nc * 4);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(A->parent, parent.data(), nc * 4, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMalloc((void **)&A->flag, nc * 4);
-        if (e == cudaSuccess)
-            e = cudaMalloc((void **)&A->gbody, nb * 4 * sizeof(double));
-        if (e == cudaSuccess)
-            e = cudaMalloc((void **)&A->gcell, nc * kCellAdj * sizeof(double));
+            e = A->get(&A->gcell, nc * kCellAdj);
         if (e == cudaSuccess && pl->dp.ewald)
-            e = cudaMalloc((void **)&A->mbar, ng * 35 * sizeof(double));
+            e = A->get(&A->mbar, ng * 35);
         if (e == cudaSuccess && pl->dp.ewald)
-            e = cudaMalloc((void **)&A->gstf, nc * kStfIndep * sizeof(double));
+            e = A->get(&A->gstf, nc * kStfIndep);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(A->leaf, 0xff, nb * 4, 0);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(A->parent, 0xff, nc * 4, 0);
+        if (e == cudaSuccess) {
+            k_adjoint_links<<<(unsigned)((nc + 127) / 128), 128>>>(S->cfirst, S->ccount, S->cchild,
+                                                                     S->cnchild, nc, A->parent, A->leaf);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(0);  // `st` does not wait for it
         if (e != cudaSuccess) {
             delete A;
             return gc::cuda_status(e, "grav_plan_adjoint_CUDA: scratch");

@@ -8,7 +8,7 @@
 // so the tables and lists are bit-identical to the host's:
 //   bounding cube     exact min / max of the FP32 positions, enlarged on the host as nlnhost.cpp
 //   Morton keys       21 bits per axis, stable radix sort of (key, input index)
-//   cells             level-synchronous octant splits of the sorted keys, one level per pass
+//   cells             level-synchronous octant splits of the sorted keys, two kernels a level
 //   moments           FP64 sums over each cell's bodies in the canonical blocked order of
 //                     nlnhost.cpp (64 bodies, 64 partials, then in order): one thread per
 //                     block at each of the three levels
@@ -180,73 +180,152 @@ __global__ void k_permute(const float4 *__restrict__ b, const int64_t *__restric
 // ------------------------------------------------------------ cells
 struct Cells {
     int64_t *first;
-    int32_t *count, *child, *nchild, *level;
+    int32_t *count, *child, *nchild;
     double *gc;    // 3 per cell
     double *side;
 };
 
-// Frontier cells [lo, lo + nf): children per octant by binary search of the
-// sorted keys (nlnhost.cpp build_cells); nk[f] their number, bounds[9 f ..]
-// the octants' first bodies.
-__global__ void k_split_count(Cells C, int64_t lo, int64_t nf, const uint64_t *__restrict__ keys,
-                              int leaf_max, int64_t *nk, int64_t *bounds) {
-    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nf)
-        return;
-    const int64_t c = lo + f;
-    nk[f] = 0;
-    const int32_t cnt = C.count[c], lev = C.level[c];
-    if (cnt <= leaf_max || lev >= KEY_LEVELS)
-        return;
-    const int shift = 3 * (KEY_LEVELS - 1 - lev);
-    int64_t a0 = C.first[c], hi = C.first[c] + cnt;
-    bounds[f * 9] = a0;
-    int k = 0;
-    for (int o = 0; o < 8; o++) {
-        int64_t a = a0, bb = hi;
-        while (a < bb) {
-            const int64_t mid = (a + bb) / 2;
-            if ((int)((keys[mid] >> shift) & 7) <= o)
-                a = mid + 1;
-            else
-                bb = mid;
-        }
-        bounds[f * 9 + o + 1] = a;
-        if (a > a0)
-            k++;
-        a0 = a;
-    }
-    nk[f] = k;
+// One level of the tree, two kernels, with the level's cells [lo, hi) in
+// device memory (state[2 l], state[2 l + 1]): the host launches every level
+// without waiting for the one before (100k-body sphere: 0.76 -> 0.25 ms; its
+// 20 levels had waited for two copies each).  A block takes a contiguous part
+// of the level, so that the children, appended in order, land as
+// nlnhost.cpp's build_cells puts them.
+constexpr int kSplitBlocks = 296;
+constexpr int kSplitThreads = 256;
+constexpr int kMaxLevels = KEY_LEVELS + 2;
+
+__device__ inline void split_part(const int64_t *state, int level, int64_t &lo, int64_t &hi,
+                                  int64_t &b, int64_t &e) {
+    lo = state[2 * level];
+    hi = state[2 * level + 1];
+    const int64_t per = (hi - lo + kSplitBlocks - 1) / kSplitBlocks;
+    b = min(hi, lo + blockIdx.x * per);
+    e = min(hi, b + per);
 }
 
-// Write the children of frontier cell f at base + off[f] .. in octant order.
-__global__ void k_split_write(Cells C, int64_t lo, int64_t nf, const int64_t *__restrict__ nk,
-                              const int64_t *__restrict__ bounds, const int64_t *__restrict__ off,
-                              int64_t base) {
-    const int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nf || nk[f] == 0)
-        return;
-    const int64_t c = lo + f;
-    C.child[c] = (int32_t)(base + off[f]);
-    C.nchild[c] = (int32_t)nk[f];
-    const double side = C.side[c];
-    int k = 0;
-    for (int o = 0; o < 8; o++) {
-        const int64_t a = bounds[f * 9 + o], b = bounds[f * 9 + o + 1];
-        if (b <= a)
-            continue;
-        const int64_t d = base + off[f] + k;
-        C.first[d] = a;
-        C.count[d] = (int32_t)(b - a);
-        C.child[d] = -1;
-        C.nchild[d] = 0;
-        C.level[d] = C.level[c] + 1;
-        C.side[d] = 0.5 * side;
-        C.gc[3 * d] = C.gc[3 * c] + ((o >> 2) & 1 ? 0.25 : -0.25) * side;
-        C.gc[3 * d + 1] = C.gc[3 * c + 1] + ((o >> 1) & 1 ? 0.25 : -0.25) * side;
-        C.gc[3 * d + 2] = C.gc[3 * c + 2] + ((o >> 0) & 1 ? 0.25 : -0.25) * side;
-        k++;
+// Children per octant by binary search of the sorted keys, a thread per cell
+// and octant: bounds[8 c + o] the end of octant o, relative to the cell's first
+// body; sums[block] the part's children.
+__global__ void __launch_bounds__(kSplitThreads)
+    k_split_count(Cells C, const int64_t *__restrict__ state, int level,
+                  const uint64_t *__restrict__ keys, int leaf_max, int32_t *bounds, int32_t *sums) {
+    int64_t lo, hi, b, e;
+    split_part(state, level, lo, hi, b, e);
+    const int o = threadIdx.x & 7;
+    int kids = 0;
+    for (int64_t c = b + threadIdx.x / 8; c < e; c += kSplitThreads / 8) {
+        const int32_t cnt = C.count[c];
+        const bool open = cnt > leaf_max && level < KEY_LEVELS;
+        const int64_t first = C.first[c];
+        int64_t a = first;
+        if (open) {
+            const int shift = 3 * (KEY_LEVELS - 1 - level);
+            int64_t bb = first + cnt;
+            while (a < bb) {
+                const int64_t mid = (a + bb) / 2;
+                if ((int)((keys[mid] >> shift) & 7) <= o)
+                    a = mid + 1;
+                else
+                    bb = mid;
+            }
+        }
+        const int32_t end = (int32_t)(a - first);
+        // a cell's eight threads are neighbours of one warp and take this turn together
+        const unsigned eight = 0xffu << (threadIdx.x & 24);
+        const int32_t before = __shfl_up_sync(eight, end, 1, 8);
+        bounds[8 * c + o] = open ? end : 0;
+        kids += open && end > (o ? before : 0) ? 1 : 0;
     }
+    typedef cub::BlockReduce<int, kSplitThreads> Reduce;
+    __shared__ typename Reduce::TempStorage tmp;
+    const int total = Reduce(tmp).Sum(kids);
+    if (threadIdx.x == 0)
+        sums[blockIdx.x] = total;
+}
+
+// The children, in order behind the level; state gets the next level's cells.
+// Beyond cap cells nothing is written and *over set.
+__global__ void __launch_bounds__(kSplitThreads)
+    k_split_write(Cells C, int64_t *state, int level, const int32_t *__restrict__ bounds,
+                  const int32_t *__restrict__ sums, int64_t cap, unsigned *over) {
+    int64_t lo, hi, b, e;
+    split_part(state, level, lo, hi, b, e);
+    typedef cub::BlockReduce<int64_t, kSplitThreads> Reduce;
+    typedef cub::BlockScan<int, kSplitThreads> Scan;
+    __shared__ union {
+        typename Reduce::TempStorage r;
+        typename Scan::TempStorage s;
+    } tmp;
+    __shared__ int64_t sh[2];
+    int64_t before = 0, all = 0;  // children of the parts before this one, and of the level
+    for (int k = threadIdx.x; k < kSplitBlocks; k += kSplitThreads) {
+        all += sums[k];
+        before += k < (int)blockIdx.x ? sums[k] : 0;
+    }
+    before = Reduce(tmp.r).Sum(before);
+    __syncthreads();
+    all = Reduce(tmp.r).Sum(all);
+    if (threadIdx.x == 0) {
+        sh[0] = before;
+        sh[1] = all;
+    }
+    __syncthreads();
+    int64_t base = hi + sh[0];
+    const bool fits = hi + sh[1] <= cap;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        state[2 * level + 2] = hi;
+        state[2 * level + 3] = fits ? hi + sh[1] : hi;
+        if (!fits)
+            *over = 1;
+    }
+    if (!fits)
+        return;
+    for (int64_t c0 = b; c0 < e; c0 += kSplitThreads) {
+        const int64_t c = c0 + threadIdx.x;
+        int nk = 0;
+        if (c < e)
+            for (int o = 0; o < 8; o++) nk += bounds[8 * c + o] > (o ? bounds[8 * c + o - 1] : 0);
+        int off, total;
+        __syncthreads();
+        Scan(tmp.s).ExclusiveSum(nk, off, total);
+        if (nk > 0) {
+            C.child[c] = (int32_t)(base + off);
+            C.nchild[c] = (int32_t)nk;
+            const double side = C.side[c];
+            const int64_t first = C.first[c];
+            int64_t d = base + off;
+            for (int o = 0; o < 8; o++) {
+                const int32_t x = o ? bounds[8 * c + o - 1] : 0, y = bounds[8 * c + o];
+                if (y <= x)
+                    continue;
+                C.first[d] = first + x;
+                C.count[d] = y - x;
+                C.child[d] = -1;
+                C.nchild[d] = 0;
+                C.side[d] = 0.5 * side;
+                C.gc[3 * d] = C.gc[3 * c] + ((o >> 2) & 1 ? 0.25 : -0.25) * side;
+                C.gc[3 * d + 1] = C.gc[3 * c + 1] + ((o >> 1) & 1 ? 0.25 : -0.25) * side;
+                C.gc[3 * d + 2] = C.gc[3 * c + 2] + ((o >> 0) & 1 ? 0.25 : -0.25) * side;
+                d++;
+            }
+        }
+        base += total;
+    }
+}
+
+__global__ void k_split_root(Cells C, int32_t n, double g0, double g1, double g2, double side,
+                             int64_t *state) {
+    C.first[0] = 0;
+    C.count[0] = n;
+    C.child[0] = -1;
+    C.nchild[0] = 0;
+    C.gc[0] = g0;
+    C.gc[1] = g1;
+    C.gc[2] = g2;
+    C.side[0] = side;
+    state[0] = 0;
+    state[1] = 1;
 }
 
 // ------------------------------------------------------------ canonical sums
@@ -304,25 +383,26 @@ __global__ void k_sum0(const Cells C, int64_t ncells, const int64_t *__restrict_
     for (int q = 0; q <= K; q++) p0[j * (K + 1) + q] = a[q];
 }
 
+// A thread per block and component: each component's partials in their order.
 template <int K>
 __global__ void k_sum1(const Cells C, int64_t ncells, const int64_t *__restrict__ o0,
                        const int64_t *__restrict__ o1, int64_t total, const double *p0,
                        double *p1) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t j = i / (K + 1);
+    const int q = (int)(i - j * (K + 1));
     if (j >= total)
         return;
     const int64_t c = owner(o1, ncells, j);
     const int64_t blk = j - o1[c];
     const int64_t nb0 = o0[c + 1] - o0[c];
-    double a[K + 1];
-    for (int q = 0; q <= K; q++) a[q] = 0.0;
+    double a = 0.0;
     const int64_t k1 = nb0 < (blk + 1) * kSumBlock ? nb0 : (blk + 1) * kSumBlock;
     for (int64_t k = blk * kSumBlock; k < k1; k++) {
-        const double *s = p0 + (o0[c] + k) * (K + 1);
-        for (int q = 0; q < K; q++) a[q] += s[q];
-        a[K] = fmax(a[K], s[K]);
+        const double s = p0[(o0[c] + k) * (K + 1) + q];
+        a = q < K ? a + s : fmax(a, s);
     }
-    for (int q = 0; q <= K; q++) p1[j * (K + 1) + q] = a[q];
+    p1[j * (K + 1) + q] = a;
 }
 
 // Level 2 of pass 1: the centre of mass (nlnhost.cpp compute_moments).
@@ -969,81 +1049,51 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     out.seconds[0] = now_s() - t0;
     t0 = now_s();
 
-    // ---- cells, level by level
-    int64_t cap = std::max<int64_t>(1024, 2 * (n / std::max(1, p.leaf_max)) + 64);
+    // ---- cells, level by level: room for two per three bodies at first (spheres and boxes
+    // with leaves of 16 need a quarter of that), four times as many where that is too few
     Cells C{};
-    auto alloc_cells = [&](Cells &D, int64_t c) -> int {
-        BC(B.get(&D.first, c));
-        BC(B.get(&D.count, c));
-        BC(B.get(&D.child, c));
-        BC(B.get(&D.nchild, c));
-        BC(B.get(&D.level, c));
-        BC(B.get(&D.gc, 3 * c));
-        BC(B.get(&D.side, c));
-        return 0;
-    };
-    if (int rc = alloc_cells(C, cap))
-        return rc;
-    {
-        const int64_t f0 = 0;
-        const int32_t cn = (int32_t)n, ch = -1, nch = 0, lv = 0;
-        double g[3];
-        for (int d = 0; d < 3; d++) g[d] = origin[d] + 0.5 * side;
-        BC(cudaMemcpyAsync(C.first, &f0, sizeof(f0), cudaMemcpyHostToDevice, st));
-        BC(cudaMemcpyAsync(C.count, &cn, sizeof(cn), cudaMemcpyHostToDevice, st));
-        BC(cudaMemcpyAsync(C.child, &ch, sizeof(ch), cudaMemcpyHostToDevice, st));
-        BC(cudaMemcpyAsync(C.nchild, &nch, sizeof(nch), cudaMemcpyHostToDevice, st));
-        BC(cudaMemcpyAsync(C.level, &lv, sizeof(lv), cudaMemcpyHostToDevice, st));
-        BC(cudaMemcpyAsync(C.gc, g, sizeof(g), cudaMemcpyHostToDevice, st));
-        BC(cudaMemcpyAsync(C.side, &side, sizeof(side), cudaMemcpyHostToDevice, st));
-        BC(cudaStreamSynchronize(st));
-    }
-    int64_t lo = 0, hi = 1;
-    while (hi > lo) {
-        out.level_start.push_back(lo);
-        const int64_t nf = hi - lo;
-        int64_t *nk = nullptr, *bounds = nullptr, *off = nullptr;
-        BC(B.get(&nk, nf));
-        BC(B.get(&off, nf));
-        BC(B.get(&bounds, 9 * nf));
-        k_split_count<<<grid_of(nf), kThreads, 0, st>>>(C, lo, nf, k_out, p.leaf_max, nk, bounds);
+    int64_t hstate[2 * (kMaxLevels + 1)];
+    for (int64_t cap = std::max<int64_t>(1024, 2 * n / 3);; cap *= 4) {
+        int32_t *bounds = nullptr, *sums = nullptr;
+        int64_t *state = nullptr;
+        BC(B.get(&C.first, cap));
+        BC(B.get(&C.count, cap));
+        BC(B.get(&C.child, cap));
+        BC(B.get(&C.nchild, cap));
+        BC(B.get(&C.gc, 3 * cap));
+        BC(B.get(&C.side, cap));
+        BC(B.get(&bounds, 8 * cap));
+        BC(B.get(&sums, kSplitBlocks));
+        BC(B.get(&state, 2 * (kMaxLevels + 1)));
+        BC(cudaMemsetAsync(state, 0, 2 * (kMaxLevels + 1) * sizeof(int64_t), st));
+        BC(cudaMemsetAsync(flag, 0, sizeof(unsigned), st));
+        k_split_root<<<1, 1, 0, st>>>(C, (int32_t)n, origin[0] + 0.5 * side, origin[1] + 0.5 * side,
+                                       origin[2] + 0.5 * side, side, state);
         BC(cudaGetLastError());
-        if (int rc = exclusive_scan(B, nk, off, nf, st))
-            return rc;
-        int64_t last_off = 0, last_nk = 0;
-        BC(cudaMemcpyAsync(&last_off, off + nf - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-        BC(cudaMemcpyAsync(&last_nk, nk + nf - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-        BC(cudaStreamSynchronize(st));
-        const int64_t total = last_off + last_nk;
-        if (total > 0) {
-            if (hi + total > cap) {  // grow the cell arrays
-                int64_t ncap = std::max(2 * cap, hi + total + 1024);
-                Cells D{};
-                if (int rc = alloc_cells(D, ncap))
-                    return rc;
-                BC(cudaMemcpyAsync(D.first, C.first, hi * sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
-                BC(cudaMemcpyAsync(D.count, C.count, hi * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-                BC(cudaMemcpyAsync(D.child, C.child, hi * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-                BC(cudaMemcpyAsync(D.nchild, C.nchild, hi * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-                BC(cudaMemcpyAsync(D.level, C.level, hi * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-                BC(cudaMemcpyAsync(D.gc, C.gc, 3 * hi * sizeof(double), cudaMemcpyDeviceToDevice, st));
-                BC(cudaMemcpyAsync(D.side, C.side, hi * sizeof(double), cudaMemcpyDeviceToDevice, st));
-                BC(cudaStreamSynchronize(st));
-                B.drop(C.first); B.drop(C.count); B.drop(C.child); B.drop(C.nchild);
-                B.drop(C.level); B.drop(C.gc); B.drop(C.side);
-                C = D;
-                cap = ncap;
-            }
-            k_split_write<<<grid_of(nf), kThreads, 0, st>>>(C, lo, nf, nk, bounds, off, hi);
+        for (int level = 0; level < kMaxLevels; level++) {
+            k_split_count<<<kSplitBlocks, kSplitThreads, 0, st>>>(C, state, level, k_out, p.leaf_max,
+                                                                   bounds, sums);
+            BC(cudaGetLastError());
+            k_split_write<<<kSplitBlocks, kSplitThreads, 0, st>>>(C, state, level, bounds, sums, cap,
+                                                                   flag);
             BC(cudaGetLastError());
         }
-        B.drop(nk);
-        B.drop(off);
+        BC(cudaMemcpyAsync(hstate, state, sizeof(hstate), cudaMemcpyDeviceToHost, st));
+        BC(cudaMemcpyAsync(&hbad, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        BC(cudaStreamSynchronize(st));
         B.drop(bounds);
-        lo = hi;
-        hi += total;
+        B.drop(sums);
+        B.drop(state);
+        if (!hbad)
+            break;
+        B.drop(C.first); B.drop(C.count); B.drop(C.child); B.drop(C.nchild); B.drop(C.gc);
+        B.drop(C.side);
     }
-    const int64_t nc = hi;
+    int64_t nc = 0;
+    for (int level = 0; level < kMaxLevels && hstate[2 * level + 1] > hstate[2 * level]; level++) {
+        out.level_start.push_back(hstate[2 * level]);
+        nc = hstate[2 * level + 1];
+    }
     out.level_start.push_back(nc);
     if (n + nc + 1 >= (int64_t)NLN_IDX_MASK)
         return gc::set_status(-1, "GPU tree build: bodies plus cells exceed 27-bit list indices");
@@ -1078,7 +1128,7 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     BC(B.get(&p1, B1 * 5));
     k_sum0<4><<<grid_of(B0), kThreads, 0, st>>>(C, nc, o0, B0, spos, smass, C.gc, p0);
     BC(cudaGetLastError());
-    k_sum1<4><<<grid_of(B1), kThreads, 0, st>>>(C, nc, o0, o1, B1, p0, p1);
+    k_sum1<4><<<grid_of(5 * B1), kThreads, 0, st>>>(C, nc, o0, o1, B1, p0, p1);
     BC(cudaGetLastError());
     k_sum2_mass<<<grid_of(nc), kThreads, 0, st>>>(C, nc, o1, p1, cen, mass);
     BC(cudaGetLastError());
@@ -1091,7 +1141,7 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
     BC(B.get(&p1, B1 * K2));
     k_sum0<NLN_NMOM><<<grid_of(B0), kThreads, 0, st>>>(C, nc, o0, B0, spos, smass, cen, p0);
     BC(cudaGetLastError());
-    k_sum1<NLN_NMOM><<<grid_of(B1), kThreads, 0, st>>>(C, nc, o0, o1, B1, p0, p1);
+    k_sum1<NLN_NMOM><<<grid_of(K2 * B1), kThreads, 0, st>>>(C, nc, o0, o1, B1, p0, p1);
     BC(cudaGetLastError());
     BC(B.get(&out.points, n + nc));
     BC(B.get(&out.qcells, nc));
