@@ -1247,6 +1247,8 @@ extern "C" int grav_plan_adjoint_CUDA(grav_plan *pl, const float *wu, float *gra
     GC_CHECK(cudaMemsetAsync(A->gcell, 0, nc * kCellAdj * sizeof(double), st));
     if (A->gstf)
         GC_CHECK(cudaMemsetAsync(A->gstf, 0, nc * kStfIndep * sizeof(double), st));
+    const bool clear = pl->queues_clear;
+    pl->queues_clear = false;
     GC_CHECK(cudaMemsetAsync(pl->dp.counters, 0, 4 * sizeof(int), st));
     AdjProblem P{};
     P.points = pl->dp.points;
@@ -1297,5 +1299,8 @@ extern "C" int grav_plan_adjoint_CUDA(grav_plan *pl, const float *wu, float *gra
         pl->dp.points, A->leaf, A->parent, pl->dp.qcells, pl->dp.hcells, A->gcell, A->flag,
         A->gbody, nb, reinterpret_cast<float4 *>(grad));
     GC_CHECK(cudaGetLastError());
+    // the queues as the evaluations leave them
+    GC_CHECK(cudaMemsetAsync(pl->dp.counters, 0, 4 * sizeof(int), st));
+    pl->queues_clear = clear;
     return 0;
 }

@@ -225,14 +225,6 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// Fold t into the compensated accumulator (hi, lo), half by half: Knuth's
-// two-sum, s + e == hi + t exactly.
-__device__ __forceinline__ void comp_add2(float2 &hi, float2 &lo, float2 t) {
-    const float2 s = add2(hi, t), bp = add2(s, neg2(hi));
-    lo = add2(lo, add2(add2(hi, neg2(add2(s, neg2(bp)))), add2(t, neg2(bp))));
-    hi = s;
-}
-
 // Running sums of one sink over this lane's records (nphi: -phi).
 struct Sum2 {
     float2 ax, ay, az, nphi;
