@@ -289,23 +289,17 @@ __device__ __forceinline__ float4 shfl_xor4(float4 v, int m) {
     return make_float4(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m),
                        __shfl_xor_sync(0xffffffffu, v.z, m), __shfl_xor_sync(0xffffffffu, v.w, m));
 }
-// A sink's running sum over the tiles of an item: (hi, lo) compensated FP32
-// (Knuth's two-sum: s + e == hi + t exactly), or plain FP32 in the plain form.
+// A sink's running sum over the tiles of an item: FP64 (its conversions and
+// adds take fewer issue slots than two-sum compensation in FP32: 1M bodies
+// 6.53 -> 6.50 ms), or plain FP32 in the plain form.
 template <bool PLAIN>
 struct Total {
-    float2 hi[2], lo[2];
-    __device__ __forceinline__ Total() { hi[0] = hi[1] = lo[0] = lo[1] = splat2(0.f); }
-    __device__ __forceinline__ void add(float4 v) {
-        const float2 t[2] = {f2(v.x, v.y), f2(v.z, v.w)};
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const float2 s = add2(hi[q], t[q]);
-            if (!PLAIN) {
-                const float2 bp = add2(s, neg2(hi[q]));
-                lo[q] = add2(lo[q], add2(add2(hi[q], neg2(add2(s, neg2(bp)))), add2(t[q], neg2(bp))));
-            }
-            hi[q] = s;
-        }
+    std::conditional_t<PLAIN, float, double> v[4] = {0, 0, 0, 0};
+    __device__ __forceinline__ void add(float4 t) {
+        v[0] += t.x;
+        v[1] += t.y;
+        v[2] += t.z;
+        v[3] += t.w;
     }
 };
 
@@ -371,9 +365,15 @@ __device__ __forceinline__ void sum_sinks(const SinkTable &T, int nsink, int lan
 template <bool PLAIN>
 __device__ __forceinline__ void store_part(const DevProblem &P, const Item &item, int lane,
                                            const Total<PLAIN> &acc) {
+    float hi[4], lo[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        hi[q] = (float)acc.v[q];
+        lo[q] = PLAIN ? 0.f : (float)(acc.v[q] - (double)hi[q]);
+    }
     float4 *dst = P.part + ((size_t)item.slot * 32 + lane) * 2;
-    dst[0] = make_float4(acc.hi[0].x, acc.hi[0].y, acc.hi[1].x, acc.hi[1].y);
-    dst[1] = make_float4(acc.lo[0].x, acc.lo[0].y, acc.lo[1].x, acc.lo[1].y);
+    dst[0] = make_float4(hi[0], hi[1], hi[2], hi[3]);
+    dst[1] = make_float4(lo[0], lo[1], lo[2], lo[3]);
 }
 
 // Coordinate of an absent record, beyond any sink: with zero mass and
