@@ -1093,7 +1093,6 @@ struct grav_plan {
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     EwStored *ewm = nullptr;
-    int64_t ewald_entries = 0;  // correction-list length
     // Group ranges of the work queue: items are sorted by cost within each
     // range, and chunk_item[k][c] is the first item of kind k in range c.
     // One range [0, ngroups) except in the pipelined end-to-end call.
@@ -1702,7 +1701,6 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
         d.ew_self = (float)(c0 - M_PI / (alpha * alpha * hp->box * hp->box * hp->box));
         d.ewald = 1;
         rc |= dev_copy<EwStored>(pl, nullptr, (size_t)ng, &pl->ewm);
-        pl->ewald_entries = hp->cptr[ng];
         // Lists are split until there are ~4 units per resident warp (10 per
         // SM), but not below 8 tiles a unit: a 16^3 box has 156 groups for
         // 1,480 warps (moments 0.16 -> 0.07 ms), a 64^3 box enough as it is.
@@ -1913,23 +1911,20 @@ int launch_moments(grav_plan *pl, const DevProblem &dp, cudaStream_t s, int per_
 // blocks per SM, sharing the SMs with them; ewald_side = -k runs them
 // (k_ewald_moments) on the evaluation's stream between the list kernels and
 // the finish pass, with the SMs to themselves, in blocks of k warps (k = 1,
-// 2 or 4) as many as fit.  Automatic (0): the side stream with 2 blocks per
-// SM while the correction list is short beside the order-4 lists, else the
-// evaluation's stream with two-warp blocks.  Measured on one B200: at 256^3
-// (MAC 1.5e-6; correction entries 1.2 % of the order-4 interactions) the
-// side stream takes 813 ms a step against 825 ms; where the moments take
-// half the order-4 kernel's time (128^3, MAC 1e-4) the side stream loses.
+// 2 or 4) as many as fit.  Automatic (0): the evaluation's stream, two-warp
+// blocks.  Since k_ewald_moments stages its rows it is the faster place at
+// every size (ms an evaluation on it, and beside the lists with 2 and 3 side
+// blocks per SM): 64^3 at MAC 1e-5 4.56, 5.19, 4.65; 128^3 at 2.5e-6 63.8,
+// 69.7, 66.2; 256^3 at 1.5e-6, where the correction list is 1.2 % of the
+// order-4 interactions, 680, 748, 703.  One, two or four warps a block differ
+// by less than 0.1 %.
 int main_moments_warps(const grav_plan *pl) {
     const int k = -pl->tune.ewald_side;
     return (k == 1 || k == 2 || k == 4) ? k : 2;
 }
 
 int side_blocks(const grav_plan *pl) {
-    if (!pl->dp.ewald || !pl->side || !pl->ewm || pl->tune.ewald_side < 0)
-        return 0;
-    if (pl->tune.ewald_side > 0)
-        return pl->tune.ewald_side;
-    return pl->ewald_entries < 0.015 * (double)pl->counts[3] ? 2 : 0;
+    return pl->dp.ewald && pl->side && pl->ewm ? std::max(0, pl->tune.ewald_side) : 0;
 }
 
 // Fork: k_ewald_moments over dp's groups on the side stream, after the work

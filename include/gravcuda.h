@@ -219,9 +219,8 @@ typedef struct grav_tuning {
                                    side stream beside the list kernels, in this many two-warp
                                    blocks per SM; -k (k = 1, 2, 4): on the evaluation's stream
                                    between the list kernels and the finish pass, with the SMs to
-                                   themselves, in blocks of k warps; 0: automatic (2 while the
-                                   correction list is under 1.5 % of the order-4 interactions,
-                                   else -2).  The results are the same either way. */
+                                   themselves, in blocks of k warps; 0: automatic (-2).  The
+                                   results are the same either way. */
 } grav_tuning;
 
 /*
