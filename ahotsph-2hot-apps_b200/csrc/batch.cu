@@ -8,8 +8,7 @@
 //   * each source record is re-centred on the same FP64 centre (with its
 //     periodic image shift) as a lane takes it up, so the inner loops subtract
 //     two small FP32 numbers;
-//   * partial sums of one tile are plain FP32, folded into a compensated
-//     (hi, lo) accumulator per tile;
+//   * partial sums of one tile are plain FP32, folded into FP64 sums per tile;
 //   * work-item partials are combined per group in FP64, in a fixed order.
 // Work decomposition: a work item is (group, kind, range of its list);
 // long lists are split so that small problems still fill the GPU; every
@@ -289,12 +288,11 @@ __device__ __forceinline__ float4 shfl_xor4(float4 v, int m) {
     return make_float4(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m),
                        __shfl_xor_sync(0xffffffffu, v.z, m), __shfl_xor_sync(0xffffffffu, v.w, m));
 }
-// A sink's running sum over the tiles of an item: FP64 (its conversions and
-// adds take fewer issue slots than two-sum compensation in FP32: 1M bodies
-// 6.53 -> 6.50 ms), or plain FP32 in the plain form.
-template <bool PLAIN>
+// A sink's running sum over the tiles of an item, in FP64: its conversions and
+// adds take fewer issue slots than two-sum compensation in FP32 (1M bodies
+// 6.53 -> 6.50 ms).
 struct Total {
-    std::conditional_t<PLAIN, float, double> v[4] = {0, 0, 0, 0};
+    double v[4] = {0, 0, 0, 0};
     __device__ __forceinline__ void add(float4 t) {
         v[0] += t.x;
         v[1] += t.y;
@@ -317,9 +315,9 @@ struct SinkSums {
 // memory once a tile.  The four evaluations of a block are one basic block
 // (a test per sink kept them from overlapping: 19.4 against 20.1 cycles per
 // point interaction, 18.5 with the registers to hold four of them).
-template <int FOLDS, bool PLAIN, class Eval>
+template <int FOLDS, class Eval>
 __device__ __forceinline__ void sum_sinks(const SinkTable &T, int nsink, int lane, SinkSums &buf,
-                                          Total<PLAIN> &acc, Eval eval) {
+                                          Total &acc, Eval eval) {
     const int sw = lane & 3, nb = nsink >> 2, rem = nsink & 3;
     const Sink *p0 = T.s + sw, *p1 = T.s + (sw ^ 1), *p2 = T.s + (sw ^ 2), *p3 = T.s + (sw ^ 3);
     float4 *out = &buf.row[0][lane];
@@ -362,14 +360,13 @@ __device__ __forceinline__ void sum_sinks(const SinkTable &T, int nsink, int lan
     __syncwarp();  // read: the next tile may write
 }
 
-template <bool PLAIN>
 __device__ __forceinline__ void store_part(const DevProblem &P, const Item &item, int lane,
-                                           const Total<PLAIN> &acc) {
+                                           const Total &acc) {
     float hi[4], lo[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         hi[q] = (float)acc.v[q];
-        lo[q] = PLAIN ? 0.f : (float)(acc.v[q] - (double)hi[q]);
+        lo[q] = (float)(acc.v[q] - (double)hi[q]);
     }
     float4 *dst = P.part + ((size_t)item.slot * 32 + lane) * 2;
     dst[0] = make_float4(hi[0], hi[1], hi[2], hi[3]);
@@ -476,8 +473,8 @@ __device__ __forceinline__ void load_cell(const unsigned char *stage, int r, boo
 // as the lanes hold their records.
 // PLAIN: the plain FP32 form the reference's lists compute in (absolute FP32
 // coordinates, nln/mac.c:1421-1561 copies cell centres as floats): sinks and
-// sources are not re-centred on the group centre and tile sums are added
-// without compensation.  It exists to be compared with the mixed form.
+// sources are not re-centred on the group centre.  It exists to be compared
+// with the mixed form.
 template <int KIND, bool PLAIN>
 __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GRAV_Q_MINB)
     k_cells(const __grid_constant__ CUtensorMap tmap, DevProblem P) {
@@ -565,7 +562,7 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
             issue(0, ent, code);
         fetch(1, ent);
         stage_sinks(sinks, P, G, c, lane);
-        Total<PLAIN> acc;
+        Total acc;
         for (int t = 0; t < ntile; t++) {
             const int nt = (int)min((int64_t)CT, nent - (int64_t)t * CT);
             const bool ok = mbar_wait_bounded(bar, phase, P.err);
@@ -587,7 +584,7 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
             // the forms of a tile are told apart outside the sink loop
             auto sums_of = [&](auto form) {
                 constexpr bool F = decltype(form)::value;
-                sum_sinks<KIND == KH ? 2 : 4, PLAIN>(sinks, G.count, lane, sums, acc, [&](const Sink &k) {
+                sum_sinks<KIND == KH ? 2 : 4>(sinks, G.count, lane, sums, acc, [&](const Sink &k) {
                     const float2 nx = f2(k.xy.x, k.xy.y), ny = f2(k.xy.z, k.xy.w), nz = k.z;
                     Sum2 A;
                     if constexpr (KIND == KH) {
@@ -687,7 +684,7 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
         copy(cur);
         fetch(item.begin + kPointTile, nxt);
         stage_sinks(sinks, P, G, c, lane);
-        Total<PLAIN> acc;
+        Total acc;
         for (int64_t k0 = item.begin; k0 < item.end; k0 += kPointTile) {
             const int np = (int)min((int64_t)NP, (item.end - k0 + 63) / 64);  // pairs in use
             MonoPair rec[NP];
@@ -723,7 +720,7 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
             fetch(k0 + 2 * kPointTile, nxt);
             // a tile of at most 128 records leaves out the other two pairs
             auto sums_of = [&](auto n) {
-                sum_sinks<8, PLAIN>(sinks, G.count, lane, sums, acc, [&](const Sink &k) {
+                sum_sinks<8>(sinks, G.count, lane, sums, acc, [&](const Sink &k) {
                     const float2 nx = f2(k.xy.x, k.xy.y), ny = f2(k.xy.z, k.xy.w), nz = k.z;
                     Sum2 A;
                     mono_pair<true>(rec[0], nx, ny, nz, e2, A);

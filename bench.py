@@ -1035,7 +1035,8 @@ def main():
     dom = max(("hexa", "quad", "point"), key=lambda k: kms[k])
     achieved = kflops[dom] / (kms[dom] * 1e-3) / 1e12
     total_tflops = float((counts * FLOPS).sum() / (ms * 1e-3) / 1e12)
-    roofline = {"bound": "fp32", "kernel": f"k_batch<{dom}>", "achieved": achieved,
+    roofline = {"bound": "fp32", "kernel": "k_points" if dom == "point" else f"k_cells<{dom}>",
+                "achieved": achieved,
                 "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                 "traffic": float(DRAM_BYTES_PER_INTERACTION[dom] * (
                     counts[3] if dom == "hexa" else counts[2] if dom == "quad" else counts[0] + counts[1])),

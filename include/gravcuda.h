@@ -199,8 +199,8 @@ typedef struct grav_problem {
     const uint32_t *zlist[4];
     /* Arithmetic of the list kernels (grav_groups_upload_CUDA and grav_groups_CUDA):
        0 = mixed (default): sinks and sources as FP32 offsets from each group's FP64
-       centre, compensated tile sums; 1 = plain FP32, the form the reference's lists
-       compute in (absolute FP32 coordinates, nln/mac.c:1421-1561; plain sums), kept
+       centre; 1 = plain FP32, the form the reference's lists
+       compute in (absolute FP32 coordinates, nln/mac.c:1421-1561), kept
        for comparison.  grav_groups_eval_dev_CUDA always runs the mixed form. */
     int precision;
 } grav_problem;
