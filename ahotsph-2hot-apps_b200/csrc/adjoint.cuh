@@ -84,6 +84,7 @@ struct AdjProblem {
     int ewald;
     const int64_t *cptr;
     const uint32_t *clist;
+    int ewsplit;             // parts of a group's correction list (warps), as in the forward
     EwTab ew;
     float ew_self;
     const EwStored *ewm;     // the forward's per-group moments
@@ -847,48 +848,34 @@ __device__ __forceinline__ float ew_D(const float *o, const float *f5, int q) {
     return q < ew::kNQ4 ? o[q] : f5[q - ew::kNQ4];
 }
 
+// The moment dual of order K, added to the cell's independent components
+// (b2 <= 1).  D is harmonic, and its interpolation keeps that, so the sums
+// over a are already trace-free in b but for the constant Laplacian of C
+// (K = 2, a = 0): nothing else is formed, and no projection is needed.
 template <int K, int SMAX>
 __device__ __forceinline__ void ew_adj_moment(const float *Mb, const float *o, const float *f5,
-                                              float *G) {
+                                              float trace, double *dst) {
     constexpr float ik = 1.f / (float)fact(K);
-#pragma unroll
-    for (int b0 = 0; b0 <= K; b0++)
-#pragma unroll
-        for (int b1 = 0; b1 <= K; b1++) {
-            if (b0 + b1 > K)
-                continue;
-            const int b2 = K - b0 - b1;
-            float acc = 0.f;
-#pragma unroll
-            for (int a0 = 0; a0 <= SMAX; a0++)
-#pragma unroll
-                for (int a1 = 0; a1 <= SMAX; a1++)
-#pragma unroll
-                    for (int a2 = 0; a2 <= SMAX; a2++) {
-                        if (a0 + a1 + a2 > SMAX)
-                            continue;
-                        acc = fmaf(Mb[ew::idx(a0, a1, a2)],
-                                   ew_D(o, f5, ew::idx(a0 + b0, a1 + b1, a2 + b2)), acc);
-                    }
-            G[ew::idx(b0, b1, b2) - ew::base(K)] = acc * ik;
-        }
-}
-
-// The trace-free part of a moment dual of order K, added to the cell's
-// independent components (a2 <= 1): 2K + 1 atomics instead of (K+1)(K+2)/2.
-template <int K>
-__device__ __forceinline__ void add_indep(float *G, double *dst) {
-    if (K == 2)
-        stf2(G);
-    else if (K == 3)
-        stf3(G);
-    else
-        stf4(G);
     int k = 0;
 #pragma unroll
-    for (int p = 0; p < mi_n(K); p++)
-        if (mi_a2(p) <= 1)
-            atomicAdd(dst + k++, (double)G[p]);
+    for (int p = 0; p < mi_n(K); p++) {
+        const int b1 = mi_a1(p), b2 = mi_a2(p), b0 = K - b1 - b2;
+        if (b2 > 1)
+            continue;
+        float acc = K == 2 && (b0 == 2 || b1 == 2) ? Mb[0] * trace * (-1.f / 3.f) : 0.f;
+#pragma unroll
+        for (int a0 = 0; a0 <= SMAX; a0++)
+#pragma unroll
+            for (int a1 = 0; a1 <= SMAX; a1++)
+#pragma unroll
+                for (int a2 = 0; a2 <= SMAX; a2++) {
+                    if (a0 + a1 + a2 > SMAX)
+                        continue;
+                    acc = fmaf(Mb[ew::idx(a0, a1, a2)],
+                               ew_D(o, f5, ew::idx(a0 + b0, a1 + b1, a2 + b2)), acc);
+                }
+        atomicAdd(dst + k++, (double)(acc * ik));
+    }
 }
 
 // N[g] += sum_{|b| = K} S[b] / b! Mbar[g - b] for |g| <= 4
@@ -918,7 +905,9 @@ __device__ __forceinline__ void ew_adj_conv(const float *S, const float *Mb, flo
 }
 
 __global__ void __launch_bounds__(64) k_adjoint_ewald_entries(AdjProblem P) {
-    const int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int64_t g = u / P.ewsplit;
+    const int part = (int)(u % P.ewsplit);
     const int lane = threadIdx.x & 31;
     __shared__ float mb_s[2][36];  // the group's Mbar, read by every lane alike
     float *Mb = mb_s[threadIdx.x >> 5];
@@ -931,7 +920,9 @@ __global__ void __launch_bounds__(64) k_adjoint_ewald_entries(AdjProblem P) {
     const nln_group G = P.groups[g];
     const double c[3] = {G.cen[0], G.cen[1], G.cen[2]};
     const uint32_t nb = (uint32_t)P.nbodies;
-    for (int64_t k = P.cptr[g] + lane; k < P.cptr[g + 1]; k += 32) {
+    const int64_t first = P.cptr[g], tiles = (P.cptr[g + 1] - first + 31) / 32;
+    const int64_t end = min(P.cptr[g + 1], first + tiles * (part + 1) / P.ewsplit * 32);
+    for (int64_t k = first + tiles * part / P.ewsplit * 32 + lane; k < end; k += 32) {
         const uint32_t ent = P.clist[k];
         const uint32_t idx = ent & NLN_IDX_MASK;
         if (idx >= (uint32_t)P.ntab[0] || (ent >> NLN_IDX_BITS) > 26u)
@@ -967,19 +958,15 @@ __global__ void __launch_bounds__(64) k_adjoint_ewald_entries(AdjProblem P) {
             float S[15];
             double *gc = P.gcell + (size_t)(idx - nb) * kCellAdj;
             double *gi = P.gstf + (size_t)(idx - nb) * kStfIndep;
-            float G[15];
             ew_quad(h->R, h->q2, S);
             ew_adj_conv<2>(S, Mb, N);
-            ew_adj_moment<2, 3>(Mb, o, f5, G);
-            add_indep<2>(G, gi);
+            ew_adj_moment<2, 3>(Mb, o, f5, P.ew.trace, gi);
             ew_oct(h->R, h->q3, S);
             ew_adj_conv<3>(S, Mb, N);
-            ew_adj_moment<3, 2>(Mb, o, f5, G);
-            add_indep<3>(G, gi + 5);
+            ew_adj_moment<3, 2>(Mb, o, f5, P.ew.trace, gi + 5);
             ew_hex(h->R, h->q4, S);
             ew_adj_conv<4>(S, Mb, N);
-            ew_adj_moment<4, 1>(Mb, o, f5, G);
-            add_indep<4>(G, gi + 12);
+            ew_adj_moment<4, 1>(Mb, o, f5, P.ew.trace, gi + 12);
             atomicAdd(gc + kAdjB2, (double)(Mb[0] * (1.f / 6.f) * P.ew.trace));
         }
         float dX[3] = {0.f, 0.f, 0.f};
@@ -1274,6 +1261,7 @@ extern "C" int grav_plan_adjoint_CUDA(grav_plan *pl, const float *wu, float *gra
     P.ewald = pl->dp.ewald;
     P.cptr = pl->dp.cptr;
     P.clist = pl->dp.clist;
+    P.ewsplit = std::max(1, pl->dp.ewsplit);
     P.ew = pl->dp.ew;
     P.ew_self = pl->dp.ew_self;
     P.ewm = pl->ewm;
@@ -1289,7 +1277,7 @@ extern "C" int grav_plan_adjoint_CUDA(grav_plan *pl, const float *wu, float *gra
     GC_CHECK(cudaGetLastError());
     if (P.ewald && ng > 0) {
         k_adjoint_ewald_groups<<<(unsigned)((ng + 3) / 4), 128, 0, st>>>(P);
-        k_adjoint_ewald_entries<<<(unsigned)((ng + 1) / 2), 64, 0, st>>>(P);
+        k_adjoint_ewald_entries<<<(unsigned)((ng * P.ewsplit + 1) / 2), 64, 0, st>>>(P);
         GC_CHECK(cudaGetLastError());
     }
     if (nc > 0)
