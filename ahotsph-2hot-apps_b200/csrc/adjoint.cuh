@@ -836,9 +836,14 @@ __global__ void k_adjoint_ewald_groups(AdjProblem P) {
     }
 }
 
-// Periodic correction, source side: one warp per group, lanes over its
-// correction entries (as ewald_moments_loop).  Per entry at y = X + shift - c
-// with the table values D (orders 0..5) there:
+// Periodic correction, source side: a warp per part of a group's correction
+// list, lanes over its entries.  The lists are split where the forward splits
+// them (too few groups for the SMs); with that, and no components formed that
+// the harmonic ones give, 1.08 -> 0.77 ms on a 32^3 box.  Bounded by its own
+// arithmetic at three warps a scheduler (168 registers): flushing the sums with
+// neighbour lanes on neighbour doubles, a third of the sectors, gave 0.74 ms
+// here but slowed the list adjoints, which share the way, by 5 to 10 %.
+// Per entry at y = X + shift - c with the table values D (orders 0..5) there:
 //   dL/dm = sum_a Mbar[a] D[a],   dL/dX_l = sum_{|g|<=4} N[g] D[g + e_l],
 //   N[g] = m Mbar[g] + sum_K sum_{|b|=K, b<=g} A_K[b]/b! Mbar[g - b],
 //   dL/dA_K[b] = (1/K!) sum_a Mbar[a] D[a + b] over the forward's terms
