@@ -4,7 +4,7 @@ The search space is grav_tuning: warps per block (4 or 8), resident blocks
 per SM (0 = as many as registers and shared memory allow, or a cap), the
 list-chunk length of each kind (the work-item size; the automatic choice
 times a scale) and, for periodic plans, where the Ewald correction moments
-run (a side stream beside the list kernels, or the finish pass).  Each
+run (a side stream beside the list kernels, or their own).  Each
 candidate is applied with grav_plan_retune_CUDA, which rebuilds only the
 work queue, and timed with CUDA events over a few evaluations; the search
 is coordinate-wise (launch shape, then chunk scale, then the moments'

@@ -199,9 +199,9 @@ typedef struct grav_problem {
     const uint32_t *zlist[4];
     /* Arithmetic of the list kernels (grav_groups_upload_CUDA and grav_groups_CUDA):
        0 = mixed (default): sinks and sources as FP32 offsets from each group's FP64
-       centre; 1 = plain FP32, the form the reference's lists
-       compute in (absolute FP32 coordinates, nln/mac.c:1421-1561), kept
-       for comparison.  grav_groups_eval_dev_CUDA always runs the mixed form. */
+       centre; 1 = plain FP32, the form the reference's lists compute in (absolute
+       FP32 coordinates, nln/mac.c:1421-1561), kept for comparison.
+       grav_groups_eval_dev_CUDA always runs the mixed form. */
     int precision;
 } grav_problem;
 
@@ -209,7 +209,7 @@ typedef struct grav_plan grav_plan;
 
 /* Tile shapes of the batched kernels (the autotuner's search space). */
 typedef struct grav_tuning {
-    int warps_per_block;        /* 4, 8 or 16 */
+    int warps_per_block;        /* 4, 8 or 16; the list kernels run in blocks of 4 for all */
     int chunk_p;                /* max point records per work item (split long lists) */
     int chunk_q;                /* max quadrupole cells per work item */
     int chunk_h;                /* max order-4 cells per work item */
