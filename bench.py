@@ -59,7 +59,7 @@ FLOPS = np.array([23, 23, 66, 217], np.float64)
 # DRAM bytes (read + write) per interaction of each list kernel, from one ncu
 # capture of the kernels on the periodic 128^3 box (MAC 1e-4); a launch's
 # traffic is this times its interactions (traffic grows with list entries)
-DRAM_BYTES_PER_INTERACTION = {"hexa": 0.2007, "quad": 0.193, "point": 0.164}
+DRAM_BYTES_PER_INTERACTION = {"hexa": 0.2013, "quad": 0.1836, "point": 0.1987}
 ALL_CONFIGS = ("plummer64k", "box128", "batch1024", "adjoint", "kdk256")
 # blocks that run only when named: the periodic adjoint alone (--adjoint-workload)
 EXTRA_CONFIGS = ("adjoint_periodic",)
