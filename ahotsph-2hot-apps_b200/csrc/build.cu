@@ -582,8 +582,8 @@ __global__ void k_groups(int64_t ng, const int64_t *first, const int32_t *count,
 // cell is decided twice.  Bounded by the FP64 decision and the scattered
 // 80-byte cell records, with the walk's parallelism 32 times the group count;
 // one thread per group had too few threads below a million bodies and wrote
-// every entry uncoalesced (both passes, 100k-body sphere 50.6 -> 2.7 ms, 96^3
-// box 71 -> 17 ms, 160^3 238 -> 121 ms).  Issue slots are 62 to 71 % busy;
+// every entry uncoalesced (both passes, 100k-body sphere 50.6 -> 1.65 ms, 96^3
+// box 71 -> 16 ms, 160^3 238 -> 117 ms).  Issue slots are 62 to 71 % busy;
 // single-precision bounds in place of the FP64 square roots changed nothing.
 constexpr int kWalkWarps = 4;
 // Stack entries per warp, of which the last NLN_WALK_STACK are kept for an
