@@ -1427,6 +1427,7 @@ int gpu_make_queue(const int64_t *const ptr[3], int64_t ng, const int64_t chunk[
         items[k] = nullptr;
         nitems[k] = 0;
     }
+    Item *made[3] = {nullptr, nullptr, nullptr};  // the caller's once nothing can fail any more
     int64_t *nfull = nullptr, *off = nullptr, *nall = nullptr, *slots = nullptr;
     uint32_t *rem = nullptr, *rem_s = nullptr;
     int32_t *gid = nullptr, *gid_s = nullptr;
@@ -1472,20 +1473,23 @@ int gpu_make_queue(const int64_t *const ptr[3], int64_t ng, const int64_t chunk[
     for (int k = 0; k < 3; k++) {
         if (!ptr[k] || tot[k] + nrem[k] == 0)
             continue;
-        BC(B.get(&items[k], tot[k] + nrem[k]));
-        nitems[k] = (int)(tot[k] + nrem[k]);
-        k_queue_full<<<grid_of(ng), kThreads, 0, st>>>(Q, k, ng, off + k * (ng + 1), slots, items[k]);
+        BC(B.get(&made[k], tot[k] + nrem[k]));
+        k_queue_full<<<grid_of(ng), kThreads, 0, st>>>(Q, k, ng, off + k * (ng + 1), slots, made[k]);
         BC(cudaGetLastError());
         if (nrem[k] > 0) {
             k_queue_rem<<<grid_of(nrem[k]), kThreads, 0, st>>>(Q, k, nrem[k], gid_s + k * ng, slots,
-                                                                items[k] + tot[k]);
+                                                                made[k] + tot[k]);
             BC(cudaGetLastError());
         }
     }
     BC(cudaStreamSynchronize(st));
     *gslot = slots;
     *nslots = tot[3];
-    for (int k = 0; k < 3; k++) B.release(items[k]);
+    for (int k = 0; k < 3; k++) {
+        items[k] = made[k];
+        nitems[k] = made[k] ? (int)(tot[k] + nrem[k]) : 0;
+        B.release(made[k]);
+    }
     B.release(slots);
     return 0;
 }

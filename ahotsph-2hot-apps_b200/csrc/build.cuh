@@ -58,7 +58,8 @@ void dev_tree_free(DevTree &t, cudaMemPool_t pool = nullptr);
 // slots group by group (a group's point items, then quadrupole, then order
 // 4), items per kind the full chunks in that order, then the groups'
 // remainders by length, longest first.  items, gslot (ngroups + 1): from the
-// pool, the caller's to free.  Enqueued on st and synchronised.
+// pool, the caller's to free; nothing (items null, gslot untouched) when it
+// fails.  Enqueued on st and synchronised.
 int gpu_make_queue(const int64_t *const ptr[3], int64_t ng, const int64_t chunk[3], cudaStream_t st,
                    cudaMemPool_t pool, Item *items[3], int nitems[3], int64_t **gslot,
                    int64_t *nslots);

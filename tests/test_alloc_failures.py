@@ -1,0 +1,88 @@
+"""CPU: what the host paths do with device memory when an allocation fails,
+on a runtime that needs no GPU (fake_cudart.cpp, preloaded in a child
+process): every buffer of a failed call is freed once and only once."""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import PKG_ROOT, REPO
+
+# a two-body plan built on the (fake) device, evaluated, and its adjoint; returns the status
+PRELUDE = """
+import ctypes, json, os, sys
+sys.path.insert(0, {pkg!r})
+import numpy as np
+from pgrav import gravcuda as gc
+from pgrav.host import Params
+L = gc.lib()
+fake = ctypes.CDLL({fake!r})
+fake.fake_allocs_before.restype = ctypes.c_long
+bodies = np.zeros((16, 4), np.float32)
+at = bodies.ctypes.data + -bodies.ctypes.data % 16
+def counts():
+    c = (ctypes.c_long * 6)()
+    fake.fake_counts(c)
+    return dict(zip(("allocs", "live", "double", "trims", "pending", "error"), c))
+def build(box):
+    p = Params(16, 32, 7, 20, 1e-3, 0.0, 0.0, box, 0, 0, 0.2, 0.0)
+    h = ctypes.c_void_p()
+    rc = L.grav_plan_build_CUDA(ctypes.byref(p), at, 2, 1e-4, 1.0, int(box > 0), None, ctypes.byref(h))
+    if rc == 0:
+        rc = L.grav_groups_eval_CUDA(h, None) or L.grav_plan_adjoint_CUDA(h, at, at, None)
+    return rc, h
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    from pgrav import _build
+    _build.build_all()
+    so = str(tmp_path_factory.mktemp("fake") / "fake_cudart.so")
+    subprocess.run([_build._cxx(), "-O1", "-std=c++17", "-fPIC", "-shared", "-o", so,
+                    os.path.join(REPO, "tests", "fake_cudart.cpp")], check=True)
+
+    def go(body):
+        code = PRELUDE.format(pkg=PKG_ROOT, fake=so) + body
+        r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600,
+                           env=dict(os.environ, LD_PRELOAD=so))
+        assert r.returncode == 0, r.stderr[-2000:]
+        return json.loads(r.stdout.splitlines()[-1])
+
+    return go
+
+
+# every allocation of a call fails in turn: status and memory counts of each
+FAIL_EACH = """
+res = []
+for box in (0.0, 1.0):
+    fake.fake_reset(0, 0)
+    rc, h = build(box)
+    assert rc == 0, rc
+    last, queue = counts()["allocs"], fake.fake_allocs_before(b"k_queue_count")
+    L.grav_plan_free(h)
+    assert counts()["live"] == 0
+    for k in {range}:
+        fake.fake_reset(k, 0)
+        rc, h = build(box)
+        if h:
+            L.grav_plan_free(h)
+        L.gravcuda_clear_status()
+        fake.cudaGetLastError()
+        res.append([box, k, rc, counts()])
+print(json.dumps(res))
+"""
+
+
+def check_freed_once(out):
+    assert len(out) >= 40
+    for box, k, rc, c in out:
+        assert rc != 0 and c["double"] == 0 and c["live"] == 0, (box, k, rc, c)
+
+
+def test_a_failed_plan_frees_every_buffer_once(run):
+    """The work queue of a device-built tree, the plan around it, its
+    evaluation and adjoint: the k-th allocation fails, for every k."""
+    check_freed_once(run(FAIL_EACH.format(range="range(queue + 1, last + 1)")))
