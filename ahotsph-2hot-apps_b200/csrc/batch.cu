@@ -2175,10 +2175,8 @@ int build_plan(const nln_params *params, const float4 *bodies, int64_t n, double
         return rc;
     DevTree T;
     const double t0 = now_s();
-    if (int rc = gpu_tree_build(*params, bodies, n, 0, T, pool)) {
-        dev_tree_free(T, pool);
+    if (int rc = gpu_tree_build(*params, bodies, n, 0, T, pool))
         return rc;
-    }
     grav_problem hp{};
     hp.nbodies = T.n;
     hp.ncells = T.ncells;

@@ -946,25 +946,9 @@ int exclusive_scan(Bufs &B, const T *in, T *out, int64_t n, cudaStream_t st) {
     return 0;
 }
 
-}  // namespace
-
-void dev_tree_free(DevTree &t, cudaMemPool_t pool) {
-    void *ps[] = {t.points, t.qcells, t.hcells, t.groups, t.list[0], t.list[1], t.list[2],
-                  t.list[3], t.order, t.cell_first, t.cell_count, t.cell_child, t.cell_nchild,
-                  t.ptr[0], t.ptr[1], t.ptr[2], t.ptr[3]};
-    for (void *p : ps)
-        if (p) {
-            if (pool)
-                cudaFreeAsync(p, 0);
-            else
-                cudaFree(p);
-        }
-    t = DevTree{};
-}
-
-int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_t st,
-                   DevTree &out, cudaMemPool_t pool) {
-    out = DevTree{};
+// The build; on failure every buffer is freed and out's pointers are stale.
+int build_tree(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_t st, DevTree &out,
+               cudaMemPool_t pool) {
     if (!bodies || n <= 0)
         return gc::set_status(-1, "GPU tree build: no bodies");
     if (p.leaf_max < 1 || p.leaf_max > 65535 || p.group_max < 1 || p.group_max > 64 ||
@@ -1337,6 +1321,17 @@ int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStr
                     dptr[0], dptr[1], dptr[2], dptr[3]};
     for (void *q : keep) B.release(q);
     return 0;
+}
+
+}  // namespace
+
+int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_t st,
+                   DevTree &out, cudaMemPool_t pool) {
+    out = DevTree{};
+    const int rc = build_tree(p, bodies, n, st, out, pool);
+    if (rc)
+        out = DevTree{};
+    return rc;
 }
 
 // ------------------------------------------------------------ work queue

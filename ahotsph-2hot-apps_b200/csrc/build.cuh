@@ -45,13 +45,13 @@ struct DevTree {
 // lists of n bodies (device float4 x, y, z, m, any order) with the
 // semantics and arithmetic of nlnhost.h's nln_tree_build + nln_tree_walk
 // (bit-identical results); enqueued on st and synchronised.  Returns 0, -1
-// for bad arguments or positions (message recorded), or a CUDA status.
+// for bad arguments or positions (message recorded), or a CUDA status; out is
+// empty then.
 // pool: when set, every device buffer comes from it (stream-ordered on st)
 // and is returned to it; the tree's buffers must then be freed with
 // cudaFreeAsync.
 int gpu_tree_build(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_t st,
                    DevTree &out, cudaMemPool_t pool = nullptr);
-void dev_tree_free(DevTree &t, cudaMemPool_t pool = nullptr);
 
 // The work queue of lists whose offsets ptr[k] (ngroups + 1 each, or null:
 // no lists of that kind) are on the device, in chunks of chunk[k] entries:

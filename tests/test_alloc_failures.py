@@ -86,3 +86,8 @@ def test_a_failed_plan_frees_every_buffer_once(run):
     """The work queue of a device-built tree, the plan around it, its
     evaluation and adjoint: the k-th allocation fails, for every k."""
     check_freed_once(run(FAIL_EACH.format(range="range(queue + 1, last + 1)")))
+
+
+def test_a_failed_tree_frees_every_buffer_once(run):
+    """The tree, its tables and its lists: the k-th allocation fails."""
+    check_freed_once(run(FAIL_EACH.format(range="range(1, queue + 1)")))
