@@ -60,6 +60,9 @@ int set_status(int code, const char *fmt, ...) {
 }
 
 int cuda_status(cudaError_t err, const char *what) {
+    // reported here: the runtime keeps a failed call's error until it is asked
+    // for, and the next launch's check would take it for its own
+    cudaGetLastError();
     return set_status((int)err, "%s: %s", what, cudaGetErrorString(err));
 }
 }  // namespace gc

@@ -91,3 +91,31 @@ def test_a_failed_plan_frees_every_buffer_once(run):
 def test_a_failed_tree_frees_every_buffer_once(run):
     """The tree, its tables and its lists: the k-th allocation fails."""
     check_freed_once(run(FAIL_EACH.format(range="range(1, queue + 1)")))
+
+
+def test_a_failed_call_does_not_fail_the_next(run):
+    """A build after one whose k-th allocation failed succeeds, for every k."""
+    out = run("""
+res = []
+fake.fake_reset(0, 0)
+rc, h = build(0.0)
+total = counts()["allocs"]
+L.grav_plan_free(h)
+for k in range(1, total + 1):
+    fake.fake_reset(k, 0)
+    rc, h = build(0.0)
+    if h:
+        L.grav_plan_free(h)
+    L.gravcuda_clear_status()
+    fake.fake_reset(0, 0)
+    again, h = build(0.0)
+    if h:
+        L.grav_plan_free(h)
+    L.gravcuda_clear_status()
+    fake.cudaGetLastError()
+    res.append([k, rc, again])
+print(json.dumps(res))
+""")
+    assert len(out) >= 60
+    for k, failed, again in out:
+        assert failed != 0 and again == 0, (k, failed, again)
