@@ -1161,7 +1161,7 @@ struct grav_adjoint_state {
     double *gbody = nullptr, *gcell = nullptr, *mbar = nullptr, *gstf = nullptr;
     template <typename T>
     cudaError_t get(T **p, size_t n) {
-        return pool ? cudaMallocFromPoolAsync((void **)p, n * sizeof(T), pool, 0)
+        return pool ? gc::pool_malloc((void **)p, n * sizeof(T), pool, 0)
                     : cudaMalloc((void **)p, n * sizeof(T));
     }
     ~grav_adjoint_state() {

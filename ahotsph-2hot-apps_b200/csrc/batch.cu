@@ -1162,15 +1162,9 @@ int dev_copy(grav_plan *pl, const T *src, size_t n, T **dst) {
     *dst = nullptr;
     if (n == 0)
         return 0;
-    if (pl->pool) {
-        if (cudaMallocFromPoolAsync((void **)dst, n * sizeof(T), pl->pool, 0) != cudaSuccess) {
-            // the pool's reserved but unused memory may be what is missing
-            cudaGetLastError();
-            cudaStreamSynchronize(0);
-            cudaMemPoolTrimTo(pl->pool, 0);
-            GC_CHECK(cudaMallocFromPoolAsync((void **)dst, n * sizeof(T), pl->pool, 0));
-        }
-    } else
+    if (pl->pool)
+        GC_CHECK(gc::pool_malloc((void **)dst, n * sizeof(T), pl->pool, 0));
+    else
         GC_CHECK(cudaMalloc((void **)dst, n * sizeof(T)));
     pl->allocs.push_back(*dst);
     if (src)
@@ -2252,8 +2246,8 @@ extern "C" int grav_build_eval_CUDA(const nln_params *params, const float *bodie
         return rc;
     float4 *dev = nullptr, *out = nullptr;
     const size_t bytes = (size_t)n * sizeof(float4);
-    GC_CHECK(cudaMallocFromPoolAsync((void **)&dev, bytes, pool, 0));
-    cudaError_t e = cudaMallocFromPoolAsync((void **)&out, bytes, pool, 0);
+    GC_CHECK(gc::pool_malloc((void **)&dev, bytes, pool, 0));
+    cudaError_t e = gc::pool_malloc((void **)&out, bytes, pool, 0);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(dev, bodies, bytes, cudaMemcpyHostToDevice, 0);
     if (e != cudaSuccess) {

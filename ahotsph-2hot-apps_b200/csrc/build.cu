@@ -75,7 +75,7 @@ struct Bufs {
     cudaError_t get(T **p, size_t n) {
         *p = nullptr;
         const size_t bytes = std::max<size_t>(1, n) * sizeof(T);
-        cudaError_t e = pool ? cudaMallocFromPoolAsync((void **)p, bytes, pool, st)
+        cudaError_t e = pool ? gc::pool_malloc((void **)p, bytes, pool, st)
                              : cudaMalloc((void **)p, bytes);
         if (e == cudaSuccess)
             held.push_back(*p);

@@ -14,6 +14,20 @@ extern int g_error_mode;
 int set_status(int code, const char *fmt, ...);
 int cuda_status(cudaError_t err, const char *what);
 
+// Device memory from a pool, stream-ordered.  The pools here keep freed memory
+// reserved: where memory runs out it may be what is missing, so it is given
+// back to the device and the allocation tried once more.
+inline cudaError_t pool_malloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t st) {
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaStreamSynchronize(st);
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    }
+    return e;
+}
+
 }  // namespace gc
 
 #define GC_CHECK(call)                                              \

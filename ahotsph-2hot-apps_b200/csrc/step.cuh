@@ -420,7 +420,7 @@ int set_tree_adopt(grav_plan *pl, const DevTree &T, cudaMemPool_t pool) {
     // the builder makes cells level by level: no order array is needed
     for (size_t l = T.level_start.size() - 1; l-- > 0;)
         S->levels.push_back({T.level_start[l], T.level_start[l + 1]});
-    cudaError_t e = cudaMallocFromPoolAsync((void **)&S->raw, (size_t)nc * kRaw * sizeof(double), pool, 0);
+    cudaError_t e = gc::pool_malloc((void **)&S->raw, (size_t)nc * kRaw * sizeof(double), pool, 0);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(0);  // other streams use it
     if (e != cudaSuccess) {

@@ -119,3 +119,27 @@ print(json.dumps(res))
     assert len(out) >= 60
     for k, failed, again in out:
         assert failed != 0 and again == 0, (k, failed, again)
+
+
+def test_the_pool_gives_its_reserve_back_first(run):
+    """The k-th allocation of a build, an evaluation and an adjoint fails until
+    the pool has given back what it keeps reserved: every call succeeds."""
+    out = run("""
+res = []
+for box in (0.0, 1.0):
+    fake.fake_reset(0, 0)
+    rc, h = build(box)
+    total = counts()["allocs"]
+    L.grav_plan_free(h)
+    for k in range(1, total + 1):
+        fake.fake_reset(k, 1)
+        rc, h = build(box)
+        res.append([box, k, rc, counts()])
+        if h:
+            L.grav_plan_free(h)
+        L.gravcuda_clear_status()
+print(json.dumps(res))
+""")
+    assert len(out) >= 150
+    for box, k, rc, c in out:
+        assert rc == 0 and c["trims"] == 1, (box, k, rc, c)
