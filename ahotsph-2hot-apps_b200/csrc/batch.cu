@@ -106,6 +106,11 @@ struct DevProblem {
     int cstride;
 };
 
+// No entry in this lane: a value that no word of a list takes.  An all-ones
+// word in a list is as invalid as the one below it, for which it passes.
+constexpr uint32_t kNone = 0xffffffffu;
+__device__ __forceinline__ uint32_t list_word(const uint32_t *p) { return min(__ldg(p), kNone - 1u); }
+
 // Image code (0..26) to the image's shift: (code / 9 - 1, code / 3 % 3 - 1,
 // code % 3 - 1) box.
 __device__ __forceinline__ void decode_shift(uint32_t code, double box, double &sx, double &sy,
@@ -634,7 +639,6 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
     const uint32_t nb = PLAIN || !P.ccen ? ntab : ntab - (uint32_t)P.ncells;  // cells from here on
     const float2 e2 = splat2(P.eps2);
     constexpr int NP = kPointTile / 64, NE = 2 * NP;  // record pairs, records per lane
-    constexpr uint32_t kNone = 0xffffffffu;           // no entry
     for (;;) {
         int it = 0;
         if (lane == 0)
@@ -650,7 +654,7 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
 #pragma unroll
             for (int j = 0; j < NE; j++) {
                 const int64_t k = k0 + 32 * j + lane;
-                e[j] = k < item.end ? __ldg(list + k) : kNone;
+                e[j] = k < item.end ? list_word(list + k) : kNone;
             }
         };
         // Start this lane's copies of its entries' records.  Entries are
@@ -831,7 +835,6 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
     EwStage *stg = reinterpret_cast<EwStage *>(ewsm + (size_t)(threadIdx.x >> 5) * kEwWarpBytes);
     const uint32_t ntab = (uint32_t)P.ntab[0];
     const uint32_t nb = ntab - (uint32_t)P.ncells;
-    constexpr uint32_t kNone = 0xffffffffu;
     // one source of the pipeline: list word (kNone: no entry in this lane)
     // and its position (FP64) with, for a body, its mass
     struct Src {
@@ -859,7 +862,7 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
         // the list word is checked where it is used, a tile after its load
         auto entry = [&](int t) -> uint32_t {
             const int64_t k = U.cb + (int64_t)(U.t0 + t) * 32 + lane;
-            return (t < ntile && k < U.ce) ? __ldg(P.clist + k) : kNone;
+            return (t < ntile && k < U.ce) ? list_word(P.clist + k) : kNone;
         };
         auto source = [&](uint32_t e) -> Src {
             Src r{kNone, 0.0, 0.0, 0.0, 0.f};
