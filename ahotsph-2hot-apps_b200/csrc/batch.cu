@@ -1857,7 +1857,9 @@ int launch_kind(grav_plan *pl, const DevProblem &dp, cudaStream_t st, Chain *cha
     GC_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int fit = 0;
     GC_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, wpb * 32, smem));
-    const int per_sm = pl->tune.blocks_per_sm > 0 ? std::min(pl->tune.blocks_per_sm, fit) : fit;
+    // a cap counts the caller's blocks, of warps_per_block warps each
+    const int64_t cap = ((int64_t)pl->tune.blocks_per_sm * pl->tune.warps_per_block + wpb - 1) / wpb;
+    const int per_sm = cap > 0 ? (int)std::min<int64_t>(cap, fit) : fit;
     const int blocks = std::min(std::max(1, per_sm) * pl->nsm, (dp.nitems[KIND] + wpb - 1) / wpb);
     CUtensorMap tm = pl->tmap[KIND];
     DevProblem d = dp;

@@ -209,11 +209,13 @@ typedef struct grav_plan grav_plan;
 
 /* Tile shapes of the batched kernels (the autotuner's search space). */
 typedef struct grav_tuning {
-    int warps_per_block;        /* 4, 8 or 16; the list kernels run in blocks of 4 for all */
+    int warps_per_block;        /* 1 to 8 (others: 8); the list kernels run in blocks of this
+                                   many warps up to 4, and of 4 beyond */
     int chunk_p;                /* max point records per work item (split long lists) */
     int chunk_q;                /* max quadrupole cells per work item */
     int chunk_h;                /* max order-4 cells per work item */
-    int blocks_per_sm;          /* persistent grid = blocks_per_sm x SM count (0: as many as fit) */
+    int blocks_per_sm;          /* persistent grids hold at most blocks_per_sm x warps_per_block
+                                   warps per SM (0: as many as fit) */
     int ewald_n;                /* Ewald table nodes per axis (0: 32) */
     int ewald_side;             /* periodic: where the Ewald correction moments run.  > 0: on a
                                    side stream beside the list kernels, in this many two-warp

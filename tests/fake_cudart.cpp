@@ -3,7 +3,8 @@
 // and an allocation can be made to fail.  It counts what a host path does
 // with its memory: live buffers, buffers freed twice, and work left on the
 // default stream.  With the emulated kernels a build sees two bodies in one
-// leaf cell, one sink group, and one list entry of every kind.
+// leaf cell, one sink group, and lists of every kind whose queue claims 8192
+// items.
 #include <stddef.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -20,6 +21,7 @@ constexpr int kOutOfMemory = 2, kInvalidValue = 1;
 std::recursive_mutex mu;
 std::map<const void *, std::string> names;     // host stub -> kernel name
 std::map<const void *, int> smem_limit;        // kernel -> its dynamic shared memory attribute
+std::map<std::string, unsigned> grids;         // kernel -> blocks of its last launch (x)
 std::map<std::string, long> first_at;          // kernel -> allocations made before its first launch
 std::set<void *> live, host_live;
 int last_error = 0;
@@ -92,7 +94,7 @@ void emulate(const std::string &f, void **a) {
         int64_t *all = arg<int64_t *>(a, 5);
         all[0] = 3;
     } else if (is("k_queue_nrem")) {
-        for (int k = 0; k < 3; k++) arg<int64_t *>(a, 2)[k] = 1;
+        for (int k = 0; k < 3; k++) arg<int64_t *>(a, 2)[k] = 8192;
     } else if (is("DeviceScanKernel")) {  // exclusive sums of the int64 counts
         const int64_t *in = arg<const int64_t *>(a, 0);
         int64_t *out = arg<int64_t *>(a, 1), s = 0;
@@ -136,6 +138,12 @@ long fake_allocs_before(const char *kernel) {
             return k.second;
     return -1;
 }
+unsigned fake_grid(const char *kernel) {
+    for (auto &k : grids)
+        if (k.first.find(kernel) != std::string::npos)
+            return k.second;
+    return 0;
+}
 int fake_smem_limit(const char *kernel) {
     for (auto &k : smem_limit)
         if (names[k.first].find(kernel) != std::string::npos)
@@ -175,8 +183,9 @@ int cudaLaunchKernel(const void *f, dim3_, dim3_, void **args, size_t, void *st)
     on(st);
     return 0;
 }
-int cudaLaunchKernelExC(const void *, const void *f, void **args) {
+int cudaLaunchKernelExC(const dim3_ *cfg, const void *f, void **args) {  // the grid comes first
     launched(f, args);
+    grids[names[f]] = cfg->x;
     return 0;
 }
 

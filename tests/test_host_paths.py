@@ -1,6 +1,6 @@
-"""CPU: what the host paths do with device memory when an allocation fails,
-on a runtime that needs no GPU (fake_cudart.cpp, preloaded in a child
-process): every buffer of a failed call is freed once and only once."""
+"""CPU: the host paths of libgravcuda.so on a runtime that needs no GPU
+(fake_cudart.cpp, preloaded in a child process): what they do with device
+memory when an allocation fails, and how they launch."""
 import json
 import os
 import subprocess
@@ -26,10 +26,11 @@ def counts():
     c = (ctypes.c_long * 6)()
     fake.fake_counts(c)
     return dict(zip(("allocs", "live", "double", "trims", "pending", "error"), c))
-def build(box):
+def build(box, tuning=None):
+    t = ctypes.byref(gc.Tuning(*tuning)) if tuning else None
     p = Params(16, 32, 7, 20, 1e-3, 0.0, 0.0, box, 0, 0, 0.2, 0.0)
     h = ctypes.c_void_p()
-    rc = L.grav_plan_build_CUDA(ctypes.byref(p), at, 2, 1e-4, 1.0, int(box > 0), None, ctypes.byref(h))
+    rc = L.grav_plan_build_CUDA(ctypes.byref(p), at, 2, 1e-4, 1.0, int(box > 0), t, ctypes.byref(h))
     if rc == 0:
         rc = L.grav_groups_eval_CUDA(h, None) or L.grav_plan_adjoint_CUDA(h, at, at, None)
     return rc, h
@@ -143,3 +144,21 @@ print(json.dumps(res))
     assert len(out) >= 150
     for box, k, rc, c in out:
         assert rc == 0 and c["trims"] == 1, (box, k, rc, c)
+
+
+def test_a_block_cap_counts_blocks_of_the_given_warps(run):
+    """blocks_per_sm caps the list kernels' resident warps at that many blocks
+    of warps_per_block warps, whatever blocks they run in (three blocks fit an
+    SM of 148 here)."""
+    caps = {"8,0": 3, "8,1": 2, "8,2": 3, "4,1": 1, "4,2": 2, "4,4": 3, "2,1": 1, "2,2": 2, "5,1": 2}
+    out = run("""
+res = []
+for w, b in %r:
+    rc, h = build(0.0, (w, 0, 0, 0, b, 0, 0))
+    assert rc == 0
+    res.append([w, b, [fake.fake_grid(k) for k in (b"k_points", b"k_cells")]])
+    L.grav_plan_free(h)
+print(json.dumps(res))
+""" % ([[int(x) for x in k.split(",")] for k in caps],))
+    for w, b, grids in out:
+        assert grids == [caps[f"{w},{b}"] * 148] * 2, (w, b, grids)
