@@ -1,10 +1,11 @@
 """Autotuner of the batched kernels' tile shapes.
 
-The search space is grav_tuning: warps per block (4 or 8), resident blocks
-per SM (0 = as many as registers and shared memory allow, or a cap), the
+The search space is grav_tuning: resident warps per SM (warps per block times
+blocks per SM; 0 blocks = as many as registers and shared memory allow), the
 list-chunk length of each kind (the work-item size; the automatic choice
-times a scale) and, for periodic plans, where the Ewald correction moments
-run (a side stream beside the list kernels, or their own).  Each
+times a scale, in whole tiles) and, for periodic plans, where the Ewald
+correction moments run (a side stream beside the list kernels, or the
+evaluation's own).  Shapes that launch alike are timed once.  Each
 candidate is applied with grav_plan_retune_CUDA, which rebuilds only the
 work queue, and timed with CUDA events over a few evaluations; the search
 is coordinate-wise (launch shape, then chunk scale, then the moments'
@@ -17,7 +18,11 @@ import numpy as np
 
 from . import gravcuda as gc
 
-TILE = 32
+TILES = (256, 128, 64)  # records of a tile of the point, quadrupole and order-4 kernels
+BLOCK_WARPS = 4         # warps of the list kernels' blocks at most
+# the kernels a stored result was measured with: a new number where their best
+# shapes change, which leaves older results unused
+KERNELS = 2
 
 
 def _time(plan, stream, reps):
@@ -34,7 +39,7 @@ def _time(plan, stream, reps):
 
 
 def _scaled(base, s):
-    return int(max(TILE, round(base * s / TILE) * TILE))
+    return [int(max(t, round(b * s / t) * t)) for b, t in zip(base, TILES)]
 
 
 def autotune(plan, reps=3, shapes=((8, 0), (4, 0), (8, 1), (8, 2), (4, 2), (4, 4)),
@@ -45,20 +50,22 @@ def autotune(plan, reps=3, shapes=((8, 0), (4, 0), (8, 1), (8, 2), (4, 2), (4, 4
     import torch
     if cache and key and os.path.exists(cache):
         table = json.load(open(cache))
-        if key in table:
+        if table.get(key, {}).get("kernels") == KERNELS:
             t = gc.Tuning(*table[key]["tuning"])
             plan.retune(t)
             return plan.tuning(), table[key]["trials"]
     stream = torch.cuda.Stream()
     base = plan.tuning()
     base_chunks = (base.chunk_p, base.chunk_q, base.chunk_h)
-    trials = []
+    trials, timed = [], {}
 
     def trial(wpb, bps, s, side=0):
-        t = gc.Tuning(wpb, _scaled(base_chunks[0], s), _scaled(base_chunks[1], s),
-                      _scaled(base_chunks[2], s), bps, base.ewald_n, side)
-        plan.retune(t)
-        ms = _time(plan, stream, reps)
+        t = gc.Tuning(wpb, *_scaled(base_chunks, s), bps, base.ewald_n, side)
+        alike = (min(wpb, BLOCK_WARPS), wpb * bps, t.chunk_p, t.chunk_q, t.chunk_h, side)
+        if alike not in timed:
+            plan.retune(t)
+            timed[alike] = _time(plan, stream, reps)
+        ms = timed[alike]
         trials.append({"warps_per_block": wpb, "blocks_per_sm": bps, "chunk_scale": s,
                        "chunks": [t.chunk_p, t.chunk_q, t.chunk_h], "ewald_side": side, "ms": ms})
         return ms
@@ -72,12 +79,12 @@ def autotune(plan, reps=3, shapes=((8, 0), (4, 0), (8, 1), (8, 2), (4, 2), (4, 4
     if getattr(plan, "ewald", False) and sides:
         best_side = min(((trial(wpb, bps, s, sd), sd) for sd in sides), default=(best_ms, 0))
         side = best_side[1] if best_side[0] < best_ms else 0
-    t = gc.Tuning(wpb, _scaled(base_chunks[0], s), _scaled(base_chunks[1], s),
-                  _scaled(base_chunks[2], s), bps, base.ewald_n, side)
+    t = gc.Tuning(wpb, *_scaled(base_chunks, s), bps, base.ewald_n, side)
     plan.retune(t)
     if cache and key:
         table = json.load(open(cache)) if os.path.exists(cache) else {}
-        table[key] = {"tuning": [t.warps_per_block, t.chunk_p, t.chunk_q, t.chunk_h,
+        table[key] = {"kernels": KERNELS,
+                      "tuning": [t.warps_per_block, t.chunk_p, t.chunk_q, t.chunk_h,
                                  t.blocks_per_sm, t.ewald_n, t.ewald_side], "trials": trials}
         with open(cache, "w") as f:
             json.dump(table, f, indent=1)
