@@ -1034,18 +1034,36 @@ int build_tree(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_
     t0 = now_s();
 
     // ---- cells, level by level: room for two per three bodies at first (spheres and boxes
-    // with leaves of 16 need a quarter of that), four times as many where that is too few
+    // with leaves of 16 need a quarter of that), four times as many where that is too few,
+    // and never more than the list indices could name
     Cells C{};
+    auto get_cells = [&](Cells &D, int64_t c) -> int {
+        BC(B.get(&D.first, c));
+        BC(B.get(&D.count, c));
+        BC(B.get(&D.child, c));
+        BC(B.get(&D.nchild, c));
+        BC(B.get(&D.gc, 3 * c));
+        BC(B.get(&D.side, c));
+        return 0;
+    };
+    auto drop_cells = [&](const Cells &D) {
+        B.drop(D.first);
+        B.drop(D.count);
+        B.drop(D.child);
+        B.drop(D.nchild);
+        B.drop(D.gc);
+        B.drop(D.side);
+    };
+    auto too_many = [] {
+        return gc::set_status(-1, "GPU tree build: bodies plus cells exceed 27-bit list indices");
+    };
     int64_t hstate[2 * (kMaxLevels + 1)];
-    for (int64_t cap = std::max<int64_t>(1024, 2 * n / 3);; cap *= 4) {
+    const int64_t most = (int64_t)NLN_IDX_MASK - n;
+    for (int64_t cap = std::min(most, std::max<int64_t>(1024, 2 * n / 3));; cap = std::min(most, 4 * cap)) {
         int32_t *bounds = nullptr, *sums = nullptr;
         int64_t *state = nullptr;
-        BC(B.get(&C.first, cap));
-        BC(B.get(&C.count, cap));
-        BC(B.get(&C.child, cap));
-        BC(B.get(&C.nchild, cap));
-        BC(B.get(&C.gc, 3 * cap));
-        BC(B.get(&C.side, cap));
+        if (int rc = get_cells(C, cap))
+            return rc;
         BC(B.get(&bounds, 8 * cap));
         BC(B.get(&sums, kSplitBlocks));
         BC(B.get(&state, 2 * (kMaxLevels + 1)));
@@ -1070,8 +1088,9 @@ int build_tree(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_
         B.drop(state);
         if (!hbad)
             break;
-        B.drop(C.first); B.drop(C.count); B.drop(C.child); B.drop(C.nchild); B.drop(C.gc);
-        B.drop(C.side);
+        if (cap == most)
+            return too_many();
+        drop_cells(C);
     }
     int64_t nc = 0;
     for (int level = 0; level < kMaxLevels && hstate[2 * level + 1] > hstate[2 * level]; level++) {
@@ -1080,7 +1099,22 @@ int build_tree(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_
     }
     out.level_start.push_back(nc);
     if (n + nc + 1 >= (int64_t)NLN_IDX_MASK)
-        return gc::set_status(-1, "GPU tree build: bodies plus cells exceed 27-bit list indices");
+        return too_many();
+    {
+        // in arrays as long as the cells: the rest of the build does without the room that
+        // was left, and the plan, which keeps four of them, too
+        Cells D{};
+        if (int rc = get_cells(D, nc))
+            return rc;
+        BC(cudaMemcpyAsync(D.first, C.first, nc * sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
+        BC(cudaMemcpyAsync(D.count, C.count, nc * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+        BC(cudaMemcpyAsync(D.child, C.child, nc * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+        BC(cudaMemcpyAsync(D.nchild, C.nchild, nc * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+        BC(cudaMemcpyAsync(D.gc, C.gc, 3 * nc * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        BC(cudaMemcpyAsync(D.side, C.side, nc * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        drop_cells(C);
+        C = D;
+    }
     out.n = n;
     out.ncells = nc;
     out.box = p.box;

@@ -23,7 +23,10 @@ std::map<const void *, std::string> names;     // host stub -> kernel name
 std::map<const void *, int> smem_limit;        // kernel -> its dynamic shared memory attribute
 std::map<std::string, unsigned> grids;         // kernel -> blocks of its last launch (x)
 std::map<std::string, long> first_at;          // kernel -> allocations made before its first launch
-std::set<void *> live, host_live;
+std::map<void *, size_t> live;
+std::set<void *> host_live;
+size_t live_bytes = 0, peak_bytes = 0;
+long long cells = 1;  // what a tree needs room for
 int last_error = 0;
 long nalloc = 0, fail_at = 0, double_frees = 0, trims = 0, pending = 0;
 bool once = false;  // the failing allocation succeeds once the pool has been trimmed
@@ -39,19 +42,24 @@ int get(void **p, size_t n) {
     nalloc++;
     if (fail_at && nalloc >= fail_at && !(once && trims))
         return ret(kOutOfMemory);
-    *p = aligned_alloc(256, (n + 511) / 256 * 256);
-    memset(*p, 0, (n + 511) / 256 * 256);
-    live.insert(*p);
+    *p = calloc(1, n + 256);
+    live[*p] = n;
+    live_bytes += n;
+    if (live_bytes > peak_bytes)
+        peak_bytes = live_bytes;
     return 0;
 }
 int put(void *p) {
     std::lock_guard<std::recursive_mutex> lk(mu);
     if (!p)
         return 0;
-    if (!live.erase(p)) {
+    const auto it = live.find(p);
+    if (it == live.end()) {
         double_frees++;
         return ret(kInvalidValue);
     }
+    live_bytes -= it->second;
+    live.erase(it);
     free(p);
     return 0;
 }
@@ -76,6 +84,9 @@ void emulate(const std::string &f, void **a) {
     if (is("k_split_root")) {  // the root alone, on level 0
         arg<int64_t *>(a, 6)[0] = 0;
         arg<int64_t *>(a, 6)[1] = 1;
+    } else if (is("k_split_write")) {
+        if (arg<int64_t>(a, 5) < cells)
+            *arg<unsigned *>(a, 6) = 1;
     } else if (is("k_runs_compact") || is("k_runs_k1")) {
     } else if (is("k_runs")) {
         arg<int64_t *>(a, 3)[0] = 1;
@@ -122,6 +133,8 @@ void fake_reset(long fail, int until_trimmed) {
     fail_at = fail;
     once = until_trimmed != 0;
     first_at.clear();
+    peak_bytes = live_bytes;
+    cells = 1;
 }
 // allocations asked for, buffers live, buffers freed twice, trims, default-stream work not
 // waited for, last error
@@ -138,6 +151,13 @@ long fake_allocs_before(const char *kernel) {
             return k.second;
     return -1;
 }
+// device bytes in use, and the most since the reset
+void fake_bytes(long *out) {
+    std::lock_guard<std::recursive_mutex> lk(mu);
+    out[0] = (long)live_bytes;
+    out[1] = (long)peak_bytes;
+}
+void fake_cells(long long need) { cells = need; }
 unsigned fake_grid(const char *kernel) {
     for (auto &k : grids)
         if (k.first.find(kernel) != std::string::npos)

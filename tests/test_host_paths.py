@@ -26,12 +26,20 @@ def counts():
     c = (ctypes.c_long * 6)()
     fake.fake_counts(c)
     return dict(zip(("allocs", "live", "double", "trims", "pending", "error"), c))
-def build(box, tuning=None):
+def used():
+    b = (ctypes.c_long * 2)()
+    fake.fake_bytes(b)
+    return list(b)
+def build(box, tuning=None, n=2):
+    data = at
+    if n > 2:
+        many = np.zeros((n + 1, 4), np.float32)
+        data = many.ctypes.data + -many.ctypes.data % 16
     t = ctypes.byref(gc.Tuning(*tuning)) if tuning else None
     p = Params(16, 32, 7, 20, 1e-3, 0.0, 0.0, box, 0, 0, 0.2, 0.0)
     h = ctypes.c_void_p()
-    rc = L.grav_plan_build_CUDA(ctypes.byref(p), at, 2, 1e-4, 1.0, int(box > 0), t, ctypes.byref(h))
-    if rc == 0:
+    rc = L.grav_plan_build_CUDA(ctypes.byref(p), data, n, 1e-4, 1.0, int(box > 0), t, ctypes.byref(h))
+    if rc == 0 and n == 2:
         rc = L.grav_groups_eval_CUDA(h, None) or L.grav_plan_adjoint_CUDA(h, at, at, None)
     return rc, h
 """
@@ -162,3 +170,24 @@ print(json.dumps(res))
 """ % ([[int(x) for x in k.split(",")] for k in caps],))
     for w, b, grids in out:
         assert grids == [caps[f"{w},{b}"] * 148] * 2, (w, b, grids)
+
+
+def test_cell_arrays_are_as_long_as_the_cells(run):
+    """Once the cells are known their arrays are cut to length: a plan of n
+    bodies and one cell holds its bodies (16 bytes each), their order (8), its
+    results (16) and little more, and a tree that would need more cells than list indices can
+    name is refused as such, after a bounded search for room."""
+    n = 3_000_000
+    held, refused, message = run("""
+n = %d
+rc, h = build(0.0, n=n)
+assert rc == 0
+held = used()[0]
+L.grav_plan_free(h)
+fake.fake_reset(0, 0)
+fake.fake_cells(ctypes.c_longlong(1 << 40))
+rc, h = build(0.0, n=n)
+print(json.dumps([held, rc, L.gravcuda_status_string().decode()]))
+""" % n)
+    assert held < 40 * n + (4 << 20), held
+    assert refused == -1 and "27-bit" in message, (refused, message)
