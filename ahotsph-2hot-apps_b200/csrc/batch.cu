@@ -2494,7 +2494,10 @@ extern "C" int grav_groups_CUDA(const grav_problem *hp, float *acc_phi) {
     return rc;
 }
 
+void dropin_release();  // dropin.cu: the sink buffers kept between walks
+
 extern "C" void grav_groups_release_CUDA(void) {
+    dropin_release();
     std::lock_guard<std::mutex> lk(g_pool_mu);
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {

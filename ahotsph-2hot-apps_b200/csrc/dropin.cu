@@ -403,7 +403,7 @@ struct State {
     int64_t nobj = 0;
     // 3 floats and (ax, ay, az, phi) per sink: set while a sink table is
     // registered; the buffers behind them are kept for the next walk until
-    // one needs larger ones or CUDA_Finalize
+    // one needs larger ones, grav_groups_release_CUDA or CUDA_Finalize
     float *devpos = nullptr;
     float4 *devaccp = nullptr;
     float *pos_buf = nullptr;
@@ -961,6 +961,8 @@ extern "C" void CUDA_Init(void *device_prop) {
                 prop.minor, prop.multiProcessorCount, prop.totalGlobalMem / 1e9);
 }
 
+void dropin_release();
+
 extern "C" void CUDA_Finalize(void) {
     std::lock_guard<std::recursive_mutex> call_lock(g_call_mu);
     grav_groups_release_CUDA();
@@ -985,11 +987,6 @@ extern "C" void CUDA_Finalize(void) {
             cudaFree(s.dev);
         s.reset();
     }
-    cudaFree(S.pos_buf);
-    cudaFree(S.acc_buf);
-    S.pos_buf = nullptr;
-    S.acc_buf = nullptr;
-    S.sink_cap = 0;
     cudaFree(S.qdev);
     cudaFree(S.derr);
     S.init = false;
@@ -998,6 +995,7 @@ extern "C" void CUDA_Finalize(void) {
     S.nobj = 0;
     S.devpos = nullptr;
     S.devaccp = nullptr;
+    dropin_release();
     S.qdev = nullptr;
     S.ncells = 0;
     S.derr = nullptr;
@@ -1087,6 +1085,18 @@ extern "C" void WalkTerminateSrcCUDA(void) {
 
 static int drain_all();
 
+// The sink buffers back to the device, unless a sink table is registered.
+void dropin_release() {
+    std::lock_guard<std::recursive_mutex> call_lock(g_call_mu);
+    if (S.devpos || (!S.pos_buf && !S.acc_buf))
+        return;
+    cudaFree(S.pos_buf);
+    cudaFree(S.acc_buf);
+    S.pos_buf = nullptr;
+    S.acc_buf = nullptr;
+    S.sink_cap = 0;
+}
+
 extern "C" void WalkInitSinkCUDA(float *btab, int stride, int64_t nobj) {
     std::lock_guard<std::recursive_mutex> call_lock(g_call_mu);
     if (ensure_init())
@@ -1102,11 +1112,7 @@ extern "C" void WalkInitSinkCUDA(float *btab, int stride, int64_t nobj) {
     S.devpos = nullptr;
     S.devaccp = nullptr;
     if (S.sink_cap < nobj) {
-        cudaFree(S.pos_buf);
-        cudaFree(S.acc_buf);
-        S.pos_buf = nullptr;
-        S.acc_buf = nullptr;
-        S.sink_cap = 0;
+        dropin_release();
         if (cudaMalloc(&S.pos_buf, (size_t)nobj * 3 * sizeof(float)) != cudaSuccess ||
             cudaMalloc(&S.acc_buf, (size_t)nobj * sizeof(float4)) != cudaSuccess) {
             gc::set_status(-1, "WalkInitSinkCUDA: device allocation failed");

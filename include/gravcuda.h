@@ -70,7 +70,12 @@ void WalkInitSrcCUDA(float *qtab, int stride, int64_t nobj);
 void WalkTerminateSrcCUDA(void);
 /* Copy sink positions (floats 1..3 of each record) to the device, zero the accumulators (nln/pgrav.cu:915-967). */
 void WalkInitSinkCUDA(float *btab, int stride, int64_t nobj);
-/* Wait for all queued work, ADD (ax, ay, az, phi) into floats 7..10 of each record (nln/pgrav.cu:969-1020). */
+/*
+ * Wait for all queued work, ADD (ax, ay, az, phi) into floats 7..10 of each
+ * record (nln/pgrav.cu:969-1020).  The device buffers (28 bytes a sink of the
+ * largest walk) are kept for the next WalkInitSinkCUDA; between walks
+ * grav_groups_release_CUDA gives them back, and CUDA_Finalize does.
+ */
 void WalkTerminateSinkCUDA(float *btab, int stride, int64_t nobj);
 
 /*
@@ -321,7 +326,11 @@ int grav_plan_problem(const grav_plan *plan, grav_problem *out);
  */
 int grav_groups_CUDA(const grav_problem *host_problem, float *acc_phi);
 
-/* Return the memory grav_groups_CUDA keeps reserved between calls on the current device. */
+/*
+ * Return the memory that is kept between calls: what grav_groups_CUDA and the
+ * device builds keep reserved on the current device, and, while no sink table
+ * is registered, the drop-in's sink buffers.
+ */
 void grav_groups_release_CUDA(void);
 
 /*

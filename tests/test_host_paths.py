@@ -191,3 +191,32 @@ print(json.dumps([held, rc, L.gravcuda_status_string().decode()]))
 """ % n)
     assert held < 40 * n + (4 << 20), held
     assert refused == -1 and "27-bit" in message, (refused, message)
+
+
+def test_sink_buffers_are_given_back_between_walks(run):
+    """The drop-in keeps its sink buffers for the next walk;
+    grav_groups_release_CUDA returns them, but not under a registered table."""
+    n = 100_000
+    idle, kept, released, again, registered, final = run("""
+n = %d
+btab = np.zeros((n, 16), np.float32)
+res = []
+L.CUDA_Init(None)
+res.append(used()[0])
+L.WalkInitSinkCUDA(btab.ctypes.data, 16, n)
+L.WalkTerminateSinkCUDA(btab.ctypes.data, 16, n)
+res.append(used()[0])
+L.grav_groups_release_CUDA()
+res.append(used()[0])
+L.WalkInitSinkCUDA(btab.ctypes.data, 16, n)
+res.append(used()[0])
+L.grav_groups_release_CUDA()
+res.append(used()[0])
+L.WalkTerminateSinkCUDA(btab.ctypes.data, 16, n)
+L.CUDA_Finalize()
+res.append(used()[0])
+assert L.gravcuda_status() == 0 and counts()["double"] == 0
+print(json.dumps(res))
+""" % n)
+    assert kept == again == registered == idle + 28 * n
+    assert released == idle and final == 0
