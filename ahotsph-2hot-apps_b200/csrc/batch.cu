@@ -1792,14 +1792,11 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     pl->hp.pptr = pl->hp.qptr = pl->hp.hptr = nullptr;
     pl->hp.plist = nullptr;
     pl->hp.qlist = pl->hp.hlist = nullptr;
-    if (pl->pool) {
-        // buffers allocated in stream order on the default stream: complete
-        // before other streams use them
-        const cudaError_t e = cudaStreamSynchronize(0);
-        if (e != cudaSuccess) {
-            grav_plan_free(pl);
-            return gc::cuda_status(e, "upload: pool allocations");
-        }
+    // pool allocations, cleared words and copies on the default stream: complete
+    // before other streams, which do not wait for it, use them
+    if (const cudaError_t e = cudaStreamSynchronize(0); e != cudaSuccess) {
+        grav_plan_free(pl);
+        return gc::cuda_status(e, "upload: default stream");
     }
     *plan_out = pl;
     t_phase[1] = now_s() - t_dev;
@@ -2082,6 +2079,7 @@ extern "C" int grav_plan_retune_CUDA(grav_plan *pl, const grav_tuning *tuning) {
     d.gslot = gs;
     if (pl->step)
         step_graph_reset(pl->step);  // a captured step holds the old queue
+    GC_CHECK(cudaStreamSynchronize(0));  // as at the end of the upload
     return rc;
 }
 

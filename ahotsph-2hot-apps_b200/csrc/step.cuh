@@ -484,6 +484,8 @@ extern "C" int grav_plan_set_tree_CUDA(grav_plan *pl, const int64_t *cell_first,
     up(&S->order, order.data(), nc);
     if (e == cudaSuccess)
         e = cudaMalloc((void **)&S->raw, (size_t)nc * kRaw * sizeof(double));
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(0);  // the copies: other streams use them
     if (e != cudaSuccess) {
         delete S;
         return gc::cuda_status(e, "grav_plan_set_tree_CUDA");

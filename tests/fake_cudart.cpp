@@ -243,10 +243,14 @@ int cudaMemPoolTrimTo(void *, size_t) {
     trims++;
     return 0;
 }
-// pageable copies end before they return
-int cudaMemcpy(void *d, const void *s, size_t n, int) {
+// kind 1, host to device: begins when the default stream is done, and may return while the copy
+// is still under way; 2, device to host: ends before it returns; 3, on the device: does not wait
+int cudaMemcpy(void *d, const void *s, size_t n, int kind) {
     memcpy(d, s, n);
-    waited(nullptr);
+    if (kind != 3)
+        waited(nullptr);
+    if (kind != 2)
+        on(nullptr);
     return 0;
 }
 int cudaMemcpyAsync(void *d, const void *s, size_t n, int, void *st) {

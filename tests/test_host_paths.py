@@ -220,3 +220,44 @@ print(json.dumps(res))
 """ % n)
     assert kept == again == registered == idle + 28 * n
     assert released == idle and final == 0
+
+
+def test_a_new_plan_leaves_nothing_on_the_default_stream(run):
+    """Streams other than the default one do not wait for it, so a plan's
+    tables and cleared words are complete when the call that makes them
+    returns: uploaded with copied lists and with lists in host memory, built
+    on the device, retuned, and with its tree links set."""
+    out = run("""
+from pgrav import ics, host
+res = {}
+pos, m = ics.grf_box(12, seed=1)
+t = host.Tree(pos, m, box=1.0, leaf_max=16, group_max=32, p2cut=7, p4cut=8, tol=1e-4)
+for in_host in (0, 1):
+    p = gc.Problem()
+    p.nbodies, p.ncells, p.ngroups = t.n, t.ncells, t.ngroups
+    p.points, p.qcells, p.hcells, p.groups = (a.ctypes.data for a in (t.points, t.qcells, t.hcells, t.groups))
+    p.pptr, p.qptr, p.hptr, p.cptr = (a.ctypes.data for a in t.ptr)
+    p.plist, p.qlist, p.hlist, p.clist = (a.ctypes.data for a in (t.plist, t.qlist, t.hlist, t.clist))
+    p.eps2, p.box, p.ewald, p.quad_phi_sign, p.lists_in_host = 1e-4, 1.0, 1, 1.0, in_host
+    h = ctypes.c_void_p()
+    fake.fake_reset(0, 0)
+    rc = L.grav_groups_upload_CUDA(ctypes.byref(p), None, ctypes.byref(h))
+    res["upload %d" % in_host] = [rc, counts()["pending"]]
+    rc = L.grav_plan_retune_CUDA(h, ctypes.byref(gc.Tuning(4, 256, 128, 64, 0, 0, 0)))
+    res["retune %d" % in_host] = [rc, counts()["pending"]]
+    links = t.cell_ranges() + t.cell_links()
+    rc = L.grav_plan_set_tree_CUDA(h, *(x.ctypes.data for x in links))
+    res["set_tree %d" % in_host] = [rc, counts()["pending"]]
+    L.grav_plan_free(h)
+fake.fake_reset(0, 0)
+p = Params(16, 32, 7, 20, 1e-3, 0.0, 0.0, 1.0, 0, 0, 0.2, 0.0)
+h = ctypes.c_void_p()
+rc = L.grav_plan_build_CUDA(ctypes.byref(p), at, 2, 1e-4, 1.0, 1, None, ctypes.byref(h))
+res["build"] = [rc, counts()["pending"]]
+rc = L.grav_plan_retune_CUDA(h, ctypes.byref(gc.Tuning(4, 256, 128, 64, 0, 0, 0)))
+res["retune built"] = [rc, counts()["pending"]]
+L.grav_plan_free(h)
+print(json.dumps(res))
+""")
+    for call, (rc, pending) in out.items():
+        assert rc == 0 and pending == 0, (call, rc, pending)
