@@ -1842,16 +1842,20 @@ int launch_kind(grav_plan *pl, const DevProblem &dp, cudaStream_t st, Chain *cha
     if (dp.nitems[KIND] == 0)
         return 0;
     const int wpb = std::min(pl->tune.warps_per_block, kListWarps);
-    size_t smem;
+    size_t warp;
     const void *kern;
     if constexpr (KIND == KP) {
-        smem = (size_t)wpb * kPointWarpBytes;
+        warp = kPointWarpBytes;
         kern = pl->plain ? (const void *)k_points<true> : (const void *)k_points<false>;
     } else {
-        smem = (size_t)wpb * CellKind<KIND>::warp_bytes;
+        warp = CellKind<KIND>::warp_bytes;
         kern = pl->plain ? (const void *)k_cells<KIND, true> : (const void *)k_cells<KIND, false>;
     }
-    GC_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the limit belongs to the kernel, not to this plan: the most that any plan needs, so that
+    // no other thread's launch finds it lowered
+    GC_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(kListWarps * warp)));
+    const size_t smem = wpb * warp;
     int fit = 0;
     GC_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, wpb * 32, smem));
     // a cap counts the caller's blocks, of warps_per_block warps each

@@ -261,3 +261,19 @@ print(json.dumps(res))
 """)
     for call, (rc, pending) in out.items():
         assert rc == 0 and pending == 0, (call, rc, pending)
+
+
+def test_a_plan_of_small_blocks_leaves_the_others_their_shared_memory(run):
+    """A kernel's shared memory limit is the process's: a plan of one-warp
+    blocks, evaluated between another thread's setting it and its launch,
+    must not lower it."""
+    out = run("""
+res = []
+for w in (8, 1, 4):
+    rc, h = build(0.0, (w, 0, 0, 0, 0, 0, 0))
+    assert rc == 0
+    res.append([fake.fake_smem_limit(k) for k in (b"k_pointsILb0", b"k_cellsILi1ELb0")])
+    L.grav_plan_free(h)
+print(json.dumps(res))
+""")
+    assert min(out[0]) > 0 and out[0] == out[1] == out[2]
