@@ -106,11 +106,6 @@ struct DevProblem {
     int cstride;
 };
 
-// No entry in this lane: a value that no word of a list takes.  An all-ones
-// word in a list is as invalid as the one below it, for which it passes.
-constexpr uint32_t kNone = 0xffffffffu;
-__device__ __forceinline__ uint32_t list_word(const uint32_t *p) { return min(__ldg(p), kNone - 1u); }
-
 // Image code (0..26) to the image's shift: (code / 9 - 1, code / 3 % 3 - 1,
 // code % 3 - 1) box.
 __device__ __forceinline__ void decode_shift(uint32_t code, double box, double &sx, double &sy,
@@ -639,6 +634,8 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
     const uint32_t nb = PLAIN || !P.ccen ? ntab : ntab - (uint32_t)P.ncells;  // cells from here on
     const float2 e2 = splat2(P.eps2);
     constexpr int NP = kPointTile / 64, NE = 2 * NP;  // record pairs, records per lane
+    // the word of an absent entry, told by its place and not by the word
+    constexpr uint32_t kBody0 = NLN_SHIFT_NONE << NLN_IDX_BITS;
     for (;;) {
         int it = 0;
         if (lane == 0)
@@ -654,21 +651,22 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
 #pragma unroll
             for (int j = 0; j < NE; j++) {
                 const int64_t k = k0 + 32 * j + lane;
-                e[j] = k < item.end ? list_word(list + k) : kNone;
+                e[j] = k < item.end ? __ldg(list + k) : kBody0;
             }
         };
         // Start this lane's copies of its entries' records.  Entries are
         // checked at upload, except in the pipelined end-to-end call: a bad
         // one becomes body 0 in the box's own image.
-        auto copy = [&](uint32_t *e) {
+        auto copy = [&](int64_t k0, uint32_t *e) {
+            const int n = (int)min((int64_t)kPointTile, item.end - k0);
             bool bad = false;
 #pragma unroll
             for (int j = 0; j < NE; j++) {
-                if (e[j] == kNone)
-                    continue;
+                if (32 * j >= n)
+                    break;
                 if ((e[j] & NLN_IDX_MASK) >= ntab || (e[j] >> NLN_IDX_BITS) > 26u) {
                     bad = true;
-                    e[j] = NLN_SHIFT_NONE << NLN_IDX_BITS;
+                    e[j] = kBody0;
                 }
                 const uint32_t idx = e[j] & NLN_IDX_MASK;
                 if (idx < nb) {
@@ -685,21 +683,22 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
         };
         uint32_t cur[NE], nxt[NE];
         fetch(item.begin, cur);
-        copy(cur);
+        copy(item.begin, cur);
         fetch(item.begin + kPointTile, nxt);
         stage_sinks(sinks, P, G, c, lane);
         Total acc;
         for (int64_t k0 = item.begin; k0 < item.end; k0 += kPointTile) {
-            const int np = (int)min((int64_t)NP, (item.end - k0 + 63) / 64);  // pairs in use
+            const int nt = (int)min((int64_t)kPointTile, item.end - k0);
+            const int np = (nt + 63) >> 6;  // pairs in use
             MonoPair rec[NP];
             cp_async_wait<0>();  // this lane's records have landed
 #pragma unroll
             for (int j = 0; j < NE; j++) {
                 if ((j >> 2) > (np - 1) >> 1)
                     break;
-                const bool live = cur[j] != kNone;
+                const bool live = 32 * j + lane < nt;
                 const uint32_t idx = cur[j] & NLN_IDX_MASK;
-                const uint32_t code = live ? cur[j] >> NLN_IDX_BITS : NLN_SHIFT_NONE;
+                const uint32_t code = cur[j] >> NLN_IDX_BITS;
                 const float4 u = stage.chunk[j][0][lane];
                 double x = u.x, y = u.y, z = u.z;
                 float m = u.w;
@@ -718,7 +717,7 @@ __global__ void __launch_bounds__(32 * kListWarps, GRAV_P_MINB) k_points(DevProb
                 set_half(rec[j >> 1].z, j & 1, live ? o[2] : kFar);
                 set_half(rec[j >> 1].m, j & 1, live ? m : 0.f);
             }
-            copy(nxt);
+            copy(k0 + kPointTile, nxt);
 #pragma unroll
             for (int j = 0; j < NE; j++) cur[j] = nxt[j];
             fetch(k0 + 2 * kPointTile, nxt);
@@ -835,6 +834,7 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
     EwStage *stg = reinterpret_cast<EwStage *>(ewsm + (size_t)(threadIdx.x >> 5) * kEwWarpBytes);
     const uint32_t ntab = (uint32_t)P.ntab[0];
     const uint32_t nb = ntab - (uint32_t)P.ncells;
+    constexpr uint32_t kNone = 0xffffffffu;
     // one source of the pipeline: list word (kNone: no entry in this lane)
     // and its position (FP64) with, for a body, its mass
     struct Src {
@@ -862,12 +862,15 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
         // the list word is checked where it is used, a tile after its load
         auto entry = [&](int t) -> uint32_t {
             const int64_t k = U.cb + (int64_t)(U.t0 + t) * 32 + lane;
-            return (t < ntile && k < U.ce) ? list_word(P.clist + k) : kNone;
+            return (t < ntile && k < U.ce) ? __ldg(P.clist + k) : kNone;
         };
-        auto source = [&](uint32_t e) -> Src {
+        auto source = [&](uint32_t e, int t) -> Src {
             Src r{kNone, 0.0, 0.0, 0.0, 0.f};
-            if (e == kNone)
+            if (e == kNone) {
+                if (t < ntile && U.cb + (int64_t)(U.t0 + t) * 32 + lane < U.ce)
+                    atomicOr(P.err, GC_DEV_BAD_INDEX);
                 return r;
+            }
             const uint32_t idx = e & NLN_IDX_MASK;
             if (idx >= ntab || (e >> NLN_IDX_BITS) > 26u) {  // as in the list kernels
                 atomicOr(P.err, GC_DEV_BAD_INDEX);
@@ -930,13 +933,13 @@ __global__ void __launch_bounds__(128) k_ewald_moments(DevProblem P) {
         };
         EwSums M;
         M.zero();
-        Staged now = issue(source(entry(0)), stg[0]), next;
-        Src s1 = source(entry(1));
+        Staged now = issue(source(entry(0), 0), stg[0]), next;
+        Src s1 = source(entry(1), 1);
         uint32_t e2 = entry(2);
         for (int t = 0; t < ntile; t++) {
             __syncwarp();  // the other stage is no longer read
             next = issue(s1, stg[(t + 1) & 1]);
-            s1 = source(e2);  // consumed by the next tile's issue
+            s1 = source(e2, t + 2);  // consumed by the next tile's issue
             e2 = entry(t + 3);
             cp_async_wait<1>();  // this lane's copies for tile t have landed
             __syncwarp();        // and the other lanes'
