@@ -1033,37 +1033,29 @@ int build_tree(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_
     out.seconds[0] = now_s() - t0;
     t0 = now_s();
 
-    // ---- cells, level by level: room for two per three bodies at first (spheres and boxes
-    // with leaves of 16 need a quarter of that), four times as many where that is too few,
-    // and never more than the list indices could name
+    // ---- cells, level by level, in room for 7 n / leaf_max cells (2 n at most): a level whose
+    // cells hold just over leaf_max bodies splits them into eight, which makes 6.5 n / leaf_max
+    // cells in the worst grids and uniform boxes tried (0.37 n with leaves of 16, 0.20 with 32;
+    // spheres 0.25 and 0.15; leaves of one body 1.5).  The plan keeps 20 of the 52 bytes a cell,
+    // room included: cutting the arrays to the count costs a build of 64k bodies 0.03 of 2.2 ms.
+    // Four times as many where that is too few (tight pairs make long chains), and never more
+    // than the list indices could name.
     Cells C{};
-    auto get_cells = [&](Cells &D, int64_t c) -> int {
-        BC(B.get(&D.first, c));
-        BC(B.get(&D.count, c));
-        BC(B.get(&D.child, c));
-        BC(B.get(&D.nchild, c));
-        BC(B.get(&D.gc, 3 * c));
-        BC(B.get(&D.side, c));
-        return 0;
-    };
-    auto drop_cells = [&](const Cells &D) {
-        B.drop(D.first);
-        B.drop(D.count);
-        B.drop(D.child);
-        B.drop(D.nchild);
-        B.drop(D.gc);
-        B.drop(D.side);
-    };
     auto too_many = [] {
         return gc::set_status(-1, "GPU tree build: bodies plus cells exceed 27-bit list indices");
     };
     int64_t hstate[2 * (kMaxLevels + 1)];
     const int64_t most = (int64_t)NLN_IDX_MASK - n;
-    for (int64_t cap = std::min(most, std::max<int64_t>(1024, 2 * n / 3));; cap = std::min(most, 4 * cap)) {
+    for (int64_t cap = std::min(most, 1024 + std::min(2 * n, 7 * n / p.leaf_max));;
+         cap = std::min(most, 4 * cap)) {
         int32_t *bounds = nullptr, *sums = nullptr;
         int64_t *state = nullptr;
-        if (int rc = get_cells(C, cap))
-            return rc;
+        BC(B.get(&C.first, cap));
+        BC(B.get(&C.count, cap));
+        BC(B.get(&C.child, cap));
+        BC(B.get(&C.nchild, cap));
+        BC(B.get(&C.gc, 3 * cap));
+        BC(B.get(&C.side, cap));
         BC(B.get(&bounds, 8 * cap));
         BC(B.get(&sums, kSplitBlocks));
         BC(B.get(&state, 2 * (kMaxLevels + 1)));
@@ -1090,7 +1082,12 @@ int build_tree(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_
             break;
         if (cap == most)
             return too_many();
-        drop_cells(C);
+        B.drop(C.first);
+        B.drop(C.count);
+        B.drop(C.child);
+        B.drop(C.nchild);
+        B.drop(C.gc);
+        B.drop(C.side);
     }
     int64_t nc = 0;
     for (int level = 0; level < kMaxLevels && hstate[2 * level + 1] > hstate[2 * level]; level++) {
@@ -1100,21 +1097,6 @@ int build_tree(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_
     out.level_start.push_back(nc);
     if (n + nc + 1 >= (int64_t)NLN_IDX_MASK)
         return too_many();
-    {
-        // in arrays as long as the cells: the rest of the build does without the room that
-        // was left, and the plan, which keeps four of them, too
-        Cells D{};
-        if (int rc = get_cells(D, nc))
-            return rc;
-        BC(cudaMemcpyAsync(D.first, C.first, nc * sizeof(int64_t), cudaMemcpyDeviceToDevice, st));
-        BC(cudaMemcpyAsync(D.count, C.count, nc * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-        BC(cudaMemcpyAsync(D.child, C.child, nc * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-        BC(cudaMemcpyAsync(D.nchild, C.nchild, nc * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-        BC(cudaMemcpyAsync(D.gc, C.gc, 3 * nc * sizeof(double), cudaMemcpyDeviceToDevice, st));
-        BC(cudaMemcpyAsync(D.side, C.side, nc * sizeof(double), cudaMemcpyDeviceToDevice, st));
-        drop_cells(C);
-        C = D;
-    }
     out.n = n;
     out.ncells = nc;
     out.box = p.box;

@@ -172,10 +172,10 @@ print(json.dumps(res))
         assert grids == [caps[f"{w},{b}"] * 148] * 2, (w, b, grids)
 
 
-def test_cell_arrays_are_as_long_as_the_cells(run):
-    """Once the cells are known their arrays are cut to length: a plan of n
-    bodies and one cell holds its bodies (16 bytes each), their order (8), its
-    results (16) and little more, and a tree that would need more cells than list indices can
+def test_cell_arrays_hold_what_the_leaves_can_make(run):
+    """A plan of n bodies in leaves of L holds its bodies (16 bytes each), their
+    order (8), its results (16), the links of at most 7 n / L cells (20) and
+    little more, and a tree that would need more cells than list indices can
     name is refused as such, after a bounded search for room."""
     n = 3_000_000
     held, refused, message = run("""
@@ -189,7 +189,7 @@ fake.fake_cells(ctypes.c_longlong(1 << 40))
 rc, h = build(0.0, n=n)
 print(json.dumps([held, rc, L.gravcuda_status_string().decode()]))
 """ % n)
-    assert held < 40 * n + (4 << 20), held
+    assert held < (40 + 20 * 7 / 16) * n + (4 << 20), held
     assert refused == -1 and "27-bit" in message, (refused, message)
 
 
