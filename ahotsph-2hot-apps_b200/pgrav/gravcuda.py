@@ -189,6 +189,8 @@ class Plan:
         if tuning is not None:
             tun = Tuning(*tuning) if not isinstance(tuning, Tuning) else tuning
         h = ctypes.c_void_p()
+        # the builder reads them on the default stream, which waits for no other
+        torch.cuda.current_stream().synchronize()
         check(lib().grav_plan_build_CUDA(ctypes.byref(params), bodies.data_ptr(), n, float(eps2),
                                          float(quad_phi_sign), int(bool(ewald)),
                                          ctypes.byref(tun) if tun is not None else None,

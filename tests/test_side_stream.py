@@ -26,6 +26,46 @@ def test_device_copies_run_on_the_current_stream(monkeypatch):
     assert calls == [("cudaMemcpyAsync", 16, 32, 64, 3, 77), ("cudaStreamSynchronize", 77)]
 
 
+def test_bodies_are_complete_before_the_build(monkeypatch):
+    """Plan.build waits for the stream that its bodies are written on, with the
+    library's and torch's calls recorded in place of a GPU."""
+    import torch
+    from pgrav import gravcuda as gc
+    calls = []
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(
+        cuda_stream=77, synchronize=lambda: calls.append("wait")))
+    monkeypatch.setattr(gc, "lib", lambda: types.SimpleNamespace(
+        grav_plan_build_CUDA=lambda *a: calls.append("build") or 0, grav_plan_free=lambda h: None))
+    gc.Plan.build(None, None, 1e-4, bodies=torch.zeros((8, 4)))
+    assert calls == ["wait", "build"]
+
+
+@pytest.mark.gpu
+def test_stepper_on_a_side_stream():
+    """A stepper made and rebuilt under a side stream that is held up before its
+    bodies are written gives the default stream's states, bit for bit."""
+    import torch
+    from pgrav import ics
+    from pgrav.step import Stepper
+    p, m = ics.plummer(3000, seed=6)
+    v = np.random.default_rng(6).normal(0, 0.1, p.shape)
+
+    def go(hold):
+        hold()
+        s = Stepper(p, v, m, 1e-4, rebuild=2, tree_kw=dict(tol=1e-4))
+        for _ in range(3):
+            hold()
+            s.run(2, 1e-3)
+        out = s.state()
+        s.free()
+        return out
+
+    want = go(lambda: None)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        got = go(lambda: torch.cuda._sleep(20_000_000))
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("box", [0.0, 1.0])
 def test_gradient_on_a_side_stream(monkeypatch, box):
