@@ -1185,6 +1185,9 @@ extern "C" int grav_plan_adjoint_CUDA(grav_plan *pl, const float *wu, float *gra
         return gc::set_status(-1, "grav_plan_adjoint_CUDA: bad arguments");
     if (!pl->step)
         return gc::set_status(-1, "grav_plan_adjoint_CUDA: no tree links (grav_plan_set_tree_CUDA)");
+    if (!has_queue(pl))
+        return gc::set_status(-1, "grav_plan_adjoint_CUDA: the plan lost its work queue in a failed "
+                                  "retune; retune it again");
     if (pl->dp.nitems[KQ] > 0 && !pl->dp.qcells)
         return gc::set_status(-1, "grav_plan_adjoint_CUDA: no quadrupole table");
     if ((pl->dp.nitems[KH] > 0 || pl->dp.ewald) && !pl->dp.hcells)

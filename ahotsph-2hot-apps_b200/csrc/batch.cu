@@ -1975,9 +1975,23 @@ int launch_finish(grav_plan *pl, const DevProblem &dp, cudaStream_t st, bool for
 }
 }  // namespace
 
+namespace {
+// A retune that ran out of memory leaves a plan without its work queue.
+bool has_queue(const grav_plan *pl) {
+    const DevProblem &d = pl->dp;
+    for (int k = 0; k < 3; k++)
+        if (d.nitems[k] > 0 && !d.items[k])
+            return false;
+    return d.part && d.gslot;
+}
+}  // namespace
+
 extern "C" int grav_groups_eval_CUDA(grav_plan *pl, void *stream) {
     if (!pl)
         return gc::set_status(-1, "grav_groups_eval_CUDA: no plan");
+    if (!has_queue(pl))
+        return gc::set_status(-1, "grav_groups_eval_CUDA: the plan lost its work queue in a failed "
+                                  "retune; retune it again");
     cudaStream_t st = (cudaStream_t)stream;
     pl->launches = 0;
     auto mark = [&](int k) -> int {

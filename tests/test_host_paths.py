@@ -277,3 +277,29 @@ for w in (8, 1, 4):
 print(json.dumps(res))
 """)
     assert min(out[0]) > 0 and out[0] == out[1] == out[2]
+
+
+def test_a_plan_without_its_queue_is_not_evaluated(run):
+    """A retune whose k-th allocation fails leaves a plan that refuses to be
+    evaluated or differentiated (its kernels would read null queues), and that
+    another retune makes whole."""
+    out = run("""
+t = ctypes.byref(gc.Tuning(4, 256, 128, 64, 0, 0, 0))
+rc, h = build(0.0)
+fake.fake_reset(0, 0)
+assert rc == 0 and L.grav_plan_retune_CUDA(h, t) == 0
+total, res = counts()["allocs"], []
+for k in range(1, total + 1):
+    fake.fake_reset(k, 0)
+    failed = L.grav_plan_retune_CUDA(h, t)
+    fake.fake_reset(0, 0)
+    res.append([k, failed, L.grav_groups_eval_CUDA(h, None), L.grav_plan_adjoint_CUDA(h, at, at, None),
+                fake.fake_allocs_before(b"k_points"), L.grav_plan_retune_CUDA(h, t),
+                L.grav_groups_eval_CUDA(h, None)])
+L.grav_plan_free(h)
+print(json.dumps(res))
+""")
+    assert len(out) >= 5
+    for k, failed, ev, adj, launched, again, after in out:
+        assert failed and ev == -1 and adj == -1 and launched == -1, (k, failed, ev, adj, launched)
+        assert again == 0 and after == 0
