@@ -1178,8 +1178,9 @@ int dev_copy(grav_plan *pl, const T *src, size_t n, T **dst) {
     return 0;
 }
 
-// Defaults: 8 warps per block, as many resident blocks as registers and
-// shared memory allow (blocks_per_sm = 0), list chunks sized automatically
+// Defaults: 8 warps per block, which the list kernels run as blocks of four,
+// as many resident as registers and shared memory allow (blocks_per_sm = 0),
+// list chunks sized automatically
 // (chunk_* = 0) from the totals once the lists are known.
 grav_tuning default_tuning() {
     grav_tuning t;
@@ -1698,9 +1699,10 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
         d.ew_self = (float)(c0 - M_PI / (alpha * alpha * hp->box * hp->box * hp->box));
         d.ewald = 1;
         rc |= dev_copy<EwStored>(pl, nullptr, (size_t)ng, &pl->ewm);
-        // Lists are split until there are ~4 units per resident warp (10 per
-        // SM), but not below 8 tiles a unit: a 16^3 box has 156 groups for
-        // 1,480 warps (moments 0.16 -> 0.07 ms), a 64^3 box enough as it is.
+        // Lists are split until there are 40 units per SM, more than three for
+        // each of its 12 resident warps, but not below 8 tiles a unit: a 16^3 box
+        // has 130 groups for 1,776 warps (moments 0.16 -> 0.07 ms), a 64^3 box
+        // enough as it is.
         const int64_t tiles = hp->cptr[ng] / (32 * ng);
         d.ewsplit = (int)std::max<int64_t>(1, std::min<int64_t>((40 * (int64_t)pl->nsm + ng - 1) / ng,
                                                                 tiles / 8));

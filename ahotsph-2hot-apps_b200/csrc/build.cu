@@ -1266,7 +1266,11 @@ int build_tree(const nln_params &p, const float4 *bodies, int64_t n, cudaStream_
         BC(cudaMemcpyAsync(&nwide, before + ng, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         BC(cudaStreamSynchronize(st));
     }
-    if (4 * nwide > ng)  // enough of them to fill the GPU whole
+    // Parts only where at most a quarter of the groups are wide.  Both passes, groups whole and
+    // in parts, ms: 30k sphere (60 of 1,350 wide) 0.75, 0.63; 100k (117 of 4,422) 1.60, 1.67; 2k
+    // (26 of 96) 0.151, 0.155; but 16^3 box (128 of 130) 0.21, 0.17 and 32^3 (all of 1,024) 0.59,
+    // 0.40: a few groups for all the SMs, which would gain from parts and are kept whole here.
+    if (4 * nwide > ng)
         nwide = 0;
     const int64_t units = ng + (kWalkParts - 1) * nwide;
     BC(B.get(&ucnt, 5 * kWalkParts * nwide));

@@ -356,9 +356,9 @@ __global__ void k_quad_index(const float *__restrict__ pos, float4 *accp, int m,
 
 // ------------------------------------------------------------ state
 // A queue slot: its stream, a device list buffer, and two page-locked
-// staging buffers used in turn; the copy out of each staging buffer records
-// an event, so reusing a staging buffer waits only for the copy that last
-// read it (two calls back), never for the slot's kernels.
+// staging buffers used in turn; what last read each of them (two calls back)
+// records an event, for which reusing it waits: the copy to the device, or,
+// where the list was read in place, the kernel.
 struct Slot {
     bool inuse = false;
     cudaStream_t stream = nullptr;
@@ -367,7 +367,8 @@ struct Slot {
     void *hbuf[2] = {nullptr, nullptr};
     cudaEvent_t copied[2] = {nullptr, nullptr};
     // staging buffer states: 0 free, 1 filled and waiting for the submitter,
-    // 2 its copy to the device issued (copied[k] recorded)
+    // 2 its copy to the device, or the kernel that reads it in place, issued (copied[k]
+    // recorded)
     std::atomic<int> bstate[2] = {{0}, {0}};
     std::atomic<int> queued{0};  // jobs of this slot not yet issued
     // recorded by the submitter after each launch (an in-place one records
@@ -462,7 +463,7 @@ bool wait_until(F done, double seconds = 120.0) {
 }
 
 // Make slot q ready for a call of `bytes`: staging buffer s.host free to
-// write (the copy that last read it has been issued and has completed),
+// write (the copy or kernel that last read it has been issued and has completed),
 // device buffer large enough.  The device buffer is only rewritten by copies
 // on the slot's own stream, which run after the kernels queued before them.
 int slot_reserve(int q, size_t bytes) {
@@ -740,8 +741,8 @@ int dispatch_list(const Routine &r, cudaStream_t st, const float *pos, float4 *a
 // ---- deferred issue: the submitter thread ----
 // grav_mn_CUDA copies its list into a slot's staging buffer and queues a
 // job; one submitter thread takes the jobs in order and issues, on the
-// slot's stream, the copy to the device, the event that frees the staging
-// buffer, and the launch.  Errors there set the status as in the calling
+// slot's stream, the copy to the device (of lists that are not read in place),
+// the launch, and the event that frees the staging buffer.  Errors there set the status as in the calling
 // thread (abort in the default error mode), and drain_all returns them.
 struct Job {
     const Routine *r;
@@ -761,8 +762,8 @@ struct Submitter {
     std::condition_variable cv;
     std::thread th;
     bool started = false;
-    // staging buffers whose copies were issued, oldest first: polled while
-    // the queue is empty and marked free when their copy has completed, so
+    // staging buffers whose readers were issued, oldest first: polled while
+    // the queue is empty and marked free when their reader has completed, so
     // the caller rarely waits on an event
     std::pair<int, int> issued[kCap];
     uint64_t issued_head = 0, issued_tail = 0;

@@ -214,9 +214,10 @@ __device__ __forceinline__ void interact(const float *__restrict__ r, float sx, 
 // pairs (nsx, nsx).  Everything works in v = source - sink = -d.
 //
 // What bounds them is the register file, not the FMA pipe: on a B200 a
-// paired FMA with three distinct operands takes three cycles a warp (two
-// with two; 49 of 74 TFLOP/s), a scalar one about 1.4.  So the forms below
-// count operand reads, not only operations.
+// paired FMA with three distinct operands takes 3.05 to 3.3 cycles a warp, by
+// the registers it gets (45 to 49 of 74 TFLOP/s), with two 2.05; a scalar one
+// 1.1 to 1.5, and 1.04.  So the forms below count operand reads, not only
+// operations.
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 splat2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }

@@ -400,9 +400,9 @@ void step_graph_reset(grav_step_state *S) {
 // The tree links of a plan whose tree was built on the device: the
 // builder's device arrays are adopted as they are (no round trip through the
 // host), and the per-cell FP64 scratch comes from the same pool.  The
-// builder makes cells level by level, so each depth is one index range and
-// the deepest-first order is those ranges in reverse; only the depths are
-// read back, to find the ranges.  The adopted arrays belong to the plan
+// builder makes cells level by level, so each depth is one index range
+// (DevTree::level_start) and the deepest-first order is those ranges in
+// reverse, without an order array.  The adopted arrays belong to the plan
 // from here on, also when this fails.
 int set_tree_adopt(grav_plan *pl, const DevTree &T, cudaMemPool_t pool) {
     const int64_t nc = pl->hp.ncells;
