@@ -1165,8 +1165,6 @@ struct grav_adjoint_state {
                     : cudaMalloc((void **)p, n * sizeof(T));
     }
     ~grav_adjoint_state() {
-        if (pool)
-            cudaDeviceSynchronize();  // an adjoint on any stream may still use them
         for (void *p : {(void *)leaf, (void *)parent, (void *)flag, (void *)gbody, (void *)gcell,
                         (void *)mbar, (void *)gstf})
             if (p) {

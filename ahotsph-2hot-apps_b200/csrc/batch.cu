@@ -2157,6 +2157,9 @@ extern "C" int grav_plan_launches(const grav_plan *pl) { return pl ? pl->launche
 extern "C" void grav_plan_free(grav_plan *pl) {
     if (!pl)
         return;
+    // work on any stream may still use what goes back to the pool (cudaFree waits by itself)
+    if (pl->pool)
+        cudaDeviceSynchronize();
     if (pl->step)
         step_state_free(pl->step);
     if (pl->adj)

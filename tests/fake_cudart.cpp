@@ -29,6 +29,7 @@ size_t live_bytes = 0, peak_bytes = 0;
 long long cells = 1;  // what a tree needs room for
 int last_error = 0;
 long nalloc = 0, fail_at = 0, double_frees = 0, trims = 0, pending = 0;
+long elsewhere = 0, freed_early = 0;  // launches on other streams, and pool buffers freed under them
 bool once = false;  // the failing allocation succeeds once the pool has been trimmed
 
 int ret(int e) {
@@ -68,6 +69,8 @@ void on(void *stream) {
     std::lock_guard<std::recursive_mutex> lk(mu);
     if (!stream)
         pending++;
+    else
+        elsewhere++;
 }
 void waited(void *stream) {
     std::lock_guard<std::recursive_mutex> lk(mu);
@@ -129,7 +132,7 @@ struct dim3_ {
 extern "C" {
 void fake_reset(long fail, int until_trimmed) {
     std::lock_guard<std::recursive_mutex> lk(mu);
-    nalloc = double_frees = trims = pending = 0;
+    nalloc = double_frees = trims = pending = elsewhere = freed_early = 0;
     fail_at = fail;
     once = until_trimmed != 0;
     first_at.clear();
@@ -157,6 +160,7 @@ void fake_bytes(long *out) {
     out[0] = (long)live_bytes;
     out[1] = (long)peak_bytes;
 }
+long fake_freed_early() { return freed_early; }
 void fake_cells(long long need) { cells = need; }
 unsigned fake_grid(const char *kernel) {
     for (auto &k : grids)
@@ -203,9 +207,15 @@ int cudaLaunchKernel(const void *f, dim3_, dim3_, void **args, size_t, void *st)
     on(st);
     return 0;
 }
-int cudaLaunchKernelExC(const dim3_ *cfg, const void *f, void **args) {  // the grid comes first
+struct launch_ {  // cudaLaunchConfig_t's first members
+    dim3_ grid, block;
+    size_t smem;
+    void *stream;
+};
+int cudaLaunchKernelExC(const launch_ *cfg, const void *f, void **args) {
     launched(f, args);
-    grids[names[f]] = cfg->x;
+    on(cfg->stream);
+    grids[names[f]] = cfg->grid.x;
     return 0;
 }
 
@@ -220,7 +230,11 @@ int cudaFree(void *p) {
     waited(nullptr);
     return put(p);
 }
-int cudaFreeAsync(void *p, void *) { return p ? put(p) : ret(kInvalidValue); }
+int cudaFreeAsync(void *p, void *) {
+    std::lock_guard<std::recursive_mutex> lk(mu);
+    freed_early += elsewhere > 0;
+    return p ? put(p) : ret(kInvalidValue);
+}
 int cudaMallocHost(void **p, size_t n) {
     *p = aligned_alloc(4096, (n + 4095) / 4096 * 4096);
     std::lock_guard<std::recursive_mutex> lk(mu);
@@ -291,7 +305,9 @@ int cudaDeviceGetAttribute(int *v, int a, int) {
     return 0;
 }
 int cudaDeviceSynchronize() {
+    std::lock_guard<std::recursive_mutex> lk(mu);
     waited(nullptr);
+    elsewhere = 0;
     return 0;
 }
 int cudaFuncGetAttributes(void *a, const void *) {  // cudaFuncAttributes: versions after 3 sizes, 2 ints

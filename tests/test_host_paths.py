@@ -303,3 +303,24 @@ print(json.dumps(res))
     for k, failed, ev, adj, launched, again, after in out:
         assert failed and ev == -1 and adj == -1 and launched == -1, (k, failed, ev, adj, launched)
         assert again == 0 and after == 0
+
+
+def test_a_plan_is_freed_after_the_work_that_uses_it(run):
+    """A device-built plan's buffers go back to the pool only when the
+    evaluation and the adjoint queued on another stream are done with them."""
+    out = run("""
+res = []
+for box in (0.0, 1.0):
+    for adjoint in (0, 1):
+        rc, h = build(box)
+        fake.cudaDeviceSynchronize()
+        fake.fake_reset(0, 0)
+        assert rc == 0 and L.grav_groups_eval_CUDA(h, 0x5000) == 0
+        if adjoint:
+            assert L.grav_plan_adjoint_CUDA(h, at, at, 0x5000) == 0
+        L.grav_plan_free(h)
+        fake.fake_freed_early.restype = ctypes.c_long
+        res.append([fake.fake_freed_early(), counts()["live"]])
+print(json.dumps(res))
+""")
+    assert out == [[0, 0]] * 4
