@@ -33,16 +33,14 @@ def memcpy_d2h(dst_array, src_ptr):
 
 def memcpy_d2d(dst_ptr, src_ptr, nbytes):
     """Copy between device buffers, the destination a tensor of torch's
-    current stream: on that stream, and complete on return, so that the
-    source may go.  (A plain cudaMemcpy runs on the legacy default stream,
-    returns before it is done, and torch's other streams do not wait for it.)"""
+    current stream: on that stream, not waited for (a plan that is freed waits
+    for it).  A plain cudaMemcpy runs on the legacy default stream, returns
+    before it is done, and torch's other streams do not wait for it."""
     import torch
     rt = _rt()
     stream = torch.cuda.current_stream().cuda_stream
     err, = rt.cudaMemcpyAsync(dst_ptr, src_ptr, nbytes,
                               rt.cudaMemcpyKind.cudaMemcpyDeviceToDevice, stream)
-    if int(err) == 0:
-        err, = rt.cudaStreamSynchronize(stream)
     if int(err) != 0:
         raise gc.GravError(f"cudaMemcpy D2D failed: {err}")
 
