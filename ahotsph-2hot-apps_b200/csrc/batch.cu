@@ -1096,6 +1096,10 @@ struct grav_plan {
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     EwStored *ewm = nullptr;
+    // a table of cell centres of the plan's own (own_centres), filled from the cell table
+    float4 *centres = nullptr;
+    const unsigned char *centres_from = nullptr;
+    int centres_stride = 0;
     // Group ranges of the work queue: items are sorted by cost within each
     // range, and chunk_item[k][c] is the first item of kind k in range c.
     // One range [0, ngroups) except in the pipelined end-to-end call.
@@ -1140,11 +1144,34 @@ int encode_cells(CUtensorMap *m, const void *base, int64_t rows) {
     return 0;
 }
 
-// The table k_points reads FP64 cell centres from, and its record size.
+// The table k_points reads FP64 cell centres and masses from, and its record size.
 const unsigned char *cell_centres(const DevProblem &d, bool quad, int &stride) {
     stride = quad ? (int)sizeof(nln_qcell) : (int)sizeof(nln_hcell);
     return quad ? reinterpret_cast<const unsigned char *>(d.qcells)
                 : reinterpret_cast<const unsigned char *>(d.hcells);
+}
+
+// A monopole's mass is the point table's.  The cell tables carry the same one
+// in every problem that this library's builders make; where a caller's differ,
+// k_points gets a table of its own (centre, mass, pad: 32 bytes a cell).
+__global__ void k_masses_differ(const float4 *__restrict__ cells, const unsigned char *__restrict__ cen,
+                                int stride, int64_t n, unsigned *differ) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool d = c < n && __float_as_uint(cells[c].w) !=
+                                __float_as_uint(reinterpret_cast<const float *>(cen + c * stride)[6]);
+    if (__any_sync(0xffffffffu, d) && (threadIdx.x & 31) == 0)
+        atomicOr(differ, 1u);
+}
+
+__global__ void k_centre_table(const float4 *__restrict__ cells, const unsigned char *__restrict__ cen,
+                               int stride, int64_t n, float4 *out) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n)
+        return;
+    const float4 *r = reinterpret_cast<const float4 *>(cen + c * stride);
+    const float4 b = r[1];
+    out[2 * c] = r[0];
+    out[2 * c + 1] = make_float4(b.x, b.y, cells[c].w, 0.f);
 }
 
 template <typename T>
@@ -1176,6 +1203,37 @@ int dev_copy(grav_plan *pl, const T *src, size_t n, T **dst) {
     if (src)
         GC_CHECK(cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice));
     return 0;
+}
+
+// After a refit too (its cell masses are the point table's own).
+int fill_centres(grav_plan *pl, cudaStream_t st) {
+    const int64_t nc = pl->dp.ncells;
+    k_centre_table<<<(unsigned)((nc + 255) / 256), 256, 0, st>>>(
+        pl->dp.points + pl->hp.nbodies, pl->centres_from, pl->centres_stride, nc, pl->centres);
+    GC_CHECK(cudaGetLastError());
+    return 0;
+}
+
+// d.ccen set: where its masses are not the point table's, a table of the
+// plan's own takes its place.  The error word, still unused, carries the answer.
+int own_centres(grav_plan *pl, int64_t nc) {
+    DevProblem &d = pl->dp;
+    unsigned differ = 0;
+    k_masses_differ<<<(unsigned)((nc + 255) / 256), 256>>>(d.points + pl->hp.nbodies, d.ccen, d.cstride,
+                                                           nc, d.err);
+    GC_CHECK(cudaGetLastError());
+    GC_CHECK(cudaMemcpy(&differ, d.err, sizeof(differ), cudaMemcpyDeviceToHost));
+    if (!differ)
+        return 0;
+    GC_CHECK(cudaMemset(d.err, 0, sizeof(unsigned)));
+    if (int rc = dev_copy<float4>(pl, nullptr, (size_t)nc * 2, &pl->centres))
+        return rc;
+    pl->centres_from = d.ccen;
+    pl->centres_stride = d.cstride;
+    d.ncells = nc;
+    d.ccen = reinterpret_cast<const unsigned char *>(pl->centres);
+    d.cstride = 2 * (int)sizeof(float4);
+    return fill_centres(pl, 0);
 }
 
 // Defaults: 8 warps per block, which the list kernels run as blocks of four,
@@ -1777,6 +1835,8 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     const bool has_q = d.qcells && hp->qptr && hp->qptr[ng];
     const bool has_h = d.hcells && hp->hptr && hp->hptr[ng];
     d.ccen = has_q || has_h ? cell_centres(d, has_q, d.cstride) : nullptr;
+    if (d.ccen && !adopt && !pl->plain)
+        rc |= own_centres(pl, np - nb);
     if (has_q)
         rc |= encode_cells<KQ>(&pl->tmap[KQ], d.qcells, hp->ncells);
     if (has_h)

@@ -357,7 +357,7 @@ int refit_enqueue(grav_plan *pl, cudaStream_t st) {
         S->raw, S->ncells, pl->hp.nbodies, const_cast<float4 *>(pl->dp.points),
         const_cast<nln_qcell *>(pl->dp.qcells), const_cast<nln_hcell *>(pl->dp.hcells));
     GC_CHECK(cudaGetLastError());
-    return 0;
+    return pl->centres ? fill_centres(pl, st) : 0;
 }
 
 int integrate_enqueue(grav_plan *pl, float *vel, const double *params, double *energy,
