@@ -23,26 +23,27 @@ class TreeGravity(torch.autograd.Function):
 
     @staticmethod
     def _plan(pos, mass, eps2, kw):
-        """The plan built on the GPU and tree position -> input index (device)."""
+        """Tree position -> input index (device), the plan built on the GPU, and
+        the current stream."""
         n = pos.shape[0]
         bodies = torch.empty((n, 4), dtype=torch.float32, device="cuda")
         bodies[:, :3] = pos.detach().to("cuda", torch.float32)
         bodies[:, 3] = mass.detach().to("cuda", torch.float32)
-        torch.cuda.synchronize()
         plan = gc.Plan.build(None, None, float(eps2), bodies=bodies, **kw)
+        stream = torch.cuda.current_stream()
         order = torch.empty(n, dtype=torch.int64, device="cuda")
-        memcpy_d2d(order.data_ptr(), plan.order_ptr(), n * 8)
-        return order, plan
+        memcpy_d2d(order.data_ptr(), plan.order_ptr(), n * 8, stream.cuda_stream)
+        return order, plan, stream
 
     @staticmethod
     def forward(ctx, pos, mass, eps2, tree_kw):
         kw = dict(tree_kw or {})
-        order, plan = TreeGravity._plan(pos, mass, eps2, kw)
+        order, plan, stream = TreeGravity._plan(pos, mass, eps2, kw)
         plan.eval()
         n = pos.shape[0]
         out_t = torch.empty((n, 4), dtype=torch.float32, device="cuda")
         torch.cuda.synchronize()
-        memcpy_d2d(out_t.data_ptr(), plan.output_ptr(), n * 16)
+        memcpy_d2d(out_t.data_ptr(), plan.output_ptr(), n * 16, stream.cuda_stream)
         plan.free()
         out = torch.empty_like(out_t)
         out[order] = out_t
@@ -54,7 +55,7 @@ class TreeGravity(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gacc, gphi):
         pos, mass = ctx.saved_tensors
-        order, plan = TreeGravity._plan(pos, mass, ctx.eps2, ctx.kw)
+        order, plan, stream = TreeGravity._plan(pos, mass, ctx.eps2, ctx.kw)
         if ctx.kw.get("ewald"):
             plan.eval()   # the correction's adjoint reads the evaluation's group moments
         n = pos.shape[0]
@@ -65,10 +66,10 @@ class TreeGravity(torch.autograd.Function):
             wu[:, 3] = gphi.detach().to("cuda", torch.float32)[order]
         grad_t = torch.empty((n, 4), dtype=torch.float32, device="cuda")
         torch.cuda.synchronize()
-        plan.adjoint(wu.data_ptr(), grad_t.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        plan.adjoint(wu.data_ptr(), grad_t.data_ptr(), stream.cuda_stream)
         grad = torch.empty_like(grad_t)
         grad[order] = grad_t
-        torch.cuda.current_stream().synchronize()
+        stream.synchronize()
         plan.free()
         dev = gacc.device if gacc is not None else gphi.device
         return grad[:, :3].to(dev), grad[:, 3].to(dev), None, None

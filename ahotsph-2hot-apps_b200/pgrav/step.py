@@ -31,16 +31,23 @@ def memcpy_d2h(dst_array, src_ptr):
     return dst_array
 
 
-def memcpy_d2d(dst_ptr, src_ptr, nbytes):
+def memcpy_d2d(dst_ptr, src_ptr, nbytes, stream=None):
     """Copy between device buffers, the destination a tensor of torch's
-    current stream: on that stream, not waited for (a plan that is freed waits
-    for it).  A plain cudaMemcpy runs on the legacy default stream, returns
-    before it is done, and torch's other streams do not wait for it."""
-    import torch
+    current stream (`stream` where the caller has it at hand), in its order.  cudaMemcpy runs on the default
+    stream and returns before it is done; on another stream, which does not
+    wait for it and in whose order a plan's buffers are not freed, the copy is
+    issued and waited for there."""
     rt = _rt()
-    stream = torch.cuda.current_stream().cuda_stream
-    err, = rt.cudaMemcpyAsync(dst_ptr, src_ptr, nbytes,
-                              rt.cudaMemcpyKind.cudaMemcpyDeviceToDevice, stream)
+    kind = rt.cudaMemcpyKind.cudaMemcpyDeviceToDevice
+    if stream is None:
+        import torch
+        stream = torch.cuda.current_stream().cuda_stream
+    if stream == 0:
+        err, = rt.cudaMemcpy(dst_ptr, src_ptr, nbytes, kind)
+    else:
+        err, = rt.cudaMemcpyAsync(dst_ptr, src_ptr, nbytes, kind, stream)
+        if int(err) == 0:
+            err, = rt.cudaStreamSynchronize(stream)
     if int(err) != 0:
         raise gc.GravError(f"cudaMemcpy D2D failed: {err}")
 

@@ -7,8 +7,9 @@ import pytest
 
 
 def test_device_copies_run_on_the_current_stream(monkeypatch):
-    """memcpy_d2d issues its copy on torch's current stream, with the runtime's
-    calls recorded in place of a GPU."""
+    """memcpy_d2d issues its copy on torch's current stream and waits there;
+    on the default stream cudaMemcpy is that copy.  The runtime's calls are
+    recorded in place of a GPU."""
     import torch
     from pgrav import step
     calls = []
@@ -18,11 +19,15 @@ def test_device_copies_run_on_the_current_stream(monkeypatch):
 
     fake = types.SimpleNamespace(
         cudaMemcpyKind=types.SimpleNamespace(cudaMemcpyDeviceToDevice=3),
-        cudaMemcpy=record("cudaMemcpy"), cudaMemcpyAsync=record("cudaMemcpyAsync"))
+        cudaMemcpy=record("cudaMemcpy"), cudaMemcpyAsync=record("cudaMemcpyAsync"),
+        cudaStreamSynchronize=record("cudaStreamSynchronize"))
     monkeypatch.setattr(step, "_rt", lambda: fake)
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=77))
-    step.memcpy_d2d(16, 32, 64)
-    assert calls == [("cudaMemcpyAsync", 16, 32, 64, 3, 77)]
+    for stream in (77, 0):
+        monkeypatch.setattr(torch.cuda, "current_stream",
+                            lambda: types.SimpleNamespace(cuda_stream=stream))
+        step.memcpy_d2d(16, 32, 64)
+    assert calls == [("cudaMemcpyAsync", 16, 32, 64, 3, 77), ("cudaStreamSynchronize", 77),
+                     ("cudaMemcpy", 16, 32, 64, 3)]
 
 
 def test_bodies_are_complete_before_the_build(monkeypatch):
