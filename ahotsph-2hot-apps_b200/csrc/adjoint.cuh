@@ -1200,6 +1200,7 @@ extern "C" int grav_plan_adjoint_CUDA(grav_plan *pl, const float *wu, float *gra
         return gc::set_status(-1, "grav_plan_adjoint_CUDA: evaluate the plan first (the "
                                   "periodic correction's adjoint reads its group moments)");
     cudaStream_t st = (cudaStream_t)stream;
+    pl->used_on(st);
     const int64_t nb = pl->hp.nbodies, nc = pl->hp.ncells, ng = pl->hp.ngroups;
     grav_step_state *S = pl->step;
     if (!pl->adj) {

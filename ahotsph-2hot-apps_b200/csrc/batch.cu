@@ -1087,6 +1087,7 @@ struct grav_plan {
     bool plain = false;                 // plain FP32 kernels (grav_problem.precision = 1)
     int integrator = 0;                 // 0: Integrate, 1: CosmoIntegrate (step.cuh)
     bool queues_clear = false;          // dp.counters are zero once the enqueued work is done
+    bool elsewhere = false;             // used on a stream that is not the default one
     bool evaluated = false;             // grav_groups_eval_CUDA has been enqueued (the
                                         // correction moments the adjoint reads are set)
     grav_step_state *step = nullptr;  // tree links, refit scratch and the step graph
@@ -1100,6 +1101,7 @@ struct grav_plan {
     float4 *centres = nullptr;
     const unsigned char *centres_from = nullptr;
     int centres_stride = 0;
+    void used_on(cudaStream_t st) { elsewhere = elsewhere || (st && st != cudaStreamLegacy); }
     // Group ranges of the work queue: items are sorted by cost within each
     // range, and chunk_item[k][c] is the first item of kind k in range c.
     // One range [0, ngroups) except in the pipelined end-to-end call.
@@ -2055,6 +2057,7 @@ extern "C" int grav_groups_eval_CUDA(grav_plan *pl, void *stream) {
         return gc::set_status(-1, "grav_groups_eval_CUDA: the plan lost its work queue in a failed "
                                   "retune; retune it again");
     cudaStream_t st = (cudaStream_t)stream;
+    pl->used_on(st);
     pl->launches = 0;
     auto mark = [&](int k) -> int {
         if (pl->timing)
@@ -2217,8 +2220,9 @@ extern "C" int grav_plan_launches(const grav_plan *pl) { return pl ? pl->launche
 extern "C" void grav_plan_free(grav_plan *pl) {
     if (!pl)
         return;
-    // work on any stream may still use what goes back to the pool (cudaFree waits by itself)
-    if (pl->pool)
+    // buffers go back to the pool in the default stream's order: work on another stream may
+    // still use them (cudaFree waits by itself)
+    if (pl->pool && pl->elsewhere)
         cudaDeviceSynchronize();
     if (pl->step)
         step_state_free(pl->step);

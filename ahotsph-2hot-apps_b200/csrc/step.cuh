@@ -345,6 +345,7 @@ struct grav_step_state {
 namespace {
 
 int refit_enqueue(grav_plan *pl, cudaStream_t st) {
+    pl->used_on(st);
     grav_step_state *S = pl->step;
     for (const auto &level : S->levels) {
         const int64_t lo = level.first, hi = level.second;
@@ -362,6 +363,7 @@ int refit_enqueue(grav_plan *pl, cudaStream_t st) {
 
 int integrate_enqueue(grav_plan *pl, float *vel, const double *params, double *energy,
                       cudaStream_t st) {
+    pl->used_on(st);
     const int64_t n = pl->hp.nbodies;
     const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)pl->nsm * 8);
     if (pl->integrator == 1)

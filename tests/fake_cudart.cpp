@@ -28,7 +28,7 @@ std::set<void *> host_live;
 size_t live_bytes = 0, peak_bytes = 0;
 long long cells = 1;  // what a tree needs room for
 int last_error = 0;
-long nalloc = 0, fail_at = 0, double_frees = 0, trims = 0, pending = 0;
+long nalloc = 0, fail_at = 0, double_frees = 0, trims = 0, pending = 0, device_waits = 0;
 long elsewhere = 0, freed_early = 0;  // launches on other streams, and pool buffers freed under them
 bool once = false;  // the failing allocation succeeds once the pool has been trimmed
 
@@ -132,7 +132,7 @@ struct dim3_ {
 extern "C" {
 void fake_reset(long fail, int until_trimmed) {
     std::lock_guard<std::recursive_mutex> lk(mu);
-    nalloc = double_frees = trims = pending = elsewhere = freed_early = 0;
+    nalloc = double_frees = trims = pending = elsewhere = freed_early = device_waits = 0;
     fail_at = fail;
     once = until_trimmed != 0;
     first_at.clear();
@@ -161,6 +161,7 @@ void fake_bytes(long *out) {
     out[1] = (long)peak_bytes;
 }
 long fake_freed_early() { return freed_early; }
+long fake_device_waits() { return device_waits; }
 void fake_cells(long long need) { cells = need; }
 unsigned fake_grid(const char *kernel) {
     for (auto &k : grids)
@@ -308,6 +309,7 @@ int cudaDeviceSynchronize() {
     std::lock_guard<std::recursive_mutex> lk(mu);
     waited(nullptr);
     elsewhere = 0;
+    device_waits++;
     return 0;
 }
 int cudaFuncGetAttributes(void *a, const void *) {  // cudaFuncAttributes: versions after 3 sizes, 2 ints

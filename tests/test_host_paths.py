@@ -306,21 +306,32 @@ print(json.dumps(res))
 
 
 def test_a_plan_is_freed_after_the_work_that_uses_it(run):
-    """A device-built plan's buffers go back to the pool only when the
-    evaluation and the adjoint queued on another stream are done with them."""
+    """A device-built plan's buffers go back to the pool only when what was
+    queued on another stream (an evaluation, an adjoint, a refit, a step) is
+    done with them; a plan used on the default stream alone, in whose order they
+    go back, does not hold the device up (a capture elsewhere would not survive
+    that)."""
     out = run("""
 res = []
+fake.fake_freed_early.restype = fake.fake_device_waits.restype = ctypes.c_long
+uses = {
+    "eval": lambda h, st: L.grav_groups_eval_CUDA(h, st),
+    "adjoint": lambda h, st: L.grav_plan_adjoint_CUDA(h, at, at, st),
+    "refit": lambda h, st: L.grav_plan_refit_CUDA(h, st),
+    "step": lambda h, st: L.grav_plan_step_CUDA(h, at, at, at, st, 0),
+}
 for box in (0.0, 1.0):
-    for adjoint in (0, 1):
-        rc, h = build(box)
-        fake.cudaDeviceSynchronize()
-        fake.fake_reset(0, 0)
-        assert rc == 0 and L.grav_groups_eval_CUDA(h, 0x5000) == 0
-        if adjoint:
-            assert L.grav_plan_adjoint_CUDA(h, at, at, 0x5000) == 0
-        L.grav_plan_free(h)
-        fake.fake_freed_early.restype = ctypes.c_long
-        res.append([fake.fake_freed_early(), counts()["live"]])
+    for name, use in uses.items():
+        for stream in (0x5000, None):
+            rc, h = build(box)
+            fake.cudaDeviceSynchronize()
+            fake.fake_reset(0, 0)
+            assert rc == 0 and use(h, stream) == 0
+            L.grav_plan_free(h)
+            res.append([name, stream is None, fake.fake_freed_early(), fake.fake_device_waits(),
+                        counts()["live"]])
 print(json.dumps(res))
 """)
-    assert out == [[0, 0]] * 4
+    assert len(out) == 16
+    for name, default, early, waits, live in out:
+        assert early == 0 and live == 0 and waits == (0 if default else 1), (name, default, early, waits)
