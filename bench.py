@@ -405,7 +405,7 @@ def config_box128(args, stream):
     """Periodic 128^3 box (GRF, P(k) ~ k^-2.5, rms displacement 0.25
     spacing), eps = spacing/50, order 4 + Ewald (FP64-built table): the
     mixed-precision kernels (FP32 offsets from FP64 group centres,
-    compensated sums) against the plain FP32 kernels (absolute FP32
+    FP64 tile sums) against the plain FP32 kernels (absolute FP32
     coordinates, plain sums) on the same lists; errors against the FP64
     Ewald-summed direct sum on 4096 random sinks."""
     from pgrav import gravcuda as gc, host, ics
@@ -1244,7 +1244,7 @@ def main():
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
                 "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": ms_max,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                "dtype": "f32 (FP64 centres, compensated sums)", "data": "synthetic (seeded)",
+                "dtype": "f32 (FP64 centres, FP64 sums of tiles)", "data": "synthetic (seeded)",
                 "config": cfg, "gpu_launches": launches * args.steps,
                 "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
                 "e2e_from_positions": e2e_pos,
