@@ -406,7 +406,7 @@ def config_box128(args, stream):
     spacing), eps = spacing/50, order 4 + Ewald (FP64-built table): the
     mixed-precision kernels (FP32 offsets from FP64 group centres,
     FP64 tile sums) against the plain FP32 kernels (absolute FP32
-    coordinates, plain sums) on the same lists; errors against the FP64
+    coordinates) on the same lists; errors against the FP64
     Ewald-summed direct sum on 4096 random sinks."""
     from pgrav import gravcuda as gc, host, ics
     w = WORKLOADS["box128"]
