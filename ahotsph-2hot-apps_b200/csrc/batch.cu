@@ -104,6 +104,9 @@ struct DevProblem {
     // or null, where the FP32 point record is used
     const unsigned char *ccen;
     int cstride;
+    // length_scale of the groups' span: the value, or the span on the device
+    float hscale;
+    const double *hscale_dev;
 };
 
 // Image code (0..26) to the image's shift: (code / 9 - 1, code / 3 % 3 - 1,
@@ -266,14 +269,36 @@ struct SinkTable {
     Sink s[32];
 };
 
-// This lane's sink offset from the group centre c, into the table.
+// Inside the order-4 kernel lengths are in units of the power of two below the
+// span of the groups: its largest terms, R^4 r^4 m, would leave FP32 in systems
+// that span some 1e5 lengths (unit masses), and its inverse powers in those of
+// 1e-7.  A power of two changes no other bits.  1 over that unit:
+__host__ __device__ inline float length_scale(double span) {
+    if (!(span > 1e-18 && span < 1e18))
+        return 1.f;
+    float s = 1.f;
+    for (; span >= 2.0; span *= 0.5) s *= 0.5f;
+    for (; span < 1.0; span *= 2.0) s *= 2.f;
+    return s;
+}
+
+// The span as the largest distance along an axis of a group's edge from `from`.
+__host__ __device__ inline double group_span(const nln_group &G, const nln_group &from) {
+    double s = 0;
+    for (int d = 0; d < 3; d++) s = fmax(s, fabs(G.cen[d] - from.cen[d]));
+    return s + G.radius;
+}
+
+// This lane's sink offset from the group centre c, into the table; `scale`: 1
+// over the kernel's unit of length.
 __device__ __forceinline__ void stage_sinks(SinkTable &T, const DevProblem &P, const nln_group &G,
-                                            const double *c, int lane) {
+                                            const double *c, int lane, float scale = 1.f) {
     __syncwarp();  // the previous item's sinks are no longer read
     if (lane < G.count) {
         const float4 s = P.points[G.first + lane];
-        const float nx = -(float)((double)s.x - c[0]), ny = -(float)((double)s.y - c[1]),
-                    nz = -(float)((double)s.z - c[2]);
+        const float nx = -scale * (float)((double)s.x - c[0]),
+                    ny = -scale * (float)((double)s.y - c[1]),
+                    nz = -scale * (float)((double)s.z - c[2]);
         T.s[lane].xy = make_float4(nx, nx, ny, ny);
         T.s[lane].z = make_float2(nz, nz);
     }
@@ -422,7 +447,7 @@ __device__ __forceinline__ void set_half(float2 &p, int h, float v) {
 
 template <int KIND>
 __device__ __forceinline__ void load_cell(const unsigned char *stage, int r, bool valid,
-                                          uint32_t code, double box, const double *c,
+                                          uint32_t code, double box, const double *c, float scale,
                                           typename CellKind<KIND>::Pair &p, int h) {
     using K = CellKind<KIND>;
     constexpr int NC = KIND == KH ? 8 : 4;
@@ -441,12 +466,14 @@ __device__ __forceinline__ void load_cell(const unsigned char *stage, int r, boo
     auto d = [&](int k) { return __hiloint2double(__float_as_int(f[k + 1]), __float_as_int(f[k])); };
     float o[3];
     recentre(d(0), d(2), d(4), code, shifted, box, c, o);
+#pragma unroll
+    for (int k = 0; k < (KIND == KH ? 3 : 0); k++) o[k] *= scale;
     auto put = [&](float2 &dst, float v) { set_half(dst, h, valid ? v : 0.f); };
     set_half(p.x, h, valid ? o[0] : kFar);
     set_half(p.y, h, valid ? o[1] : kFar);
     set_half(p.z, h, valid ? o[2] : kFar);
     put(p.m, f[6]);
-    const float R = f[7], c2 = -3.0f * R * R;
+    const float R = KIND == KH ? scale * f[7] : f[7], c2 = -3.0f * R * R;
 #pragma unroll
     for (int k = 0; k < 5; k++) put(p.q[k], c2 * f[8 + k]);
     if constexpr (KIND == KQ) {
@@ -496,7 +523,8 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
     __syncwarp();
     const uint32_t *list = P.list[KIND];
     const uint32_t ntab = (uint32_t)P.ntab[KIND];
-    const float2 e2 = splat2(P.eps2);
+    const float scale = KIND == KH ? (P.hscale_dev ? length_scale(*P.hscale_dev) : P.hscale) : 1.f;
+    const float2 e2 = splat2(P.eps2 * (scale * scale));
     uint32_t phase = 0;
     for (;;) {
         int it = 0;
@@ -561,7 +589,7 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
         if (ntile > 0)
             issue(0, ent, code);
         fetch(1, ent);
-        stage_sinks(sinks, P, G, c, lane);
+        stage_sinks(sinks, P, G, c, lane, scale);
         Total acc;
         for (int t = 0; t < ntile; t++) {
             const int nt = (int)min((int64_t)CT, nent - (int64_t)t * CT);
@@ -576,7 +604,7 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
             for (int h = 0; h < NE; h++)
                 if (h < 2 || nt > 64 * (h >> 1))
                     load_cell<KIND>(stage, 32 * h + lane, 32 * h + lane < nt, code[h], P.box, c,
-                                    rec[h >> 1], h & 1);
+                                    scale, rec[h >> 1], h & 1);
             __syncwarp();  // the stage is free: start the next copies, then compute
             if (t + 1 < ntile)
                 issue(t + 1, ent, code);
@@ -602,6 +630,10 @@ __global__ void __launch_bounds__(32 * kListWarps, KIND == KH ? GRAV_H_MINB : GR
                 sums_of(std::true_type());
             else
                 sums_of(std::false_type());
+        }
+        if constexpr (KIND == KH) {
+            for (int k = 0; k < 3; k++) acc.v[k] *= (double)scale * scale;
+            acc.v[3] *= scale;
         }
         store_part(P, item, lane, acc);
     }
@@ -1431,9 +1463,11 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
 
     // validate everything the kernels will index
     int bad_group = 0;
-#pragma omp parallel for schedule(static) reduction(| : bad_group)
+    double span = 0;
+#pragma omp parallel for schedule(static) reduction(| : bad_group) reduction(max : span)
     for (int64_t g = 0; g < ng; g++) {
         const nln_group &G = hp->groups[g];
+        span = std::max(span, group_span(G, hp->groups[0]));
         if (G.count < 1 || G.count > 32 || G.first < 0 || G.first + G.count > nb)
             bad_group |= 1;
         if (hp->pptr[g + 1] < hp->pptr[g] || (hp->qptr && hp->qptr[g + 1] < hp->qptr[g]) ||
@@ -1852,6 +1886,7 @@ int upload_impl(const grav_problem *hp, const grav_tuning *tuning, grav_plan **p
     d.eps2 = (float)hp->eps2;
     d.qsh = 0.5f * (hp->quad_phi_sign == 0.0f ? 1.0f : hp->quad_phi_sign);
     d.box = hp->box;
+    d.hscale = length_scale(span);
     pl->hp.points = nullptr;
     pl->hp.qcells = nullptr;
     pl->hp.hcells = nullptr;
@@ -2618,6 +2653,7 @@ constexpr int kMaxDevices = 64;
 struct DevScratch {
     int *counters;      // 4 queue heads: must be 0 when the kernels start
     unsigned *err;      // device error word: must be 0 when the kernels start
+    double *span;       // of the groups: must be 0 when the setup starts
     Item *items[3];
     nln_group *groups;  // checked copy of the caller's groups
     int64_t *gslot;
@@ -2695,6 +2731,11 @@ __global__ void k_dev_setup(const nln_group *__restrict__ groups, const int64_t 
         G.count = 1;
     }
     S.groups[g] = G;
+    // not negative: their bits are in their order
+    const double span = group_span(G, groups[0]);
+    if (span > 0)
+        atomicMax(reinterpret_cast<unsigned long long *>(S.span),
+                  (unsigned long long)__double_as_longlong(span));
     int rank = 0;
     for (int k = 0; k < 3; k++) {
         if (!ptr[k])
@@ -2744,6 +2785,7 @@ extern "C" int grav_groups_eval_dev_CUDA(const grav_problem *dp, float *acc_phi,
     size_t off = 0;
     S.counters = reinterpret_cast<int *>(base);
     S.err = reinterpret_cast<unsigned *>(base + 4 * sizeof(int));
+    S.span = reinterpret_cast<double *>(base + 8 * sizeof(int));
     off = 256;
     for (int k = 0; k < 3; k++) {
         S.items[k] = reinterpret_cast<Item *>(base + off);
@@ -2782,6 +2824,7 @@ extern "C" int grav_groups_eval_dev_CUDA(const grav_problem *dp, float *acc_phi,
     d.eps2 = (float)dp->eps2;
     d.qsh = 0.5f * (dp->quad_phi_sign == 0.0f ? 1.0f : dp->quad_phi_sign);
     d.box = dp->box;
+    d.hscale_dev = S.span;
     d.err = S.err;
     d.cptr = nullptr;
     d.clist = nullptr;
